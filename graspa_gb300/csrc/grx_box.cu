@@ -2,6 +2,7 @@
 // factors and FP64 totals (drift checks).
 #include <algorithm>
 #include <atomic>
+#include <climits>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -122,6 +123,14 @@ void refresh_dev(grx_box* b) {
   d.ctab_base = b->ctab_base;
   d.ctab_n = b->ctab_n;
   d.ctabf = b->ctabf;
+  const Tables64* t64 = b->t64.get();
+  d.g64 = t64 ? t64->g : nullptr;
+  d.g64_base = t64 ? t64->g_base : 0;
+  d.g64_n = t64 ? t64->g_n : 0;
+  d.h64 = t64 ? t64->h : nullptr;
+  d.h64_base = t64 ? t64->h_base : 0;
+  d.h64_n = t64 ? t64->h_n : 0;
+  d.img = reinterpret_cast<const double4*>(b->ff64 + (size_t)d.ntypes * d.ntypes);
   d.qdf = b->qdf;
   d.ffdf = b->ffdf;
   d.ffdf2 = b->ffdf2;
@@ -600,16 +609,31 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
     }
     const double h = 0.5 * wmin * (1.0 - 1e-4);
     d.half_wmin2 = (float)(h * h);
+    // The FP64 form takes a pair's lattice image from FP32 fractions of the hi parts (each
+    // within 2^-13 A of its coordinate) unless the fraction is this close to a tie.
+    d.tie = (float)(0.5 - (1e-5 + 4e-4 / wmin));
+  }
+  {
+    int64_t bits;
+    std::memcpy(&bits, &ff.overlap_criteria, 8);
+    d.overlap_hi = ff.overlap_criteria > 0.0 ? (int)(bits >> 32) : INT_MIN;
   }
 
   const int nt2 = ff.ntypes * ff.ntypes;
-  std::vector<FFPair64> f64(nt2);
+  std::vector<FFPair64> f64(nt2 + 27);  // the lattice vectors of BoxDev::img follow the pair table
+  static_assert(sizeof(FFPair64) == sizeof(double4), "lattice vectors share the pair table's allocation");
+  for (int i = 0; i < 27; ++i) {
+    const double nx = i % 3 - 1, ny = i / 3 % 3 - 1, nz = i / 9 - 1;
+    double v[3];
+    for (int k = 0; k < 3; ++k) v[k] = nx * g.cell[k] + ny * g.cell[3 + k] + nz * g.cell[6 + k];
+    f64[nt2 + i] = FFPair64{v[0], v[1], v[2], 0.0};
+  }
   std::vector<double> c10(nt2, 0.0);
   std::vector<float4> f32(nt2);
   for (int r = 0; r < nt2; ++r) {
-    f64[r].a = ff.epsilon[r];
+    f64[r].a = ff.use_1264 ? ff.epsilon[r] : 4.0 * ff.epsilon[r];
     f64[r].b = ff.sigma[r];
-    f64[r].c = ff.z ? ff.z[r] : 0.0;
+    f64[r].c = ff.use_1264 ? (ff.z ? ff.z[r] : 0.0) : ff.sigma[r] * ff.sigma[r];
     f64[r].shift = ff.shift[r];
     if (ff.c10) c10[r] = ff.c10[r];
     const double s2 = ff.sigma[r] * ff.sigma[r];
@@ -641,7 +665,7 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
   if ((e = dev_alloc(b, (void**)&b->scale, n * sizeof(double))) != cudaSuccess) return fail(e, "alloc scale");
   if ((e = dev_alloc(b, (void**)&b->charge, n * sizeof(double))) != cudaSuccess) return fail(e, "alloc charge");
   if ((e = dev_alloc(b, (void**)&b->d_size, GRX_MAX_COMPONENTS * sizeof(int))) != cudaSuccess) return fail(e, "alloc sizes");
-  if ((e = dev_alloc(b, (void**)&b->ff64, nt2 * sizeof(FFPair64))) != cudaSuccess) return fail(e, "alloc ff64");
+  if ((e = dev_alloc(b, (void**)&b->ff64, f64.size() * sizeof(FFPair64))) != cudaSuccess) return fail(e, "alloc ff64");
   if ((e = dev_alloc(b, (void**)&b->ffc10, nt2 * sizeof(double))) != cudaSuccess) return fail(e, "alloc ffc10");
   if ((e = dev_alloc(b, (void**)&b->ff32, nt2 * sizeof(float4))) != cudaSuccess) return fail(e, "alloc ff32");
   if ((e = dev_alloc(b, (void**)&b->ffdf, nt2 * sizeof(float4))) != cudaSuccess) return fail(e, "alloc ffdf");
@@ -669,7 +693,7 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
   cudaMemset(b->s_fw, 0, nv * sizeof(double2));
   cudaMemset(b->s_ads, 0, nv * sizeof(double2));
   cudaMemset(b->s_tmp, 0, nv * sizeof(double2));
-  cudaMemcpy(b->ff64, f64.data(), nt2 * sizeof(FFPair64), cudaMemcpyHostToDevice);
+  cudaMemcpy(b->ff64, f64.data(), f64.size() * sizeof(FFPair64), cudaMemcpyHostToDevice);
   cudaMemcpy(b->ffc10, c10.data(), nt2 * sizeof(double), cudaMemcpyHostToDevice);
   cudaMemcpy(b->ff32, f32.data(), nt2 * sizeof(float4), cudaMemcpyHostToDevice);
   cudaMemcpy(b->ffdf, fdf.data(), nt2 * sizeof(float4), cudaMemcpyHostToDevice);
@@ -688,6 +712,11 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
       grx_box_destroy(b);
       return st;
     }
+    double diag = 0.0;  // no image picked by rounded fractions is longer than half the summed edges
+    for (int k = 0; k < 3; ++k)
+      diag += 0.5 * std::sqrt(g.cell[3 * k] * g.cell[3 * k] + g.cell[3 * k + 1] * g.cell[3 * k + 1] +
+                              g.cell[3 * k + 2] * g.cell[3 * k + 2]);
+    attach_tables64(b, g.alpha, ff.cutoff_coul_sq, diag * diag);
   }
   refresh_dev(b);
   *out = b;
@@ -714,7 +743,7 @@ grx_status grx_box_footprint(const grx_box_desc* desc, size_t* bytes) {
   const size_t nv = std::max(tmp.nvec, 1), na = std::max(tmp.nact, 1);
   size_t t = al(n * sizeof(double4)) + 2 * al(n * sizeof(float4)) + al(n * sizeof(int2)) + 2 * al(n * sizeof(double)) +
              al(n * sizeof(float2)) + al(GRX_MAX_COMPONENTS * sizeof(int));
-  t += al(nt2 * sizeof(FFPair64)) + al(nt2 * sizeof(double)) + 2 * al(nt2 * sizeof(float4)) + al(nt2 * sizeof(float2));
+  t += al((nt2 + 27) * sizeof(FFPair64)) + al(nt2 * sizeof(double)) + 2 * al(nt2 * sizeof(float4)) + al(nt2 * sizeof(float2));
   t += al(na * sizeof(int4)) + al(na * sizeof(double)) + 3 * al(nv * sizeof(double2)) + 2 * al(na * sizeof(float4)) +
        al(na * sizeof(float2));
   t += al(ntiles * sizeof(float4)) + al(ntiles * sizeof(int4));

@@ -1,10 +1,23 @@
 // grx_host.h -- host-side box object shared by the libgrx translation units.
 #pragma once
 
+#include <memory>
 #include <vector>
 #include <string>
 
 #include "grx_internal.cuh"
+
+namespace grx {
+// Device copies of the FP64 tables of one (device, alpha, cutoff^2, largest image distance^2):
+// freed when the last holder (a box, or an arena for its boxes) lets go.
+struct Tables64 {
+  int device = 0;
+  double2* g = nullptr;
+  double2* h = nullptr;
+  int g_base = 0, g_n = 0, h_base = 0, h_n = 0;
+  ~Tables64();
+};
+}  // namespace grx
 
 struct grx_box {
   grx::BoxDev dev{};
@@ -87,6 +100,7 @@ struct grx_box {
   double* ctab = nullptr;
   int ctab_n = 0, ctab_base = 0;
   double ctab_maxrel = 0.0;
+  std::shared_ptr<const grx::Tables64> t64;  // FP64 Coulomb tables, shared by boxes of equal parameters
 
   // scratch (grown on demand)
   double* scratch = nullptr;
@@ -111,6 +125,11 @@ cudaError_t dev_alloc(grx_box* b, void** p, size_t bytes);
 // for replicas) and marks them valid.
 grx_status ewald_df_refresh(grx_box* b);
 void dev_free(grx_box* b, void* p);
+// The FP64 Coulomb tables of the box (grx_table.cu); without device memory for them the box
+// runs on the library functions.
+void attach_tables64(grx_box* b, double alpha, double cut2, double smax);
+// Keeps the tables of an arena's boxes until the arena goes (retiring a box must not free device memory).
+void arena_keep(grx_arena* a, const std::shared_ptr<const Tables64>& t);
 // Voxel candidate lists of the machine's host atoms (grx_voxel.cu), rebuilt after the tiles.
 grx_status build_voxels(grx_box* b);
 }  // namespace grx

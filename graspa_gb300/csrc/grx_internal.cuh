@@ -22,9 +22,12 @@
 
 namespace grx {
 
-struct FFPair64 {  // per type pair, FP64: {eps or C12, sigma or C6, z or C4, shift}
+struct FFPair64 {  // per type pair, FP64: {4 eps or C12, sigma or C6, C4 (12-6-4) or sigma^2 (12-6), shift}
   double a, b, c, shift;
 };
+
+// Pieces of the FP64 tables (grx_table.cu): high-word bits below the index, 2^(20 - shift) per octave.
+constexpr int kShiftG64 = 11, kShiftH64 = 12;
 
 struct BoxDev {
   // geometry
@@ -102,6 +105,17 @@ struct BoxDev {
   const float2* qdf;     // q * scaleCoul, hi/lo
   const float4* ffdf;    // {4 eps hi, lo, 1/sigma^2 hi, lo}
   const float2* ffdf2;   // {shift hi, lo}
+  // FP64 form: g(s) and h(s) = erf(alpha sqrt s)/sqrt s as piecewise quintics indexed by the
+  // high word of the FP64 s (grx_table.cu); n = 0: no table
+  const double2* g64;    // per piece {c0, c1}, {c2, c3}, {c4, c5} in u = s - centre
+  int g64_base;
+  int g64_n;
+  const double2* h64;
+  int h64_base;
+  int h64_n;
+  const double4* img;    // 27 lattice vectors n, entry (nx+1) + 3 (ny+1) + 9 (nz+1)
+  float tie;             // |fraction - nearest integer| above which FP32 does not pick the image
+  int overlap_hi;        // high word of a positive overlap criterion, else INT_MIN
   float2 cut_vdw2_df;
   float2 cut_coul2_df;
   const float4* ewA;     // per active k {re hi, re lo, im hi, im lo} of temp * S_ads
@@ -235,7 +249,7 @@ __device__ __forceinline__ double vdw64(const BoxDev& b, int row, double rr, dou
     const double ri12 = ri6 * ri6;
     return scaling * (f.a * ri12 - f.b * ri6 + b.ffc10[row] * ri10 + f.c * ri4 - f.shift);
   }
-  const double arg1 = 4.0 * f.a;
+  const double arg1 = f.a;
   const double arg2 = f.b * f.b;
   const double temp = rr / arg2;
   const double temp3 = temp * temp * temp;
@@ -270,8 +284,17 @@ struct Bead {
   double scale;        // LJ lambda
   float2 pq;           // prefactor * q as double-float
   int type;
-  int unit;            // scale == 1
+  int unit;            // bit 0: scale == 1; bit 1: every |h| < kNearCoord
 };
+
+// Coordinates below this bound: the hi parts are exact multiples of 2^-12 in FP32, as are the
+// differences of two of them. The FP64 form screens and picks images in FP32 only within it.
+constexpr float kNearCoord = 2048.0f;
+
+__host__ __device__ __forceinline__ int bead_unit(double scale, float3 h) {
+  return (scale == 1.0 ? 1 : 0) |
+         (fabsf(h.x) < kNearCoord && fabsf(h.y) < kNearCoord && fabsf(h.z) < kNearCoord ? 2 : 0);
+}
 
 __device__ __forceinline__ void split_coord(double x, float& h, float& l) {
   const double hd = rint(x * GRX_GRID_COORD) * (1.0 / GRX_GRID_COORD);
@@ -289,7 +312,7 @@ __device__ __forceinline__ void make_bead(Bead& bd, double x, double y, double z
   const double pq = prefactor * q;
   const float ph = __double2float_rn(pq);
   bd.pq = make_float2(ph, __double2float_rn(pq - (double)ph));
-  bd.unit = scale == 1.0;
+  bd.unit = bead_unit(scale, bd.h);
 }
 
 // Energy of one (atom, bead) pair. Returns true when the pair is inside a cutoff;

@@ -109,7 +109,7 @@ static grx_status stage_beads(const grx_trials* t, size_t first_bead, size_t nbe
     const double pq = prefactor * bd.q;
     const float ph = (float)pq;
     bd.pq = make_float2(ph, (float)(pq - (double)ph));
-    bd.unit = bd.scale == 1.0;
+    bd.unit = bead_unit(bd.scale, bd.h);
   }
   return GRX_OK;
 }
