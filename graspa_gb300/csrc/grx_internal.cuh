@@ -207,36 +207,6 @@ __device__ __forceinline__ void pbc64(const BoxDev& b, double& x, double& y, dou
   }
 }
 
-// Split-coordinate minimum image: (dh, dl) = hi and lo parts of a displacement.
-// The integer image shift is chosen from the FP32 sum with the reference's
-// rounding rule; the shift is applied to both parts so dh stays exact.
-__device__ __forceinline__ void pbc_split(const BoxDev& b, float3& dh, float3& dl) {
-  const float x = dh.x + dl.x, y = dh.y + dl.y, z = dh.z + dl.z;
-  float nx, ny, nz;
-  if (b.cubic) {
-    nx = (float)(int)(x * b.invf[0] + ((x >= 0.f) ? 0.5f : -0.5f));
-    ny = (float)(int)(y * b.invf[4] + ((y >= 0.f) ? 0.5f : -0.5f));
-    nz = (float)(int)(z * b.invf[8] + ((z >= 0.f) ? 0.5f : -0.5f));
-    dh.x -= nx * b.cell_hi[0]; dl.x -= nx * b.cell_lo[0];
-    dh.y -= ny * b.cell_hi[4]; dl.y -= ny * b.cell_lo[4];
-    dh.z -= nz * b.cell_hi[8]; dl.z -= nz * b.cell_lo[8];
-  } else {
-    const float sx = b.invf[0] * x + b.invf[3] * y + b.invf[6] * z;
-    const float sy = b.invf[1] * x + b.invf[4] * y + b.invf[7] * z;
-    const float sz = b.invf[2] * x + b.invf[5] * y + b.invf[8] * z;
-    nx = (float)(int)(sx + ((sx >= 0.f) ? 0.5f : -0.5f));
-    ny = (float)(int)(sy + ((sy >= 0.f) ? 0.5f : -0.5f));
-    nz = (float)(int)(sz + ((sz >= 0.f) ? 0.5f : -0.5f));
-    // hi parts: cell_hi on the 2^-12 grid, small integer multiples stay exact
-    dh.x -= nx * b.cell_hi[0]; dh.x -= ny * b.cell_hi[3]; dh.x -= nz * b.cell_hi[6];
-    dh.y -= nx * b.cell_hi[1]; dh.y -= ny * b.cell_hi[4]; dh.y -= nz * b.cell_hi[7];
-    dh.z -= nx * b.cell_hi[2]; dh.z -= ny * b.cell_hi[5]; dh.z -= nz * b.cell_hi[8];
-    dl.x -= nx * b.cell_lo[0] + ny * b.cell_lo[3] + nz * b.cell_lo[6];
-    dl.y -= nx * b.cell_lo[1] + ny * b.cell_lo[4] + nz * b.cell_lo[7];
-    dl.z -= nx * b.cell_lo[2] + ny * b.cell_lo[5] + nz * b.cell_lo[8];
-  }
-}
-
 // ---------------------------------------------------------------- potentials
 // VDW(), maths.cuh:452-494 (FP64, soft-core lambda and 12-6-4 mode).
 __device__ __forceinline__ double vdw64(const BoxDev& b, int row, double rr, double scaling) {
@@ -315,104 +285,10 @@ __device__ __forceinline__ void make_bead(Bead& bd, double x, double y, double z
   bd.unit = bead_unit(scale, bd.h);
 }
 
-// Energy of one (atom, bead) pair. Returns true when the pair is inside a cutoff;
-// adds to vdw / real and sets `flag` on overlap (VDW_Coulomb.cu:1290-1322).
 // Atom arrays by storage index: host atoms may live in a parent box (replicas).
 __device__ __forceinline__ double4 atom_pos64(const BoxDev& b, int i) { return i < b.host_end ? b.hpos64[i] : b.pos64[i]; }
 __device__ __forceinline__ int2 atom_meta(const BoxDev& b, int i) { return i < b.host_end ? b.hmeta[i] : b.meta[i]; }
 __device__ __forceinline__ double atom_scale(const BoxDev& b, int i) { return i < b.host_end ? b.hscale[i] : b.scale[i]; }
-
-template <int PREC>
-__device__ __forceinline__ void pair_energy(const BoxDev& b, int i, const Bead& bd, int rowbase,
-                                            double& vdw, double& real, int& flag) {
-  const bool host = i < b.host_end;
-  const double4* P64 = host ? b.hpos64 : b.pos64;
-  const float4* HI = host ? b.hhi : b.hi;
-  const float4* LO = host ? b.hlo : b.lo;
-  const int2* META = host ? b.hmeta : b.meta;
-  const double* SC = host ? b.hscale : b.scale;
-  if (PREC == GRX_FP64) {
-    const double4 p = P64[i];
-    double x = p.x - bd.x, y = p.y - bd.y, z = p.z - bd.z;
-    pbc64(b, x, y, z);
-    const double rr = x * x + y * y + z * z;
-    const int2 mt = META[i];
-    if (rr < b.cut_vdw2) {
-      const double e = vdw64(b, mt.x * b.ntypes + bd.type, rr, SC[i] * bd.scale);
-      if (e > b.overlap) flag = 1;
-      if (rr < 0.01) flag = 1;
-      vdw += e;
-    }
-    if (!b.no_charges && rr < b.cut_coul2) real += coul64(b, p.w * bd.q, rr);
-  } else {
-    const float4 ah = HI[i];
-    const float4 al = LO[i];
-    float3 dh = make_float3(ah.x - bd.h.x, ah.y - bd.h.y, ah.z - bd.h.z);
-    float3 dl = make_float3(al.x - bd.l.x, al.y - bd.l.y, al.z - bd.l.z);
-    pbc_split(b, dh, dl);
-    const float fx = dh.x + dl.x, fy = dh.y + dl.y, fz = dh.z + dl.z;
-    const float rr32 = fx * fx + fy * fy + fz * fz;
-    if (rr32 >= b.screen2) return;
-    const int2 mt = META[i];
-    const int row = mt.x * b.ntypes + bd.type;
-    if (PREC == GRX_MIXED) {
-      const double x = (double)dh.x + (double)dl.x;
-      const double y = (double)dh.y + (double)dl.y;
-      const double z = (double)dh.z + (double)dl.z;
-      const double rr = x * x + y * y + z * z;
-      if (rr < b.cut_vdw2) {
-        const float4 f = b.ff32[row];
-        const bool unit = (al.w == 1.0f) && (bd.scale == 1.0) && !b.use_1264;
-        double e;
-        if (unit && (float)rr > f.w) e = (double)vdw32(f, (float)rr);
-        else e = vdw64(b, row, rr, SC[i] * bd.scale);
-        if (e > b.overlap) flag = 1;
-        if (rr < 0.01) flag = 1;
-        vdw += e;
-      }
-      if (!b.no_charges && rr < b.cut_coul2) real += coul64(b, P64[i].w * bd.q, rr);
-    } else {  // GRX_FP32
-      const float sc = al.w * (float)bd.scale;
-      if (rr32 < b.cut_vdw2f) {
-        float e;
-        if (sc == 1.0f && !b.use_1264) e = vdw32(b.ff32[row], rr32);
-        else e = (float)vdw64(b, row, (double)rr32, (double)sc);
-        if (e > (float)b.overlap) flag = 1;
-        if (rr32 < 0.01f) flag = 1;
-        vdw += (double)e;
-      }
-      if (!b.no_charges && rr32 < b.cut_coul2f) real += (double)coul32(b, ah.w * (float)bd.q, rr32);
-    }
-  }
-}
-
-// One pass of trial beads over every live atom. Thread t owns bead t % nb and lane
-// t / nb; lanes (of this block, offset by lane0, strided by lane_stride across
-// blocks) walk the atoms of every component. acc = {hg_vdw, hg_real, gg_vdw,
-// gg_real} of the thread's bead; `flag` is set on overlap. Atoms of
-// (component, newmol) and (excl_comp, excl_mol) are skipped, as in
-// Calculate_Multiple_Trial_Energy_VDWReal (VDW_Coulomb.cu:1274-1276).
-template <int PREC>
-__device__ __forceinline__ void bead_pass(const BoxDev& b, const Bead& bd, int lane, int lane_stride,
-                                          int component, int newmol, int excl_comp, int excl_mol,
-                                          double acc[4], int& flag) {
-  for (int c = 0; c < b.ncomp; ++c) {
-    const int n = b.comp_size[c];
-    const int off = b.comp_off[c];
-    const bool check_mol = (c == component) || (c == excl_comp);
-    double v = 0.0, r = 0.0;
-#pragma unroll 2
-    for (int i = lane; i < n; i += lane_stride) {
-      if (check_mol) {
-        const int mol = atom_meta(b, off + i).y;
-        if ((c == excl_comp && mol == excl_mol) || (c == component && mol == newmol)) continue;
-      }
-      pair_energy<PREC>(b, off + i, bd, 0, v, r, flag);
-    }
-    if (c < b.nhost) { acc[0] += v; acc[1] += r; }
-    else { acc[2] += v; acc[3] += r; }
-  }
-}
 
 // ---------------------------------------------------------------- reductions
 // Deterministic block sum of one double per thread (fixed shuffle tree).

@@ -16,9 +16,8 @@
 //    (once per device, with the box's device made current for the call and the
 //    caller's device restored after); make that first call before any stream capture
 //    is started;
-//  * all calls share the one array and it keeps the last call's contents. The
-//    parts that must start at zero (overlap flags) are cleared on every call.
-//    Calls that overlap on the GPU (two host threads, two streams) race on the
+//  * all calls share the one array and it keeps the last call's contents; every call
+//    writes what it reads. Calls that overlap on the GPU (two host threads, two streams) race on the
 //    array: issue them one after another.
 // The box itself is created beforehand with grx_box_create (which allocates once).
 #include <mutex>
@@ -40,14 +39,12 @@ constexpr size_t kOffScaleCoul = kOffCharge + kNoallocBeads * 8;        // doubl
 constexpr size_t kOffType = kOffScaleCoul + kNoallocBeads * 8;          // size_t[B]
 constexpr size_t kOffBeads = kOffType + kNoallocBeads * 8;              // Bead[B]
 constexpr size_t kBeadBytes = ((kNoallocBeads * sizeof(Bead)) + 255) / 256 * 256;
-constexpr size_t kOffPart = kOffBeads + kBeadBytes;                     // double[4*B]
-constexpr size_t kOffFlags = kOffPart + 4 * kNoallocBeads * 8;          // int[B]
-constexpr size_t kOffOut = kOffFlags + kNoallocBeads * 4;               // double[4*B]
+constexpr size_t kOffOut = kOffBeads + kBeadBytes;                      // double[4*B]
 constexpr size_t kOffOver = kOffOut + 4 * kNoallocBeads * 8;            // uint8[B]
 constexpr size_t kNeed = kOffOver + kNoallocBeads;
 
 static_assert(kNeed <= GRX_NOALLOC_SCRATCH_BYTES, "scratch array too small for its layout");
-static_assert(kOffScale % 256 == 0 && kOffBeads % 256 == 0 && kOffPart % 256 == 0 && kOffOut % 256 == 0,
+static_assert(kOffScale % 256 == 0 && kOffBeads % 256 == 0 && kOffOut % 256 == 0,
               "scratch blocks must stay aligned");
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[GRX_NOALLOC_SCRATCH_BYTES];
@@ -103,22 +100,6 @@ __global__ void noalloc_beads_kernel(const double* pos, const double* scale, con
   make_bead(beads[j], pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], q * scc, sc, (int)type[j], prefactor);
 }
 
-__global__ void noalloc_reduce_kernel(const double* part, const int* flags, int nb, int chain, double* out,
-                                      unsigned char* over) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ntr = nb / chain;
-  if (w >= ntr * 4) return;
-  const int t = w >> 2, q = w & 3;
-  double s = 0.0;
-  for (int a = 0; a < chain; ++a) s += part[(size_t)(t * chain + a) * 4 + q];
-  out[t * 4 + q] = s;
-  if (q == 0) {
-    int f = 0;
-    for (int a = 0; a < chain; ++a) f |= flags[t * chain + a];
-    over[t] = f ? 1 : 0;
-  }
-}
-
 }  // namespace
 }  // namespace grx
 
@@ -156,8 +137,6 @@ extern "C" grx_status grx_trial_energies_noalloc(grx_box* b, const grx_trials* t
   double* scale_coul = reinterpret_cast<double*>(base + kOffScaleCoul);
   size_t* type = reinterpret_cast<size_t*>(base + kOffType);
   Bead* beads = reinterpret_cast<Bead*>(base + kOffBeads);
-  double* part = reinterpret_cast<double*>(base + kOffPart);
-  int* flags = reinterpret_cast<int*>(base + kOffFlags);
   double* dout = reinterpret_cast<double*>(base + kOffOut);
   unsigned char* dover = base + kOffOver;
   GRX_CHECK_CUDA(cudaMemcpyAsync(pos, t->pos, 3 * nb * sizeof(double), cudaMemcpyDefault, s), "noalloc: stage pos");
@@ -169,20 +148,24 @@ extern "C" grx_status grx_trial_energies_noalloc(grx_box* b, const grx_trials* t
     GRX_CHECK_CUDA(cudaMemcpyAsync(scale_coul, t->scale_coul, nb * sizeof(double), cudaMemcpyDefault, s),
                    "noalloc: stage scaleCoul");
   GRX_CHECK_CUDA(cudaMemcpyAsync(type, t->type, nb * sizeof(size_t), cudaMemcpyDefault, s), "noalloc: stage type");
-  GRX_CHECK_CUDA(cudaMemsetAsync(flags, 0, nb * sizeof(int), s), "noalloc: clear flags");
   noalloc_beads_kernel<<<(nb + 127) / 128, 128, 0, s>>>(pos, scale, charge, scale_coul, type, nb, t->scale != nullptr,
                                                         t->charge != nullptr, t->scale_coul != nullptr,
                                                         b->dev.prefactor, beads);
-  const int ec = (int)exclude_comp, em = (int)exclude_molid, nm = (int)t->molid;
-  if (prec == GRX_FP64)
-    trial_bead_kernel<GRX_FP64><<<nb, GRX_THREADS, 0, s>>>(b->dev, beads, component, nm, ec, em, part, flags);
-  else if (prec == GRX_MIXED)
-    trial_bead_kernel<GRX_MIXED><<<nb, GRX_THREADS, 0, s>>>(b->dev, beads, component, nm, ec, em, part, flags);
-  else
-    trial_bead_kernel<GRX_FP32><<<nb, GRX_THREADS, 0, s>>>(b->dev, beads, component, nm, ec, em, part, flags);
   const int ntr = (int)t->ntrials;
-  noalloc_reduce_kernel<<<(ntr * 4 + 127) / 128, 128, 0, s>>>(part, flags, nb, (int)t->chainsize, dout, dover);
-  count_launch(3);
+  TrialArgs a{};
+  a.beads = beads;
+  a.chain = (int)t->chainsize;
+  a.component = component;
+  a.mol[0] = (int)t->molid;
+  a.split = ntr;
+  a.excl_comp = (int)exclude_comp;
+  a.excl_mol = (int)exclude_molid;
+  a.out = dout;
+  a.over = dover;
+  if (prec == GRX_FP64) launch_trials<GRX_FP64>(b->dev, a, ntr, s);
+  else if (prec == GRX_MIXED) launch_trials<GRX_MIXED>(b->dev, a, ntr, s);
+  else launch_trials<GRX_FP32>(b->dev, a, ntr, s);
+  count_launch(2);
   GRX_CHECK_CUDA(cudaGetLastError(), "grx_trial_energies_noalloc: launch");
   GRX_CHECK_CUDA(cudaMemcpyAsync(out, dout, ntr * sizeof(grx_trial_energy), cudaMemcpyDefault, s),
                  "noalloc: read energies");

@@ -1,5 +1,6 @@
 // grx_pair.cu -- stand-alone pair-energy entry points: CBMC trial energies and the
-// single-molecule move delta (the reference's per-move kernels, one call each).
+// single-molecule move delta (the reference's per-move kernels, one call each). Both run
+// trial_kernel (grx_warp.cuh); a move delta is two trials, the new molecule and the old one.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -8,74 +9,6 @@
 #include "grx_warp.cuh"
 
 namespace grx {
-
-// Fixed-order reduction: trial t, quantity q = sum over blocks, then chain beads.
-__global__ void trial_reduce_kernel(const double* part, const int* flags, int nblk, int nb, int chain,
-                                    double* out, int* tflag) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ntr = nb / chain;
-  if (w >= ntr * 4) return;
-  const int t = w >> 2, q = w & 3;
-  double s = 0.0;
-  for (int a = 0; a < chain; ++a) {
-    const int bead = t * chain + a;
-    double sb = 0.0;
-    for (int k = 0; k < nblk; ++k) sb += part[((size_t)k * nb + bead) * 4 + q];
-    s += sb;
-  }
-  out[t * 4 + q] = s;
-  if (q == 0) {
-    int f = 0;
-    for (int a = 0; a < chain; ++a) f |= flags[t * chain + a];
-    tflag[t] = f;
-  }
-}
-
-// Single-molecule delta: beads [0, ms) are the new molecule, [ms, 2 ms) the old
-// one; slot of an atom: HH / HG / GG by its component and the moved component
-// (mc_single_particle.h:142-170). part[block][6], flag from new beads only.
-template <int PREC>
-__global__ void __launch_bounds__(GRX_THREADS) single_body_kernel(BoxDev b, const Bead* beads, int ms,
-                                                                  int do_new, int do_old, int component,
-                                                                  int new_mol, int old_mol, double* part,
-                                                                  int* flag_out) {
-  __shared__ double sbuf[32];
-  const int nb = 2 * ms;
-  const int nl = blockDim.x / nb;
-  const int tid = threadIdx.x;
-  double e[6] = {0, 0, 0, 0, 0, 0};
-  int flag = 0;
-  if (tid < nl * nb) {
-    const int bead = tid % nb;
-    const bool is_new = bead < ms;
-    if ((is_new && do_new) || (!is_new && do_old)) {
-      const Bead bd = beads[bead];
-      const bool moved_host = component < b.nhost;
-      const int mol = is_new ? new_mol : old_mol;
-      for (int c = 0; c < b.ncomp; ++c) {
-        const bool host = c < b.nhost;
-        const int slot = moved_host ? (host ? 0 : 1) : (host ? 1 : 2);
-        const int n = b.comp_size[c];
-        const int off = b.comp_off[c];
-        double v = 0.0, r = 0.0;
-        int f = 0;
-        for (int i = blockIdx.x * nl + tid / nb; i < n; i += gridDim.x * nl) {
-          if (c == component && b.meta[off + i].y == mol) continue;
-          pair_energy<PREC>(b, off + i, bd, 0, v, r, f);
-        }
-        const double sg = is_new ? 1.0 : -1.0;
-        e[2 * slot] += sg * v;
-        e[2 * slot + 1] += sg * r;
-        if (is_new) flag |= f;
-      }
-    }
-  }
-  if (flag) atomicOr(flag_out, 1);
-  for (int k = 0; k < 6; ++k) {
-    const double v = block_sum(e[k], sbuf);
-    if (tid == 0) part[6 * blockIdx.x + k] = v;
-  }
-}
 
 static void host_split(double x, float& h, float& l) {
   const double hd = std::nearbyint(x * GRX_GRID_COORD) / GRX_GRID_COORD;
@@ -114,10 +47,12 @@ static grx_status stage_beads(const grx_trials* t, size_t first_bead, size_t nbe
   return GRX_OK;
 }
 
-template <int PREC>
-static void launch_trial_pass(grx_box* b, const Bead* beads, int nb, int comp, int newmol, int ec, int em,
-                              double* part, int* flags) {
-  trial_bead_kernel<PREC><<<nb, GRX_THREADS, 0, b->stream>>>(b->dev, beads, comp, newmol, ec, em, part, flags);
+static void run_trials(grx_box* b, const TrialArgs& a, int ntrials, int prec) {
+  if (prec == GRX_FP64) launch_trials<GRX_FP64>(b->dev, a, ntrials, b->stream);
+  else if (prec == GRX_MIXED) launch_trials<GRX_MIXED>(b->dev, a, ntrials, b->stream);
+  else if (prec == kMixed64) launch_trials<kMixed64>(b->dev, a, ntrials, b->stream);
+  else launch_trials<GRX_FP32>(b->dev, a, ntrials, b->stream);
+  count_launch();
 }
 
 }  // namespace grx
@@ -139,48 +74,38 @@ grx_status grx_trial_energies(grx_box* b, const grx_trials* t, int32_t component
   refresh_dev(b);
   const size_t ch = t->chainsize;
   const size_t per_chunk = std::max<size_t>(1, GRX_MAX_TRIAL_BEADS / ch);
-  std::vector<double> host_out;
-  std::vector<int> host_flag;
+  std::vector<double> eo(4 * t->ntrials);
+  std::vector<uint8_t> fo(t->ntrials);
   for (size_t t0 = 0; t0 < t->ntrials; t0 += per_chunk) {
     const size_t ntr = std::min(per_chunk, t->ntrials - t0);
     const int nb = (int)(ntr * ch);
     std::vector<Bead> beads;
     grx_status st = stage_beads(t, t0 * ch, nb, b->dev.prefactor, beads);
     if (st) return st;
-    const int nblk = 1;
     const size_t bead_bytes = (nb * sizeof(Bead) + 255) / 256 * 256;
-    const size_t part_bytes = ((size_t)nblk * nb * 4 * sizeof(double) + 255) / 256 * 256;
-    const size_t flag_bytes = ((size_t)nb * sizeof(int) + 255) / 256 * 256;
-    const size_t out_bytes = ntr * 4 * sizeof(double) + ntr * sizeof(int);
-    st = ensure_scratch(b, bead_bytes + part_bytes + flag_bytes + out_bytes + 256);
+    const size_t out_bytes = (ntr * 4 * sizeof(double) + 255) / 256 * 256;
+    st = ensure_scratch(b, bead_bytes + out_bytes + ntr);
     if (st) return st;
     char* base = (char*)b->scratch;
-    Bead* d_beads = (Bead*)base;
-    double* part = (double*)(base + bead_bytes);
-    int* flags = (int*)(base + bead_bytes + part_bytes);
-    double* d_out = (double*)(base + bead_bytes + part_bytes + flag_bytes);
-    int* d_tflag = (int*)(d_out + ntr * 4);
-    GRX_CHECK_CUDA(cudaMemcpyAsync(d_beads, beads.data(), nb * sizeof(Bead), cudaMemcpyHostToDevice, b->stream), "upload beads");
-    GRX_CHECK_CUDA(cudaMemsetAsync(flags, 0, nb * sizeof(int), b->stream), "clear flags");
-    const int ec = (int)exclude_comp, em = (int)exclude_molid;
-    if (prec == GRX_FP64) launch_trial_pass<GRX_FP64>(b, d_beads, nb, component, (int)t->molid, ec, em, part, flags);
-    else if (prec == GRX_MIXED) launch_trial_pass<GRX_MIXED>(b, d_beads, nb, component, (int)t->molid, ec, em, part, flags);
-    else launch_trial_pass<GRX_FP32>(b, d_beads, nb, component, (int)t->molid, ec, em, part, flags);
-    trial_reduce_kernel<<<(int)((ntr * 4 + 127) / 128), 128, 0, b->stream>>>(part, flags, nblk, nb, (int)ch, d_out, d_tflag);
-    count_launch(2);
+    TrialArgs a{};
+    a.beads = (Bead*)base;
+    a.chain = (int)ch;
+    a.component = component;
+    a.mol[0] = (int)t->molid;
+    a.split = (int)ntr;
+    a.excl_comp = (int)exclude_comp;
+    a.excl_mol = (int)exclude_molid;
+    a.out = (double*)(base + bead_bytes);
+    a.over = (unsigned char*)(base + bead_bytes + out_bytes);
+    GRX_CHECK_CUDA(cudaMemcpyAsync(base, beads.data(), nb * sizeof(Bead), cudaMemcpyHostToDevice, b->stream), "upload beads");
+    run_trials(b, a, (int)ntr, prec);
     GRX_CHECK_CUDA(cudaGetLastError(), "trial energy launch");
-    std::vector<double> eo(ntr * 4);
-    std::vector<int> fo(ntr);
-    GRX_CHECK_CUDA(cudaMemcpyAsync(eo.data(), d_out, ntr * 4 * sizeof(double), cudaMemcpyDeviceToHost, b->stream), "read energies");
-    GRX_CHECK_CUDA(cudaMemcpyAsync(fo.data(), d_tflag, ntr * sizeof(int), cudaMemcpyDeviceToHost, b->stream), "read flags");
+    GRX_CHECK_CUDA(cudaMemcpyAsync(eo.data() + 4 * t0, a.out, ntr * 4 * sizeof(double), cudaMemcpyDeviceToHost, b->stream), "read energies");
+    GRX_CHECK_CUDA(cudaMemcpyAsync(fo.data() + t0, a.over, ntr, cudaMemcpyDeviceToHost, b->stream), "read flags");
     GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "trial energies");
-    host_out.insert(host_out.end(), eo.begin(), eo.end());
-    host_flag.insert(host_flag.end(), fo.begin(), fo.end());
   }
-  std::vector<uint8_t> f8(t->ntrials);
-  for (size_t k = 0; k < t->ntrials; ++k) f8[k] = host_flag[k] ? 1 : 0;
-  GRX_CHECK_CUDA(cudaMemcpy(out, host_out.data(), t->ntrials * sizeof(grx_trial_energy), cudaMemcpyDefault), "write energies");
-  GRX_CHECK_CUDA(cudaMemcpy(overlap, f8.data(), t->ntrials, cudaMemcpyDefault), "write flags");
+  GRX_CHECK_CUDA(cudaMemcpy(out, eo.data(), t->ntrials * sizeof(grx_trial_energy), cudaMemcpyDefault), "write energies");
+  GRX_CHECK_CUDA(cudaMemcpy(overlap, fo.data(), t->ntrials, cudaMemcpyDefault), "write flags");
   return GRX_OK;
 }
 
@@ -200,36 +125,37 @@ grx_status grx_single_body_energy(grx_box* b, const grx_trials* old_mol, const g
   st = stage_beads(old_mol, 0, ms, b->dev.prefactor, ob_);
   if (st) return st;
   nb_.insert(nb_.end(), ob_.begin(), ob_.end());
-  size_t total_atoms = 0;
-  for (int c = 0; c < b->ncomp; ++c) total_atoms += b->cap[c];
-  const int nl = GRX_THREADS / (int)(2 * ms);
-  int nblk = (int)std::min<size_t>((total_atoms + (size_t)nl * 16 - 1) / ((size_t)nl * 16), 2 * (size_t)sm_count(b));
-  nblk = std::max(nblk, 1);
   const size_t bead_bytes = (2 * ms * sizeof(Bead) + 255) / 256 * 256;
-  st = ensure_scratch(b, bead_bytes + 6 * nblk * sizeof(double) + 256);
+  st = ensure_scratch(b, bead_bytes + 256);
   if (st) return st;
-  Bead* d_beads = (Bead*)b->scratch;
-  double* part = (double*)((char*)b->scratch + bead_bytes);
-  int* d_flag = (int*)(part + 6 * nblk);
-  GRX_CHECK_CUDA(cudaMemcpyAsync(d_beads, nb_.data(), 2 * ms * sizeof(Bead), cudaMemcpyHostToDevice, b->stream), "upload beads");
-  GRX_CHECK_CUDA(cudaMemsetAsync(d_flag, 0, sizeof(int), b->stream), "clear flag");
-  const int nm = (int)new_mol->molid, om = (int)old_mol->molid;
-  if (prec == GRX_FP64)
-    single_body_kernel<GRX_FP64><<<nblk, GRX_THREADS, 0, b->stream>>>(b->dev, d_beads, (int)ms, do_new, do_old, component, nm, om, part, d_flag);
-  else if (prec == GRX_MIXED)
-    single_body_kernel<GRX_MIXED><<<nblk, GRX_THREADS, 0, b->stream>>>(b->dev, d_beads, (int)ms, do_new, do_old, component, nm, om, part, d_flag);
-  else
-    single_body_kernel<GRX_FP32><<<nblk, GRX_THREADS, 0, b->stream>>>(b->dev, d_beads, (int)ms, do_new, do_old, component, nm, om, part, d_flag);
-  count_launch();
+  // two trials: the new molecule and the old one, each without the atoms of its own molecule id
+  TrialArgs a{};
+  a.beads = (Bead*)b->scratch;
+  a.chain = (int)ms;
+  a.component = component;
+  a.mol[0] = (int)new_mol->molid;
+  a.mol[1] = (int)old_mol->molid;
+  a.split = 1;
+  a.excl_comp = -1;
+  a.excl_mol = -1;
+  a.out = (double*)((char*)b->scratch + bead_bytes);
+  a.over = (unsigned char*)(a.out + 8);
+  GRX_CHECK_CUDA(cudaMemcpyAsync(b->scratch, nb_.data(), 2 * ms * sizeof(Bead), cudaMemcpyHostToDevice, b->stream), "upload beads");
+  run_trials(b, a, 2, prec == GRX_MIXED ? kMixed64 : (int)prec);
   GRX_CHECK_CUDA(cudaGetLastError(), "single body launch");
-  std::vector<double> parts(6 * nblk);
-  int flag = 0;
-  GRX_CHECK_CUDA(cudaMemcpyAsync(parts.data(), part, 6 * nblk * sizeof(double), cudaMemcpyDeviceToHost, b->stream), "read partials");
-  GRX_CHECK_CUDA(cudaMemcpyAsync(&flag, d_flag, sizeof(int), cudaMemcpyDeviceToHost, b->stream), "read flag");
+  struct { double e[8]; unsigned char over[8]; } r;
+  GRX_CHECK_CUDA(cudaMemcpyAsync(&r, a.out, sizeof(r), cudaMemcpyDeviceToHost, b->stream), "read energies");
   GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "single body");
+  // HH / HG / GG by the atom's component and the moved one (mc_single_particle.h:142-170)
   double e[6] = {0, 0, 0, 0, 0, 0};
-  for (int k = 0; k < nblk; ++k)
-    for (int q = 0; q < 6; ++q) e[q] += parts[6 * k + q];
+  const int host_slot = component < b->nhost ? 0 : 2;
+  for (int q = 0; q < 4; ++q) {
+    double d = 0.0;
+    if (do_new) d += r.e[q];
+    if (do_old) d -= r.e[4 + q];
+    e[host_slot + q] = d;
+  }
+  const int flag = do_new && r.over[0];
   GRX_CHECK_CUDA(cudaMemcpy(out6, e, 6 * sizeof(double), cudaMemcpyDefault), "write energies");
   uint8_t f8 = flag ? 1 : 0;
   GRX_CHECK_CUDA(cudaMemcpy(overlap, &f8, 1, cudaMemcpyDefault), "write flag");

@@ -19,6 +19,12 @@ namespace grx {
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kQueue = 64;  // ring buffer entries per warp
 
+// The mixed form of the single-molecule delta: split FP32 screening and FP32 LJ outside 1.1
+// sigma as in GRX_MIXED, displacement, LJ inside and real-space Coulomb in FP64. A move's two
+// configurations share nearly all of their energy, so the double-float Coulomb of the trial
+// passes would show in their difference.
+constexpr int kMixed64 = 3;
+
 // ---------------------------------------------------------------- voxel-list staging
 // A warp walking a bead's voxel list stages the next 8 chunks (256 entries) into its own shared
 // buffer with one bulk copy (cp.async.bulk, completion on an mbarrier) instead of one dependent
@@ -351,7 +357,29 @@ __device__ __forceinline__ void pair_dense(const BoxDev& b, bool host, int i, co
     float3 dh = make_float3(ah.x - bd.h.x, ah.y - bd.h.y, ah.z - bd.h.z);
     float3 dl = make_float3(al.x - bd.l.x, al.y - bd.l.y, al.z - bd.l.z);
     image_split(b, dh, dl);
-    if constexpr (PREC == GRX_MIXED) {
+    if constexpr (PREC == kMixed64) {
+      const double x = (double)dh.x + (double)dl.x;
+      const double y = (double)dh.y + (double)dl.y;
+      const double z = (double)dh.z + (double)dl.z;
+      const double rr = x * x + y * y + z * z;
+      if (rr < b.cut_vdw2) {
+        const float4 f = b.ff32[row];
+        const bool unit = sc1 && (bd.unit & 1) && !b.use_1264;
+        double e;
+        if (unit && (float)rr > f.w) e = (double)vdw32(f, (float)rr);
+        else e = vdw64_cold(b, row, rr, (host ? b.hscale : b.scale)[i] * bd.scale);
+        if (e > b.overlap) flag = 1;
+        if (rr < 0.01) flag = 1;
+        acc.v += e;
+      }
+      if (!b.no_charges && rr < b.cut_coul2) {
+        const int k = table64_piece<kShiftG64>(rr, b.g64_base);
+        double g;
+        if ((unsigned)k < (unsigned)b.g64_n) g = table64<kShiftG64>(b.g64, k, rr);
+        else g = coul_g_cold(b, rr);
+        acc.r = fma((host ? b.hpos64 : b.pos64)[i].w, g, acc.r);
+      }
+    } else if constexpr (PREC == GRX_MIXED) {
       const df s = df_norm2_split(dh, dl);
       if (df_lt(s, df{b.cut_vdw2_df.x, b.cut_vdw2_df.y})) {
         const float4 f = b.ff32[row];
@@ -699,7 +727,7 @@ __device__ __forceinline__ void warp_store(const LaneAcc<PREC>& h, const LaneAcc
     double d = 0.0, e = 0.0;
     if (with_guests) { d = warp_sum(g.v); e = warp_sum(g.r); }
     if (lane == 0) {
-      const double f = PREC == GRX_FP64 ? pq64 : 1.0;  // FP64 real parts: sums of q_atom g
+      const double f = PREC == GRX_FP64 || PREC == kMixed64 ? pq64 : 1.0;  // FP64 real parts: sums of q_atom g
       out4[0] = a; out4[1] = c * f; out4[2] = d; out4[3] = e * f;
     }
   }
@@ -908,34 +936,132 @@ __device__ __forceinline__ void reduce_items(const double* ipart, const int* ifl
   }
 }
 
-// Trial energies of one bead per block, the launch behind grx_trial_energies and
-// grx_trial_energies_noalloc (both entry points run this one kernel, so they give the
-// same sums); per-bead sums go to part[bead][4] and the overlap flag to flags[bead].
+// ---------------------------------------------------------------- single passes
+// One trial (`chain` beads in shared memory) against every atom by a cluster of kTrialCtas CTAs
+// of kTrialWarps warps. A host-driven call has 1 to 64 trials and its time is latency, so the
+// pass is cut into 32 items spread over eight SMs (one block per bead left 142 of 152 SMs idle
+// on a ten-trial step); the split depends on the chain length alone, so a trial's sums are the
+// same whatever else the call holds. The CTAs write their partial slots into CTA 0, whose warp q
+// adds quantity q over the slots.
+constexpr int kTrialCtas = 8;
+constexpr int kTrialWarps = 4;
+constexpr int kTrialItems = kTrialCtas * kTrialWarps;
+constexpr int kTrialSlots = kTrialItems + GRX_MAX_TRIAL_BEADS;
+
+// One block copies a descriptor (a kernel parameter) into shared memory, where the out-of-line
+// pass reads it through a pointer. The caller synchronises.
+template <class T>
+__device__ __forceinline__ void copy_words(T* dst, const T* src) {
+  static_assert(sizeof(T) % 8 == 0, "copied in 8-byte words");
+  for (int k = threadIdx.x; k < (int)(sizeof(T) / 8); k += blockDim.x)
+    reinterpret_cast<unsigned long long*>(dst)[k] = reinterpret_cast<const unsigned long long*>(src)[k];
+}
+
+struct TrialWork {
+  double ipart[kTrialSlots * 4];
+  int iflag[kTrialSlots];
+  int qbuf[kTrialWarps * kQueue];
+  int counter;
+};
+
+// Called by every thread of the cluster after `beads` is filled and before any barrier that
+// publishes it. In CTA 0, lane 0 of warp q < 4 returns quantity q (hg_vdw, hg_real, gg_vdw,
+// gg_real) in `sum` and the overlap flag in `flag`.
 template <int PREC>
-__global__ void __launch_bounds__(GRX_THREADS) trial_bead_kernel(BoxDev b, const Bead* beads, int component,
-                                                                 int newmol, int excl_comp, int excl_mol,
-                                                                 double* part, int* flags) {
-  __shared__ double ipart[kMaxItems * 4];
-  __shared__ int iflag[kMaxItems];
-  __shared__ int qbuf[(GRX_THREADS / 32) * kQueue];
-  __shared__ int counter;
-  if (threadIdx.x == 0) counter = 0;
-  __syncthreads();
-  const PassSplit sp = pass_split(b, 1, GRX_THREADS / 32, 4);
-  const int nch = (int)sp.items;  // one bead: slot = item
-  block_bead_pass<PREC>(b, beads + blockIdx.x, 1, component, newmol, excl_comp, excl_mol, qbuf, ipart, iflag,
-                        &counter, sp);
-  __syncthreads();
-  if (threadIdx.x < 4) {
-    double s = 0.0;
-    for (int c = 0; c < nch; ++c) s += item_get<PREC>(ipart, c * 4 + threadIdx.x);
-    part[blockIdx.x * 4 + threadIdx.x] = s;
+__device__ __forceinline__ void trial_cluster_pass(const BoxDev& b, const Bead* beads, TrialWork& W, int chain,
+                                                   int component, int newmol, int excl_comp, int excl_mol, double& sum,
+                                                   int& flag) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned rank = cluster_rank();
+  const PassSplit sp = pass_split(b, chain, kTrialItems, 1);
+  const int nslot = (int)sp.items + chain;
+  if (rank == 0) {  // a slot between two beads may stay unwritten
+    for (int k = tid; k < nslot * 4; k += blockDim.x) W.ipart[k] = 0.0;
+    for (int k = tid; k < nslot; k += blockDim.x) W.iflag[k] = 0;
   }
-  if (threadIdx.x == 0) {
-    int f = 0;
-    for (int c = 0; c < nch; ++c) f |= iflag[c];
-    flags[blockIdx.x] = f;
+  if (tid == 0) W.counter = 0;
+  __syncthreads();
+  cluster_sync_all();
+  int i0, i1;
+  cluster_items(sp, kTrialCtas, rank, i0, i1);
+  if (i0 < i1 && sp.nu > 0) {
+    block_bead_pass<PREC>(b, beads, chain, component, newmol, excl_comp, excl_mol, W.qbuf, W.ipart, W.iflag, &W.counter,
+                          sp, i0, i1);
+    __syncthreads();
+    if (rank != 0) {
+      unsigned lo, hi;
+      double* dst = cluster_map(W.ipart, 0);
+      int* df = cluster_map(W.iflag, 0);
+      for (int item = i0; item < i1; ++item) {  // the slots this CTA wrote, gaps left out
+        sp.range((unsigned)item, lo, hi);
+        const int b0 = (int)(lo / sp.nu), b1 = (int)((hi - 1u) / sp.nu);
+        for (int k = tid; k < 5 * (b1 - b0 + 1); k += blockDim.x) {
+          const int slot = item + b0 + k / 5, f = k % 5;
+          if (f < 4) dst[slot * 4 + f] = W.ipart[slot * 4 + f];
+          else df[slot] = W.iflag[slot];
+        }
+      }
+    }
   }
+  __syncthreads();
+  cluster_sync_all();
+  sum = 0.0;
+  flag = 0;
+  if (rank == 0 && warp < 4) {
+    for (int s = lane; s < nslot; s += 32) {
+      sum += item_get<PREC>(W.ipart, s * 4 + warp);
+      flag |= W.iflag[s];
+    }
+    sum = warp_sum(sum);
+    flag = __any_sync(kFull, flag != 0) ? 1 : 0;
+  }
+}
+
+// Trial energies behind grx_trial_energies, grx_trial_energies_noalloc and
+// grx_single_body_energy (they run this one kernel, so they give the same sums): one cluster
+// per trial; trial t leaves out the atoms of (component, mol[t < split ? 0 : 1]).
+struct TrialArgs {
+  const Bead* beads;
+  int chain;
+  int component;
+  int mol[2];
+  int split;
+  int excl_comp;
+  int excl_mol;
+  double* out;          // 4 per trial
+  unsigned char* over;  // 1 per trial
+};
+
+template <int PREC>
+__global__ void __cluster_dims__(kTrialCtas, 1, 1) __launch_bounds__(kTrialWarps * 32)
+    trial_kernel(const __grid_constant__ BoxDev box, const __grid_constant__ TrialArgs a) {
+  extern __shared__ double2 trial_smem[];
+  Bead* beads = reinterpret_cast<Bead*>(trial_smem);
+  __shared__ TrialWork W;
+  __shared__ BoxDev b;
+  copy_words(&b, &box);
+  const int t = (int)blockIdx.x / kTrialCtas;
+  const int nw = a.chain * (int)(sizeof(Bead) / 8);
+  const double* src = reinterpret_cast<const double*>(a.beads + (size_t)t * a.chain);
+  for (int k = threadIdx.x; k < nw; k += blockDim.x) reinterpret_cast<double*>(beads)[k] = src[k];
+  __syncthreads();
+  double sum;
+  int flag;
+  trial_cluster_pass<PREC>(b, beads, W, a.chain, a.component, a.mol[t < a.split ? 0 : 1], a.excl_comp, a.excl_mol, sum,
+                           flag);
+  const int warp = threadIdx.x >> 5;
+  if (cluster_rank() == 0 && warp < 4 && (threadIdx.x & 31) == 0) {
+    a.out[4 * t + warp] = sum;
+    if (warp == 0) a.over[t] = (unsigned char)flag;
+  }
+}
+
+static_assert(sizeof(Bead) % 8 == 0, "beads are staged in 8-byte words");
+
+// Enqueues the pass over ntrials trials (ntrials >= 1).
+template <int PREC>
+static inline void launch_trials(const BoxDev& b, const TrialArgs& a, int ntrials, cudaStream_t s) {
+  trial_kernel<PREC><<<ntrials * kTrialCtas, kTrialWarps * 32, a.chain * sizeof(Bead), s>>>(b, a);
 }
 
 }  // namespace grx
