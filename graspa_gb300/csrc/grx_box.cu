@@ -457,6 +457,36 @@ static void build_kvectors(grx_box* b, const grx_box_geometry& g) {
     b->h_ktemp.push_back(factor * std::exp((-0.25 / alpha_sq) * rksq) / rksq);
   }
   b->nact = (int)b->h_kact.size();
+  // rows (runs of kact with one kx, ky; the cutoff is convex, so kz is contiguous but for the
+  // origin) and groups of rows with at most 128 columns and 32 rows (a block of sk_kernel)
+  b->h_krow.clear();
+  b->h_kgroup.clear();
+  for (int j = 0; j < b->nact;) {
+    int e = j + 1;
+    while (e < b->nact && b->h_kact[e].x == b->h_kact[j].x && b->h_kact[e].y == b->h_kact[j].y &&
+           (b->h_kact[e].z == b->h_kact[e - 1].z + 1 || (b->h_kact[j].x == 0 && b->h_kact[j].y == 0 &&
+                                                         b->h_kact[e - 1].z == -1 && b->h_kact[e].z == 1)))
+      ++e;
+    KRow r{};
+    r.kx = b->h_kact[j].x;
+    r.ky = b->h_kact[j].y;
+    r.lo = b->h_kact[j].z;
+    r.hi = b->h_kact[e - 1].z;
+    r.first = j;
+    r.ncol = std::max(std::abs(r.lo), std::abs(r.hi)) + 1;
+    const int k = (int)b->h_krow.size();
+    if (b->h_kgroup.empty() || k - b->h_kgroup.back().x >= 32 ||
+        b->h_krow.back().col + b->h_krow.back().ncol + r.ncol > 128) {
+      b->h_kgroup.push_back(make_int2(k, k));
+      r.col = 0;
+    } else {
+      r.col = b->h_krow.back().col + b->h_krow.back().ncol;
+    }
+    b->h_kgroup.back().y = k + 1;
+    b->h_krow.push_back(r);
+    j = e;
+  }
+  b->n_kgroups = (int)b->h_kgroup.size();
 }
 
 }  // namespace grx
@@ -677,6 +707,8 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
   const size_t nv = std::max(b->nvec, 1), na = std::max(b->nact, 1);
   if ((e = dev_alloc(b, (void**)&b->kact, na * sizeof(int4))) != cudaSuccess) return fail(e, "alloc kact");
   if ((e = dev_alloc(b, (void**)&b->ktemp, na * sizeof(double))) != cudaSuccess) return fail(e, "alloc ktemp");
+  if ((e = dev_alloc(b, (void**)&b->krow, (b->h_krow.size() + 1) * sizeof(KRow))) != cudaSuccess) return fail(e, "alloc k rows");
+  if ((e = dev_alloc(b, (void**)&b->kgroup, (b->h_kgroup.size() + 1) * sizeof(int2))) != cudaSuccess) return fail(e, "alloc k groups");
   if ((e = dev_alloc(b, (void**)&b->s_fw, nv * sizeof(double2))) != cudaSuccess) return fail(e, "alloc s_fw");
   if ((e = dev_alloc(b, (void**)&b->s_ads, nv * sizeof(double2))) != cudaSuccess) return fail(e, "alloc s_ads");
   if ((e = dev_alloc(b, (void**)&b->s_tmp, nv * sizeof(double2))) != cudaSuccess) return fail(e, "alloc s_tmp");
@@ -704,6 +736,8 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
   if (b->nact) {
     cudaMemcpy(b->kact, b->h_kact.data(), b->nact * sizeof(int4), cudaMemcpyHostToDevice);
     cudaMemcpy(b->ktemp, b->h_ktemp.data(), b->nact * sizeof(double), cudaMemcpyHostToDevice);
+    cudaMemcpy(b->krow, b->h_krow.data(), b->h_krow.size() * sizeof(KRow), cudaMemcpyHostToDevice);
+    cudaMemcpy(b->kgroup, b->h_kgroup.data(), b->h_kgroup.size() * sizeof(int2), cudaMemcpyHostToDevice);
   }
   if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return fail(e, "box upload");
   if (!ff.no_charges) {
@@ -744,6 +778,7 @@ grx_status grx_box_footprint(const grx_box_desc* desc, size_t* bytes) {
   size_t t = al(n * sizeof(double4)) + 2 * al(n * sizeof(float4)) + al(n * sizeof(int2)) + 2 * al(n * sizeof(double)) +
              al(n * sizeof(float2)) + al(GRX_MAX_COMPONENTS * sizeof(int));
   t += al((nt2 + 27) * sizeof(FFPair64)) + al(nt2 * sizeof(double)) + 2 * al(nt2 * sizeof(float4)) + al(nt2 * sizeof(float2));
+  t += al((tmp.h_krow.size() + 1) * sizeof(KRow)) + al((tmp.h_kgroup.size() + 1) * sizeof(int2));
   t += al(na * sizeof(int4)) + al(na * sizeof(double)) + 3 * al(nv * sizeof(double2)) + 2 * al(na * sizeof(float4)) +
        al(na * sizeof(float2));
   t += al(ntiles * sizeof(float4)) + al(ntiles * sizeof(int4));
@@ -840,7 +875,7 @@ grx_status grx_box_destroy(grx_box* b) {
     return GRX_OK;
   }
   void* ptrs[] = {b->pos64, b->hi, b->lo, b->meta, b->scale, b->charge, b->d_size, b->ff64,
-                  b->ffc10, b->ff32, b->kact, b->ktemp, b->s_fw, b->s_ads, b->s_tmp,
+                  b->ffc10, b->ff32, b->kact, b->ktemp, b->krow, b->kgroup, b->s_fw, b->s_ads, b->s_tmp,
                   b->scratch, b->d_results, b->tile_c, b->tile_r, b->ctab, b->ctabf, b->qdf,
                   b->ffdf, b->ffdf2, b->ewA, b->ewF, b->ewT, b->vmeta, b->vlist, b->hrec, b->htype};
   for (void* p : ptrs) dev_free(b, p);
@@ -946,6 +981,9 @@ grx_status grx_box_set_component(grx_box* b, int32_t comp, const grx_atoms* a, i
     b->h_charge[o + i] = q[i];
     b->h_scale_coul[o + i] = scc[i];
   }
+  b->many_mols[comp] = 0;
+  for (size_t i = 1; comp < b->nhost && i < a->size; ++i)
+    if (mol[i] != mol[0]) b->many_mols[comp] = 1;
   b->size[comp] = (int)a->size;
   b->stored[comp] = nst;
   b->rigid[comp] = rigid;

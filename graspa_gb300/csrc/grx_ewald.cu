@@ -5,6 +5,7 @@
 #include <vector>
 
 #include "grx_host.h"
+#include "grx_warp.cuh"
 
 namespace grx {
 
@@ -25,34 +26,31 @@ __device__ __forceinline__ int comp_of(const CompRanges& r, int j, int& local) {
   return c;
 }
 
-// eik tables of every live atom: e^{i k s} for k = 0..kmax per axis by the
-// recurrence of Initialize_Vectors (Ewald_Energy_Functions.h:42-95).
-__global__ void eik_tables_kernel(BoxDev b, CompRanges r, double2* ex, double2* ey, double2* ez) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+// eik tables of the live atoms [r.first, r.n): e^{i k s} for k = 0..kmax per axis by the
+// recurrence of Initialize_Vectors (Ewald_Energy_Functions.h:42-95). x tables carry the charge
+// (q e^{i kx s}); x and y are [k][atom], z is [atom][k], as sk_kernel reads them.
+__global__ void eik_tables_kernel(BoxDev b, CompRanges r, int first, double2* ex, double2* ey, double2* ez) {
+  const int j = first + blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= r.n) return;
   int local;
   const int c = comp_of(r, j, local);
   const double4 p = atom_pos64(b, r.off[c] + local);
   const double PI2 = 2.0 * 3.14159265358979323846;
-  double s[3];
-  s[0] = (b.inv[0] * p.x + b.inv[3] * p.y + b.inv[6] * p.z) * PI2;
-  s[1] = (b.inv[1] * p.x + b.inv[4] * p.y + b.inv[7] * p.z) * PI2;
-  s[2] = (b.inv[2] * p.x + b.inv[5] * p.y + b.inv[8] * p.z) * PI2;
-  double2* t[3] = {ex, ey, ez};
-  for (int d = 0; d < 3; ++d) {
-    const int km = b.kmax[d];
-    const size_t n = r.n;
-    t[d][j] = make_double2(1.0, 0.0);
-    if (km >= 1) {
-      double sn, cs;
-      sincos(s[d], &sn, &cs);
-      const double2 e1 = make_double2(cs, sn);
-      t[d][j + n] = e1;
-      double2 e = e1;
-      for (int k = 2; k <= km; ++k) {
-        e = cmul(e, e1);
-        t[d][j + k * n] = e;
-      }
+  const int d = blockIdx.y;  // one axis per thread: the recurrence is a serial chain
+  const double s = (b.inv[d] * p.x + b.inv[3 + d] * p.y + b.inv[6 + d] * p.z) * PI2;
+  const int km = b.kmax[d];
+  const size_t n = r.n;
+  double2* t = d == 0 ? ex + j : (d == 1 ? ey + j : ez + (size_t)j * (km + 1));
+  const size_t stride = d == 2 ? 1 : n;
+  double2 e = d == 0 ? make_double2(p.w, 0.0) : make_double2(1.0, 0.0);
+  t[0] = e;
+  if (km >= 1) {
+    double sn, cs;
+    sincos(s, &sn, &cs);
+    const double2 e1 = make_double2(cs, sn);
+    for (int k = 1; k <= km; ++k) {
+      e = cmul(e, e1);
+      t[k * stride] = e;
     }
   }
 }
@@ -66,31 +64,132 @@ __device__ __forceinline__ double2 eik_term(const double2* ex, const double2* ey
   return cmul(cmul(ex[j + n * (size_t)kx], y), z);
 }
 
-// Structure factors per active k, split framework / adsorbate (Ewald_Total,
-// ewald_preparation.h:128-147). One block per active k, deterministic sums.
-__global__ void __launch_bounds__(GRX_THREADS) sk_kernel(BoxDev b, CompRanges r, const double2* ex,
-                                                         const double2* ey, const double2* ez) {
+// Structure factors (Ewald_Total, ewald_preparation.h:128-147). A block holds the columns
+// (kx, ky, |kz|) of a few (kx, ky) rows, one per thread, and walks one chunk of atoms in tiles
+// of 32: the tile's q X Y products are formed once per row in shared memory, and a column's
+// four real sums with Re Z and Im Z give both +kz and -kz, two FP64 FMAs per (k, atom) where
+// the direct product of three factors takes ten. FP64 issue (two lanes per SM and clock)
+// bounds it. Chunks hold framework or adsorbate atoms only; their partial S(k) go to `part`
+// [chunk][active k], or straight into the structure factors when there is one chunk of each.
+constexpr int kSkCols = 128;
+constexpr int kSkRows = 32;
+constexpr int kSkTile = 32;
+
+struct SkChunks {
+  int n, nhost, n_host_chunks;  // atoms, framework atoms, chunks of them (0 when the framework's S is a parent's)
+  int host_len, guest_len;      // atoms per chunk
+};
+
+__global__ void __launch_bounds__(kSkCols) sk_kernel(BoxDev b, SkChunks c, const KRow* rows, const int2* groups,
+                                                     const double2* ex, const double2* ey, const double2* ez,
+                                                     double2* part) {
+  __shared__ double2 P[kSkRows][kSkTile + 1];
+  __shared__ KRow R[kSkRows];
+  const int tid = threadIdx.x;
+  const int2 g = groups[blockIdx.x];
+  const int nr = g.y - g.x;
+  for (int k = tid; k < nr; k += blockDim.x) R[k] = rows[g.x + k];
+  __syncthreads();
+  int row = 0;
+  while (row + 1 < nr && tid >= R[row + 1].col) ++row;
+  const int az = tid - R[row].col;
+  const bool live = az < R[row].ncol;
+  const int chunk = blockIdx.y;
+  const bool host = chunk < c.n_host_chunks;
+  const int a0 = host ? chunk * c.host_len : c.nhost + (chunk - c.n_host_chunks) * c.guest_len;
+  const int a1 = host ? min(a0 + c.host_len, c.nhost) : min(a0 + c.guest_len, c.n);
+  const int kz1 = b.kmax[2] + 1;
+  const double2* z = ez + (live ? az : 0);
+  double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
+  for (int t0 = a0; t0 < a1; t0 += kSkTile) {
+    for (int e = tid; e < nr * kSkTile; e += blockDim.x) {
+      const int k = e / kSkTile, at = e % kSkTile, j = t0 + at;
+      double2 v = make_double2(0.0, 0.0);
+      if (j < a1) {
+        double2 y = ey[(size_t)abs(R[k].ky) * c.n + j];
+        if (R[k].ky < 0) y.y = -y.y;
+        v = cmul(ex[(size_t)R[k].kx * c.n + j], y);
+      }
+      P[k][at] = v;
+    }
+    __syncthreads();
+    if (live) {
+      const int m = min(kSkTile, a1 - t0);
+      const double2* zt = z + (size_t)t0 * kz1;
+#pragma unroll 4
+      for (int at = 0; at < m; ++at) {
+        const double2 v = P[row][at], w = zt[(size_t)at * kz1];
+        s0 = fma(v.x, w.x, s0);
+        s1 = fma(v.y, w.y, s1);
+        s2 = fma(v.x, w.y, s2);
+        s3 = fma(v.y, w.x, s3);
+      }
+    }
+    __syncthreads();
+  }
+  if (!live) return;
+  double2* out = part ? part + (size_t)chunk * b.nact : nullptr;
+  double2* in_place = host ? b.s_fw : b.s_ads;
+  auto put = [&](int j, double2 v) {
+    if (out) out[j] = v;
+    else in_place[b.kact[j].w] = v;
+  };
+  const int jp = R[row].index(az), jm = az ? R[row].index(-az) : -1;
+  if (jp >= 0) put(jp, make_double2(s0 - s1, s2 + s3));
+  if (jm >= 0) put(jm, make_double2(s0 + s1, s3 - s2));
+}
+
+// Sums the chunks of every active k in order, writes S(k) and adds the Fourier energies
+// (Ewald_Total, ewald_preparation.h:150-161): epart per block {gg, hh, hg}.
+__global__ void __launch_bounds__(GRX_THREADS) sk_reduce_kernel(BoxDev b, const double2* part, int nh, int ng,
+                                                                double* epart) {
   __shared__ double sbuf[32];
-  const int4 k = b.kact[blockIdx.x];
-  double fr = 0, fi = 0, ar = 0, ai = 0;
-  const int nhost_atoms = r.base[r.nhost];
-  for (int j = threadIdx.x; j < r.n; j += blockDim.x) {
-    int local;
-    const int c = comp_of(r, j, local);
-    const double q = atom_pos64(b, r.off[c] + local).w;
-    const double2 t = eik_term(ex, ey, ez, r.n, j, k.x, k.y, k.z);
-    if (j < nhost_atoms) { fr += q * t.x; fi += q * t.y; }
-    else { ar += q * t.x; ai += q * t.y; }
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  double gg = 0.0, hh = 0.0, hg = 0.0;
+  if (j < b.nact) {
+    const int slot = b.kact[j].w;
+    double2 f, a;
+    if (part) {
+      f = a = make_double2(0.0, 0.0);
+      for (int k = 0; k < nh; ++k) {
+        const double2 v = part[(size_t)k * b.nact + j];
+        f.x += v.x; f.y += v.y;
+      }
+      for (int k = nh; k < nh + ng; ++k) {
+        const double2 v = part[(size_t)k * b.nact + j];
+        a.x += v.x; a.y += v.y;
+      }
+      if (b.shared_host) f = b.s_fw[slot];  // a replica reads its parent's
+      else b.s_fw[slot] = f;
+      b.s_ads[slot] = a;
+    } else {
+      f = b.s_fw[slot];
+      a = b.s_ads[slot];
+    }
+    b.s_tmp[slot] = a;
+    const double t = b.ktemp[j];
+    gg = t * (a.x * a.x + a.y * a.y);
+    hh = t * (f.x * f.x + f.y * f.y);
+    hg = t * (f.x * a.x + f.y * a.y) * 2.0;
   }
-  fr = block_sum(fr, sbuf);
-  fi = block_sum(fi, sbuf);
-  ar = block_sum(ar, sbuf);
-  ai = block_sum(ai, sbuf);
+  gg = block_sum(gg, sbuf);
+  hh = block_sum(hh, sbuf);
+  hg = block_sum(hg, sbuf);
   if (threadIdx.x == 0) {
-    if (!b.shared_host) b.s_fw[k.w] = make_double2(fr, fi);  // a replica reads its parent's
-    b.s_ads[k.w] = make_double2(ar, ai);
-    b.s_tmp[k.w] = make_double2(ar, ai);
+    epart[3 * blockIdx.x] = gg;
+    epart[3 * blockIdx.x + 1] = hh;
+    epart[3 * blockIdx.x + 2] = hg;
   }
+}
+
+// h(s) = erf(alpha sqrt s) / sqrt s from the table, by the library outside it.
+static __device__ __noinline__ double excl_h_cold(const BoxDev& b, double s) {
+  const double r = sqrt(s);
+  return erf(b.alpha * r) / r;
+}
+__device__ __forceinline__ double excl_h(const BoxDev& b, double s) {
+  const int k = table64_piece<kShiftH64>(s, b.h64_base);
+  return (unsigned)k < (unsigned)b.h64_n ? table64<kShiftH64>(b.h64, k, s) : excl_h_cold(b, s);
 }
 
 // Self energy and intramolecular erf exclusion per atom (ewald_preparation.h:189-249),
@@ -114,8 +213,7 @@ __global__ void __launch_bounds__(GRX_THREADS) self_excl_kernel(BoxDev b, CompRa
       const double4 q = atom_pos64(b, r.off[c] + l2);
       double x = p.x - q.x, y = p.y - q.y, z = p.z - q.z;
       pbc64(b, x, y, z);
-      const double rr = sqrt(x * x + y * y + z * z);
-      const double e = b.prefactor * p.w * q.w * erf(b.alpha * rr) / rr;
+      const double e = b.prefactor * p.w * q.w * excl_h(b, x * x + y * y + z * z);
       ea += e;
       if (c < r.nhost) eh += e;
     }
@@ -133,82 +231,138 @@ __global__ void __launch_bounds__(GRX_THREADS) self_excl_kernel(BoxDev b, CompRa
 }
 
 // Intramolecular erf exclusion of the molecules of one component with more than
-// kBigMolecule atoms (a framework is one such molecule): the pairs i < j of each
-// molecule spread over the whole grid instead of one thread per atom.
+// kBigMolecule atoms (a framework is one such molecule): the pairs i < j of each molecule in
+// 64 x 64 tiles, atoms of the j tile in shared memory. FP64 issue bounds it, so a pair takes
+// its image from FP32 fractions (image64) and erf(alpha r) / r from the table: 16 FP64
+// operations where sqrt, erf and the division took about 100.
 // part per block: [excl_all, excl_host].
+constexpr int kExclTile = 64;
+
 __global__ void __launch_bounds__(GRX_THREADS) big_excl_kernel(BoxDev b, CompRanges r, int c, double* part) {
   __shared__ double sbuf[32];
+  __shared__ double4 J[kExclTile];
+  __shared__ float4 H[kExclTile];
+  const int tid = threadIdx.x;
   const int ms = r.molsize[c];
   const int n = r.base[c + 1] - r.base[c];
   const long long nmol = (n + ms - 1) / ms;
-  const long long npair = nmol * (long long)ms * ms;
+  const long long T = (ms + kExclTile - 1) / kExclTile, per = T * (T + 1) / 2;
+  const float4* hi = c < r.nhost ? b.hhi : b.hi;
+  constexpr int kParts = GRX_THREADS / kExclTile, kSpan = kExclTile / kParts;
   double ea = 0.0;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < npair;
-       p += (long long)gridDim.x * blockDim.x) {
-    const long long m = p / ((long long)ms * ms);
-    const int rem = (int)(p - m * (long long)ms * ms);
-    const int i = rem / ms, j = rem - i * ms;
-    const int li = (int)(m * ms) + i, lj = (int)(m * ms) + j;
-    if (j <= i || lj >= n) continue;
-    const double4 a = atom_pos64(b, r.off[c] + li);
-    const double4 q = atom_pos64(b, r.off[c] + lj);
-    double x = a.x - q.x, y = a.y - q.y, z = a.z - q.z;
-    pbc64(b, x, y, z);
-    const double rr = sqrt(x * x + y * y + z * z);
-    ea += b.prefactor * a.w * q.w * erf(b.alpha * rr) / rr;
+  for (long long p = blockIdx.x; p < nmol * per; p += gridDim.x) {
+    const long long m = p / per;
+    const long long t = p - m * per;  // row-major upper triangle, counted from its last row
+    const long long u = per - 1 - t;
+    long long k = (long long)((sqrtf(8.0f * (float)u + 1.0f) - 1.0f) * 0.5f);
+    while (k * (k + 1) / 2 > u) --k;
+    while ((k + 1) * (k + 2) / 2 <= u) ++k;
+    const int ti = (int)(T - 1 - k), tj = (int)(T - 1 - (u - k * (k + 1) / 2));
+    const int m0 = (int)(m * ms), mend = min(m0 + ms, n);
+    const int i0 = m0 + ti * kExclTile, j0 = m0 + tj * kExclTile;
+    __syncthreads();
+    if (tid < kExclTile) {
+      const int j = j0 + tid;
+      const bool in = j < mend;
+      J[tid] = in ? atom_pos64(b, r.off[c] + j) : make_double4(0.0, 0.0, 0.0, 0.0);
+      H[tid] = in ? hi[r.off[c] + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    __syncthreads();
+    const int i = i0 + tid % kExclTile, s0 = tid / kExclTile * kSpan;
+    if (i < mend) {
+      const double4 a = atom_pos64(b, r.off[c] + i);
+      const float4 ah = hi[r.off[c] + i];
+      const bool near = fabsf(ah.x) < kNearCoord && fabsf(ah.y) < kNearCoord && fabsf(ah.z) < kNearCoord;
+      double e = 0.0;
+      for (int s = s0; s < s0 + kSpan; ++s) {
+        const int j = j0 + s;
+        if (j <= i || j >= mend) continue;
+        const double4 q = J[s];
+        const float4 qh = H[s];
+        double x = a.x - q.x, y = a.y - q.y, z = a.z - q.z;
+        image64(b, near, ah.x - qh.x, ah.y - qh.y, ah.z - qh.z, x, y, z);
+        e = fma(q.w, excl_h(b, x * x + y * y + z * z), e);
+      }
+      ea = fma(a.w, e, ea);
+    }
   }
-  ea = block_sum(ea, sbuf);
-  if (threadIdx.x == 0) {
+  ea = block_sum(ea * b.prefactor, sbuf);
+  if (tid == 0) {
     part[2 * blockIdx.x + 0] = ea;
     part[2 * blockIdx.x + 1] = c < r.nhost ? ea : 0.0;
   }
 }
 
-// Total VDW + real Coulomb over ordered pairs with factor 0.5 (VDWReal_Total_CPU,
-// VDW_Coulomb.cu:34-226; device form Total_VDW_Coulomb_Energy :1580-1665).
-// part per block: hh_v hh_r hg_v hg_r gg_v gg_r, then per block an overlap flag (a pair
-// with an adsorbate atom above the overlap criterion or closer than 0.1 A,
-// VDWCoulEnergy_Total :1385-1386).
-__global__ void __launch_bounds__(GRX_THREADS) vdw_real_total_kernel(BoxDev b, CompRanges r, double* part) {
+// VDW + real Coulomb of one adsorbate atom per cluster against every atom outside its
+// molecule, through the trial pass (VDWReal_Total_CPU, VDW_Coulomb.cu:34-226; device form
+// Total_VDW_Coulomb_Energy :1580-1665): hg sums as they are, gg sums count every pair twice.
+// part per atom: hg_v hg_r gg_v gg_r and the overlap flag (a pair above the overlap criterion
+// or closer than 0.1 A, VDWCoulEnergy_Total :1385-1386) as the fifth value.
+__global__ void __cluster_dims__(kTrialCtas, 1, 1) __launch_bounds__(kTrialWarps * 32)
+    guest_total_kernel(const __grid_constant__ BoxDev box, const __grid_constant__ CompRanges r, double* part) {
+  __shared__ TrialWork W;
+  __shared__ BoxDev b;
+  __shared__ Bead bead;
+  __shared__ int who[2];
+  copy_words(&b, &box);
+  __syncthreads();
+  const int t = (int)blockIdx.x / kTrialCtas;
+  if (threadIdx.x == 0) {
+    int local;
+    const int c = comp_of(r, r.base[r.nhost] + t, local);
+    const int i = r.off[c] + local;
+    const double4 p = b.pos64[i];
+    const int2 m = b.meta[i];
+    make_bead(bead, p.x, p.y, p.z, p.w, b.scale[i], m.x, b.prefactor);
+    who[0] = c;
+    who[1] = m.y;
+  }
+  __syncthreads();
+  double sum;
+  int flag;
+  trial_cluster_pass<GRX_FP64>(b, &bead, W, 1, who[0], who[1], -1, -1, sum, flag);
+  const int warp = threadIdx.x >> 5;
+  if (cluster_rank() == 0 && warp < 4 && (threadIdx.x & 31) == 0) {
+    part[5 * t + warp] = warp < 2 ? sum : 0.5 * sum;
+    if (warp == 0) part[5 * t + 4] = flag ? 1.0 : 0.0;
+  }
+}
+
+// VDW + real Coulomb between framework atoms of different molecules or components (ordered
+// pairs, factor 0.5); launched only when there are such pairs. Thread i, blockIdx.y a slice of
+// the j atoms. part per block: hh_v hh_r.
+__global__ void __launch_bounds__(GRX_THREADS) host_total_kernel(BoxDev b, CompRanges r, double* part) {
   __shared__ double sbuf[32];
+  const int nh = r.base[r.nhost];
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  double e[6] = {0, 0, 0, 0, 0, 0};
-  int ovl = 0;
-  if (j < r.n) {
+  LaneAcc<GRX_FP64> acc;
+  double q = 0.0;
+  int flag = 0;
+  if (j < nh) {
     int li;
     const int ci = comp_of(r, j, li);
     const int ii = r.off[ci] + li;
     const double4 p = atom_pos64(b, ii);
     const int2 mi = atom_meta(b, ii);
-    const double si = atom_scale(b, ii);
-    for (int cj = 0; cj < r.ncomp; ++cj) {
-      int it;
-      if (ci < r.nhost || cj < r.nhost) it = (!(ci < r.nhost) || !(cj < r.nhost)) ? 1 : 0;
-      else it = 2;
-      const int nj = r.base[cj + 1] - r.base[cj];
-      for (int lj = 0; lj < nj; ++lj) {
-        const int jj = r.off[cj] + lj;
-        const int2 mj = atom_meta(b, jj);
-        if (mi.y == mj.y && ci == cj) continue;
-        const double4 q = atom_pos64(b, jj);
-        double x = p.x - q.x, y = p.y - q.y, z = p.z - q.z;
-        pbc64(b, x, y, z);
-        const double rr = x * x + y * y + z * z;
-        if (rr < b.cut_vdw2) {
-          const double ev = vdw64(b, mi.x * b.ntypes + mj.x, rr, si * atom_scale(b, jj));
-          e[2 * it] += 0.5 * ev;
-          if (it > 0 && (ev > b.overlap || rr < 0.01)) ovl = 1;
-        }
-        if (!b.no_charges && rr < b.cut_coul2) e[2 * it + 1] += 0.5 * coul64(b, p.w * q.w, rr);
-      }
+    Bead bd;
+    make_bead(bd, p.x, p.y, p.z, p.w, atom_scale(b, ii), mi.x, b.prefactor);
+    q = b.prefactor * p.w;
+    const int per = (nh + gridDim.y - 1) / gridDim.y;
+    const int j1 = min(nh, (int)(blockIdx.y + 1) * per);
+    for (int jc = blockIdx.y * per; jc < j1; ++jc) {
+      int lj;
+      const int cj = comp_of(r, jc, lj);
+      const int jj = r.off[cj] + lj;
+      if (ci == cj && atom_meta(b, jj).y == mi.y) continue;
+      if (pair_screen<GRX_FP64, true>(b, jj, bd)) pair_dense<GRX_FP64>(b, true, jj, bd, acc, flag);
     }
   }
-  for (int k = 0; k < 6; ++k) {
-    const double v = block_sum(e[k], sbuf);
-    if (threadIdx.x == 0) part[6 * blockIdx.x + k] = v;
+  const double v = block_sum(0.5 * acc.v, sbuf), e = block_sum(0.5 * q * acc.r, sbuf);
+  if (threadIdx.x == 0) {
+    const int k = blockIdx.y * gridDim.x + blockIdx.x;
+    part[2 * k] = v;
+    part[2 * k + 1] = e;
   }
-  ovl = __syncthreads_or(ovl);
-  if (threadIdx.x == 0) part[6 * gridDim.x + blockIdx.x] = ovl ? 1.0 : 0.0;
 }
 
 // Fourier delta of one move (Fourier_Ewald_Diff, Ewald_Energy_Functions.h:280-397):
@@ -308,6 +462,147 @@ static grx_status sync_sizes(grx_box* b) {
   return GRX_OK;
 }
 
+// Structure factors and Fourier totals (out8), and with `pairs` the VDW + real Coulomb totals
+// {hh_v, hh_r, hg_v, hg_r, gg_v, gg_r} and the overlap flag: every kernel enqueued, one read back.
+static grx_status totals(grx_box* b, double* out8, double* pairs, uint8_t* overlap) {
+  grx_status st = sync_sizes(b);
+  if (st) return st;
+  refresh_dev(b);
+  const CompRanges r = ranges(b);
+  const size_t n = std::max(r.n, 1);
+  const size_t ntab = (size_t)(b->dev.kmax[0] + b->dev.kmax[1] + b->dev.kmax[2] + 3) * n;
+  const int sms = sm_count(b);
+  const int nhost = r.base[r.nhost], nguest = r.n - nhost;
+  const int nblk_atoms = (r.n + GRX_THREADS - 1) / GRX_THREADS;
+  const int nblk_big = 4 * sms;
+  const int nblk_k = (b->nact + GRX_THREADS - 1) / GRX_THREADS;
+  // framework pairs count only between molecules or components
+  int host_comps = 0;
+  bool host_pairs = false;
+  for (int c = 0; c < r.nhost; ++c) {
+    if (b->size[c] > 0) ++host_comps;
+    host_pairs = host_pairs || b->many_mols[c];
+  }
+  host_pairs = pairs && (host_pairs || host_comps > 1);
+  const int hx = (nhost + GRX_THREADS - 1) / GRX_THREADS;
+  const int hy = host_pairs ? std::max(1, std::min(64, 4 * sms / std::max(hx, 1))) : 0;
+  std::vector<int> big;
+  for (int c = 0; c < r.ncomp; ++c)
+    if (r.molsize[c] > kBigMolecule && r.base[c + 1] - r.base[c] >= 2) big.push_back(c);
+  // result doubles: self + small exclusions, large exclusions, Fourier energies, pair totals
+  const size_t o_big = 4 * (size_t)std::max(nblk_atoms, 1), o_k = o_big + 2 * (size_t)nblk_big * big.size(),
+               o_pair = o_k + 3 * (size_t)nblk_k, o_host = o_pair + (pairs ? 5 * (size_t)nguest : 0),
+               n_out = o_host + 2 * (size_t)hx * hy;
+  // chunks of atoms: about eight blocks of sk_kernel per SM, at least one tile each
+  SkChunks ck{};
+  ck.n = (int)n;
+  ck.nhost = nhost;
+  const int fw_atoms = b->parent ? 0 : nhost;
+  const bool sums = b->nact > 0 && r.n > 0;
+  auto split = [&](int want) {
+    auto len = [&](int atoms) {
+      const int per = (int)(((int64_t)(fw_atoms + nguest) + want - 1) / want);
+      return std::max(kSkTile, std::min((per + kSkTile - 1) / kSkTile * kSkTile, (std::max(atoms, 1) + kSkTile - 1) / kSkTile * kSkTile));
+    };
+    ck.host_len = len(fw_atoms);
+    ck.guest_len = len(nguest);
+    ck.n_host_chunks = fw_atoms ? (fw_atoms + ck.host_len - 1) / ck.host_len : 0;
+    return ck.n_host_chunks + (nguest ? (nguest + ck.guest_len - 1) / ck.guest_len : 0);
+  };
+  int nchunks = 0;
+  size_t part_bytes = 0;
+  if (sums) {
+    nchunks = split(std::max(1, 8 * sms / std::max(b->n_kgroups, 1)));
+    part_bytes = (size_t)nchunks * b->nact * sizeof(double2);
+  }
+  const size_t fixed = ntab * sizeof(double2) + n_out * sizeof(double);
+  st = ensure_scratch(b, fixed + part_bytes);
+  if (st == GRX_ERR_OUT_OF_MEMORY && part_bytes) {  // one chunk of each kind writes S(k) in place
+    ck.host_len = std::max(kSkTile, fw_atoms);
+    ck.guest_len = std::max(kSkTile, nguest);
+    ck.n_host_chunks = fw_atoms ? 1 : 0;
+    nchunks = ck.n_host_chunks + (nguest ? 1 : 0);
+    part_bytes = 0;
+    st = ensure_scratch(b, fixed);
+  }
+  if (st) return st;
+  double2* ex = (double2*)b->scratch;
+  double2* ey = ex + (size_t)(b->dev.kmax[0] + 1) * n;
+  double2* ez = ey + (size_t)(b->dev.kmax[1] + 1) * n;
+  double* out = (double*)(ex + ntab);
+  double2* part = part_bytes ? (double2*)(out + (n_out + 1) / 2 * 2) : nullptr;
+  cudaStream_t s = b->stream;
+  if (!b->parent)  // a replica's framework structure factor is its parent's, shared by every replica
+    GRX_CHECK_CUDA(cudaMemsetAsync(b->s_fw, 0, b->nvec * sizeof(double2), s), "clear S_fw");
+  GRX_CHECK_CUDA(cudaMemsetAsync(b->s_ads, 0, b->nvec * sizeof(double2), s), "clear S_ads");
+  GRX_CHECK_CUDA(cudaMemsetAsync(b->s_tmp, 0, b->nvec * sizeof(double2), s), "clear S_tmp");
+  std::vector<double> h(n_out, 0.0);
+  if (sums) {
+    const int first = b->parent ? nhost : 0;
+    if (r.n > first)
+      eik_tables_kernel<<<dim3((r.n - first + 127) / 128, 3), 128, 0, s>>>(b->dev, r, first, ex, ey, ez);
+    if (nchunks)
+      sk_kernel<<<dim3(b->n_kgroups, nchunks), kSkCols, 0, s>>>(b->dev, ck, b->krow, b->kgroup, ex, ey, ez, part);
+    count_launch((r.n > first) + (nchunks > 0));
+  }
+  if (b->nact > 0) {
+    sk_reduce_kernel<<<nblk_k, GRX_THREADS, 0, s>>>(b->dev, part, ck.n_host_chunks, nchunks - ck.n_host_chunks, out + o_k);
+    count_launch();
+  }
+  if (r.n > 0) {
+    self_excl_kernel<<<nblk_atoms, GRX_THREADS, 0, s>>>(b->dev, r, out);
+    count_launch();
+    for (size_t g = 0; g < big.size(); ++g) {
+      big_excl_kernel<<<nblk_big, GRX_THREADS, 0, s>>>(b->dev, r, big[g], out + o_big + 2 * (size_t)nblk_big * g);
+      count_launch();
+    }
+  }
+  if (pairs && nguest > 0) {
+    guest_total_kernel<<<nguest * kTrialCtas, kTrialWarps * 32, 0, s>>>(b->dev, r, out + o_pair);
+    count_launch();
+  }
+  if (host_pairs && nhost > 0) {
+    host_total_kernel<<<dim3(hx, hy), GRX_THREADS, 0, s>>>(b->dev, r, out + o_host);
+    count_launch();
+  }
+  GRX_CHECK_CUDA(cudaGetLastError(), "totals launch");
+  if (r.n > 0 || b->nact > 0)
+    GRX_CHECK_CUDA(cudaMemcpyAsync(h.data(), out, n_out * sizeof(double), cudaMemcpyDeviceToHost, s), "read totals");
+  GRX_CHECK_CUDA(cudaStreamSynchronize(s), "totals");
+  double gg = 0, hh = 0, hg = 0;
+  for (int k = 0; k < nblk_k; ++k) {
+    gg += h[o_k + 3 * k]; hh += h[o_k + 3 * k + 1]; hg += h[o_k + 3 * k + 2];
+  }
+  double sa = 0, sh = 0, ea = 0, eh = 0;
+  for (int k = 0; k < nblk_atoms; ++k) {
+    sa += h[4 * k]; sh += h[4 * k + 1]; ea += h[4 * k + 2]; eh += h[4 * k + 3];
+  }
+  if (r.n > 0)
+    for (size_t k = 0; k < (size_t)nblk_big * big.size(); ++k) {
+      ea += h[o_big + 2 * k];
+      eh += h[o_big + 2 * k + 1];
+    }
+  out8[0] = gg; out8[1] = hh; out8[2] = hg;
+  out8[3] = sa; out8[4] = sh; out8[5] = -ea; out8[6] = -eh;
+  out8[7] = (double)b->nact;
+  b->sk_valid = true;
+  b->ewdf_valid = false;
+  if (pairs) {
+    for (int q = 0; q < 6; ++q) pairs[q] = 0.0;
+    *overlap = 0;
+    for (int t = 0; t < nguest; ++t) {
+      for (int q = 0; q < 4; ++q) pairs[2 + q] += h[o_pair + 5 * (size_t)t + q];
+      if (h[o_pair + 5 * (size_t)t + 4] != 0.0) *overlap = 1;
+    }
+    if (host_pairs)
+      for (int k = 0; k < hx * hy; ++k) {
+        pairs[0] += h[o_host + 2 * (size_t)k];
+        pairs[1] += h[o_host + 2 * (size_t)k + 1];
+      }
+  }
+  return GRX_OK;
+}
+
 }  // namespace grx
 
 using namespace grx;
@@ -316,108 +611,18 @@ extern "C" {
 
 grx_status grx_ewald_total(grx_box* b, double* out8) {
   GRX_REQUIRE(b && out8, "grx_ewald_total: null argument");
-  grx_status st = sync_sizes(b);
-  if (st) return st;
-  refresh_dev(b);
-  CompRanges r = ranges(b);
-  const size_t n = std::max(r.n, 1);
-  const size_t ntab = (size_t)(b->dev.kmax[0] + b->dev.kmax[1] + b->dev.kmax[2] + 3) * n;
-  const int nblk_atoms = (r.n + GRX_THREADS - 1) / GRX_THREADS;
-  const int nblk_big = 4 * sm_count(b);
-  const size_t part_doubles = 4 * (size_t)std::max(nblk_atoms, 1) + 2 * (size_t)nblk_big * GRX_MAX_COMPONENTS;
-  st = ensure_scratch(b, ntab * sizeof(double2) + part_doubles * sizeof(double));
-  if (st) return st;
-  double2* ex = (double2*)b->scratch;
-  double2* ey = ex + (size_t)(b->dev.kmax[0] + 1) * n;
-  double2* ez = ey + (size_t)(b->dev.kmax[1] + 1) * n;
-  double* part = (double*)(ex + ntab);
-  if (r.n > 0) {
-    eik_tables_kernel<<<nblk_atoms, GRX_THREADS, 0, b->stream>>>(b->dev, r, ex, ey, ez);
-    count_launch();
-  }
-  if (!b->parent)  // a replica's framework structure factor is its parent's, shared by every replica
-    GRX_CHECK_CUDA(cudaMemsetAsync(b->s_fw, 0, b->nvec * sizeof(double2), b->stream), "clear S_fw");
-  GRX_CHECK_CUDA(cudaMemsetAsync(b->s_ads, 0, b->nvec * sizeof(double2), b->stream), "clear S_ads");
-  GRX_CHECK_CUDA(cudaMemsetAsync(b->s_tmp, 0, b->nvec * sizeof(double2), b->stream), "clear S_tmp");
-  if (b->nact > 0 && r.n > 0) {
-    sk_kernel<<<b->nact, GRX_THREADS, 0, b->stream>>>(b->dev, r, ex, ey, ez);
-    count_launch();
-  }
-  std::vector<double> parts(part_doubles, 0.0);
-  std::vector<int> big;
-  if (r.n > 0) {
-    self_excl_kernel<<<nblk_atoms, GRX_THREADS, 0, b->stream>>>(b->dev, r, part);
-    count_launch();
-    double* pbig = part + 4 * (size_t)std::max(nblk_atoms, 1);
-    for (int c = 0; c < r.ncomp; ++c) {
-      if (r.molsize[c] <= kBigMolecule || r.base[c + 1] - r.base[c] < 2) continue;
-      big_excl_kernel<<<nblk_big, GRX_THREADS, 0, b->stream>>>(b->dev, r, c, pbig + 2 * (size_t)nblk_big * big.size());
-      count_launch();
-      big.push_back(c);
-    }
-    GRX_CHECK_CUDA(cudaMemcpyAsync(parts.data(), part, part_doubles * sizeof(double), cudaMemcpyDeviceToHost,
-                                   b->stream), "read self/exclusion");
-  }
-  std::vector<double2> sfw(b->nvec), sads(b->nvec);
-  GRX_CHECK_CUDA(cudaMemcpyAsync(sfw.data(), b->s_fw, b->nvec * sizeof(double2), cudaMemcpyDeviceToHost, b->stream), "read S_fw");
-  GRX_CHECK_CUDA(cudaMemcpyAsync(sads.data(), b->s_ads, b->nvec * sizeof(double2), cudaMemcpyDeviceToHost, b->stream), "read S_ads");
-  GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "ewald total");
-  // energies in slot order, FP64 (Ewald_Total, ewald_preparation.h:150-161)
-  double gg = 0, hh = 0, hg = 0;
-  for (int j = 0; j < b->nact; ++j) {
-    const int s = b->h_kact[j].w;
-    const double t = b->h_ktemp[j];
-    const double2 a = sads[s], f = sfw[s];
-    gg += t * (a.x * a.x + a.y * a.y);
-    hh += t * (f.x * f.x + f.y * f.y);
-    hg += t * (f.x * a.x + f.y * a.y) * 2.0;
-  }
-  double sa = 0, sh = 0, ea = 0, eh = 0;
-  for (int k = 0; k < nblk_atoms; ++k) {
-    sa += parts[4 * k]; sh += parts[4 * k + 1]; ea += parts[4 * k + 2]; eh += parts[4 * k + 3];
-  }
-  const double* pb = parts.data() + 4 * (size_t)std::max(nblk_atoms, 1);
-  for (size_t g = 0; g < big.size(); ++g)
-    for (int k = 0; k < nblk_big; ++k) {
-      ea += pb[2 * (nblk_big * g + k)];
-      eh += pb[2 * (nblk_big * g + k) + 1];
-    }
-  out8[0] = gg; out8[1] = hh; out8[2] = hg;
-  out8[3] = sa; out8[4] = sh; out8[5] = -ea; out8[6] = -eh;
-  out8[7] = (double)b->nact;
-  b->sk_valid = true;
-  b->ewdf_valid = false;
-  return GRX_OK;
+  return totals(b, out8, nullptr, nullptr);
 }
 
 grx_status grx_total_energy(grx_box* b, grx_energy* out) { return grx_total_energy_overlap(b, out, nullptr); }
 
 grx_status grx_total_energy_overlap(grx_box* b, grx_energy* out, uint8_t* overlap) {
   GRX_REQUIRE(b && out, "grx_total_energy: null argument");
-  double ew[8];
-  grx_status st = grx_ewald_total(b, ew);
+  double ew[8], e[6];
+  uint8_t ovl = 0;
+  grx_status st = totals(b, ew, e, &ovl);
   if (st) return st;
-  CompRanges r = ranges(b);
-  const int nblk = std::max((r.n + GRX_THREADS - 1) / GRX_THREADS, 1);
-  st = ensure_scratch(b, 7 * (size_t)nblk * sizeof(double));
-  if (st) return st;
-  double* part = b->scratch;
-  std::vector<double> parts(7 * (size_t)nblk, 0.0);
-  if (r.n > 0) {
-    vdw_real_total_kernel<<<nblk, GRX_THREADS, 0, b->stream>>>(b->dev, r, part);
-    count_launch();
-    GRX_CHECK_CUDA(cudaMemcpyAsync(parts.data(), part, parts.size() * sizeof(double),
-                                   cudaMemcpyDeviceToHost, b->stream), "read totals");
-  }
-  GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "totals");
-  double e[6] = {0, 0, 0, 0, 0, 0};
-  for (int k = 0; k < nblk; ++k)
-    for (int q = 0; q < 6; ++q) e[q] += parts[6 * k + q];
-  if (overlap) {
-    *overlap = 0;
-    for (int k = 0; k < nblk; ++k)
-      if (parts[6 * (size_t)nblk + k] != 0.0) *overlap = 1;
-  }
+  if (overlap) *overlap = ovl;
   out->hh_vdw = e[0]; out->hh_real = e[1];
   out->hg_vdw = e[2]; out->hg_real = e[3];
   out->gg_vdw = e[4]; out->gg_real = e[5];

@@ -36,6 +36,7 @@ struct grx_box {
   int size[GRX_MAX_COMPONENTS] = {};
   int rigid[GRX_MAX_COMPONENTS] = {};
   int has_charge[GRX_MAX_COMPONENTS] = {};
+  int many_mols[GRX_MAX_COMPONENTS] = {};  // host components: live atoms of more than one molecule id
   size_t stored[GRX_MAX_COMPONENTS] = {};  // atoms written to storage (template included)
   double excl_intra[GRX_MAX_COMPONENTS] = {};
   double excl_self[GRX_MAX_COMPONENTS] = {};
@@ -61,6 +62,11 @@ struct grx_box {
   double2* s_ads = nullptr;
   double2* s_tmp = nullptr;
   int nvec = 0, nact = 0;
+  grx::KRow* krow = nullptr;   // (kx, ky) rows of the active k, and groups of rows for sk_kernel
+  int2* kgroup = nullptr;
+  int n_kgroups = 0;
+  std::vector<grx::KRow> h_krow;
+  std::vector<int2> h_kgroup;
   std::vector<int4> h_kact;
   std::vector<double> h_ktemp;
   bool sk_valid = false;

@@ -132,6 +132,18 @@ struct BoxDev {
   double2* s_tmp;
 };
 
+// One (kx, ky) row of the active k vectors, which sit in kact by rows with kz ascending from lo
+// to hi (only the origin is left out): columns |kz| = 0 .. ncol - 1, numbered from `col` within
+// the row's group of sk_kernel.
+struct KRow {
+  int kx, ky, lo, hi, first, col, ncol, pad_;
+  __host__ __device__ __forceinline__ int index(int kz) const {  // in kact, -1 when not active
+    if (kz < lo || kz > hi) return -1;
+    if (kx == 0 && ky == 0) return kz == 0 ? -1 : first + (kz - lo) - (kz > 0 && lo <= 0 ? 1 : 0);
+    return first + (kz - lo);
+  }
+};
+
 // ---------------------------------------------------------------- Philox
 // Philox4x32-10 (Salmon et al., SC'11). Counter {slot, move lo, move hi, stream},
 // key = seed: the same stream layout as the test oracle.
