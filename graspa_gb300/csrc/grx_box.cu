@@ -119,7 +119,6 @@ void refresh_dev(grx_box* b) {
   d.tile_c = b->tile_c;
   d.tile_r = b->tile_r;
   d.ntiles = b->ntiles;
-  d.ctab = b->ctab;
   d.ctab_base = b->ctab_base;
   d.ctab_n = b->ctab_n;
   d.ctabf = b->ctabf;
@@ -184,13 +183,10 @@ static void pbc_host(const BoxDev& b, double* d) {
 // polynomials in s = r^2. Pieces follow the FP32 bit pattern of s (64 per octave) from
 // s = 0.25 A^2 to just past the cutoff, so the device finds its piece with one shift of
 // the FP32 bits. Each piece is the degree-5 interpolant at Chebyshev nodes, fitted in
-// long double from erfcl; the worst relative error found on a dense sample is kept in
-// ctab_maxrel (about 1e-14 for the benchmark systems).
+// long double from erfcl (about 1e-14 of g for the benchmark systems).
 struct CoulombTable {
   int base = 0, n = 0;
-  double maxrel = 0.0;
-  std::vector<double> tab;  // 8 per piece: s0, 1/width, 6 coefficients
-  std::vector<float4> tf;   // the double-float copy
+  std::vector<float4> tf;  // per piece {c0 hi, c0 lo, c1 hi, c1 lo}, {c2, c3, c4, c5} in t = (s - s0) / width
 };
 
 static void fit_coulomb_table(double alpha, double cut2, CoulombTable& T);
@@ -217,13 +213,9 @@ static grx_status build_coulomb_table(grx_box* b, double alpha, double cut2) {
   const CoulombTable& T = coulomb_table(alpha, cut2);
   b->ctab_base = T.base;
   b->ctab_n = T.n;
-  b->ctab_maxrel = T.maxrel;
-  GRX_CHECK_CUDA(dev_alloc(b, (void**)&b->ctab, T.tab.size() * sizeof(double)), "alloc Coulomb table");
-  GRX_CHECK_CUDA(cudaMemcpy(b->ctab, T.tab.data(), T.tab.size() * sizeof(double), cudaMemcpyHostToDevice),
-                 "upload Coulomb table");
-  GRX_CHECK_CUDA(dev_alloc(b, (void**)&b->ctabf, T.tf.size() * sizeof(float4)), "alloc Coulomb table (float pairs)");
+  GRX_CHECK_CUDA(dev_alloc(b, (void**)&b->ctabf, T.tf.size() * sizeof(float4)), "alloc Coulomb table");
   GRX_CHECK_CUDA(cudaMemcpy(b->ctabf, T.tf.data(), T.tf.size() * sizeof(float4), cudaMemcpyHostToDevice),
-                 "upload Coulomb table (float pairs)");
+                 "upload Coulomb table");
   return GRX_OK;
 }
 
@@ -235,10 +227,9 @@ static void fit_coulomb_table(double alpha, double cut2, CoulombTable& T) {
   std::memcpy(&hi_bits, &s_hi, 4);
   const int base = (int)(lo_bits >> 17);
   const int n = (int)(hi_bits >> 17) - base + 2;
-  std::vector<double> tab(8 * (size_t)n);
+  T.tf.resize(2 * (size_t)n);
   const long double PI = 3.141592653589793238462643383279502884L;
   auto g = [&](long double sv) { const long double r = sqrtl(sv); return erfcl((long double)alpha * r) / r; };
-  double maxrel = 0.0;
   for (int k = 0; k < n; ++k) {
     const uint32_t ab = (uint32_t)(base + k) << 17, bb = (uint32_t)(base + k + 1) << 17;
     float fa, fb;
@@ -263,37 +254,17 @@ static void fit_coulomb_table(double alpha, double cut2, CoulombTable& T) {
         for (int q = c; q < 7; ++q) A[r][q] -= f * A[c][q];
       }
     }
-    double* e = &tab[8 * (size_t)k];
-    e[0] = (double)s0;
-    e[1] = (double)(1.0L / w);
-    for (int c = 0; c < 6; ++c) e[2 + c] = (double)(A[c][6] / A[c][c]);
-    for (int m = 0; m <= 16; ++m) {
-      const double sv = e[0] + (double)w * (m / 16.0);
-      const double t = (sv - e[0]) * e[1];
-      const double pv = e[2] + t * (e[3] + t * (e[4] + t * (e[5] + t * (e[6] + t * e[7]))));
-      const long double ex = g(sv);
-      maxrel = std::max(maxrel, (double)fabsl((pv - ex) / ex));
+    double e[6];
+    float h[6];
+    for (int c = 0; c < 6; ++c) {
+      e[c] = (double)(A[c][6] / A[c][c]);
+      h[c] = (float)e[c];
     }
+    T.tf[2 * k] = make_float4(h[0], (float)(e[0] - (double)h[0]), h[1], (float)(e[1] - (double)h[1]));
+    T.tf[2 * k + 1] = make_float4(h[2], h[3], h[4], h[5]);
   }
   T.base = base;
   T.n = n;
-  T.maxrel = maxrel;
-  // double-float copy: s0 and 1/width are exact floats (width is a power of two)
-  std::vector<float4> tf(4 * (size_t)n);
-  for (int k = 0; k < n; ++k) {
-    const double* e = &tab[8 * (size_t)k];
-    float2 c[6];
-    for (int j = 0; j < 6; ++j) {
-      const float h = (float)e[2 + j];
-      c[j] = make_float2(h, (float)(e[2 + j] - (double)h));
-    }
-    tf[4 * k + 0] = make_float4((float)e[0], (float)e[1], c[0].x, c[0].y);
-    tf[4 * k + 1] = make_float4(c[1].x, c[1].y, c[2].x, c[2].y);
-    tf[4 * k + 2] = make_float4(c[3].x, c[3].y, c[4].x, c[4].y);
-    tf[4 * k + 3] = make_float4(c[5].x, c[5].y, 0.0f, 0.0f);
-  }
-  T.tab = std::move(tab);
-  T.tf = std::move(tf);
 }
 
 // Storage order of host atoms: recursive bisection of the wrapped Cartesian positions
@@ -789,8 +760,7 @@ grx_status grx_box_footprint(const grx_box_desc* desc, size_t* bytes) {
     uint32_t lb, hb;
     std::memcpy(&lb, &s_lo, 4);
     std::memcpy(&hb, &s_hi, 4);
-    const size_t np = (size_t)((int)(hb >> 17) - (int)(lb >> 17) + 2);
-    t += al(8 * np * sizeof(double)) + al(4 * np * sizeof(float4));
+    t += al(2 * (size_t)((int)(hb >> 17) - (int)(lb >> 17) + 2) * sizeof(float4));
   }
   t += al((size_t)1 << 20) + al(1024 * sizeof(grx_widom_result));  // first scratch and result buffers
   *bytes = t;
@@ -876,7 +846,7 @@ grx_status grx_box_destroy(grx_box* b) {
   }
   void* ptrs[] = {b->pos64, b->hi, b->lo, b->meta, b->scale, b->charge, b->d_size, b->ff64,
                   b->ffc10, b->ff32, b->kact, b->ktemp, b->krow, b->kgroup, b->s_fw, b->s_ads, b->s_tmp,
-                  b->scratch, b->d_results, b->tile_c, b->tile_r, b->ctab, b->ctabf, b->qdf,
+                  b->scratch, b->d_results, b->tile_c, b->tile_r, b->ctabf, b->qdf,
                   b->ffdf, b->ffdf2, b->ewA, b->ewF, b->ewT, b->vmeta, b->vlist, b->hrec, b->htype};
   for (void* p : ptrs) dev_free(b, p);
   if (b->pinned) cudaFreeHost(b->pinned);

@@ -97,15 +97,12 @@ struct grx_box {
   uint16_t* htype = nullptr;
   float4* ffdf = nullptr;    // per type pair {4eps hi, lo, 1/sigma^2 hi, lo}
   float2* ffdf2 = nullptr;   // per type pair {shift hi, lo}
-  float4* ctabf = nullptr;   // Coulomb table, 4 float4 per piece
+  float4* ctabf = nullptr;   // Coulomb table, 2 float4 per piece
   float4* ewA = nullptr;     // per active k: temp * S_ads as double-float complex
   float4* ewF = nullptr;     // per active k: temp * S_fw
   float2* ewT = nullptr;     // per active k: temp
   bool ewdf_valid = false;
-  // Coulomb table
-  double* ctab = nullptr;
   int ctab_n = 0, ctab_base = 0;
-  double ctab_maxrel = 0.0;
   std::shared_ptr<const grx::Tables64> t64;  // FP64 Coulomb tables, shared by boxes of equal parameters
 
   // scratch (grown on demand)

@@ -95,13 +95,11 @@ struct BoxDev {
   int ew_rows;           // GCMC Ewald delta through (kx, ky) row products (shared memory sized for it)
   float wperp[3];        // perpendicular widths of the cell (distances between lattice planes)
   float half_wmin2;      // (min width / 2)^2, shrunk for FP32 rounding
-  // real-space Coulomb table: g(s) = erfc(alpha sqrt s)/sqrt s, piecewise quintic in
-  // s = r^2, 64 pieces per octave indexed by the FP32 bit pattern of s
-  const double* ctab;    // per piece {s0, 1/width, c0..c5}
+  // double-float data of the mixed-precision dense path; g(s) = erfc(alpha sqrt s)/sqrt s as
+  // piecewise quintics in s = r^2, 64 pieces per octave indexed by the FP32 bits of s
+  const float4* ctabf;   // per piece {c0 hi, c0 lo, c1 hi, c1 lo}, {c2, c3, c4, c5} in t = (s - s0) / width
   int ctab_base;
   int ctab_n;
-  // double-float data of the mixed-precision dense path
-  const float4* ctabf;   // per piece {s0, 1/width, c0 hi, c0 lo}, {c1 hi, lo, c2 hi, lo}, ...
   const float2* qdf;     // q * scaleCoul, hi/lo
   const float4* ffdf;    // {4 eps hi, lo, 1/sigma^2 hi, lo}
   const float2* ffdf2;   // {shift hi, lo}

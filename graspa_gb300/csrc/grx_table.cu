@@ -14,6 +14,7 @@
 // rounding error of the argument taken out, so an evaluation carries about one rounding where
 // erfc(alpha sqrt s) / sqrt s amplifies that of alpha sqrt s by 2 alpha^2 s. Against 80-bit
 // values over 0.26 A^2 to the cutoff (alpha 0.265, 12 A): rms 1.0e-16, library form 4.5e-16.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <map>
