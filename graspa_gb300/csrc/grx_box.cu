@@ -149,6 +149,7 @@ void refresh_dev(grx_box* b) {
   d.vox = h->vox_on;
   d.vmeta = h->vmeta;
   d.vlist = h->vlist;
+  d.vshift = reinterpret_cast<const float4*>(h->vmeta) + (size_t)h->vn[0] * h->vn[1] * h->vn[2];
   for (int k = 0; k < 3; ++k) d.vn[k] = h->vn[k];
   d.vchunks = h->vchunks;
 }

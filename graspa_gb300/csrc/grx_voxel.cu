@@ -207,18 +207,25 @@ grx_status build_voxels(grx_box* b) {
   std::vector<uint32_t> flat;
   flat.reserve(total);
   for (const auto& l : lists) flat.insert(flat.end(), l.begin(), l.end());
-  // 8 zero entries of padding: the pass stages list ranges with bulk copies rounded out to
-  // 16-byte boundaries, which may read up to 3 entries past the last list
-  flat.insert(flat.end(), 8, 0u);
+  // the lattice vectors of the 512 shift codes follow the voxel records
+  meta.resize(nvox + 512);
+  static_assert(sizeof(int4) == sizeof(float4), "shift vectors share the voxel records' allocation");
+  float4* shift = reinterpret_cast<float4*>(meta.data() + nvox);
+  for (int c = 0; c < 512; ++c) {
+    const double n[3] = {(c & 7) - 4.0, ((c >> 3) & 7) - 4.0, (c >> 6) - 4.0};
+    float v[3];
+    for (int k = 0; k < 3; ++k) v[k] = (float)(n[0] * d.cell_hi[k] + n[1] * d.cell_hi[3 + k] + n[2] * d.cell_hi[6 + k]);
+    shift[c] = make_float4(v[0], v[1], v[2], 0.0f);
+  }
   if (b->arena) {  // in an arena the lists are optional: take them only with room to spare
     size_t used = 0, largest = 0;
     grx_arena_usage(b->arena, &used, &largest, nullptr);
-    if (largest < nvox * sizeof(int4) + flat.size() * sizeof(uint32_t) + kArenaHeadroom) {
+    if (largest < meta.size() * sizeof(int4) + flat.size() * sizeof(uint32_t) + kArenaHeadroom) {
       refresh_dev(b);
       return GRX_OK;
     }
   }
-  if (dev_alloc(b, (void**)&b->vmeta, nvox * sizeof(int4)) != cudaSuccess ||
+  if (dev_alloc(b, (void**)&b->vmeta, meta.size() * sizeof(int4)) != cudaSuccess ||
       dev_alloc(b, (void**)&b->vlist, flat.size() * sizeof(uint32_t)) != cudaSuccess) {
     cudaGetLastError();  // no room: the tile path serves the box
     dev_free(b, b->vmeta);
@@ -228,7 +235,7 @@ grx_status build_voxels(grx_box* b) {
     refresh_dev(b);
     return GRX_OK;
   }
-  GRX_CHECK_CUDA(cudaMemcpy(b->vmeta, meta.data(), nvox * sizeof(int4), cudaMemcpyHostToDevice), "upload voxels");
+  GRX_CHECK_CUDA(cudaMemcpy(b->vmeta, meta.data(), meta.size() * sizeof(int4), cudaMemcpyHostToDevice), "upload voxels");
   GRX_CHECK_CUDA(cudaMemcpy(b->vlist, flat.data(), flat.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
                  "upload voxel lists");
   for (int k = 0; k < 3; ++k) b->vn[k] = nv[k];

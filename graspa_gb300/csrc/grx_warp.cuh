@@ -25,75 +25,6 @@ constexpr int kQueue = 64;  // ring buffer entries per warp
 // passes would show in their difference.
 constexpr int kMixed64 = 3;
 
-// ---------------------------------------------------------------- voxel-list staging
-// A warp walking a bead's voxel list stages the next 8 chunks (256 entries) into its own shared
-// buffer with one bulk copy (cp.async.bulk, completion on an mbarrier) instead of one dependent
-// global load per chunk. The copied range is rounded out to 16-byte boundaries (the list array
-// carries 8 entries of padding), so the buffer holds up to 264 entries.
-constexpr int kStageChunks = 8;
-constexpr int kStageBuf = 32 * kStageChunks + 8;
-struct alignas(16) VoxStage {
-  unsigned buf[kStageBuf];
-  unsigned long long mbar;
-  unsigned phase;  // parity of the mbarrier phase the next copy completes
-  unsigned ok;     // 0 after a wait gave up: the warp reads the lists directly from then on
-};
-constexpr int kStageSpin = 1 << 20;  // try_wait rounds before a wait gives up
-
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-  return static_cast<unsigned>(__cvta_generic_to_shared(p));
-}
-// Called by one thread per stage before first use, then fenced and barrier-synchronised.
-__device__ __forceinline__ void stage_init(VoxStage& st) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&st.mbar)) : "memory");
-  st.phase = 0;
-  st.ok = 1;
-}
-__device__ __forceinline__ void stage_fence_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-// Lane 0: expect `bytes` on the mbarrier and start the bulk copy of [src, src + bytes).
-__device__ __forceinline__ void stage_issue(VoxStage& st, const unsigned* src, unsigned bytes) {
-  const unsigned mb = smem_addr(&st.mbar);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the warp's reads of the old contents first
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(mb), "r"(bytes) : "memory");
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(smem_addr(st.buf)), "l"(src), "r"(bytes), "r"(mb) : "memory");
-}
-// Wait for the phase `parity` of the stage's mbarrier, at most kStageSpin rounds; true when done.
-__device__ __forceinline__ bool stage_wait(const VoxStage& st, unsigned parity) {
-  const unsigned mb = smem_addr(&st.mbar);
-  for (int it = 0; it < kStageSpin; ++it) {
-    unsigned done;
-    asm volatile("{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(done) : "r"(mb), "r"(parity) : "memory");
-    if (done) return true;
-  }
-  return false;
-}
-
-// The whole warp stages list entries [a0, a1) (absolute indices): one bulk copy of the range
-// rounded out to 16 bytes, issued by lane 0, awaited by every lane. Returns the first staged
-// entry, or -1 when the wait gave up (after waiting once more for the copy); the stage is then
-// switched off and the warp reads the lists directly. Out of line: it runs once per 8 chunks.
-static __device__ __noinline__ int stage_refill(VoxStage* st, const unsigned* vlist, unsigned a0, unsigned a1) {
-  const int lane = threadIdx.x & 31;
-  const unsigned g0 = a0 & ~3u, g1 = (a1 + 3u) & ~3u;
-  __syncwarp();
-  if (lane == 0) stage_issue(*st, vlist + g0, (g1 - g0) * 4u);
-  __syncwarp();
-  const unsigned par = st->phase;
-  const bool done = __all_sync(kFull, stage_wait(*st, par));
-  if (lane == 0) st->phase = par ^ 1u;
-  if (!done) {
-    stage_wait(*st, par);
-    if (lane == 0) st->ok = 0;
-  }
-  __syncwarp();
-  return done ? (int)g0 : -1;
-}
-
 // Round to the nearest integer with two FP32 instructions (|x| < 2^22): adding
 // 1.5*2^23 moves the fraction out of the mantissa. Differs from the reference's
 // int-cast rounding only at exact half-cell ties, which lie beyond the cutoff.
@@ -280,62 +211,132 @@ template <int PREC> __device__ __forceinline__ double acc_value(const LaneAcc<PR
   else return vdw ? a.v : a.r;
 }
 
-// Dense evaluation of one screened pair: exact cutoff tests, LJ, real Coulomb,
-// overlap flag (VDW_Coulomb.cu:1287-1322). `host`: atom i is a framework (host) atom, else a
-// guest atom; the arrays are selected at run time so that a work item has one inlined copy
-// of this evaluation for both kinds of atoms and for full and final batches (the hot code of
-// a move then fits the instruction cache better).
+// Dense evaluation of one screened pair in the split forms, from its displacement (dh, dl): exact
+// cutoff tests, LJ, real Coulomb, overlap flag (VDW_Coulomb.cu:1287-1322). row: type pair; sc1: the
+// atom's scale is 1; qa: its charge as a float pair.
 template <int PREC>
-__device__ __forceinline__ void pair_dense(const BoxDev& b, bool host, int i, const Bead& bd, LaneAcc<PREC>& acc,
-                                           int& flag) {
-  if constexpr (PREC == GRX_FP64) {
-    float4 ah;
-    double4 p;
-    int ty;
-    bool sc1;
-    if (host) {
-      ah = b.hrec[2 * i];
-      p = b.hpos64[i];
-      const unsigned t = b.htype[i];
-      ty = (int)(t & 0x7fffu);
-      sc1 = !(t & 0x8000u);
-    } else {
-      ah = b.hi[i];
-      p = b.pos64[i];
-      ty = b.meta[i].x;
-      sc1 = __double_as_longlong(b.scale[i]) == 0x3ff0000000000000ll;
-    }
-    double x = p.x - bd.x, y = p.y - bd.y, z = p.z - bd.z;
-    image64(b, (bd.unit & 2) != 0, ah.x - bd.h.x, ah.y - bd.h.y, ah.z - bd.h.z, x, y, z);
+__device__ __forceinline__ void pair_core(const BoxDev& b, bool host, int i, const Bead& bd, float3 dh, float3 dl,
+                                          int row, bool sc1, float2 qa, LaneAcc<PREC>& acc, int& flag) {
+  if constexpr (PREC == kMixed64) {
+    const double x = (double)dh.x + (double)dl.x;
+    const double y = (double)dh.y + (double)dl.y;
+    const double z = (double)dh.z + (double)dl.z;
     const double rr = x * x + y * y + z * z;
-    // non-negative doubles (and NaN above all of them) order as their words do
-    const unsigned long long rb = (unsigned long long)__double_as_longlong(rr);
-    const int rh = __double2hiint(rr);
-    if (rb < (unsigned long long)__double_as_longlong(b.cut_vdw2)) {
-      const int row = ty * b.ntypes + bd.type;
+    if (rr < b.cut_vdw2) {
+      const float4 f = b.ff32[row];
+      const bool unit = sc1 && (bd.unit & 1) && !b.use_1264;
       double e;
-      if (sc1 && (bd.unit & 1) && !b.use_1264 && rh >= 0x3fd00000) {  // full molecules, r >= 0.5 A
-        const double2* f = reinterpret_cast<const double2*>(b.ff64 + row);
-        const double2 f0 = __ldg(f), f1 = __ldg(f + 1);  // {4 eps, sigma}, {sigma^2, shift}
-        const double r = recip64(rr);
-        double u = f1.x * r;
-        u = fma(fma(-rr, u, f1.x), r, u);  // sigma^2 / r^2, the rounding of the product taken out
-        const double u3 = u * u * u;
-        e = fma(f0.x, fma(u3, u3, -u3), -f1.y);
-      } else {
-        e = vdw64_cold(b, row, rr, (host ? b.hscale : b.scale)[i] * bd.scale);
-      }
-      if (__double2hiint(e) >= b.overlap_hi && e > b.overlap) flag = 1;
-      if (rh <= 0x3f847ae1 && rr < 0.01) flag = 1;
+      if (unit && (float)rr > f.w) e = (double)vdw32(f, (float)rr);
+      else e = vdw64_cold(b, row, rr, (host ? b.hscale : b.scale)[i] * bd.scale);
+      if (e > b.overlap) flag = 1;
+      if (rr < 0.01) flag = 1;
       acc.v += e;
     }
-    if (!b.no_charges && rb < (unsigned long long)__double_as_longlong(b.cut_coul2)) {
+    if (!b.no_charges && rr < b.cut_coul2) {
       const int k = table64_piece<kShiftG64>(rr, b.g64_base);
       double g;
       if ((unsigned)k < (unsigned)b.g64_n) g = table64<kShiftG64>(b.g64, k, rr);
       else g = coul_g_cold(b, rr);
-      acc.r = fma(p.w, g, acc.r);  // prefactor * q_bead applied once per item
+      acc.r = fma((host ? b.hpos64 : b.pos64)[i].w, g, acc.r);
     }
+  } else if constexpr (PREC == GRX_MIXED) {
+    const df s = df_norm2_split(dh, dl);
+    if (df_lt(s, df{b.cut_vdw2_df.x, b.cut_vdw2_df.y})) {
+      const float4 f = b.ff32[row];
+      const bool unit = sc1 && (bd.unit & 1) && !b.use_1264;
+      df e;
+      if (unit && s.hi > f.w) e = df{vdw32(f, s.hi), 0.0f};
+      else if (unit) {
+        const float2 c = lj_df_cold(b, row, s.hi, s.lo);
+        e = df{c.x, c.y};
+      }
+      else e = df_from(vdw64_cold(b, row, df_to(s), (host ? b.hscale : b.scale)[i] * bd.scale));
+      if (e.hi > b.overlapf) flag = 1;
+      if (s.hi < 0.01f) flag = 1;
+      df_accumulate(acc.v, e.hi, e.lo);
+    }
+    if (!b.no_charges && df_lt(s, df{b.cut_coul2_df.x, b.cut_coul2_df.y})) {
+      df g;
+      const int k = (__float_as_int(s.hi) >> 17) - b.ctab_base;
+      if ((unsigned)k < (unsigned)b.ctab_n) g = coul_table_df(b, k, s);
+      else g = df_from(coul_g_cold(b, df_to(s)));
+      const df e = two_prod(g.hi, qa.x);  // prefactor * q_bead applied once per item
+      df_accumulate(acc.r, e.hi, __fmaf_rn(g.hi, qa.y, __fmaf_rn(g.lo, qa.x, e.lo)));
+    }
+  } else {  // GRX_FP32
+    const float fx = dh.x + dl.x, fy = dh.y + dl.y, fz = dh.z + dl.z;
+    const float rr32 = fx * fx + fy * fy + fz * fz;
+    if (rr32 < b.cut_vdw2f) {
+      const float sc = (sc1 ? 1.0f : (float)(host ? b.hscale : b.scale)[i]) * (float)bd.scale;
+      float e;
+      if (sc == 1.0f && !b.use_1264) e = vdw32(b.ff32[row], rr32);
+      else e = (float)vdw64(b, row, (double)rr32, (double)sc);
+      if (e > b.overlapf) flag = 1;
+      if (rr32 < 0.01f) flag = 1;
+      acc.v += (double)e;
+    }
+    if (!b.no_charges && rr32 < b.cut_coul2f) acc.r += (double)coul32(b, qa.x * (float)bd.q, rr32);
+  }
+}
+
+// The same in FP64 (host: atom i is a framework atom, else a guest).
+__device__ __forceinline__ void pair_fp64(const BoxDev& b, bool host, int i, const Bead& bd, LaneAcc<GRX_FP64>& acc,
+                                          int& flag) {
+  float4 ah;
+  double4 p;
+  int ty;
+  bool sc1;
+  if (host) {
+    ah = b.hrec[2 * i];
+    p = b.hpos64[i];
+    const unsigned t = b.htype[i];
+    ty = (int)(t & 0x7fffu);
+    sc1 = !(t & 0x8000u);
+  } else {
+    ah = b.hi[i];
+    p = b.pos64[i];
+    ty = b.meta[i].x;
+    sc1 = __double_as_longlong(b.scale[i]) == 0x3ff0000000000000ll;
+  }
+  double x = p.x - bd.x, y = p.y - bd.y, z = p.z - bd.z;
+  image64(b, (bd.unit & 2) != 0, ah.x - bd.h.x, ah.y - bd.h.y, ah.z - bd.h.z, x, y, z);
+  const double rr = x * x + y * y + z * z;
+  // non-negative doubles (and NaN above all of them) order as their words do
+  const unsigned long long rb = (unsigned long long)__double_as_longlong(rr);
+  const int rh = __double2hiint(rr);
+  if (rb < (unsigned long long)__double_as_longlong(b.cut_vdw2)) {
+    const int row = ty * b.ntypes + bd.type;
+    double e;
+    if (sc1 && (bd.unit & 1) && !b.use_1264 && rh >= 0x3fd00000) {  // full molecules, r >= 0.5 A
+      const double2* f = reinterpret_cast<const double2*>(b.ff64 + row);
+      const double2 f0 = __ldg(f), f1 = __ldg(f + 1);  // {4 eps, sigma}, {sigma^2, shift}
+      const double r = recip64(rr);
+      double u = f1.x * r;
+      u = fma(fma(-rr, u, f1.x), r, u);  // sigma^2 / r^2, the rounding of the product taken out
+      const double u3 = u * u * u;
+      e = fma(f0.x, fma(u3, u3, -u3), -f1.y);
+    } else {
+      e = vdw64_cold(b, row, rr, (host ? b.hscale : b.scale)[i] * bd.scale);
+    }
+    if (__double2hiint(e) >= b.overlap_hi && e > b.overlap) flag = 1;
+    if (rh <= 0x3f847ae1 && rr < 0.01) flag = 1;
+    acc.v += e;
+  }
+  if (!b.no_charges && rb < (unsigned long long)__double_as_longlong(b.cut_coul2)) {
+    const int k = table64_piece<kShiftG64>(rr, b.g64_base);
+    double g;
+    if ((unsigned)k < (unsigned)b.g64_n) g = table64<kShiftG64>(b.g64, k, rr);
+    else g = coul_g_cold(b, rr);
+    acc.r = fma(p.w, g, acc.r);  // prefactor * q_bead applied once per item
+  }
+}
+
+// Atom i with the image of rounded fractions: framework atoms of the tile path, guests.
+template <int PREC>
+__device__ __forceinline__ void pair_dense(const BoxDev& b, bool host, int i, const Bead& bd, LaneAcc<PREC>& acc,
+                                           int& flag) {
+  if constexpr (PREC == GRX_FP64) {
+    pair_fp64(b, host, i, bd, acc, flag);
   } else {
     // host atoms from their records (one 32-byte sector: split position and charge, plus the
     // 2-byte type); guest atoms from the per-field arrays
@@ -357,70 +358,10 @@ __device__ __forceinline__ void pair_dense(const BoxDev& b, bool host, int i, co
       sc1 = al.w == 1.0f;
       qa = b.qdf[i];
     }
-    const int row = ty * b.ntypes + bd.type;
     float3 dh = make_float3(ah.x - bd.h.x, ah.y - bd.h.y, ah.z - bd.h.z);
     float3 dl = make_float3(al.x - bd.l.x, al.y - bd.l.y, al.z - bd.l.z);
     image_split(b, dh, dl);
-    if constexpr (PREC == kMixed64) {
-      const double x = (double)dh.x + (double)dl.x;
-      const double y = (double)dh.y + (double)dl.y;
-      const double z = (double)dh.z + (double)dl.z;
-      const double rr = x * x + y * y + z * z;
-      if (rr < b.cut_vdw2) {
-        const float4 f = b.ff32[row];
-        const bool unit = sc1 && (bd.unit & 1) && !b.use_1264;
-        double e;
-        if (unit && (float)rr > f.w) e = (double)vdw32(f, (float)rr);
-        else e = vdw64_cold(b, row, rr, (host ? b.hscale : b.scale)[i] * bd.scale);
-        if (e > b.overlap) flag = 1;
-        if (rr < 0.01) flag = 1;
-        acc.v += e;
-      }
-      if (!b.no_charges && rr < b.cut_coul2) {
-        const int k = table64_piece<kShiftG64>(rr, b.g64_base);
-        double g;
-        if ((unsigned)k < (unsigned)b.g64_n) g = table64<kShiftG64>(b.g64, k, rr);
-        else g = coul_g_cold(b, rr);
-        acc.r = fma((host ? b.hpos64 : b.pos64)[i].w, g, acc.r);
-      }
-    } else if constexpr (PREC == GRX_MIXED) {
-      const df s = df_norm2_split(dh, dl);
-      if (df_lt(s, df{b.cut_vdw2_df.x, b.cut_vdw2_df.y})) {
-        const float4 f = b.ff32[row];
-        const bool unit = sc1 && (bd.unit & 1) && !b.use_1264;
-        df e;
-        if (unit && s.hi > f.w) e = df{vdw32(f, s.hi), 0.0f};
-        else if (unit) {
-          const float2 c = lj_df_cold(b, row, s.hi, s.lo);
-          e = df{c.x, c.y};
-        }
-        else e = df_from(vdw64_cold(b, row, df_to(s), (host ? b.hscale : b.scale)[i] * bd.scale));
-        if (e.hi > b.overlapf) flag = 1;
-        if (s.hi < 0.01f) flag = 1;
-        df_accumulate(acc.v, e.hi, e.lo);
-      }
-      if (!b.no_charges && df_lt(s, df{b.cut_coul2_df.x, b.cut_coul2_df.y})) {
-        df g;
-        const int k = (__float_as_int(s.hi) >> 17) - b.ctab_base;
-        if ((unsigned)k < (unsigned)b.ctab_n) g = coul_table_df(b, k, s);
-        else g = df_from(coul_g_cold(b, df_to(s)));
-        const df e = two_prod(g.hi, qa.x);  // prefactor * q_bead applied once per item
-        df_accumulate(acc.r, e.hi, __fmaf_rn(g.hi, qa.y, __fmaf_rn(g.lo, qa.x, e.lo)));
-      }
-    } else {  // GRX_FP32
-      const float fx = dh.x + dl.x, fy = dh.y + dl.y, fz = dh.z + dl.z;
-      const float rr32 = fx * fx + fy * fy + fz * fz;
-      if (rr32 < b.cut_vdw2f) {
-        const float sc = (host ? (sc1 ? 1.0f : (float)b.hscale[i]) : al.w) * (float)bd.scale;
-        float e;
-        if (sc == 1.0f && !b.use_1264) e = vdw32(b.ff32[row], rr32);
-        else e = (float)vdw64(b, row, (double)rr32, (double)sc);
-        if (e > b.overlapf) flag = 1;
-        if (rr32 < 0.01f) flag = 1;
-        acc.v += (double)e;
-      }
-      if (!b.no_charges && rr32 < b.cut_coul2f) acc.r += (double)coul32(b, ah.w * (float)bd.q, rr32);
-    }
+    pair_core<PREC>(b, host, i, bd, dh, dl, ty * b.ntypes + bd.type, sc1, qa, acc, flag);
   }
 }
 
@@ -429,10 +370,11 @@ __device__ __forceinline__ void pair_dense(const BoxDev& b, bool host, int i, co
 // {vdw, real} of the host and the guest atoms (valid on every lane, summed later); flag is
 // per lane.
 //
-// A generator step screens up to 32 candidates of the current phase (host, then guests) and
-// appends the ones inside the screening radius to the warp's ring buffer. Whenever 32 are
-// queued, or the phase has no candidates left, the warp evaluates the next batch at the one
-// dense site; a phase ends with its buffer drained. Batches are the queue order, so the sums
+// Candidates are screened 32 at a time (host, then guests) and the ones inside the screening
+// radius appended to the warp's ring buffer; whenever 32 are queued, or the phase has no
+// candidates left, the warp evaluates the next batch at the phase's one dense site. Whole
+// chunks of voxel-list entries that lie inside the cutoff for the whole voxel (half of a
+// silica bead's list) go to the dense site directly. Batches come in list order, so the sums
 // do not depend on how the candidates were produced.
 //
 // Early overlap rejection: with `dead` (the bead's trial's flag in shared memory, null
@@ -445,15 +387,14 @@ template <int PREC, bool VOX>
 __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t0, int t1, int g0, int g1,
                                           int component, int newmol, int excl_comp, int excl_mol, int* q,
                                           LaneAcc<PREC>& hacc, LaneAcc<PREC>& gacc, int& flag,
-                                          volatile int* dead, VoxStage* stage) {
+                                          volatile int* dead) {
   const int lane = threadIdx.x & 31;
   const unsigned lt = (1u << lane) - 1u;
   unsigned head = 0, tail = 0;
-  // the trial is dead (checked by lane 0, the answer shared, so the warp stays converged)
-  auto is_dead = [&]() { return dead && __shfl_sync(kFull, lane == 0 ? *dead : 0, 0) > 0; };
-  // after a dense batch: an overlap found by this warp kills the trial
-  auto found_overlap = [&]() {
-    if (!dead || !__any_sync(kFull, flag != 0)) return false;
+  // the trial is dead: marked by another warp, or an overlap found by this one (which marks it).
+  // One vote, so the warp stays converged.
+  auto stop = [&]() {
+    if (!dead || !__any_sync(kFull, flag != 0 || *dead > 0)) return false;
     if (lane == 0) *dead = 1;
     return true;
   };
@@ -462,23 +403,17 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
     if (in) q[(tail + __popc(m & lt)) & (kQueue - 1)] = i;
     tail += __popc(m);
   };
+  // the next queued batch: entry of this lane (stale past n), n taken
+  auto pop = [&](int& n) {
+    n = (int)min(tail - head, 32u);
+    __syncwarp();
+    const int j = q[(head + lane) & (kQueue - 1)];
+    __syncwarp();
+    head += (unsigned)n;
+    return j;
+  };
+  if (stop()) return;
   const float bx = bd.h.x + bd.l.x, by = bd.h.y + bd.l.y, bz = bd.h.z + bd.l.z;
-
-  // host generator state. VOX: chunks [ch, cend) of the bead's voxel list; entries below
-  // vm.y are inside the cutoff for every bead of the voxel (queued unscreened), the others are
-  // screened at the stored image against the bead wrapped into the home cell. Tiles: groups of
-  // 32 tiles from `base`, culled one per lane; `mask` holds the group's surviving tiles.
-  int ch = t0, cend = t0;
-  int win_off = 0, win_end = t0;  // staged list window: entry j at buf[j + win_off], chunks below win_end
-  if (stage && !stage->ok) stage = nullptr;
-  int4 vm = make_int4(0, 0, 0, 0);
-  float wx = 0.f, wy = 0.f, wz = 0.f;
-  bool hcheck = false;
-  int base = t0;
-  unsigned mask = 0;
-  float sx = 0.f, sy = 0.f, sz = 0.f;  // this lane's tile: image shift of the bead
-  bool one_image = false;
-  int4 trl = make_int4(0, 0, -1, 0);   // this lane's tile range, shuffled to the warp below
   if constexpr (VOX) {
     if (t1 > t0) {
       const float fx = b.invf[0] * bx + b.invf[3] * by + b.invf[6] * bz;
@@ -488,56 +423,65 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
       const int ix = min(b.vn[0] - 1, max(0, (int)((fx - mx) * (float)b.vn[0])));
       const int iy = min(b.vn[1] - 1, max(0, (int)((fy - my) * (float)b.vn[1])));
       const int iz = min(b.vn[2] - 1, max(0, (int)((fz - mz) * (float)b.vn[2])));
-      vm = b.vmeta[(iz * b.vn[1] + iy) * b.vn[0] + ix];
-      wx = bd.h.x - (mx * b.cellf[0] + my * b.cellf[3] + mz * b.cellf[6]);
-      wy = bd.h.y - (mx * b.cellf[1] + my * b.cellf[4] + mz * b.cellf[7]);
-      wz = bd.h.z - (mx * b.cellf[2] + my * b.cellf[5] + mz * b.cellf[8]);
-      hcheck = component < b.nhost || (excl_comp >= 0 && excl_comp < b.nhost);
-      cend = min(t1, (vm.z + 31) >> 5);
+      const int4 vm = b.vmeta[(iz * b.vn[1] + iy) * b.vn[0] + ix];
+      // the bead in the home cell, for the screen (hi parts: grid multiples, exact)
+      const float3 wh = make_float3(
+          __fmaf_rn(-mz, b.cell_hi[6], __fmaf_rn(-my, b.cell_hi[3], __fmaf_rn(-mx, b.cell_hi[0], bd.h.x))),
+          __fmaf_rn(-mz, b.cell_hi[7], __fmaf_rn(-my, b.cell_hi[4], __fmaf_rn(-mx, b.cell_hi[1], bd.h.y))),
+          __fmaf_rn(-mz, b.cell_hi[8], __fmaf_rn(-my, b.cell_hi[5], __fmaf_rn(-mx, b.cell_hi[2], bd.h.z))));
+      const bool hcheck = component < b.nhost || (excl_comp >= 0 && excl_comp < b.nhost);
+      int ch = t0;
+      const int cend = min(t1, (vm.z + 31) >> 5);
+      const int sure_end = hcheck ? t0 : min(cend, vm.y >> 5);  // chunks of entries inside the cutoff
+      const unsigned* list = b.vlist + vm.x + lane;
+      auto load = [&](int c) { return c < cend && 32 * c + lane < vm.z ? __ldg(list + 32 * c) : 0u; };
+      unsigned next = load(ch);  // one chunk ahead: the list load is off the gather's path
+      for (;;) {
+        unsigned w;
+        int n;
+        if (ch < sure_end) {
+          w = next;
+          n = 32;
+          next = load(++ch);
+        } else {
+          while (tail - head < 32u && ch < cend) {  // screen at the stored image
+            const int j = (ch << 5) + lane;
+            const unsigned c = next;
+            next = load(++ch);
+            bool in = j < vm.z;
+            if (in && (j >= vm.y || hcheck)) {
+              const int i = (int)(c & 0xFFFFFu);
+              if (j >= vm.y) {
+                const float4 ah = b.hrec[2 * i];
+                const float4 sh = __ldg(b.vshift + (c >> 20));
+                const float x = (ah.x - wh.x) - sh.x, y = (ah.y - wh.y) - sh.y, z = (ah.z - wh.z) - sh.z;
+                in = x * x + y * y + z * z < b.screen2 || (PREC == GRX_FP64 && !(bd.unit & 2));
+              }
+              if (in && hcheck) {  // a host component is moved or excluded: skip its molecule
+                int tz = 0;
+                while (tz + 1 < b.nhost && i >= b.comp_off[tz + 1]) ++tz;
+                const int mol = b.hmeta[i].y;
+                if ((tz == excl_comp && mol == excl_mol) || (tz == component && mol == newmol)) in = false;
+              }
+            }
+            push(in, (int)c);
+          }
+          if (tail == head) break;
+          w = (unsigned)pop(n);
+        }
+        if (lane < n) pair_dense<PREC>(b, true, (int)(w & 0xFFFFFu), bd, hacc, flag);
+        if (stop()) return;
+      }
     }
-  }
-  // one host step: screen the next chunk / surviving tile; false when none is left
-  auto host_step = [&]() -> bool {
-    if constexpr (VOX) {
-      if (ch >= cend) return false;
-      if (stage && ch >= win_end) {  // stage chunks [ch, ch + 8) of the list (clipped to cend)
-        const int g0 = stage_refill(stage, b.vlist, (unsigned)vm.x + 32u * (unsigned)ch,
-                                    (unsigned)vm.x + (unsigned)min(32 * min(ch + kStageChunks, cend), vm.z));
-        if (g0 >= 0) {
-          win_off = vm.x - g0;
-          win_end = min(ch + kStageChunks, cend);
-        } else {
-          stage = nullptr;
-        }
-      }
-      const int j = (ch << 5) + lane;
-      ++ch;
-      bool in = false;
-      int i = 0;
-      if (j < vm.z) {
-        const unsigned w = stage ? stage->buf[j + win_off] : __ldg(b.vlist + vm.x + j);
-        i = (int)(w & 0xFFFFFu);
-        if (j < vm.y) {
-          in = true;
-        } else {
-          const float nx = (float)((int)((w >> 20) & 7u) - 4), ny = (float)((int)((w >> 23) & 7u) - 4),
-                      nz = (float)((int)((w >> 26) & 7u) - 4);
-          const float4 ah = b.hrec[2 * i];
-          const float x = ah.x - wx - (nx * b.cellf[0] + ny * b.cellf[3] + nz * b.cellf[6]);
-          const float y = ah.y - wy - (nx * b.cellf[1] + ny * b.cellf[4] + nz * b.cellf[7]);
-          const float z = ah.z - wz - (nx * b.cellf[2] + ny * b.cellf[5] + nz * b.cellf[8]);
-          in = x * x + y * y + z * z < b.screen2 || (PREC == GRX_FP64 && !(bd.unit & 2));
-        }
-        if (in && hcheck) {  // a host component is moved or excluded: skip its molecule
-          int tz = 0;
-          while (tz + 1 < b.nhost && i >= b.comp_off[tz + 1]) ++tz;
-          const int mol = b.hmeta[i].y;
-          if ((tz == excl_comp && mol == excl_mol) || (tz == component && mol == newmol)) in = false;
-        }
-      }
-      push(in, i);
-      return true;
-    } else {
+  } else {
+    // Groups of 32 tiles from `base`, culled one per lane; `mask` holds the group's surviving tiles.
+    int base = t0;
+    unsigned mask = 0;
+    float sx = 0.f, sy = 0.f, sz = 0.f;  // this lane's tile: image shift of the bead
+    bool one_image = false;
+    int4 trl = make_int4(0, 0, -1, 0);   // this lane's tile range, shuffled to the warp below
+    // screen the next surviving tile; false when none is left
+    auto host_step = [&]() -> bool {
       // Tiles are tested 32 at a time, one per lane; survivors are then screened one tile at
       // a time by the whole warp. When a tile lies inside one periodic image of the bead
       // (stored positions compact, the tile sphere clear of the rounding boundaries), the
@@ -625,48 +569,32 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
       }
       push(in, i);
       return true;
-    }
-  };
-  // one batch at the phase's dense site: 32 queued pairs, or the final ones when the phase has
-  // no candidates left (got false); true when the warp must stop (the trial overlaps)
-  auto batch = [&](bool host, bool got, LaneAcc<PREC>& acc) -> bool {
-    const unsigned avail = tail - head;
-    if (avail >= 32u || (!got && avail > 0u)) {
-      const int n = (int)min(avail, 32u);
-      __syncwarp();
-      const int j = q[(head + lane) & (kQueue - 1)];  // entries past n are stale and unused
-      __syncwarp();
-      if (lane < n) pair_dense<PREC>(b, host, j, bd, acc, flag);
-      head += (unsigned)n;
-      if (found_overlap()) return true;
-    }
-    return false;
-  };
-  if (t1 > t0) {
+    };
+    bool more = t1 > t0;
     for (;;) {
-      if (is_dead()) return;
-      const bool got = host_step();
-      if (batch(true, got, hacc)) return;
-      if (!got && tail == head) break;
+      while (more && tail - head < 32u) more = host_step();
+      if (tail == head) break;
+      int n;
+      const int j = pop(n);
+      if (lane < n) pair_dense<PREC>(b, true, j, bd, hacc, flag);
+      if (stop()) return;
     }
   }
   if (g1 <= g0) return;
-  head = tail = 0;
   // guest atoms [g0, g1) of the concatenated adsorbate components: component gc, its atoms
   // [gi, ghi) still to screen (indices within the component), gbase = the first concatenated
   // guest index after gc
   int gc = b.nhost, gbase = 0, gi = 0, ghi = 0;
   for (;;) {
-    if (is_dead()) return;
-    bool got = false;
-    while (gi >= ghi && gc < b.ncomp && gbase < g1) {  // next component overlapping [g0, g1)
-      const int n = b.comp_size[gc];
-      gi = max(g0 - gbase, 0);
-      ghi = min(g1 - gbase, n);
-      gbase += n;
-      ++gc;
-    }
-    if (gi < ghi) {
+    while (tail - head < 32u) {
+      while (gi >= ghi && gc < b.ncomp && gbase < g1) {  // next component overlapping [g0, g1)
+        const int n = b.comp_size[gc];
+        gi = max(g0 - gbase, 0);
+        ghi = min(g1 - gbase, n);
+        gbase += n;
+        ++gc;
+      }
+      if (gi >= ghi) break;
       const int c = gc - 1;
       const int i = b.comp_off[c] + gi + lane;
       bool in = false;
@@ -680,10 +608,12 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
       }
       gi += 32;
       push(in, i);
-      got = true;
     }
-    if (batch(false, got, gacc)) return;
-    if (!got && tail == head) return;
+    if (tail == head) return;
+    int n;
+    const int j = pop(n);
+    if (lane < n) pair_dense<PREC>(b, false, j, bd, gacc, flag);
+    if (stop()) return;
   }
 }
 
@@ -787,8 +717,7 @@ template <int PREC, bool VOX>
 __device__ __noinline__ void block_bead_pass_impl(const BoxDev& b, const Bead* beads, int nb, int component,
                                                      int newmol, int excl_comp, int excl_mol, int* qbuf,
                                                      double* ipart, int* iflag, int* counter, PassSplit sp,
-                                                     int item0, int item1, int chain, int* dead,
-                                                     VoxStage* stages) {
+                                                     int item0, int item1, int chain, int* dead) {
   if (item1 < 0) item1 = (int)sp.items;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int* q = qbuf + warp * kQueue;
@@ -821,8 +750,7 @@ __device__ __noinline__ void block_bead_pass_impl(const BoxDev& b, const Bead* b
       // trials of `chain` beads; dead[t] < 0: evaluated in full, else the early-exit flag
       volatile int* dt = nullptr;
       if (dead && dead[bead / chain] >= 0) dt = dead + bead / chain;
-      warp_item<PREC, VOX>(b, bd, t0, t1, g0, g1, component, newmol, excl_comp, excl_mol, q, hacc, gacc, flag, dt,
-                           stages ? stages + warp : nullptr);
+      warp_item<PREC, VOX>(b, bd, t0, t1, g0, g1, component, newmol, excl_comp, excl_mol, q, hacc, gacc, flag, dt);
       const unsigned fm = __ballot_sync(kFull, flag != 0);
       warp_store<PREC>(hacc, gacc, ipart + (item + bead) * 4, df{bd.pq.x, bd.pq.y},
                        b.prefactor * bd.q, g1 > g0);
@@ -840,13 +768,13 @@ template <int PREC>
 __device__ __forceinline__ void block_bead_pass(const BoxDev& b, const Bead* beads, int nb, int component, int newmol,
                                                 int excl_comp, int excl_mol, int* qbuf, double* ipart, int* iflag,
                                                 int* counter, PassSplit sp, int item0 = 0, int item1 = -1,
-                                                int chain = 1, int* dead = nullptr, VoxStage* stages = nullptr) {
+                                                int chain = 1, int* dead = nullptr) {
   if (b.vox)
     block_bead_pass_impl<PREC, true>(b, beads, nb, component, newmol, excl_comp, excl_mol, qbuf, ipart, iflag,
-                                     counter, sp, item0, item1, chain, dead, stages);
+                                     counter, sp, item0, item1, chain, dead);
   else
     block_bead_pass_impl<PREC, false>(b, beads, nb, component, newmol, excl_comp, excl_mol, qbuf, ipart, iflag,
-                                      counter, sp, item0, item1, chain, dead, nullptr);
+                                      counter, sp, item0, item1, chain, dead);
 }
 
 // ---------------------------------------------------------------- thread-block clusters
