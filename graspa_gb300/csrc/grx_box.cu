@@ -111,6 +111,8 @@ void refresh_dev(grx_box* b) {
   d.nvec = b->nvec;
   d.nact = b->nact;
   d.kact = b->kact;
+  d.kcol = b->kcol;
+  d.ncol = b->ncol;
   d.ktemp = b->ktemp;
   d.s_fw = b->s_fw;
   d.s_ads = b->s_ads;
@@ -433,6 +435,7 @@ static void build_kvectors(grx_box* b, const grx_box_geometry& g) {
   // origin) and groups of rows with at most 128 columns and 32 rows (a block of sk_kernel)
   b->h_krow.clear();
   b->h_kgroup.clear();
+  b->h_kcol.clear();
   for (int j = 0; j < b->nact;) {
     int e = j + 1;
     while (e < b->nact && b->h_kact[e].x == b->h_kact[j].x && b->h_kact[e].y == b->h_kact[j].y &&
@@ -456,8 +459,14 @@ static void build_kvectors(grx_box* b, const grx_box_geometry& g) {
     }
     b->h_kgroup.back().y = k + 1;
     b->h_krow.push_back(r);
+    const int slot0 = (r.kx * (2 * kym + 1) + r.ky + kym) * (2 * kzm + 1) + kzm;
+    for (int az = 0; az < r.ncol; ++az) {
+      const int jp = r.index(az), jm = az ? r.index(-az) : -1;
+      if (jp >= 0 || jm >= 0) b->h_kcol.push_back(make_int4(r.kx | (r.ky + 128) << 8 | az << 16, jp, jm, slot0));
+    }
     j = e;
   }
+  b->ncol = (int)b->h_kcol.size();
   b->n_kgroups = (int)b->h_kgroup.size();
 }
 
@@ -680,6 +689,7 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
   if ((e = dev_alloc(b, (void**)&b->kact, na * sizeof(int4))) != cudaSuccess) return fail(e, "alloc kact");
   if ((e = dev_alloc(b, (void**)&b->ktemp, na * sizeof(double))) != cudaSuccess) return fail(e, "alloc ktemp");
   if ((e = dev_alloc(b, (void**)&b->krow, (b->h_krow.size() + 1) * sizeof(KRow))) != cudaSuccess) return fail(e, "alloc k rows");
+  if ((e = dev_alloc(b, (void**)&b->kcol, (b->h_kcol.size() + 1) * sizeof(int4))) != cudaSuccess) return fail(e, "alloc k columns");
   if ((e = dev_alloc(b, (void**)&b->kgroup, (b->h_kgroup.size() + 1) * sizeof(int2))) != cudaSuccess) return fail(e, "alloc k groups");
   if ((e = dev_alloc(b, (void**)&b->s_fw, nv * sizeof(double2))) != cudaSuccess) return fail(e, "alloc s_fw");
   if ((e = dev_alloc(b, (void**)&b->s_ads, nv * sizeof(double2))) != cudaSuccess) return fail(e, "alloc s_ads");
@@ -709,6 +719,7 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
     cudaMemcpy(b->kact, b->h_kact.data(), b->nact * sizeof(int4), cudaMemcpyHostToDevice);
     cudaMemcpy(b->ktemp, b->h_ktemp.data(), b->nact * sizeof(double), cudaMemcpyHostToDevice);
     cudaMemcpy(b->krow, b->h_krow.data(), b->h_krow.size() * sizeof(KRow), cudaMemcpyHostToDevice);
+    cudaMemcpy(b->kcol, b->h_kcol.data(), b->h_kcol.size() * sizeof(int4), cudaMemcpyHostToDevice);
     cudaMemcpy(b->kgroup, b->h_kgroup.data(), b->h_kgroup.size() * sizeof(int2), cudaMemcpyHostToDevice);
   }
   if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return fail(e, "box upload");
@@ -750,6 +761,7 @@ grx_status grx_box_footprint(const grx_box_desc* desc, size_t* bytes) {
   size_t t = al(n * sizeof(double4)) + 2 * al(n * sizeof(float4)) + al(n * sizeof(int2)) + 2 * al(n * sizeof(double)) +
              al(n * sizeof(float2)) + al(GRX_MAX_COMPONENTS * sizeof(int));
   t += al((nt2 + 27) * sizeof(FFPair64)) + al(nt2 * sizeof(double)) + 2 * al(nt2 * sizeof(float4)) + al(nt2 * sizeof(float2));
+  t += al((tmp.h_kcol.size() + 1) * sizeof(int4));
   t += al((tmp.h_krow.size() + 1) * sizeof(KRow)) + al((tmp.h_kgroup.size() + 1) * sizeof(int2));
   t += al(na * sizeof(int4)) + al(na * sizeof(double)) + 3 * al(nv * sizeof(double2)) + 2 * al(na * sizeof(float4)) +
        al(na * sizeof(float2));
@@ -846,7 +858,7 @@ grx_status grx_box_destroy(grx_box* b) {
     return GRX_OK;
   }
   void* ptrs[] = {b->pos64, b->hi, b->lo, b->meta, b->scale, b->charge, b->d_size, b->ff64,
-                  b->ffc10, b->ff32, b->kact, b->ktemp, b->krow, b->kgroup, b->s_fw, b->s_ads, b->s_tmp,
+                  b->ffc10, b->ff32, b->kact, b->ktemp, b->krow, b->kgroup, b->kcol, b->s_fw, b->s_ads, b->s_tmp,
                   b->scratch, b->d_results, b->tile_c, b->tile_r, b->ctabf, b->qdf,
                   b->ffdf, b->ffdf2, b->ewA, b->ewF, b->ewT, b->vmeta, b->vlist, b->hrec, b->htype};
   for (void* p : ptrs) dev_free(b, p);

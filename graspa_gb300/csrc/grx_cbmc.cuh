@@ -13,6 +13,7 @@
 //                     (Ewald_Energy_Functions.h:162-185, 280-397)
 #pragma once
 
+#include "grx_ewcol.cuh"
 #include "grx_warp.cuh"
 
 namespace grx {
@@ -52,7 +53,6 @@ struct CbmcWork {
   double sbuf[32];
   double ewx[8][2];  // per-CTA Fourier partials {same, cross} of a cluster
   double wsum[2][NW];
-  float2 qd[2 * kMolWork];
   int counter;
   long long cfg;    // trial configurations evaluated since the caller last cleared it
   long long cbeads; // their beads
@@ -299,103 +299,35 @@ __device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, d
 // ---------------------------------------------------------------- Ewald
 // Fourier delta of the na moved atoms in W.mx/my/mz/mq (old atoms carry -q):
 // dS(k) = sum q e^{ik.r}; same = sum temp (|S + dS|^2 - |S|^2), cross = sum temp
-// Re(S_cross dS*), S_same = adsorbate block (guest moves). The FP64 form follows
-// the reference arithmetic; the other forms evaluate dS and both sums in
+// Re(S_cross dS*), S_same = adsorbate block (guest moves), by columns of k (grx_ewcol.cuh). The
+// FP64 form keeps the reference arithmetic; the other forms evaluate dS and both sums in
 // double-float on the FP32 pipe against temp*S tables (ewA, ewF). When s_out is
 // given, S_same + dS is staged there (FP64) for a later commit. Results on thread 0.
-// With CL > 1 each CTA of the cluster takes a contiguous range of the active k (its
-// range of S is staged, and later committed, by that CTA alone); the CTAs' partial sums
-// are exchanged through distributed shared memory and added in rank order by every CTA.
+// With CL > 1 each CTA of the cluster takes a contiguous range of the columns; the CTAs' partial
+// sums are exchanged through distributed shared memory and added in rank order by every CTA, and
+// the cluster barriers before a commit publish the staged S.
 template <int PREC, class WK, bool ROWS = false, int CL = 1>
 __device__ __noinline__ void ewald_move(const BoxDev& b, WK& W, int na, double2* eik, double2* s_out,
                                            double& same, double& cross) {
   const int tid = threadIdx.x;
-  int k0 = 0, k1 = b.nact;
-  if constexpr (CL > 1) cluster_k_range(b.nact, CL, cluster_rank(), k0, k1);
-  const int kx1 = b.kmax[0] + 1, ky1 = b.kmax[1] + 1;
-  double2* ex = eik;
-  double2* ey = ex + kx1 * na;
-  double2* ez = ey + ky1 * na;
-  const double PI2 = 2.0 * 3.14159265358979323846;
-  if (tid < 3 * na) {  // eik recurrence per atom and axis (Initialize_Vectors_thread)
-    const int at = tid % na, d = tid / na;
-    const double f = b.inv[d] * W.mx[at] + b.inv[3 + d] * W.my[at] + b.inv[6 + d] * W.mz[at];
-    const int km = b.kmax[d];
-    if constexpr (PREC == GRX_FP64) {
-      double2* tab = d == 0 ? ex : (d == 1 ? ey : ez);
-      tab[at] = make_double2(1.0, 0.0);
-      if (km >= 1) {
-        double sn, cs;
-        sincos(f * PI2, &sn, &cs);
-        const double2 e1 = make_double2(cs, sn);
-        double2 e = e1;
-        tab[at + na] = e1;
-        for (int k = 2; k <= km; ++k) {
-          e = cmul(e, e1);
-          tab[at + k * na] = e;
-        }
-      }
-    } else {  // straight into the double-float tables read below (the FP64 ones are not used)
-      float4* f0 = reinterpret_cast<float4*>(eik);
-      float4* tab = f0 + (d == 0 ? 0 : (d == 1 ? kx1 * na : (kx1 + ky1) * na));
-      df_eik_row(f, km, tab + at, na);
-    }
-  }
+  int c0 = 0, c1 = b.ncol;
+  if constexpr (CL > 1) cluster_k_range(b.ncol, CL, cluster_rank(), c0, c1);
+  eik_fill<PREC == GRX_FP64>(b, na, W.mx, W.my, W.mz, W.mq, eik, tid, blockDim.x);
   __syncthreads();
   same = 0.0;
   cross = 0.0;
   if constexpr (PREC == GRX_FP64) {
-    for (int j = k0 + tid; j < k1; j += blockDim.x) {
-      const int4 k = b.kact[j];
-      double2 dsk = make_double2(0.0, 0.0);
-      for (int at = 0; at < na; ++at) {
-        double2 y = ey[at + na * abs(k.y)];
-        if (k.y < 0) y.y = -y.y;
-        double2 z = ez[at + na * abs(k.z)];
-        if (k.z < 0) z.y = -z.y;
-        const double2 t = cmul(cmul(ex[at + na * k.x], y), z);
-        dsk.x += W.mq[at] * t.x;
-        dsk.y += W.mq[at] * t.y;
-      }
-      const double tmp = b.ktemp[j];
-      const double2 ov = b.s_ads[k.w];
-      const double2 nv = make_double2(ov.x + dsk.x, ov.y + dsk.y);
-      same += tmp * (nv.x * nv.x + nv.y * nv.y);
-      same -= tmp * (ov.x * ov.x + ov.y * ov.y);
-      const double2 xv = b.s_fw[k.w];
-      cross += tmp * (xv.x * dsk.x + xv.y * dsk.y);
-      if (s_out) s_out[k.w] = nv;
-    }
-    same = block_sum(same, W.sbuf);
-    cross = block_sum(cross, W.sbuf);
+    EwSums64 e;
+    ewald_columns(b, na, eik, c0 + tid, c1, blockDim.x, s_out, e);
+    same = block_sum(e.same, W.sbuf);
+    cross = block_sum(e.cross, W.sbuf);
   } else {
-    float4* fx = reinterpret_cast<float4*>(eik);
-    const int ntab = (b.kmax[0] + b.kmax[1] + b.kmax[2] + 3) * na;
-    if (tid < na) { const df q = df_from(W.mq[tid]); W.qd[tid] = make_float2(q.hi, q.lo); }
-    __syncthreads();
-    const float4* fy = fx + kx1 * na;
-    const float4* fz = fy + ky1 * na;
-    df sm = {0.f, 0.f}, cr = {0.f, 0.f};
-    if constexpr (ROWS) {
-      // energy terms of one k from its dS: sm += 2 Re(temp S* dS) + temp |dS|^2,
-      // cr += Re(temp S_fw* dS); optionally stage S + dS (FP64, compensated)
-      auto k_energy = [&](int j, int slot, const df& cre, const df& cim) {
-        const float4 A = b.ewA[j], F = b.ewF[j];
-        const float2 T = b.ewT[j];
-        const df reA = df_add(df_mul(df{A.x, A.y}, cre), df_mul(df{A.z, A.w}, cim));
-        const df n2 = df_add(df_mul(cre, cre), df_mul(cim, cim));
-        sm = df_add(sm, df_add(df{2.f * reA.hi, 2.f * reA.lo}, df_mul(df{T.x, T.y}, n2)));
-        cr = df_add(cr, df_add(df_mul(df{F.x, F.y}, cre), df_mul(df{F.z, F.w}, cim)));
-        if (s_out) {
-          const double2 ov = b.s_ads[slot];
-          s_out[slot] = make_double2(ov.x + df_to(cre), ov.y + df_to(cim));
-        }
-      };
-
-      // q X(kx) Y(ky) per (kx, ky) row and atom, then one complex product with Z(kz) per
-      // (k, atom); threads keep one k each, as in the direct form
+    const float4* fx = reinterpret_cast<const float4*>(eik);
+    float4* rxy = nullptr;
+    if constexpr (ROWS) {  // q X(kx) Y(ky) per (kx, ky) row and atom
+      rxy = reinterpret_cast<float4*>(eik) + (b.kmax[0] + b.kmax[1] + b.kmax[2] + 3) * na;
+      const float4* fy = fx + (b.kmax[0] + 1) * na;
       const int ny = 2 * b.kmax[1] + 1, nrow = ew_rows(b.kmax);
-      float4* rxy = fx + ntab;
       for (int e = tid; e < nrow * na; e += blockDim.x) {
         const int row = e / na, at = e - row * na;
         const int kx = row / ny, ky = row - kx * ny - b.kmax[1];
@@ -403,60 +335,15 @@ __device__ __noinline__ void ewald_move(const BoxDev& b, WK& W, int na, double2*
         const float4 X = fx[at + na * kx], Y = fy[at + na * abs(ky)];
         const df xr = {X.x, X.y}, xi = {X.z, X.w};
         const df yr = {Y.x, Y.y}, yi = {s * Y.z, s * Y.w};
-        const df q = {W.qd[at].x, W.qd[at].y};
-        const df pr = df_mul(q, df_add(df_mul(xr, yr), df_mul(df{-xi.hi, -xi.lo}, yi)));
-        const df pi = df_mul(q, df_add(df_mul(xr, yi), df_mul(xi, yr)));
+        const df pr = df_add(df_mul(xr, yr), df_mul(df{-xi.hi, -xi.lo}, yi));
+        const df pi = df_add(df_mul(xr, yi), df_mul(xi, yr));
         rxy[e] = make_float4(pr.hi, pr.lo, pi.hi, pi.lo);
       }
       __syncthreads();
-      for (int j = k0 + tid; j < k1; j += blockDim.x) {
-        const int4 k = b.kact[j];
-        const float4* P = rxy + (k.x * ny + k.y + b.kmax[1]) * na;
-        const int az = abs(k.z);
-        const float sz = k.z < 0 ? -1.f : 1.f;
-        df cre = {0.f, 0.f}, cim = {0.f, 0.f};
-#pragma unroll 1
-        for (int at = 0; at < na; ++at) {
-          const float4 R = P[at], Z = fz[at + na * az];
-          const df pr = {R.x, R.y}, pi = {R.z, R.w};
-          const df zr = {Z.x, Z.y}, zi = {sz * Z.z, sz * Z.w};
-          cre = df_add(cre, df_add(df_mul(pr, zr), df_mul(df{-pi.hi, -pi.lo}, zi)));
-          cim = df_add(cim, df_add(df_mul(pr, zi), df_mul(pi, zr)));
-        }
-        k_energy(j, k.w, cre, cim);
-      }
-    } else {
-      for (int j = k0 + tid; j < k1; j += blockDim.x) {
-        const int4 k = b.kact[j];
-        df cre = {0.f, 0.f}, cim = {0.f, 0.f};
-        const int ay = abs(k.y), az = abs(k.z);
-        const float sy = k.y < 0 ? -1.f : 1.f, sz = k.z < 0 ? -1.f : 1.f;
-#pragma unroll 1
-        for (int at = 0; at < na; ++at) {
-          const float4 X = fx[at + na * k.x], Y = fy[at + na * ay], Z = fz[at + na * az];
-          const df xr = {X.x, X.y}, xi = {X.z, X.w};
-          const df yr = {Y.x, Y.y}, yi = {sy * Y.z, sy * Y.w};
-          const df zr = {Z.x, Z.y}, zi = {sz * Z.z, sz * Z.w};
-          const df pr = df_add(df_mul(xr, yr), df_mul(df{-xi.hi, -xi.lo}, yi));
-          const df pi = df_add(df_mul(xr, yi), df_mul(xi, yr));
-          const df tr = df_add(df_mul(pr, zr), df_mul(df{-pi.hi, -pi.lo}, zi));
-          const df ti = df_add(df_mul(pr, zi), df_mul(pi, zr));
-          const df q = {W.qd[at].x, W.qd[at].y};
-          cre = df_add(cre, df_mul(q, tr));
-          cim = df_add(cim, df_mul(q, ti));
-        }
-        const float4 A = b.ewA[j], F = b.ewF[j];
-        const float2 T = b.ewT[j];
-        const df reA = df_add(df_mul(df{A.x, A.y}, cre), df_mul(df{A.z, A.w}, cim));
-        const df n2 = df_add(df_mul(cre, cre), df_mul(cim, cim));
-        sm = df_add(sm, df_add(df{2.f * reA.hi, 2.f * reA.lo}, df_mul(df{T.x, T.y}, n2)));
-        cr = df_add(cr, df_add(df_mul(df{F.x, F.y}, cre), df_mul(df{F.z, F.w}, cim)));
-        if (s_out) {  // compensated update: FP64 S plus the double-float dS
-          const double2 ov = b.s_ads[k.w];
-          s_out[k.w] = make_double2(ov.x + df_to(cre), ov.y + df_to(cim));
-        }
-      }
     }
+    EwSumsDf e;
+    ewald_columns<ROWS>(b, na, fx, rxy, c0 + tid, c1, blockDim.x, s_out, e);
+    df sm = ew_same(e), cr = e.c;
     sm = warp_sum_df(sm);
     cr = warp_sum_df(cr);
     if ((tid & 31) == 0) { W.wsum[0][tid >> 5] = df_to(sm); W.wsum[1][tid >> 5] = df_to(cr); }

@@ -65,6 +65,9 @@ struct grx_box {
   grx::KRow* krow = nullptr;   // (kx, ky) rows of the active k, and groups of rows for sk_kernel
   int2* kgroup = nullptr;
   int n_kgroups = 0;
+  int4* kcol = nullptr;        // columns (kx, ky, |kz|) of the active k
+  int ncol = 0;
+  std::vector<int4> h_kcol;
   std::vector<grx::KRow> h_krow;
   std::vector<int2> h_kgroup;
   std::vector<int4> h_kact;

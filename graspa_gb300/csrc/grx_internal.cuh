@@ -126,6 +126,9 @@ struct BoxDev {
   int nact;
   const int4* kact;     // kx, ky, kz, slot
   const double* ktemp;  // factor * exp(-k^2/4a^2)/k^2 per active k
+  const int4* kcol;     // columns of the active k (see grx_ewcol.cuh): {kx | ky+128 << 8 | |kz| << 16, index of +|kz|,
+                        // of -|kz| (-1: not active, or |kz| = 0), slot of kz = 0}
+  int ncol;
   double2* s_fw;
   double2* s_ads;
   double2* s_tmp;

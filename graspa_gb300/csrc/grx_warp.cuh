@@ -180,13 +180,6 @@ __device__ __forceinline__ df coul_table_df(const BoxDev& b, int k, df s) {
   return {g.hi, __fadd_rn(g.lo, __fadd_rn(m.lo, c0.y))};
 }
 
-// a += h + l, a kept as an unnormalised pair: the exact error of the hi sum joins the low part.
-__device__ __forceinline__ void df_accumulate(df& a, float h, float l) {
-  const df s = two_sum(a.hi, h);
-  a.hi = s.hi;
-  a.lo = __fadd_rn(a.lo, __fadd_rn(s.lo, l));
-}
-
 // Cold paths of the mixed-precision pair evaluation, kept out of line so the inlined copies of
 // pair_dense stay small: LJ inside 1.1 sigma (double-float), LJ with a non-unit scaling or the
 // 12-6-4 form, and g(s) outside the Coulomb table's range.

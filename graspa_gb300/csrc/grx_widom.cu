@@ -13,6 +13,7 @@
 #include <cmath>
 #include <vector>
 
+#include "grx_ewcol.cuh"
 #include "grx_host.h"
 #include "grx_warp.cuh"
 
@@ -245,96 +246,18 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
     }
     // 6. Ewald delta of the chosen molecule (insertion: no old atoms)
     if (s_ok && a.charged && !b.no_charges && b.nact > 0) {
-      const int kx1 = b.kmax[0] + 1, ky1 = b.kmax[1] + 1;
-      double2* ex = eik_s;
-      double2* ey = ex + kx1 * ms;
-      double2* ez = ey + ky1 * ms;
-      const double PI2 = 2.0 * 3.14159265358979323846;
-      if (tid < 3 * ms) {
-        const int at = tid % ms, d = tid / ms;
-        const double f = b.inv[d] * newx[at] + b.inv[3 + d] * newy[at] + b.inv[6 + d] * newz[at];
-        const int km = b.kmax[d];
-        if constexpr (PREC == GRX_FP64) {
-          double2* tab = d == 0 ? ex : (d == 1 ? ey : ez);
-          tab[at] = make_double2(1.0, 0.0);
-          if (km >= 1) {
-            double sn, cs;
-            sincos(f * PI2, &sn, &cs);
-            const double2 e1 = make_double2(cs, sn);
-            double2 e = e1;
-            tab[at + ms] = e1;
-            for (int k = 2; k <= km; ++k) {
-              e = cmul(e, e1);
-              tab[at + k * ms] = e;
-            }
-          }
-        } else {  // straight into the double-float tables (after the FP64 ones)
-          float4* f0 = reinterpret_cast<float4*>(ez + (b.kmax[2] + 1) * ms);
-          float4* tab = f0 + (d == 0 ? 0 : (d == 1 ? kx1 * ms : (kx1 + ky1) * ms));
-          df_eik_row(f, km, tab + at, ms);
-        }
-      }
+      eik_fill<PREC == GRX_FP64>(b, ms, newx, newy, newz, newq, eik_s, tid, blockDim.x);
       __syncthreads();
       double same = 0.0, cross = 0.0;
       if constexpr (PREC == GRX_FP64) {
-        for (int j = tid; j < b.nact; j += blockDim.x) {
-          const int4 k = b.kact[j];
-          double2 cn = make_double2(0.0, 0.0);
-          for (int at = 0; at < ms; ++at) {
-            double2 y = ey[at + ms * abs(k.y)];
-            if (k.y < 0) y.y = -y.y;
-            double2 z = ez[at + ms * abs(k.z)];
-            if (k.z < 0) z.y = -z.y;
-            const double2 t = cmul(cmul(ex[at + ms * k.x], y), z);
-            cn.x += newq[at] * t.x;
-            cn.y += newq[at] * t.y;
-          }
-          const double tmp = b.ktemp[j];
-          const double2 ov = b.s_ads[k.w];
-          const double2 nv = make_double2(ov.x + cn.x, ov.y + cn.y);
-          same += tmp * (nv.x * nv.x + nv.y * nv.y);
-          same -= tmp * (ov.x * ov.x + ov.y * ov.y);
-          const double2 xv = b.s_fw[k.w];
-          cross += tmp * (xv.x * cn.x + xv.y * cn.y);
-        }
-        same = block_sum(same, sbuf);
-        cross = block_sum(cross, sbuf);
+        EwSums64 e;
+        ewald_columns(b, ms, eik_s, tid, b.ncol, blockDim.x, nullptr, e);
+        same = block_sum(e.same, sbuf);
+        cross = block_sum(e.cross, sbuf);
       } else {
-        // double-float copies of the eik tables (same shared buffer, after the FP64 ones)
-        float4* fx = reinterpret_cast<float4*>(ez + (b.kmax[2] + 1) * ms);
-        __shared__ float2 qd[GRX_MAX_MOLSIZE];
-        if (tid < ms) { const df q = df_from(newq[tid]); qd[tid] = make_float2(q.hi, q.lo); }
-        __syncthreads();
-        const float4* fy = fx + kx1 * ms;
-        const float4* fz = fy + ky1 * ms;
-        df sm = {0.f, 0.f}, cr = {0.f, 0.f};
-        for (int j = tid; j < b.nact; j += blockDim.x) {
-          const int4 k = b.kact[j];
-          df cre = {0.f, 0.f}, cim = {0.f, 0.f};
-          const int ay = abs(k.y), az = abs(k.z);
-          const float sy = k.y < 0 ? -1.f : 1.f, sz = k.z < 0 ? -1.f : 1.f;
-          for (int at = 0; at < ms; ++at) {
-            const float4 X = fx[at + ms * k.x], Y = fy[at + ms * ay], Z = fz[at + ms * az];
-            const df xr = {X.x, X.y}, xi = {X.z, X.w};
-            const df yr = {Y.x, Y.y}, yi = {sy * Y.z, sy * Y.w};
-            const df zr = {Z.x, Z.y}, zi = {sz * Z.z, sz * Z.w};
-            // (x*y)*z, then charge
-            const df pr = df_add(df_mul(xr, yr), df_mul(df{-xi.hi, -xi.lo}, yi));
-            const df pi = df_add(df_mul(xr, yi), df_mul(xi, yr));
-            const df tr = df_add(df_mul(pr, zr), df_mul(df{-pi.hi, -pi.lo}, zi));
-            const df ti = df_add(df_mul(pr, zi), df_mul(pi, zr));
-            const df q = {qd[at].x, qd[at].y};
-            cre = df_add(cre, df_mul(q, tr));
-            cim = df_add(cim, df_mul(q, ti));
-          }
-          const float4 A = b.ewA[j], F = b.ewF[j];
-          const float2 T = b.ewT[j];
-          // same: 2 Re(A dS*) + temp |dS|^2 ; cross: Re(F dS*)
-          const df reA = df_add(df_mul(df{A.x, A.y}, cre), df_mul(df{A.z, A.w}, cim));
-          const df n2 = df_add(df_mul(cre, cre), df_mul(cim, cim));
-          sm = df_add(sm, df_add(df{2.f * reA.hi, 2.f * reA.lo}, df_mul(df{T.x, T.y}, n2)));
-          cr = df_add(cr, df_add(df_mul(df{F.x, F.y}, cre), df_mul(df{F.z, F.w}, cim)));
-        }
+        EwSumsDf e;
+        ewald_columns<false>(b, ms, reinterpret_cast<const float4*>(eik_s), nullptr, tid, b.ncol, blockDim.x, nullptr, e);
+        df sm = ew_same(e), cr = e.c;
         // block sums: warp tree in double-float, then FP64 over the 8 warp partials
         sm = warp_sum_df(sm);
         cr = warp_sum_df(cr);
@@ -428,8 +351,8 @@ static grx_status widom_launch(grx_box* b, const grx_widom_desc* d, uint64_t fir
   a.stream = d->stream;
   a.first_move = first_move;
   a.n = (int64_t)n;
-  const size_t smem = (size_t)(b->dev.kmax[0] + b->dev.kmax[1] + b->dev.kmax[2] + 3) * ms *
-                      (sizeof(double2) + sizeof(float4));
+  const size_t smem = (size_t)(b->dev.kmax[0] + b->dev.kmax[1] + b->dev.kmax[2] + 3) * ms * sizeof(double2);
+  static_assert(sizeof(double2) == sizeof(float4), "eik entries of both forms");
   if (!b->ewdf_valid && b->nact > 0) {
     ewald_df_refresh_kernel<<<std::max(1, std::min((b->nact + 255) / 256, sm_count(b))), 256, 0, b->stream>>>(
         b->dev, b->ewA, b->ewF, b->ewT);
