@@ -82,6 +82,28 @@ grx_status ensure_pinned(grx_box* b, size_t bytes) {
   return GRX_OK;
 }
 
+static bool plain_host(const void* p) {
+  cudaPointerAttributes a;
+  if (!p) return false;  // the runtime reports it
+  if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+  cudaGetLastError();
+  return false;
+}
+
+grx_status fetch(void* dst, const void* src, size_t bytes, const char* what) {
+  if (bytes == 0) return GRX_OK;
+  if (plain_host(src)) std::memcpy(dst, src, bytes);
+  else GRX_CHECK_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDefault), what);
+  return GRX_OK;
+}
+
+grx_status deliver(void* dst, const void* src, size_t bytes, const char* what) {
+  if (bytes == 0) return GRX_OK;
+  if (plain_host(dst)) std::memcpy(dst, src, bytes);
+  else GRX_CHECK_CUDA(cudaMemcpy(dst, src, bytes, cudaMemcpyDefault), what);
+  return GRX_OK;
+}
+
 grx_status ensure_results(grx_box* b, size_t n) {
   if (n <= b->results_cap) return GRX_OK;
   dev_free(b, b->d_results);

@@ -318,7 +318,7 @@ __device__ __noinline__ void ewald_move(const BoxDev& b, WK& W, int na, double2*
   cross = 0.0;
   if constexpr (PREC == GRX_FP64) {
     EwSums64 e;
-    ewald_columns(b, na, eik, c0 + tid, c1, blockDim.x, s_out, e);
+    ewald_columns(b, na, eik, c0 + tid, c1, blockDim.x, b.s_ads, b.s_fw, s_out, e);
     same = block_sum(e.same, W.sbuf);
     cross = block_sum(e.cross, W.sbuf);
   } else {

@@ -4,6 +4,7 @@
 #include <cmath>
 #include <vector>
 
+#include "grx_ewcol.cuh"
 #include "grx_host.h"
 #include "grx_warp.cuh"
 
@@ -53,15 +54,6 @@ __global__ void eik_tables_kernel(BoxDev b, CompRanges r, int first, double2* ex
       t[k * stride] = e;
     }
   }
-}
-
-__device__ __forceinline__ double2 eik_term(const double2* ex, const double2* ey, const double2* ez,
-                                            size_t n, size_t j, int kx, int ky, int kz) {
-  double2 y = ey[j + n * (size_t)abs(ky)];
-  if (ky < 0) y.y = -y.y;
-  double2 z = ez[j + n * (size_t)abs(kz)];
-  if (kz < 0) z.y = -z.y;
-  return cmul(cmul(ex[j + n * (size_t)kx], y), z);
 }
 
 // Structure factors (Ewald_Total, ewald_preparation.h:128-147). A block holds the columns
@@ -365,67 +357,25 @@ __global__ void __launch_bounds__(GRX_THREADS) host_total_kernel(BoxDev b, CompR
   }
 }
 
-// Fourier delta of one move (Fourier_Ewald_Diff, Ewald_Energy_Functions.h:280-397):
-// every block rebuilds the eik tables of the few moved atoms in shared memory, then
-// handles a strided subset of the active k. part per block: {same, cross}.
-struct MoveAtoms {
-  int n_old, n_new;
-  double x[2 * GRX_MAX_MOLSIZE], y[2 * GRX_MAX_MOLSIZE], z[2 * GRX_MAX_MOLSIZE], q[2 * GRX_MAX_MOLSIZE];
-};
+// Fourier delta of one move (Fourier_Ewald_Diff, Ewald_Energy_Functions.h:280-397) by columns of
+// k (grx_ewcol.cuh): every block rebuilds the eik tables of the few moved atoms in shared
+// memory, then takes a strided subset of the columns. A call is latency, so the blocks are small
+// (two warps, at most two blocks an SM): 12 on the silica box, where one thread per k made 6.
+// at: x, y, z, q of the moved atoms (the old ones with their charges negated), in pinned host
+// memory, as is part, per block {same, cross}.
+constexpr int kDeltaThreads = 64;
 
-__global__ void __launch_bounds__(GRX_THREADS) ewald_delta_kernel(BoxDev b, const MoveAtoms* mv,
-                                                                  const double2* s_same,
-                                                                  const double2* s_cross,
-                                                                  double2* s_out, double* part) {
+__global__ void __launch_bounds__(kDeltaThreads) ewald_delta_kernel(const __grid_constant__ BoxDev b, const double* at,
+                                                                    int na, const double2* s_same,
+                                                                    const double2* s_cross, double2* s_out, double* part) {
   extern __shared__ double2 eik_s[];
   __shared__ double sbuf[32];
-  const int na = mv->n_old + mv->n_new;
-  const int kx1 = b.kmax[0] + 1, ky1 = b.kmax[1] + 1;
-  double2* ex = eik_s;
-  double2* ey = ex + kx1 * na;
-  double2* ez = ey + ky1 * na;
-  const double PI2 = 2.0 * 3.14159265358979323846;
-  for (int t = threadIdx.x; t < 3 * na; t += blockDim.x) {
-    const int a = t % na, d = t / na;
-    const double px = mv->x[a], py = mv->y[a], pz = mv->z[a];
-    const double s = (b.inv[d] * px + b.inv[3 + d] * py + b.inv[6 + d] * pz) * PI2;
-    double2* tab = d == 0 ? ex : (d == 1 ? ey : ez);
-    const int km = b.kmax[d];
-    tab[a] = make_double2(1.0, 0.0);
-    if (km >= 1) {
-      double sn, cs;
-      sincos(s, &sn, &cs);
-      const double2 e1 = make_double2(cs, sn);
-      double2 e = e1;
-      tab[a + na] = e1;
-      for (int k = 2; k <= km; ++k) {
-        e = cmul(e, e1);
-        tab[a + k * na] = e;
-      }
-    }
-  }
+  eik_fill<true>(b, na, at, at + na, at + 2 * na, at + 3 * na, eik_s, threadIdx.x, blockDim.x);
   __syncthreads();
-  double same = 0.0, cross = 0.0;
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < b.nact; j += gridDim.x * blockDim.x) {
-    const int4 k = b.kact[j];
-    double2 co = make_double2(0, 0), cn = make_double2(0, 0);
-    for (int a = 0; a < na; ++a) {
-      const double2 t = eik_term(ex, ey, ez, na, a, k.x, k.y, k.z);
-      const double q = mv->q[a];
-      if (a < mv->n_old) { co.x += q * t.x; co.y += q * t.y; }
-      else { cn.x += q * t.x; cn.y += q * t.y; }
-    }
-    const double tmp = b.ktemp[j];
-    const double2 ov = s_same[k.w];
-    const double2 nv = make_double2(ov.x + cn.x - co.x, ov.y + cn.y - co.y);
-    same += tmp * (nv.x * nv.x + nv.y * nv.y);
-    same -= tmp * (ov.x * ov.x + ov.y * ov.y);
-    s_out[k.w] = nv;
-    const double2 xv = s_cross[k.w];
-    cross += tmp * (xv.x * (cn.x - co.x) + xv.y * (cn.y - co.y));
-  }
-  same = block_sum(same, sbuf);
-  cross = block_sum(cross, sbuf);
+  EwSums64 e;
+  ewald_columns(b, na, eik_s, blockIdx.x * blockDim.x + threadIdx.x, b.ncol, gridDim.x * blockDim.x, s_same, s_cross, s_out,
+                e);
+  const double same = block_sum(e.same, sbuf), cross = block_sum(e.cross, sbuf);
   if (threadIdx.x == 0) {
     part[2 * blockIdx.x] = same;
     part[2 * blockIdx.x + 1] = cross;
@@ -643,41 +593,32 @@ static grx_status ewald_delta_run(grx_box* b, const double* old_pos, const doubl
                                   const double* new_pos, const double* new_qs, size_t n_new, const double2* same,
                                   const double2* cross, double& s_same, double& s_cross) {
   s_same = s_cross = 0.0;
-  MoveAtoms mv{};
-  mv.n_old = (int)n_old;
-  mv.n_new = (int)n_new;
-  std::vector<double> op(3 * n_old), oq(n_old), np_(3 * n_new), nq(n_new);
-  if (n_old) {
-    GRX_CHECK_CUDA(cudaMemcpy(op.data(), old_pos, 3 * n_old * sizeof(double), cudaMemcpyDefault), "read old pos");
-    GRX_CHECK_CUDA(cudaMemcpy(oq.data(), old_qs, n_old * sizeof(double), cudaMemcpyDefault), "read old q");
-  }
-  if (n_new) {
-    GRX_CHECK_CUDA(cudaMemcpy(np_.data(), new_pos, 3 * n_new * sizeof(double), cudaMemcpyDefault), "read new pos");
-    GRX_CHECK_CUDA(cudaMemcpy(nq.data(), new_qs, n_new * sizeof(double), cudaMemcpyDefault), "read new q");
-  }
-  for (size_t a = 0; a < n_old; ++a) { mv.x[a] = op[3 * a]; mv.y[a] = op[3 * a + 1]; mv.z[a] = op[3 * a + 2]; mv.q[a] = oq[a]; }
-  for (size_t a = 0; a < n_new; ++a) {
-    mv.x[n_old + a] = np_[3 * a]; mv.y[n_old + a] = np_[3 * a + 1]; mv.z[n_old + a] = np_[3 * a + 2]; mv.q[n_old + a] = nq[a];
-  }
-  const int nblk = std::max(1, std::min((b->nact + GRX_THREADS - 1) / GRX_THREADS, sm_count(b)));
-  grx_status st = ensure_scratch(b, sizeof(MoveAtoms) + 2 * (size_t)nblk * sizeof(double) + 256);
+  const size_t na = n_old + n_new;
+  std::vector<double> pos(3 * na), q(na);
+  grx_status st = fetch(pos.data(), old_pos, 3 * n_old * sizeof(double), "read old pos");
+  if (!st) st = fetch(q.data(), old_qs, n_old * sizeof(double), "read old q");
+  if (!st) st = fetch(pos.data() + 3 * n_old, new_pos, 3 * n_new * sizeof(double), "read new pos");
+  if (!st) st = fetch(q.data() + n_old, new_qs, n_new * sizeof(double), "read new q");
   if (st) return st;
-  MoveAtoms* d_mv = (MoveAtoms*)b->scratch;
-  double* part = (double*)((char*)b->scratch + (sizeof(MoveAtoms) + 255) / 256 * 256);
-  GRX_CHECK_CUDA(cudaMemcpyAsync(d_mv, &mv, sizeof(MoveAtoms), cudaMemcpyHostToDevice, b->stream), "upload move");
   refresh_dev(b);
-  const int na = (int)(n_old + n_new);
-  const size_t smem = (size_t)(b->dev.kmax[0] + b->dev.kmax[1] + b->dev.kmax[2] + 3) * std::max(na, 1) * sizeof(double2);
-  std::vector<double> parts(2 * nblk, 0.0);
+  const int nblk = std::max(1, std::min((b->ncol + kDeltaThreads - 1) / kDeltaThreads, 2 * sm_count(b)));
+  st = ensure_pinned(b, (4 * na + 2 * (size_t)nblk) * sizeof(double));
+  if (st) return st;
+  double* at = (double*)b->pinned;
+  double* part = at + 4 * na;
+  for (size_t a = 0; a < na; ++a) {
+    for (int k = 0; k < 3; ++k) at[k * na + a] = pos[3 * a + k];
+    at[3 * na + a] = a < n_old ? -q[a] : q[a];
+  }
   if (b->nact > 0 && na > 0) {
-    ewald_delta_kernel<<<nblk, GRX_THREADS, smem, b->stream>>>(b->dev, d_mv, same, cross, b->s_tmp, part);
+    const size_t smem = (size_t)(b->dev.kmax[0] + b->dev.kmax[1] + b->dev.kmax[2] + 3) * na * sizeof(double2);
+    ewald_delta_kernel<<<nblk, kDeltaThreads, smem, b->stream>>>(b->dev, at, (int)na, same, cross, b->s_tmp, part);
     count_launch();
     GRX_CHECK_CUDA(cudaGetLastError(), "ewald delta launch");
-    GRX_CHECK_CUDA(cudaMemcpyAsync(parts.data(), part, 2 * nblk * sizeof(double), cudaMemcpyDeviceToHost, b->stream),
-                   "read ewald partials");
   }
   GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "ewald delta");
-  for (int k = 0; k < nblk; ++k) { s_same += parts[2 * k]; s_cross += parts[2 * k + 1]; }
+  if (b->nact > 0 && na > 0)
+    for (int k = 0; k < nblk; ++k) { s_same += part[2 * k]; s_cross += part[2 * k + 1]; }
   return GRX_OK;
 }
 
@@ -722,13 +663,14 @@ grx_status grx_ewald_delta_lambda(grx_box* b, int32_t comp, const double* pos, c
   out2[0] = out2[1] = 0.0;
   if (b->dev.no_charges && !b->has_charge[comp]) return GRX_OK;
   std::vector<double> hq(n), qo(n), qn(n);
-  GRX_CHECK_CUDA(cudaMemcpy(hq.data(), charge, n * sizeof(double), cudaMemcpyDefault), "read charges");
+  grx_status st = fetch(hq.data(), charge, n * sizeof(double), "read charges");
+  if (st) return st;
   for (size_t a = 0; a < n; ++a) {  // Fourier_Ewald_Diff_LambdaChange: the same atoms, old and new scaleCoul
     qo[a] = hq[a] * scale_coul_old;
     qn[a] = hq[a] * scale_coul_new;
   }
   double s_same = 0, s_cross = 0;
-  grx_status st = ewald_delta_run(b, pos, qo.data(), n, pos, qn.data(), n, use_staged ? b->s_tmp : b->s_ads, b->s_fw,
+  st = ewald_delta_run(b, pos, qo.data(), n, pos, qn.data(), n, use_staged ? b->s_tmp : b->s_ads, b->s_fw,
                                   s_same, s_cross);
   if (st) return st;
   // GPU_EwaldDifference_LambdaChange (:782-785): exclusion times the change of scaleCoul^2

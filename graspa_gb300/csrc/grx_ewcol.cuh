@@ -58,9 +58,9 @@ struct EwSumsDf { df a = {0.f, 0.f}, n = {0.f, 0.f}, c = {0.f, 0.f}; };  // A.dS
 
 __device__ __forceinline__ df df_neg(df a) { return {-a.hi, -a.lo}; }
 
-// FP64: same = sum temp (|S + dS|^2 - |S|^2), cross = sum temp Re(S_fw dS*), S + dS to s_out.
+// FP64: same = sum temp (|S + dS|^2 - |S|^2), cross = sum temp Re(S_cross dS*), S + dS to s_out.
 __device__ __forceinline__ void ewald_columns(const BoxDev& b, int na, const double2* tab, int first, int end, int stride,
-                                              double2* s_out, EwSums64& e) {
+                                              const double2* s_same, const double2* s_cross, double2* s_out, EwSums64& e) {
   const double2* ey = tab + (b.kmax[0] + 1) * na;
   const double2* ez = ey + (b.kmax[1] + 1) * na;
   for (int col = first; col < end; col += stride) {
@@ -84,7 +84,7 @@ __device__ __forceinline__ void ewald_columns(const BoxDev& b, int na, const dou
       const int slot = h ? c.w - az : c.w + az;
       const double2 ds = h ? make_double2(sa + sb, sd - sc) : make_double2(sa - sb, sc + sd);
       const double t = b.ktemp[j];
-      const double2 ov = b.s_ads[slot], xv = b.s_fw[slot];
+      const double2 ov = s_same[slot], xv = s_cross[slot];
       const double2 nv = make_double2(ov.x + ds.x, ov.y + ds.y);
       e.same += t * (nv.x * nv.x + nv.y * nv.y);
       e.same -= t * (ov.x * ov.x + ov.y * ov.y);

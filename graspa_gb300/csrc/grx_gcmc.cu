@@ -680,10 +680,21 @@ struct MolWrite {
 
 // Update_insertion_data_Parallel / update_translation_position (mc_utilities.h:191-234,
 // 285-292): one thread per atom writes every stored representation.
-__global__ void write_molecule_kernel(BoxDev b, int comp, int first, int ms, int mol, int grow, MolWrite m) {
+// Checks against the live count on the device, so the call needs no read back before its launch.
+// status (pinned host memory): {error, live atoms of every component after the call}; dry: check only.
+__global__ void write_molecule_kernel(BoxDev b, int comp, int off, int ms, long long mol, long long cap, int dry, MolWrite m,
+                                      int* status) {
   const int a = threadIdx.x;
-  if (a < ms) store_atom(b, first + a, m.x[a], m.y[a], m.z[a], m.q[a], 1.0, 1.0, m.type[a], mol);
-  if (grow && a == 0) const_cast<int*>(b.comp_size)[comp] += ms;
+  const int n = b.comp_size[comp];
+  const int err = mol > n / ms ? GRX_ERR_INVALID_ARG : ((mol + 1) * ms > cap ? GRX_ERR_CAPACITY : GRX_OK);
+  const bool grow = mol == n / ms;
+  __syncwarp();
+  if (!err && !dry) {
+    if (a < ms) store_atom(b, off + (int)mol * ms + a, m.x[a], m.y[a], m.z[a], m.q[a], 1.0, 1.0, m.type[a], (int)mol);
+    if (grow && a == 0) const_cast<int*>(b.comp_size)[comp] = n + ms;
+  }
+  if (a == 0) status[0] = err;
+  if (a < b.ncomp) status[1 + a] = a == comp ? (!err && !dry && grow ? n + ms : n) : b.comp_size[a];
 }
 
 // Update_deletion_data_Parallel (mc_utilities.h:163-189): the last molecule moves
@@ -702,34 +713,36 @@ extern "C" grx_status grx_box_write_molecule(grx_box* b, int32_t comp, size_t mo
   GRX_REQUIRE(comp >= b->nhost && comp < b->ncomp, "grx_box_write_molecule: not an adsorbate component");
   const size_t ms = b->molsize[comp];
   GRX_REQUIRE(ms >= 1 && ms <= (size_t)kMolWork, "grx_box_write_molecule: molecule size must be 1..32");
-  GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "write_molecule sync");
-  GRX_CHECK_CUDA(cudaMemcpy(b->size, b->d_size, GRX_MAX_COMPONENTS * sizeof(int), cudaMemcpyDeviceToHost),
-                 "read sizes");
-  const size_t n = (size_t)b->size[comp] / ms;
-  GRX_REQUIRE(mol <= n, "grx_box_write_molecule: molecule index beyond the count");
-  if ((mol + 1) * ms > b->cap[comp]) {
-    set_error("grx_box_write_molecule: component %d capacity %zu exhausted", comp, b->cap[comp]);
-    return GRX_ERR_CAPACITY;
-  }
   MolWrite m{};
+  bool types_ok = true;
   for (size_t a = 0; a < ms; ++a) {
     m.x[a] = pos[3 * a];
     m.y[a] = pos[3 * a + 1];
     m.z[a] = pos[3 * a + 2];
     m.q[a] = charge[a];
-    GRX_REQUIRE(type[a] < (size_t)b->dev.ntypes, "grx_box_write_molecule: atom type out of range");
+    types_ok = types_ok && type[a] < (size_t)b->dev.ntypes;
     m.type[a] = (int)type[a];
-    if (charge[a] != 0.0) b->has_charge[comp] = 1;
   }
   refresh_dev(b);
-  const int grow = mol == n ? 1 : 0;
-  write_molecule_kernel<<<1, 32, 0, b->stream>>>(b->dev, comp, (int)(b->off[comp] + mol * ms), (int)ms, (int)mol,
-                                                 grow, m);
+  grx_status st = ensure_pinned(b, (1 + GRX_MAX_COMPONENTS) * sizeof(int));
+  if (st) return st;
+  int* status = (int*)b->pinned;
+  const long long index = (long long)std::min<size_t>(mol, (size_t)1 << 40);
+  write_molecule_kernel<<<1, 32, 0, b->stream>>>(b->dev, comp, (int)b->off[comp], (int)ms, index, (long long)b->cap[comp],
+                                                 types_ok ? 0 : 1, m, status);
   count_launch();
   GRX_CHECK_CUDA(cudaGetLastError(), "write_molecule launch");
-  if (grow) b->size[comp] += (int)ms;
-  b->stored[comp] = std::max(b->stored[comp], (mol + 1) * ms);
   GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "write_molecule");
+  for (int c = 0; c < b->ncomp; ++c) b->size[c] = status[1 + c];
+  GRX_REQUIRE(status[0] != GRX_ERR_INVALID_ARG, "grx_box_write_molecule: molecule index beyond the count");
+  if (status[0] == GRX_ERR_CAPACITY) {
+    set_error("grx_box_write_molecule: component %d capacity %zu exhausted", comp, b->cap[comp]);
+    return GRX_ERR_CAPACITY;
+  }
+  GRX_REQUIRE(types_ok, "grx_box_write_molecule: atom type out of range");
+  for (size_t a = 0; a < ms; ++a)
+    if (charge[a] != 0.0) b->has_charge[comp] = 1;
+  b->stored[comp] = std::max(b->stored[comp], (mol + 1) * ms);
   return GRX_OK;
 }
 

@@ -121,6 +121,10 @@ namespace grx {
 grx_status ensure_scratch(grx_box* b, size_t bytes);
 grx_status ensure_pinned(grx_box* b, size_t bytes);
 grx_status ensure_results(grx_box* b, size_t n);
+// Between a caller's array and host memory of ours: plain host memory by memcpy, anything the
+// CUDA runtime knows (device, managed, pinned) through it.
+grx_status fetch(void* dst, const void* src, size_t bytes, const char* what);
+grx_status deliver(void* dst, const void* src, size_t bytes, const char* what);
 void refresh_dev(grx_box* b);
 int sm_count(grx_box* b);
 void* arena_alloc(grx_arena* a, size_t bytes);

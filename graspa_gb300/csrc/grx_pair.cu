@@ -3,6 +3,7 @@
 // trial_kernel (grx_warp.cuh); a move delta is two trials, the new molecule and the old one.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "grx_host.h"
@@ -16,35 +17,42 @@ static void host_split(double x, float& h, float& l) {
   l = (float)(x - hd);
 }
 
-static grx_status stage_beads(const grx_trials* t, size_t first_bead, size_t nbeads, double prefactor,
-                              std::vector<Bead>& out) {
-  const size_t nall = t->ntrials * t->chainsize;
-  std::vector<double> pos(3 * nall), sc(nall, 1.0), q(nall, 0.0), scc(nall, 1.0);
-  std::vector<size_t> ty(nall, 0);
-  if (nall) {
-    GRX_CHECK_CUDA(cudaMemcpy(pos.data(), t->pos, 3 * nall * sizeof(double), cudaMemcpyDefault), "read bead pos");
-    if (t->scale) GRX_CHECK_CUDA(cudaMemcpy(sc.data(), t->scale, nall * sizeof(double), cudaMemcpyDefault), "read bead scale");
-    if (t->charge) GRX_CHECK_CUDA(cudaMemcpy(q.data(), t->charge, nall * sizeof(double), cudaMemcpyDefault), "read bead charge");
-    if (t->scale_coul) GRX_CHECK_CUDA(cudaMemcpy(scc.data(), t->scale_coul, nall * sizeof(double), cudaMemcpyDefault), "read bead scaleCoul");
-    GRX_CHECK_CUDA(cudaMemcpy(ty.data(), t->type, nall * sizeof(size_t), cudaMemcpyDefault), "read bead type");
-  }
-  out.resize(nbeads);
-  for (size_t k = 0; k < nbeads; ++k) {
-    const size_t j = first_bead + k;
+// The caller's bead arrays [0, nall) on the host.
+struct HostBeads {
+  std::vector<double> pos, scale, charge, scale_coul;
+  std::vector<size_t> type;
+};
+
+static grx_status read_beads(const grx_trials* t, size_t nall, HostBeads& h) {
+  h.pos.resize(3 * nall);
+  h.scale.assign(nall, 1.0);
+  h.charge.assign(nall, 0.0);
+  h.scale_coul.assign(nall, 1.0);
+  h.type.resize(nall);
+  grx_status st = fetch(h.pos.data(), t->pos, 3 * nall * sizeof(double), "read bead pos");
+  if (!st && t->scale) st = fetch(h.scale.data(), t->scale, nall * sizeof(double), "read bead scale");
+  if (!st && t->charge) st = fetch(h.charge.data(), t->charge, nall * sizeof(double), "read bead charge");
+  if (!st && t->scale_coul) st = fetch(h.scale_coul.data(), t->scale_coul, nall * sizeof(double), "read bead scaleCoul");
+  if (!st) st = fetch(h.type.data(), t->type, nall * sizeof(size_t), "read bead type");
+  return st;
+}
+
+static void make_beads(const HostBeads& h, size_t first, size_t n, double prefactor, Bead* out) {
+  for (size_t k = 0; k < n; ++k) {
+    const size_t j = first + k;
     Bead& bd = out[k];
-    bd.x = pos[3 * j]; bd.y = pos[3 * j + 1]; bd.z = pos[3 * j + 2];
+    bd.x = h.pos[3 * j]; bd.y = h.pos[3 * j + 1]; bd.z = h.pos[3 * j + 2];
     host_split(bd.x, bd.h.x, bd.l.x);
     host_split(bd.y, bd.h.y, bd.l.y);
     host_split(bd.z, bd.h.z, bd.l.z);
-    bd.q = q[j] * scc[j];
-    bd.scale = sc[j];
-    bd.type = (int)ty[j];
+    bd.q = h.charge[j] * h.scale_coul[j];
+    bd.scale = h.scale[j];
+    bd.type = (int)h.type[j];
     const double pq = prefactor * bd.q;
     const float ph = (float)pq;
     bd.pq = make_float2(ph, (float)(pq - (double)ph));
     bd.unit = bead_unit(bd.scale, bd.h);
   }
-  return GRX_OK;
 }
 
 static void run_trials(grx_box* b, const TrialArgs& a, int ntrials, int prec) {
@@ -76,17 +84,18 @@ grx_status grx_trial_energies(grx_box* b, const grx_trials* t, int32_t component
   const size_t per_chunk = std::max<size_t>(1, GRX_MAX_TRIAL_BEADS / ch);
   std::vector<double> eo(4 * t->ntrials);
   std::vector<uint8_t> fo(t->ntrials);
+  HostBeads h;
+  grx_status st = read_beads(t, t->ntrials * ch, h);
+  if (st) return st;
   for (size_t t0 = 0; t0 < t->ntrials; t0 += per_chunk) {
     const size_t ntr = std::min(per_chunk, t->ntrials - t0);
     const int nb = (int)(ntr * ch);
-    std::vector<Bead> beads;
-    grx_status st = stage_beads(t, t0 * ch, nb, b->dev.prefactor, beads);
+    // the kernel reads the beads from and writes the sums to pinned host memory: one launch, no copies
+    const size_t bead_bytes = nb * sizeof(Bead);
+    st = ensure_pinned(b, bead_bytes + ntr * (4 * sizeof(double) + 1));
     if (st) return st;
-    const size_t bead_bytes = (nb * sizeof(Bead) + 255) / 256 * 256;
-    const size_t out_bytes = (ntr * 4 * sizeof(double) + 255) / 256 * 256;
-    st = ensure_scratch(b, bead_bytes + out_bytes + ntr);
-    if (st) return st;
-    char* base = (char*)b->scratch;
+    char* base = (char*)b->pinned;
+    make_beads(h, t0 * ch, nb, b->dev.prefactor, (Bead*)base);
     TrialArgs a{};
     a.beads = (Bead*)base;
     a.chain = (int)ch;
@@ -96,17 +105,16 @@ grx_status grx_trial_energies(grx_box* b, const grx_trials* t, int32_t component
     a.excl_comp = (int)exclude_comp;
     a.excl_mol = (int)exclude_molid;
     a.out = (double*)(base + bead_bytes);
-    a.over = (unsigned char*)(base + bead_bytes + out_bytes);
-    GRX_CHECK_CUDA(cudaMemcpyAsync(base, beads.data(), nb * sizeof(Bead), cudaMemcpyHostToDevice, b->stream), "upload beads");
+    a.over = (unsigned char*)(a.out + 4 * ntr);
     run_trials(b, a, (int)ntr, prec);
     GRX_CHECK_CUDA(cudaGetLastError(), "trial energy launch");
-    GRX_CHECK_CUDA(cudaMemcpyAsync(eo.data() + 4 * t0, a.out, ntr * 4 * sizeof(double), cudaMemcpyDeviceToHost, b->stream), "read energies");
-    GRX_CHECK_CUDA(cudaMemcpyAsync(fo.data() + t0, a.over, ntr, cudaMemcpyDeviceToHost, b->stream), "read flags");
     GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "trial energies");
+    std::memcpy(eo.data() + 4 * t0, a.out, ntr * 4 * sizeof(double));
+    std::memcpy(fo.data() + t0, a.over, ntr);
   }
-  GRX_CHECK_CUDA(cudaMemcpy(out, eo.data(), t->ntrials * sizeof(grx_trial_energy), cudaMemcpyDefault), "write energies");
-  GRX_CHECK_CUDA(cudaMemcpy(overlap, fo.data(), t->ntrials, cudaMemcpyDefault), "write flags");
-  return GRX_OK;
+  st = deliver(out, eo.data(), t->ntrials * sizeof(grx_trial_energy), "write energies");
+  if (!st) st = deliver(overlap, fo.data(), t->ntrials, "write flags");
+  return st;
 }
 
 grx_status grx_single_body_energy(grx_box* b, const grx_trials* old_mol, const grx_trials* new_mol,
@@ -119,18 +127,18 @@ grx_status grx_single_body_energy(grx_box* b, const grx_trials* old_mol, const g
               "grx_single_body_energy: molecule size out of range");
   GRX_REQUIRE(do_new || do_old, "grx_single_body_energy: nothing to do");
   refresh_dev(b);
-  std::vector<Bead> nb_, ob_;
-  grx_status st = stage_beads(new_mol, 0, ms, b->dev.prefactor, nb_);
+  HostBeads hn, ho;
+  grx_status st = read_beads(new_mol, ms, hn);
+  if (!st) st = read_beads(old_mol, ms, ho);
+  const size_t bead_bytes = 2 * ms * sizeof(Bead);
+  if (!st) st = ensure_pinned(b, bead_bytes + 8 * sizeof(double) + 8);
   if (st) return st;
-  st = stage_beads(old_mol, 0, ms, b->dev.prefactor, ob_);
-  if (st) return st;
-  nb_.insert(nb_.end(), ob_.begin(), ob_.end());
-  const size_t bead_bytes = (2 * ms * sizeof(Bead) + 255) / 256 * 256;
-  st = ensure_scratch(b, bead_bytes + 256);
-  if (st) return st;
+  Bead* beads = (Bead*)b->pinned;
+  make_beads(hn, 0, ms, b->dev.prefactor, beads);
+  make_beads(ho, 0, ms, b->dev.prefactor, beads + ms);
   // two trials: the new molecule and the old one, each without the atoms of its own molecule id
   TrialArgs a{};
-  a.beads = (Bead*)b->scratch;
+  a.beads = beads;
   a.chain = (int)ms;
   a.component = component;
   a.mol[0] = (int)new_mol->molid;
@@ -138,28 +146,26 @@ grx_status grx_single_body_energy(grx_box* b, const grx_trials* old_mol, const g
   a.split = 1;
   a.excl_comp = -1;
   a.excl_mol = -1;
-  a.out = (double*)((char*)b->scratch + bead_bytes);
+  a.out = (double*)((char*)b->pinned + bead_bytes);
   a.over = (unsigned char*)(a.out + 8);
-  GRX_CHECK_CUDA(cudaMemcpyAsync(b->scratch, nb_.data(), 2 * ms * sizeof(Bead), cudaMemcpyHostToDevice, b->stream), "upload beads");
   run_trials(b, a, 2, prec == GRX_MIXED ? kMixed64 : (int)prec);
   GRX_CHECK_CUDA(cudaGetLastError(), "single body launch");
-  struct { double e[8]; unsigned char over[8]; } r;
-  GRX_CHECK_CUDA(cudaMemcpyAsync(&r, a.out, sizeof(r), cudaMemcpyDeviceToHost, b->stream), "read energies");
   GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "single body");
+  const double* r = a.out;
   // HH / HG / GG by the atom's component and the moved one (mc_single_particle.h:142-170)
   double e[6] = {0, 0, 0, 0, 0, 0};
   const int host_slot = component < b->nhost ? 0 : 2;
   for (int q = 0; q < 4; ++q) {
     double d = 0.0;
-    if (do_new) d += r.e[q];
-    if (do_old) d -= r.e[4 + q];
+    if (do_new) d += r[q];
+    if (do_old) d -= r[4 + q];
     e[host_slot + q] = d;
   }
-  const int flag = do_new && r.over[0];
-  GRX_CHECK_CUDA(cudaMemcpy(out6, e, 6 * sizeof(double), cudaMemcpyDefault), "write energies");
-  uint8_t f8 = flag ? 1 : 0;
-  GRX_CHECK_CUDA(cudaMemcpy(overlap, &f8, 1, cudaMemcpyDefault), "write flag");
-  return GRX_OK;
+  const int flag = do_new && a.over[0];
+  st = deliver(out6, e, 6 * sizeof(double), "write energies");
+  const uint8_t f8 = flag ? 1 : 0;
+  if (!st) st = deliver(overlap, &f8, 1, "write flag");
+  return st;
 }
 
 }  // extern "C"

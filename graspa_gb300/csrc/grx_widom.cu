@@ -251,7 +251,7 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
       double same = 0.0, cross = 0.0;
       if constexpr (PREC == GRX_FP64) {
         EwSums64 e;
-        ewald_columns(b, ms, eik_s, tid, b.ncol, blockDim.x, nullptr, e);
+        ewald_columns(b, ms, eik_s, tid, b.ncol, blockDim.x, b.s_ads, b.s_fw, nullptr, e);
         same = block_sum(e.same, sbuf);
         cross = block_sum(e.cross, sbuf);
       } else {

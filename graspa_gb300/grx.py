@@ -250,11 +250,18 @@ def check(status, what=""):
 
 
 def _d(a):
-    return a.ctypes.data_as(_dp)
+    """Pointer to a C-contiguous float64 array (kept alive by the pointer)."""
+    try:
+        return C.pointer(C.c_double.from_buffer(a))
+    except (TypeError, ValueError):  # read-only or empty
+        return a.ctypes.data_as(_dp)
 
 
 def _sz(a):
-    return a.ctypes.data_as(_szp)
+    try:
+        return C.pointer(C.c_size_t.from_buffer(a))
+    except (TypeError, ValueError):
+        return a.ctypes.data_as(_szp)
 
 
 def geometry_from_system(system):
@@ -519,8 +526,7 @@ class Box:
         flag = np.zeros(ntrials, dtype=np.uint8)
         check(self.L.grx_trial_energies(self.h, C.byref(t), component, excl_comp, excl_molid, prec, out,
                                         flag.ctypes.data_as(_u8p)), "grx_trial_energies")
-        e = np.array([[o.hg_vdw, o.hg_real, o.gg_vdw, o.gg_real] for o in out])
-        return e, flag
+        return (np.frombuffer(out).reshape(ntrials, 4).copy() if ntrials else np.array([])), flag
 
     def trial_energies_noalloc(self, pos, charge, types, molid, ntrials, chainsize, component, prec=GRX_FP64,
                                excl_comp=-1, excl_molid=-1, scale=None, scale_coul=None):
@@ -537,8 +543,7 @@ class Box:
         st = self.L.grx_trial_energies_noalloc(self.h, C.byref(t), component, excl_comp, excl_molid, prec, out,
                                                flag.ctypes.data_as(_u8p))
         check(st, "grx_trial_energies_noalloc")
-        e = np.array([[o.hg_vdw, o.hg_real, o.gg_vdw, o.gg_real] for o in out])
-        return e, flag
+        return (np.frombuffer(out).reshape(ntrials, 4).copy() if ntrials else np.array([])), flag
 
     def single_body(self, old, new, component, do_new=1, do_old=1, prec=GRX_FP64):
         """old/new: dict(pos, charge, type, molid[, scale, scale_coul])."""
