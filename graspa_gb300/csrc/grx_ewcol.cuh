@@ -58,7 +58,7 @@ struct EwSumsDf { df a = {0.f, 0.f}, n = {0.f, 0.f}, c = {0.f, 0.f}; };  // A.dS
 
 __device__ __forceinline__ df df_neg(df a) { return {-a.hi, -a.lo}; }
 
-// FP64: same = sum temp (|S + dS|^2 - |S|^2), cross = sum temp Re(S_cross dS*), S + dS to s_out.
+// FP64: same = sum temp (|S + dS|^2 - |S|^2) = sum temp dS.(2 S + dS), cross = sum temp Re(S_cross dS*), S + dS to s_out.
 __device__ __forceinline__ void ewald_columns(const BoxDev& b, int na, const double2* tab, int first, int end, int stride,
                                               const double2* s_same, const double2* s_cross, double2* s_out, EwSums64& e) {
   const double2* ey = tab + (b.kmax[0] + 1) * na;
@@ -86,9 +86,9 @@ __device__ __forceinline__ void ewald_columns(const BoxDev& b, int na, const dou
       const double t = b.ktemp[j];
       const double2 ov = s_same[slot], xv = s_cross[slot];
       const double2 nv = make_double2(ov.x + ds.x, ov.y + ds.y);
-      e.same += t * (nv.x * nv.x + nv.y * nv.y);
-      e.same -= t * (ov.x * ov.x + ov.y * ov.y);
-      e.cross += t * (xv.x * ds.x + xv.y * ds.y);
+      // |S + dS|^2 - |S|^2 without the cancellation of the two squares
+      e.same = fma(t, fma(ds.x, ov.x + nv.x, ds.y * (ov.y + nv.y)), e.same);
+      e.cross = fma(t, fma(xv.x, ds.x, xv.y * ds.y), e.cross);
       if (s_out) s_out[slot] = nv;
     }
   }
