@@ -88,6 +88,18 @@ __device__ __forceinline__ bool pair_screen(const BoxDev& b, int i, const Bead& 
   return screen_hi<PREC>(b, HOST ? b.hrec[2 * i] : b.hi[i], bd);
 }
 
+// 32 read-only bytes in one load. The gathers of the pair evaluation go to a different line for
+// most lanes, so their cost is line lookups, one per lane and load: a record or table piece of
+// two float4 in one 256-bit load takes half of them.
+__device__ __forceinline__ void load32(const float4* p, float4& a, float4& c) {
+  unsigned long long q0, q1, q2, q3;
+  asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(q0), "=l"(q1), "=l"(q2), "=l"(q3) : "l"(p));
+  a = make_float4(__uint_as_float((unsigned)q0), __uint_as_float((unsigned)(q0 >> 32)), __uint_as_float((unsigned)q1),
+                  __uint_as_float((unsigned)(q1 >> 32)));
+  c = make_float4(__uint_as_float((unsigned)q2), __uint_as_float((unsigned)(q2 >> 32)), __uint_as_float((unsigned)q3),
+                  __uint_as_float((unsigned)(q3 >> 32)));
+}
+
 // ---------------------------------------------------------------- FP64 pairs
 // An SM retires two FP64 lanes per clock, so a warp's FP64 instruction takes 16 cycles of the
 // SM and the FP64 form is bound by how many a pair needs. Images come from FP32 fractions and
@@ -164,8 +176,8 @@ __device__ __forceinline__ df lj_df(const BoxDev& b, int row, df rr) {
 // batch of 456 chains x 50 steps, with the accumulation below: 7.13 -> 6.77 ms, 20,000 Widom
 // insertions 6.61 -> 5.85 ms.
 __device__ __forceinline__ df coul_table_df(const BoxDev& b, int k, df s) {
-  const float4* c = b.ctabf + 2 * k;
-  const float4 c0 = __ldg(c), c1 = __ldg(c + 1);
+  float4 c0, c1;
+  load32(b.ctabf + 2 * k, c0, c1);
   const int bits = __float_as_int(s.hi);
   const float inv = __int_as_float((260 << 23) - (bits & 0x7f800000));  // 64 / 2^exponent
   const float t = __fmul_rn(__fsub_rn(s.hi, __int_as_float(bits & ~0x1ffff)), inv), tl = __fmul_rn(s.lo, inv);
@@ -338,9 +350,8 @@ __device__ __forceinline__ void pair_dense(const BoxDev& b, bool host, int i, co
     bool sc1;  // the atom's scale is 1
     float2 qa;
     if (host) {
-      ah = b.hrec[2 * i];
-      al = b.hrec[2 * i + 1];
-      const unsigned t = b.htype[i];
+      load32(b.hrec + 2 * i, ah, al);
+      const unsigned t = __ldg(b.htype + i);
       ty = (int)(t & 0x7fffu);
       sc1 = !(t & 0x8000u);
       qa = make_float2(ah.w, al.w);
