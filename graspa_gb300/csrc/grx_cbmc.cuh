@@ -46,7 +46,7 @@ struct CbmcWork {
   int qbuf[NW * kQueue];
   double te[kMaxTrials * 4];
   int tflag[kMaxTrials];
-  double sel_ws[kMaxTrials], sel_wa[kMaxTrials];
+  double sel_wa[kMaxTrials];
   // moved atoms of the Ewald delta: [0, n_old) leave (charge stored negated),
   // [n_old, n_old + n_new) arrive
   double mx[2 * kMolWork], my[2 * kMolWork], mz[2 * kMolWork], mq[2 * kMolWork];
@@ -215,79 +215,22 @@ __device__ __noinline__ void trial_pass_excl(const BoxDev& b, WK& W, int nb, int
 // Insertion: log-sum-exp selection with the uniform u (SelectTrialPosition) and the
 // 1e-150 failure test. Retrace (deletion): the first trial without overlap is the
 // existing configuration and no selection is drawn. `stored` is added to the sum
-// before averaging (the reinsertion retrace's StoredR, mc_widom.h:363-366). Exponentials are evaluated one
-// trial per lane; sums and the cumulative search stay sequential in trial order.
+// before averaging (the reinsertion retrace's StoredR, mc_widom.h:363-366).
 template <class WK>
 __device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, double u, double navg,
                                             bool retrace, double stored = 0.0) {
   if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    double lw[2];
-    bool ok[2];
-    double mx = -INFINITY;
-    int cnt = 0;
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int t = lane + 32 * r;
-      ok[r] = t < nt && !W.tflag[t];
-      lw[r] = -INFINITY;
-      if (ok[r]) {
-        double tot = W.te[4 * t] + W.te[4 * t + 2];
-        if (bias) tot += W.te[4 * t + 1] + W.te[4 * t + 3];
-        lw[r] = __dmul_rn(-beta, tot);
-        mx = fmax(mx, lw[r]);
-        ++cnt;
-      }
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    }
-#pragma unroll 1
-    for (int r = 0; r < 2; ++r) {
-      const int t = lane + 32 * r;
-      if (t < nt) {
-        W.sel_ws[t] = ok[r] ? exp_move(__dsub_rn(lw[r], mx)) : 0.0;
-        W.sel_wa[t] = ok[r] ? exp_move(lw[r]) : 0.0;
-      }
-    }
-    __syncwarp();
-    if (lane == 0) {
-      W.nok = cnt;
+    const StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u, retrace, W.sel_wa);
+    if (threadIdx.x == 0) {
+      W.nok = c.nok;
       W.ok = 0;
-      if (cnt > 0) {
-        int s = -1;
-        if (retrace) {
-#pragma unroll 1
-          for (int t = 0; t < nt; ++t)
-            if (!W.tflag[t]) { s = t; break; }
-        } else {
-          double sum = 0.0;
-#pragma unroll 1
-          for (int t = 0; t < nt; ++t)
-            if (!W.tflag[t]) sum += W.sel_ws[t];
-          const double wsel = u * sum;
-          int left = cnt;
-          double cum = 0.0;
-#pragma unroll 1
-          for (int t = 0; t < nt; ++t) {
-            if (W.tflag[t]) continue;
-            cum += W.sel_ws[t];
-            s = t;
-            --left;
-            if (!(cum < wsel) || left == 0) break;
-          }
-        }
-        double w = 0.0;
-#pragma unroll 1
-        for (int t = 0; t < nt; ++t)
-          if (!W.tflag[t]) w += W.sel_wa[t];
-        W.wraw = w;
-        if (retrace || !(w < 1e-150)) {
-          double avg = (w + stored) / navg;
-          if (!bias) avg *= exp_move(-beta * (W.te[4 * s + 1] + W.te[4 * s + 3]));
+      if (c.nok > 0) {
+        W.wraw = c.w;
+        if (retrace || !(c.w < 1e-150)) {
+          double avg = (c.w + stored) / navg;
+          if (!bias) avg *= exp_move(-beta * (W.te[4 * c.sel + 1] + W.te[4 * c.sel + 3]));
           W.ok = 1;
-          W.sel = s;
+          W.sel = c.sel;
           W.w = avg;
         }
       }

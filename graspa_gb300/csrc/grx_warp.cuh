@@ -11,6 +11,8 @@
 // order of every sum is fixed by the ballot order, so results are deterministic.
 #pragma once
 
+#include <limits.h>
+
 #include "grx_internal.cuh"
 #include "grx_df.cuh"
 
@@ -628,7 +630,7 @@ __device__ __forceinline__ double warp_sum(double x) {
   return x;
 }
 
-// Out of line: called once per work item and per Ewald delta, so one copy serves them all.
+// Out of line: called once per Ewald delta, so one copy serves them all.
 static __device__ __noinline__ float2 warp_sum_df_out(float hi, float lo) {
   df x = {hi, lo};
   for (int o = 16; o > 0; o >>= 1) {
@@ -643,33 +645,141 @@ __device__ __forceinline__ df warp_sum_df(df x) {
   return df{r.x, r.y};
 }
 
+__device__ __forceinline__ df lane_add(df a, df b) { return df_add(a, b); }
+__device__ __forceinline__ double lane_add(double a, double b) { return a + b; }
+__device__ __forceinline__ df lane_xor(df x, int o) {
+  return {__shfl_xor_sync(kFull, x.hi, o), __shfl_xor_sync(kFull, x.lo, o)};
+}
+__device__ __forceinline__ double lane_xor(double x, int o) { return __shfl_xor_sync(kFull, x, o); }
+
+// One exchange of a transposed sum: lanes with bit `o` clear keep a, the others b, and each
+// receives its partner's share of what it keeps.
+template <class T>
+__device__ __forceinline__ T lane_fold(T a, T b, int o) {
+  const bool up = (threadIdx.x & o) != 0;
+  const T keep = up ? b : a, send = up ? a : b;
+  return lane_add(keep, lane_xor(send, o));
+}
+
+// Warp sums of a work item's four accumulators: host vdw and real on lanes 0 and 16, guest vdw
+// and real on lanes 8 and 24. Folding two sums into one register per exchange takes 7 additions
+// (5 without guests) where four separate trees take 20. Out of line: one copy per form.
+template <class T>
+static __device__ __noinline__ T item_sums(T hv, T hr, T gv, T gr, bool guests) {
+  T x = lane_fold(hv, hr, 16);
+  if (guests) x = lane_fold(x, lane_fold(gv, gr, 16), 8);
+  else x = lane_add(x, lane_xor(x, 8));
+  for (int o = 4; o > 0; o >>= 1) x = lane_add(x, lane_xor(x, o));
+  return x;
+}
+
+// The sums of one work item into its slot {hg_vdw, hg_real, gg_vdw, gg_real}. The mixed and FP64
+// forms accumulate sum q_atom * g(r); the bead factor prefactor * q_bead is applied here, once.
 template <int PREC>
 __device__ __forceinline__ void warp_store(const LaneAcc<PREC>& h, const LaneAcc<PREC>& g, double* out4, df pq,
                                            double pq64, bool with_guests) {
   const int lane = threadIdx.x & 31;
-  if constexpr (PREC == GRX_MIXED) {
-    // the mixed form accumulates sum q_atom * g(r); the bead factor prefactor*q_bead
-    // is applied here, once
-    const df a = warp_sum_df(h.v), c = warp_sum_df(h.r);
-    df d = {0.f, 0.f}, e = {0.f, 0.f};
-    if (with_guests) { d = warp_sum_df(g.v); e = warp_sum_df(g.r); }
-    if (lane == 0) {  // stored as float pairs in the 8-byte slots (item_get converts)
-      float2* o = reinterpret_cast<float2*>(out4);
-      const df cq = df_mul(c, pq), eq = df_mul(e, pq);
-      o[0] = make_float2(a.hi, a.lo);
-      o[1] = make_float2(cq.hi, cq.lo);
-      o[2] = make_float2(d.hi, d.lo);
-      o[3] = make_float2(eq.hi, eq.lo);
-    }
+  const bool real = lane >= 16, guest = (lane & 8) != 0;
+  const auto x = item_sums(h.v, h.r, g.v, g.r, with_guests);
+  if ((lane & 7) != 0) return;
+  const int k = (real ? 1 : 0) + (guest ? 2 : 0);
+  if constexpr (PREC == GRX_MIXED) {  // stored as float pairs in the 8-byte slots (item_get converts)
+    const df v = real ? df_mul(x, pq) : x;
+    reinterpret_cast<float2*>(out4)[k] = guest && !with_guests ? make_float2(0.f, 0.f) : make_float2(v.hi, v.lo);
   } else {
-    const double a = warp_sum(h.v), c = warp_sum(h.r);
-    double d = 0.0, e = 0.0;
-    if (with_guests) { d = warp_sum(g.v); e = warp_sum(g.r); }
-    if (lane == 0) {
-      const double f = PREC == GRX_FP64 || PREC == kMixed64 ? pq64 : 1.0;  // FP64 real parts: sums of q_atom g
-      out4[0] = a; out4[1] = c * f; out4[2] = d; out4[3] = e * f;
+    const double f = real && (PREC == GRX_FP64 || PREC == kMixed64) ? pq64 : 1.0;
+    out4[k] = guest && !with_guests ? 0.0 : x * f;
+  }
+}
+
+// ---------------------------------------------------------------- Rosenbluth step
+// Selection and weight of one CBMC step over nt <= 64 trials by one warp (SelectTrialPosition,
+// mc_widom.h:14-39, and the sums of CBMC_FirstBead_Finish, :330-376): the trial without overlap
+// that the uniform u picks from the shifted weights (with `retrace` the first one), the number of
+// trials without overlap and the unshifted weight sum; wa[t] is trial t's weight. Every trial is
+// two lanes' worth at most, the cumulative sum a warp scan and the unshifted weights the shifted
+// ones times exp(max), so a step is one exp and five additions deep; a serial walk over the trials
+// took two exps and three additions per trial, each a full FP64 latency on one lane.
+struct StepChoice {
+  int sel, nok;
+  double w;
+};
+
+static __device__ __noinline__ StepChoice choose_trial(const double* te, const int* tflag, int nt, double beta, int bias,
+                                                       double u, bool retrace, double* wa) {
+  const int lane = threadIdx.x & 31;
+  double lw[2], e[2] = {0.0, 0.0};
+  bool ok[2];
+  // order-preserving words: an integer maximum instead of FP64 comparisons
+  long long top = LLONG_MIN;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int t = lane + 32 * r;
+    ok[r] = t < nt && !tflag[t];
+    lw[r] = 0.0;
+    if (ok[r]) {
+      double tot = te[4 * t] + te[4 * t + 2];
+      if (bias) tot += te[4 * t + 1] + te[4 * t + 3];
+      lw[r] = __dmul_rn(-beta, tot);
+      const long long w = __double_as_longlong(lw[r]);
+      top = max(top, w ^ ((w >> 63) & 0x7fffffffffffffffll));
     }
   }
+  const unsigned ok0 = __ballot_sync(kFull, ok[0]), ok1 = __ballot_sync(kFull, ok[1]);
+  StepChoice c;
+  c.nok = __popc(ok0) + __popc(ok1);
+  c.sel = -1;
+  c.w = 0.0;
+  if (c.nok == 0) {
+    for (int t = lane; t < nt; t += 32) wa[t] = 0.0;
+    __syncwarp();
+    return c;
+  }
+  for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(kFull, top, o));
+  const double mx = __longlong_as_double(top ^ ((top >> 63) & 0x7fffffffffffffffll));
+  double scale;
+  if (nt < 32) {  // the last lane is free for exp(max)
+    const double x = exp_move(lane == 31 ? mx : (ok[0] ? __dsub_rn(lw[0], mx) : 0.0));
+    scale = __shfl_sync(kFull, x, 31);
+    e[0] = ok[0] ? x : 0.0;
+  } else {
+    scale = exp_move(mx);
+#pragma unroll 1
+    for (int r = 0; r < 2; ++r) {
+      const double x = exp_move(ok[r] ? __dsub_rn(lw[r], mx) : 0.0);
+      e[r] = ok[r] ? x : 0.0;
+    }
+  }
+  double c0 = e[0], c1 = 0.0;
+  for (int o = 1; o < 32; o <<= 1) {
+    const double v = __shfl_up_sync(kFull, c0, o);
+    if (lane >= o) c0 += v;
+  }
+  double sum = __shfl_sync(kFull, c0, 31);
+  if (nt > 32) {
+    c1 = e[1];
+    for (int o = 1; o < 32; o <<= 1) {
+      const double v = __shfl_up_sync(kFull, c1, o);
+      if (lane >= o) c1 += v;
+    }
+    c1 += sum;
+    sum = __shfl_sync(kFull, c1, 31);
+  }
+  const double wsel = u * sum;
+  const unsigned m0 = __ballot_sync(kFull, ok[0] && (retrace || !(c0 < wsel))),
+                 m1 = __ballot_sync(kFull, ok[1] && (retrace || !(c1 < wsel)));
+  if (m0) c.sel = __ffs(m0) - 1;
+  else if (m1) c.sel = 31 + __ffs(m1);
+  else c.sel = ok1 ? 63 - __clz(ok1) : 31 - __clz(ok0);  // rounding left the sum below u * sum: the last one
+  const bool finite = scale < INFINITY;  // weights beyond the range of exp: one by one
+#pragma unroll 1
+  for (int r = 0; r < 2; ++r) {
+    const int t = lane + 32 * r;
+    if (t < nt) wa[t] = finite ? scale * e[r] : (ok[r] ? exp_move(lw[r]) : 0.0);
+  }
+  c.w = mx > -INFINITY || mx != mx ? scale * sum : 0.0;  // every energy +inf: no weight
+  __syncwarp();
+  return c;
 }
 
 // Live adsorbate atoms of the box, and the 32-atom work units a bead pass covers

@@ -42,65 +42,15 @@ struct WidomArgs {
   uint32_t stream;
 };
 
-// Log-sum-exp selection and weight of one CBMC step (SelectTrialPosition,
-// mc_widom.h:14-39, and CBMC_FirstBead_Finish :330-376, insertion branch), computed by
-// warp 0: the exponentials are evaluated one trial per lane, the sums and the cumulative
-// search stay sequential in trial order on lane 0, as in the reference's host loop.
-// Results are valid on lane 0.
+// Weight of one CBMC step by one warp (insertion branch); true when a trial was chosen.
 __device__ bool select_trial_warp(const double* te, const int* tflag, int nt, double beta, int bias,
-                                  double u, double navg, int& sel, double& wavg, int& nok, double* ws,
-                                  double* wa) {
-  const int lane = threadIdx.x & 31;
-  double lw[2];
-  bool ok[2];
-  double mx = -INFINITY;
-  int cnt = 0;
-  for (int r = 0; r < 2; ++r) {
-    const int t = lane + 32 * r;
-    ok[r] = t < nt && !tflag[t];
-    lw[r] = -INFINITY;
-    if (ok[r]) {
-      double tot = te[4 * t] + te[4 * t + 2];
-      if (bias) tot += te[4 * t + 1] + te[4 * t + 3];
-      lw[r] = __dmul_rn(-beta, tot);
-      mx = fmax(mx, lw[r]);
-      ++cnt;
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) {
-    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-  }
-  for (int r = 0; r < 2; ++r) {
-    const int t = lane + 32 * r;
-    if (t < nt) {
-      ws[t] = ok[r] ? exp(__dsub_rn(lw[r], mx)) : 0.0;
-      wa[t] = ok[r] ? exp(lw[r]) : 0.0;
-    }
-  }
-  __syncwarp();
-  nok = cnt;
-  if (lane != 0 || cnt == 0) return false;
-  double sum = 0.0;
-  for (int t = 0; t < nt; ++t)
-    if (!tflag[t]) sum += ws[t];
-  const double wsel = u * sum;
-  int s = -1, left = cnt;
-  double cum = 0.0;
-  for (int t = 0; t < nt; ++t) {
-    if (tflag[t]) continue;
-    cum += ws[t];
-    s = t;
-    --left;
-    if (!(cum < wsel) || left == 0) break;
-  }
-  double w = 0.0;
-  for (int t = 0; t < nt; ++t)
-    if (!tflag[t]) w += wa[t];
-  if (w < 1e-150) return false;
-  sel = s;
-  double avg = w / navg;
-  if (!bias) avg *= exp(-beta * (te[4 * s + 1] + te[4 * s + 3]));
+                                  double u, double navg, int& sel, double& wavg, int& nok, double* wa) {
+  const StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false, wa);
+  nok = c.nok;
+  if ((threadIdx.x & 31) != 0 || c.nok == 0 || c.w < 1e-150) return false;
+  sel = c.sel;
+  double avg = c.w / navg;
+  if (!bias) avg *= exp(-beta * (te[4 * c.sel + 1] + te[4 * c.sel + 3]));
   wavg = avg;
   return true;
 }
@@ -142,7 +92,7 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
   __shared__ double newx[GRX_MAX_MOLSIZE], newy[GRX_MAX_MOLSIZE], newz[GRX_MAX_MOLSIZE], newq[GRX_MAX_MOLSIZE];
   __shared__ grx_widom_result res;
   __shared__ int s_ok;
-  __shared__ double sel_ws[kMaxTrials], sel_wa[kMaxTrials];
+  __shared__ double sel_wa[kMaxTrials];
   extern __shared__ double2 eik_s[];
 
   const int tid = threadIdx.x;
@@ -184,7 +134,7 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
       int sel = -1, nok = 0;
       double w = 0.0;
       const bool ok = select_trial_warp(te, tflag, nt, a.beta, b.vdw_real_bias, u01(selw[0]), (double)nt, sel, w,
-                                        nok, sel_ws, sel_wa);
+                                        nok, sel_wa);
       if (tid == 0) res.n_ok_first = nok;
       if (ok && w > 1e-150) {
         s_ok = 1;
@@ -226,7 +176,7 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
         int sel = -1, nok = 0;
         double w = 0.0;
         const bool ok = select_trial_warp(te, tflag, no, a.beta, b.vdw_real_bias, u01(selw[1]), (double)no, sel, w,
-                                          nok, sel_ws, sel_wa);
+                                          nok, sel_wa);
         if (tid == 0) res.n_ok_orient = nok;
         if (tid == 0 && ok) {
           res.sel_orient = sel;
