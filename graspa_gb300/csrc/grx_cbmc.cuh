@@ -54,6 +54,7 @@ struct CbmcWork {
   double ewx[8][2];  // per-CTA Fourier partials {same, cross} of a cluster
   double wsum[2][NW];
   int counter;
+  int staged;             // s_tmp holds the dS of a charged move: 1 not committed, 2 committed (0: none yet)
   long long cfg;    // trial configurations evaluated since the caller last cleared it
   long long cbeads; // their beads
   int ok;       // step constructed
@@ -244,8 +245,8 @@ __device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, d
 // dS(k) = sum q e^{ik.r}; same = sum temp (|S + dS|^2 - |S|^2), cross = sum temp
 // Re(S_cross dS*), S_same = adsorbate block (guest moves), by columns of k (grx_ewcol.cuh). The
 // FP64 form keeps the reference arithmetic; the other forms evaluate dS and both sums in
-// double-float on the FP32 pipe against temp*S tables (ewA, ewF). When s_out is
-// given, S_same + dS is staged there (FP64) for a later commit. Results on thread 0.
+// double-float on the FP32 pipe against temp*S tables (ewA, ewF). In s_out (by slot) the FP64
+// form stages S_same + dS, the others dS as float pairs, for a later commit. Results on thread 0.
 // With CL > 1 each CTA of the cluster takes a contiguous range of the columns; the CTAs' partial
 // sums are exchanged through distributed shared memory and added in rank order by every CTA, and
 // the cluster barriers before a commit publish the staged S.
@@ -285,7 +286,8 @@ __device__ __noinline__ void ewald_move(const BoxDev& b, WK& W, int na, double2*
       __syncthreads();
     }
     EwSumsDf e;
-    ewald_columns<ROWS>(b, na, fx, rxy, c0 + tid, c1, blockDim.x, s_out, e);
+    ewald_columns<ROWS>(b, na, fx, rxy, c0 + tid, c1, blockDim.x, reinterpret_cast<float4*>(s_out), e);
+    if (tid == 0) W.staged = 1;
     df sm = ew_same(e), cr = e.c;
     sm = warp_sum_df(sm);
     cr = warp_sum_df(cr);
@@ -312,22 +314,44 @@ __device__ __noinline__ void ewald_move(const BoxDev& b, WK& W, int na, double2*
   __syncthreads();
 }
 
+// S + dS of one slot from a staged dS (FP64).
+__device__ __forceinline__ double2 staged_sum(double2 v, float4 d) {
+  return make_double2(v.x + (wide(d.x) + wide(d.y)), v.y + (wide(d.z) + wide(d.w)));
+}
+
 // Make the staged structure factor current and refresh its double-float table (in a
-// cluster, the CTA's own range of k).
-template <int CL = 1>
-__device__ __noinline__ void commit_sk(const BoxDev& b, const double2* s_tmp) {
+// cluster, the CTA's own range of k). staged: the workspace's mark of a staged dS.
+template <int PREC, int CL = 1>
+__device__ __noinline__ void commit_sk(const BoxDev& b, const double2* s_tmp, int* staged) {
   float4* ewA = const_cast<float4*>(b.ewA);
   int k0 = 0, k1 = b.nact;
   if constexpr (CL > 1) cluster_k_range(b.nact, CL, cluster_rank(), k0, k1);
   for (int j = k0 + threadIdx.x; j < k1; j += blockDim.x) {
     const int slot = b.kact[j].w;
-    const double2 v = s_tmp[slot];
+    double2 v;
+    if constexpr (PREC == GRX_FP64) v = s_tmp[slot];
+    else v = staged_sum(b.s_ads[slot], reinterpret_cast<const float4*>(s_tmp)[slot]);
     b.s_ads[slot] = v;
     const double t = b.ktemp[j];
     const df ar = df_from(t * v.x), ai = df_from(t * v.y);
     ewA[j] = make_float4(ar.hi, ar.lo, ai.hi, ai.lo);
   }
+  if (threadIdx.x == 0) *staged = 2;
   __syncthreads();
+}
+
+// After the last step: the staged vector as the box's callers know it, S of the last move evaluated
+// (its S + dS when it was rejected). Called with the block (in a cluster, the cluster) synchronised.
+template <int PREC, int CL>
+__device__ __forceinline__ void settle_staged(const BoxDev& b, int staged) {
+  if (PREC == GRX_FP64 || staged == 0) return;
+  int k0 = 0, k1 = b.nact;
+  if constexpr (CL > 1) cluster_k_range(b.nact, CL, cluster_rank(), k0, k1);
+  for (int j = k0 + threadIdx.x; j < k1; j += blockDim.x) {
+    const int slot = b.kact[j].w;
+    const double2 v = b.s_ads[slot];
+    b.s_tmp[slot] = staged == 2 ? v : staged_sum(v, reinterpret_cast<const float4*>(b.s_tmp)[slot]);
+  }
 }
 
 // Write one atom into the box storage (all representations).

@@ -25,6 +25,13 @@ __device__ __forceinline__ df df_from(double x) {
 
 __device__ __forceinline__ double df_to(df a) { return (double)a.hi + (double)a.lo; }
 
+// A float as a double by its bits (the conversion instruction issues at the FP64 rate).
+__device__ __forceinline__ double wide(float x) {
+  const unsigned b = __float_as_uint(x);
+  if ((b & 0x7f800000u) - 0x00800000u >= 0x7f000000u) return (double)x;  // zero, below normal, inf, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
 __device__ __forceinline__ df fast_two_sum(float a, float b) {  // |a| >= |b|
   const float s = __fadd_rn(a, b);
   const float e = __fsub_rn(b, __fsub_rn(s, a));

@@ -94,11 +94,12 @@ __device__ __forceinline__ void ewald_columns(const BoxDev& b, int na, const dou
   }
 }
 
-// Double-float: the sums against the temp * S tables (ewA, ewF, ewT); S + dS (FP64, compensated) to
-// s_out. rows: the (kx, ky) products of ROWS.
+// Double-float: the sums against the temp * S tables (ewA, ewF, ewT); dS as a float pair per part to
+// ds_out by slot (only an accepted move needs S + dS, and its FP64 additions cost as much as all
+// the rest of a k). rows: the (kx, ky) products of ROWS.
 template <bool ROWS>
 __device__ __forceinline__ void ewald_columns(const BoxDev& b, int na, const float4* tab, const float4* rows, int first,
-                                              int end, int stride, double2* s_out, EwSumsDf& e) {
+                                              int end, int stride, float4* ds_out, EwSumsDf& e) {
   const float4* fy = tab + (b.kmax[0] + 1) * na;
   const float4* fz = fy + (b.kmax[1] + 1) * na;
   for (int col = first; col < end; col += stride) {
@@ -144,11 +145,7 @@ __device__ __forceinline__ void ewald_columns(const BoxDev& b, int na, const flo
       df_mac(e.n, df{T.x, T.y}, n2);
       df_mac(e.c, df{F.x, F.y}, re);
       df_mac(e.c, df{F.z, F.w}, im);
-      if (s_out) {
-        const int slot = h ? c.w - az : c.w + az;
-        const double2 ov = b.s_ads[slot];
-        s_out[slot] = make_double2(ov.x + df_to(re), ov.y + df_to(im));
-      }
+      if (ds_out) ds_out[h ? c.w - az : c.w + az] = make_float4(re.hi, re.lo, im.hi, im.lo);
     }
   }
 }

@@ -248,7 +248,7 @@ __device__ __noinline__ void identity_swap_step(const BoxDev& b, const GcmcArgs*
       } else if (tid < msn) {  // same species: the new configuration replaces the old one
         store_position(b, o0 + tid, W.mx[mso + tid], W.my[mso + tid], W.mz[mso + tid]);
       }
-      if (charged) commit_sk<CL>(b, b.s_tmp);
+      if (charged) commit_sk<PREC, CL>(b, b.s_tmp, &W.staged);
       if (tid == 0) {
         ST[eo].identity_out[1]++;
         ST[en].identity_in[1]++;
@@ -293,6 +293,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
     b = boxes[box];
     W.cfg = 0;
     W.cbeads = 0;
+    W.staged = 0;
   }
   if (tid < nm) {
     A[tid] = args[e0 + tid];
@@ -371,7 +372,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
       if constexpr (CL > 1) cluster_sync_all();  // every CTA past its reads of this move
       if (s_accept) {
         if (tid < ms) store_position(b, m0 + tid, W.mx[ms + tid], W.my[ms + tid], W.mz[ms + tid]);
-        if (a.charged) commit_sk<CL>(b, b.s_tmp);
+        if (a.charged) commit_sk<PREC, CL>(b, b.s_tmp, &W.staged);
         if (tid == 0) {
           st.accepted[kind]++;
           st.energy[0] += s_dE[0]; st.energy[1] += s_dE[1]; st.energy[2] += s_dE[2];
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
       if constexpr (CL > 1) cluster_sync_all();  // every CTA past its reads of this move
       if (s_accept) {
         if (tid < ms) store_position(b, m0 + tid, W.mx[ms + tid], W.my[ms + tid], W.mz[ms + tid]);
-        if (a.charged) commit_sk<CL>(b, b.s_tmp);
+        if (a.charged) commit_sk<PREC, CL>(b, b.s_tmp, &W.staged);
         if (tid == 0) {
           st.accepted[4]++;
           st.energy[0] += s_dE[0]; st.energy[1] += s_dE[1]; st.energy[2] += s_dE[2];
@@ -575,7 +576,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
           __syncthreads();
           if (tid == 0) comp_size[comp] = (N - 1) * ms;
         }
-        if (a.charged) commit_sk<CL>(b, b.s_tmp);
+        if (a.charged) commit_sk<PREC, CL>(b, b.s_tmp, &W.staged);
         if (tid == 0) {
           st.accepted[kind]++;
           st.energy[0] += s_dE[0]; st.energy[1] += s_dE[1]; st.energy[2] += s_dE[2];
@@ -597,6 +598,8 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
     }
     __syncthreads();
   }
+  if constexpr (CL > 1) cluster_sync_all();  // every CTA's staged parts
+  settle_staged<PREC, CL>(b, W.staged);
   if (tid < nm && (CL == 1 || cluster_rank() == 0)) {  // accumulate into the caller's running statistics
     grx_gcmc_stats& o = stats[e0 + tid];
     for (int k = 0; k < 5; ++k) {
