@@ -86,7 +86,7 @@ struct BoxDev {
   const int4* vmeta;     // per voxel {first entry, sure atoms, all atoms, 0}
   const unsigned* vlist; // entries: storage index | lattice shift << 20
   const float4* vshift;  // lattice vector of every shift code, hi parts
-  int vox;
+  int vox;               // 0 tile path, 1 entries carry their image, 2 images by rounded fractions
   int vn[3];             // voxels along a, b, c
   int vchunks;           // 32-entry chunks of the longest list
   int cull;              // tile culling on

@@ -13,6 +13,12 @@
 // box's 32-atom tiles; the dense evaluation still applies the exact cutoff tests, so the
 // lists change which pairs are screened, never which pairs count.
 //
+// A cell narrower than 2 r_list (or host atoms stored far outside the home cell) has no such unique
+// image. Its lists (mode 2) hold an atom once, whenever the image that rounded fractions pick for
+// some bead of the voxel may lie within the screening radius; "sure" atoms are those whose picked
+// image is the same for every bead of the voxel and inside the cutoff, and the others are
+// screened with the rounded fractions, as the tile path does.
+//
 // Entry: bits 0-19 the atom's storage index, bits 20-28 the shift (nx + 4) | (ny + 4) << 3
 // | (nz + 4) << 6, n in [-4, 3], the image being r - nx a - ny b - nz c. Lists are built on
 // the host (threads over voxels; tile spheres prune the atoms) when the host atoms change,
@@ -53,15 +59,16 @@ inline double image(const Geo& G, double* d, int* n, double half_wmin) {
 }
 
 constexpr double kMargin = 0.02;                  // A, on the voxel bounding radius
+constexpr double kTieMargin = 1e-3;               // fractional, on a voxel's half extent (mode 2)
 constexpr size_t kArenaHeadroom = 4u << 20;       // arena bytes left free for the box's other buffers
 
 }  // namespace
 
 // Voxel grid of a cell: the finest edge g in {1.5, 2, 2.5, 3, 4} A whose lists fit the byte
-// cap max_bytes (estimated from the host-atom density) and leave the cell wider than 2 r_list. Returns
-// false when none does (the tile path then serves the box).
-static bool choose_voxels(const double* C, double volume, int nh_atoms, double r_screen, size_t max_bytes, Geo& G,
-                          double& half_wmin, int nv[3], double& h, double& est_bytes) {
+// cap max_bytes (estimated from the host-atom density). unique: only grids that leave the cell wider
+// than 2 r_list. Returns false when none does.
+static bool choose_voxels(const double* C, double volume, int nh_atoms, double r_screen, size_t max_bytes, bool unique,
+                          Geo& G, double& half_wmin, int nv[3], double& h, double& est_bytes) {
   const double av[3] = {C[0], C[1], C[2]}, bv[3] = {C[3], C[4], C[5]}, cv[3] = {C[6], C[7], C[8]};
   auto cross_norm = [](const double* u, const double* v) {
     const double x = u[1] * v[2] - u[2] * v[1], y = u[2] * v[0] - u[0] * v[2], z = u[0] * v[1] - u[1] * v[0];
@@ -87,9 +94,10 @@ static bool choose_voxels(const double* C, double volume, int nh_atoms, double r
         hm = std::max(hm, 0.5 * std::sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]));
       }
     hm += kMargin;
-    if (r_screen + hm + kMargin >= half_wmin) return false;  // coarser voxels only make the bound worse
+    if (unique && r_screen + hm + kMargin >= half_wmin) return false;  // coarser voxels only make the bound worse
     const double rl = r_screen + hm;
-    const double est = (double)n[0] * n[1] * n[2] * (dens * 4.18879 * rl * rl * rl * 1.25 + 32.0) * 4.0 +
+    const double per = unique ? dens * 4.18879 * rl * rl * rl * 1.25 : std::min((double)nh_atoms, dens * 4.18879 * rl * rl * rl * 1.5);
+    const double est = (double)n[0] * n[1] * n[2] * (per + 32.0) * 4.0 +
                        (double)n[0] * n[1] * n[2] * 16.0;
     if (est <= (double)max_bytes) {
       for (int k = 0; k < 3; ++k) nv[k] = n[k];
@@ -125,7 +133,17 @@ grx_status build_voxels(grx_box* b) {
   const double r_screen = std::sqrt((double)d.screen2);
   int nv[3] = {0, 0, 0};
   double h = 0.0, half_wmin = 0.0, est = 0.0;
-  if (!choose_voxels(C, d.volume, nh_atoms, r_screen, b->vox_max_bytes, G, half_wmin, nv, h, est)) {
+  // host atoms must lie within four cells of the home cell for the 3-bit shifts of mode 1
+  bool near_home = true;
+  for (int i = 0; i < nh_atoms && near_home; ++i)
+    for (int k = 0; k < 3; ++k) {
+      const double f = G.inv[k] * b->h_pos[3 * i] + G.inv[3 + k] * b->h_pos[3 * i + 1] + G.inv[6 + k] * b->h_pos[3 * i + 2];
+      if (!(f >= -2.5 && f <= 2.5)) near_home = false;
+    }
+  int mode = 0;
+  if (near_home && choose_voxels(C, d.volume, nh_atoms, r_screen, b->vox_max_bytes, true, G, half_wmin, nv, h, est)) mode = 1;
+  else if (choose_voxels(C, d.volume, nh_atoms, r_screen, b->vox_max_bytes, false, G, half_wmin, nv, h, est)) mode = 2;
+  if (!mode) {
     refresh_dev(b);
     return GRX_OK;
   }
@@ -153,6 +171,30 @@ grx_status build_voxels(grx_box* b) {
         for (int i = tr.x; i < tr.y; ++i) {
           double da[3] = {b->h_pos[3 * i] - c[0], b->h_pos[3 * i + 1] - c[1], b->h_pos[3 * i + 2] - c[2]};
           int m[3];
+          if (mode == 2) {
+            // the images that rounded fractions may pick for a bead of the voxel: the remainder of
+            // the centre, and across a tie on each axis that the voxel's extent reaches
+            double f[3], v[3];
+            int tie[3], nt = 0;
+            for (int k = 0; k < 3; ++k) {
+              f[k] = G.inv[k] * da[0] + G.inv[3 + k] * da[1] + G.inv[6 + k] * da[2];
+              f[k] -= rnd_away(f[k]);
+              if (std::fabs(f[k]) > 0.5 - (0.5 / nv[k] + kTieMargin)) tie[nt++] = k;
+            }
+            double r2 = 1e300;
+            for (int c = 0; c < (1 << nt); ++c) {
+              double g[3] = {f[0], f[1], f[2]};
+              for (int q = 0; q < nt; ++q)
+                if (c >> q & 1) g[tie[q]] -= g[tie[q]] >= 0.0 ? 1.0 : -1.0;
+              for (int j = 0; j < 3; ++j) v[j] = G.cell[j] * g[0] + G.cell[3 + j] * g[1] + G.cell[6 + j] * g[2];
+              r2 = std::min(r2, v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
+            }
+            const double r = std::sqrt(r2);
+            if (r > r_list) continue;
+            if (nt == 0 && r <= r_sure) sure.push_back({i, (uint32_t)i});
+            else maybe.push_back({i, (uint32_t)i});
+            continue;
+          }
           image(G, da, m, half_wmin);
           // the rounded image is the nearest one for any image within r_list < w_min / 2
           const double r = std::sqrt(da[0] * da[0] + da[1] * da[1] + da[2] * da[2]);
@@ -175,17 +217,6 @@ grx_status build_voxels(grx_box* b) {
       nsure[v] = (int)sure.size();
     }
   };
-  // host atoms must lie within four cells of the home cell for the 3-bit shifts
-  for (int i = 0; i < nh_atoms; ++i) {
-    double s[3];
-    for (int k = 0; k < 3; ++k)
-      s[k] = G.inv[k] * b->h_pos[3 * i] + G.inv[3 + k] * b->h_pos[3 * i + 1] + G.inv[6 + k] * b->h_pos[3 * i + 2];
-    for (int k = 0; k < 3; ++k)
-      if (s[k] < -2.5 || s[k] > 2.5) {
-        refresh_dev(b);
-        return GRX_OK;
-      }
-  }
   const int nthr = std::max(1, std::min<int>(16, (int)std::thread::hardware_concurrency()));
   {
     std::vector<std::thread> th;
@@ -240,7 +271,7 @@ grx_status build_voxels(grx_box* b) {
                  "upload voxel lists");
   for (int k = 0; k < 3; ++k) b->vn[k] = nv[k];
   b->vchunks = (maxn + 31) / 32;
-  b->vox_on = 1;
+  b->vox_on = mode;
   b->vox_entries = total;
   refresh_dev(b);
   return GRX_OK;
@@ -263,7 +294,7 @@ extern "C" grx_status grx_box_set_voxel_lists(grx_box* b, int32_t mode) {
 extern "C" grx_status grx_box_get_voxel_lists(grx_box* b, int32_t* on, int32_t* dims, int64_t* entries) {
   GRX_REQUIRE(b && on, "grx_box_get_voxel_lists: null argument");
   const grx_box* h = b->parent ? b->parent : b;
-  *on = h->vox_on;
+  *on = h->vox_on ? 1 : 0;
   if (dims)
     for (int k = 0; k < 3; ++k) dims[k] = h->vox_on ? h->vn[k] : 0;
   if (entries) *entries = h->vox_on ? (int64_t)h->vox_entries : 0;

@@ -459,9 +459,13 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
               const int i = (int)(c & 0xFFFFFu);
               if (j >= vm.y) {
                 const float4 ah = b.hrec[2 * i];
-                const float4 sh = __ldg(b.vshift + (c >> 20));
-                const float x = (ah.x - wh.x) - sh.x, y = (ah.y - wh.y) - sh.y, z = (ah.z - wh.z) - sh.z;
-                in = x * x + y * y + z * z < b.screen2 || (PREC == GRX_FP64 && !(bd.unit & 2));
+                if (b.vox == 2) {
+                  in = screen_hi<PREC>(b, ah, bd);
+                } else {
+                  const float4 sh = __ldg(b.vshift + (c >> 20));
+                  const float x = (ah.x - wh.x) - sh.x, y = (ah.y - wh.y) - sh.y, z = (ah.z - wh.z) - sh.z;
+                  in = x * x + y * y + z * z < b.screen2 || (PREC == GRX_FP64 && !(bd.unit & 2));
+                }
               }
               if (in && hcheck) {  // a host component is moved or excluded: skip its molecule
                 int tz = 0;

@@ -211,10 +211,11 @@ grx_status grx_box_create_replica(grx_box* parent, grx_box** out);
  * point of the voxel, with its periodic image, the atoms inside the cutoff for the whole
  * voxel first. The pair engine then walks a bead's voxel list instead of culling the
  * framework's 32-atom tiles (the cutoff tests stay exact, so results change only in the
- * summation order). Built by default when the lists fit 32 MB and the cell is wider than
- * twice the list radius; mode 0 frees them (tile path), mode 1 rebuilds them. Refused on
- * a box with replicas (they share the lists). No counterpart in the reference (it tests
- * every framework atom per trial). get: on (0/1), voxels per axis, list entries. */
+ * summation order). In a cell narrower than twice the list radius an entry's image is the
+ * one of rounded fractions, as on the tile path. Built by default when the lists fit 32 MB;
+ * mode 0 frees them (tile path), mode 1 rebuilds them. Refused on a box with replicas (they
+ * share the lists). No counterpart in the reference (it tests every framework atom per
+ * trial). get: on (0/1), voxels per axis, list entries. */
 grx_status grx_box_set_voxel_lists(grx_box* box, int32_t mode);
 grx_status grx_box_get_voxel_lists(grx_box* box, int32_t* on, int32_t* dims, int64_t* entries);
 
