@@ -38,6 +38,12 @@ struct Geo {
   double cell[9], inv[9], w[3];
 };
 
+struct Cand {  // a candidate of one voxel: storage index, list entry, distance of its image from the centre
+  int i;
+  uint32_t e;
+  float r;
+};
+
 // Fractional rounding of the reference's PBC (round half away from zero).
 inline double rnd_away(double s) { return (double)(int)(s + (s >= 0.0 ? 0.5 : -0.5)); }
 
@@ -154,7 +160,7 @@ grx_status build_voxels(grx_box* b) {
   std::vector<int> nsure(nvox, 0);
   const int ntile = b->ntiles;
   auto work = [&](int v0, int v1) {
-    std::vector<std::pair<int, uint32_t>> sure, maybe;
+    std::vector<Cand> sure, maybe;
     for (int v = v0; v < v1; ++v) {
       const int ix = v % nv[0], iy = (v / nv[0]) % nv[1], iz = v / (nv[0] * nv[1]);
       const double f[3] = {(ix + 0.5) / nv[0], (iy + 0.5) / nv[1], (iz + 0.5) / nv[2]};
@@ -191,8 +197,8 @@ grx_status build_voxels(grx_box* b) {
             }
             const double r = std::sqrt(r2);
             if (r > r_list) continue;
-            if (nt == 0 && r <= r_sure) sure.push_back({i, (uint32_t)i});
-            else maybe.push_back({i, (uint32_t)i});
+            if (nt == 0 && r <= r_sure) sure.push_back({i, (uint32_t)i, (float)r});
+            else maybe.push_back({i, (uint32_t)i, (float)r});
             continue;
           }
           image(G, da, m, half_wmin);
@@ -204,16 +210,20 @@ grx_status build_voxels(grx_box* b) {
           if (!ok) continue;  // never taken: host atoms were checked to lie near the home cell
           const uint32_t e = (uint32_t)i | ((uint32_t)(m[0] + 4) << 20) | ((uint32_t)(m[1] + 4) << 23) |
                              ((uint32_t)(m[2] + 4) << 26);
-          if (r <= r_sure) sure.push_back({i, e});
-          else maybe.push_back({i, e});
+          if (r <= r_sure) sure.push_back({i, e, (float)r});
+          else maybe.push_back({i, e, (float)r});
         }
       }
-      std::sort(sure.begin(), sure.end());
-      std::sort(maybe.begin(), maybe.end());
+      const size_t nf = std::min<size_t>(32, sure.size());
+      std::partial_sort(sure.begin(), sure.begin() + nf, sure.end(),
+                        [](const Cand& x, const Cand& y) { return x.r < y.r || (x.r == y.r && x.e < y.e); });
+      auto by_index = [](const Cand& x, const Cand& y) { return x.i < y.i || (x.i == y.i && x.e < y.e); };
+      std::sort(sure.begin() + nf, sure.end(), by_index);
+      std::sort(maybe.begin(), maybe.end(), by_index);
       std::vector<uint32_t>& out = lists[v];
       out.reserve(sure.size() + maybe.size());
-      for (const auto& p : sure) out.push_back(p.second);
-      for (const auto& p : maybe) out.push_back(p.second);
+      for (const Cand& p : sure) out.push_back(p.e);
+      for (const Cand& p : maybe) out.push_back(p.e);
       nsure[v] = (int)sure.size();
     }
   };
