@@ -669,6 +669,7 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
     f64[r].c = ff.use_1264 ? (ff.z ? ff.z[r] : 0.0) : ff.sigma[r] * ff.sigma[r];
     f64[r].shift = ff.shift[r];
     if (ff.c10) c10[r] = ff.c10[r];
+    if (!ff.use_1264) b->sigma_max = std::max(b->sigma_max, ff.sigma[r]);
     const double s2 = ff.sigma[r] * ff.sigma[r];
     f32[r] = make_float4((float)(4.0 * ff.epsilon[r]), s2 > 0 ? (float)(1.0 / s2) : INFINITY,
                          (float)ff.shift[r], (float)(1.21 * s2));

@@ -85,6 +85,7 @@ struct grx_box {
   // candidate lists of host atoms per voxel (grx_voxel.cu); a replica uses its parent's
   int vox_mode = 1;          // 1: build them when they fit, 0: tile path only
   size_t vox_max_bytes = 32u << 20;  // byte cap of the lists (coarser voxels to stay below it)
+  double sigma_max = 0.0;    // largest sigma of the type pairs (0: 12-6-4 tables)
   int vox_on = 0;            // 0 no lists, 1 entries with their image, 2 images by rounded fractions
   int vn[3] = {0, 0, 0};
   int vchunks = 0;

@@ -8,24 +8,25 @@
 // image the bead sees it (the cell is wider than 2 r_list, so that image is unique).
 // Atoms whose image lies within (screening radius - bounding radius) of the centre are
 // inside the cutoff for every bead of the voxel: they come first in the list and go to
-// the dense evaluation without the FP32 screen; the others are screened with the stored
-// shift. A bead pass walks its voxel's list in 32-atom chunks instead of culling the
+// the dense evaluation without the FP32 screen, the ones near the centre (1.1 sigma from some
+// bead of the voxel) ahead of the rest: the pairs that take the out-of-line LJ then share a batch
+// or two instead of falling into half of them, and an overlap shows at once. The others are
+// screened with the stored shift. A bead pass walks its voxel's list in 32-atom chunks instead of culling the
 // box's 32-atom tiles; the dense evaluation still applies the exact cutoff tests, so the
 // lists change which pairs are screened, never which pairs count.
 //
-// A cell narrower than 2 r_list (or host atoms stored far outside the home cell) has no such unique
-// image. Its lists (mode 2) hold an atom once, whenever the image that rounded fractions pick for
+// A cell narrower than 2 r_list (or host atoms stored cells away from the home cell) has no such
+// unique image. Its lists (mode 2) hold an atom once, whenever the image that rounded fractions pick for
 // some bead of the voxel may lie within the screening radius; "sure" atoms are those whose picked
 // image is the same for every bead of the voxel and inside the cutoff, and the others are
 // screened with the rounded fractions, as the tile path does.
 //
 // Entry: bits 0-19 the atom's storage index, bits 20-28 the shift (nx + 4) | (ny + 4) << 3
 // | (nz + 4) << 6, n in [-4, 3], the image being r - nx a - ny b - nz c. Lists are built on
-// the host (threads over voxels; tile spheres prune the atoms) when the host atoms change,
-// and shared with the box's replicas.
+// the device when the host atoms change (a warp per voxel counts, the host sums, the warp writes;
+// host threads took 10 to 20 ms a box), and shared with the box's replicas.
 #include <algorithm>
 #include <cmath>
-#include <thread>
 #include <vector>
 
 #include "grx_host.h"
@@ -37,32 +38,6 @@ namespace {
 struct Geo {
   double cell[9], inv[9], w[3];
 };
-
-struct Cand {  // a candidate of one voxel: storage index, list entry, distance of its image from the centre
-  int i;
-  uint32_t e;
-  float r;
-};
-
-// Fractional rounding of the reference's PBC (round half away from zero).
-inline double rnd_away(double s) { return (double)(int)(s + (s >= 0.0 ? 0.5 : -0.5)); }
-
-// Displacement d (in) to its rounded image (out), with the lattice integers n; returns
-// a lower bound of the distance to the nearest image (exact when |d_out| <= w_min / 2).
-inline double image(const Geo& G, double* d, int* n, double half_wmin) {
-  double s[3];
-  for (int k = 0; k < 3; ++k) s[k] = G.inv[k] * d[0] + G.inv[3 + k] * d[1] + G.inv[6 + k] * d[2];
-  double r[3];
-  for (int k = 0; k < 3; ++k) {
-    const double m = rnd_away(s[k]);
-    n[k] = (int)m;
-    r[k] = s[k] - m;
-  }
-  for (int j = 0; j < 3; ++j) d[j] = G.cell[j] * r[0] + G.cell[3 + j] * r[1] + G.cell[6 + j] * r[2];
-  const double len = std::sqrt(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-  if (len <= half_wmin) return len;
-  return std::max(std::fabs(r[0]) * G.w[0], std::max(std::fabs(r[1]) * G.w[1], std::fabs(r[2]) * G.w[2]));
-}
 
 constexpr double kMargin = 0.02;                  // A, on the voxel bounding radius
 constexpr double kTieMargin = 1e-3;               // fractional, on a voxel's half extent (mode 2)
@@ -115,6 +90,83 @@ static bool choose_voxels(const double* C, double volume, int nh_atoms, double r
   return false;
 }
 
+struct VoxelScan {
+  int mode;
+  int nv[3];
+  float tie[3];  // mode 2: |fraction| of the centre above which the voxel reaches across the tie
+  float r_list, r_sure, r_near;
+};
+
+constexpr int kVoxelWarps = 8;
+
+// One warp per voxel walks the framework atoms in storage order, one per lane. Without `list` it
+// counts: meta {0, sure, all, near}. With it, meta holds the first entry too, and the warp
+// writes the groups near, sure and the rest behind each other. FP32 on the hi parts: its errors
+// (1e-3 A and 1e-5 of a fraction) stay inside the margins of the radii and of the ties.
+__global__ void __launch_bounds__(32 * kVoxelWarps) voxel_scan_kernel(const __grid_constant__ BoxDev b,
+                                                                      const __grid_constant__ VoxelScan p, int4* meta,
+                                                                      unsigned* list) {
+  const int v = blockIdx.x * kVoxelWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (v >= p.nv[0] * p.nv[1] * p.nv[2]) return;
+  const unsigned lt = (1u << lane) - 1u;
+  const float fx = ((v % p.nv[0]) + 0.5f) / p.nv[0], fy = ((v / p.nv[0] % p.nv[1]) + 0.5f) / p.nv[1],
+              fz = ((v / (p.nv[0] * p.nv[1])) + 0.5f) / p.nv[2];
+  const float cx = b.cellf[0] * fx + b.cellf[3] * fy + b.cellf[6] * fz;
+  const float cy = b.cellf[1] * fx + b.cellf[4] * fy + b.cellf[7] * fz;
+  const float cz = b.cellf[2] * fx + b.cellf[5] * fy + b.cellf[8] * fz;
+  const int4 m = list ? meta[v] : make_int4(0, 0, 0, 0);
+  int at[3] = {m.x, m.x + m.w, m.x + m.y};  // next entry of near, sure, the rest
+  int n[3] = {0, 0, 0};
+  for (int c = 0; c < b.nhost; ++c) {
+    const int end = b.comp_off[c] + b.comp_size[c];
+    for (int i0 = b.comp_off[c]; i0 < end; i0 += 32) {
+      const int i = i0 + lane;
+      int group = -1;
+      unsigned code = 4u | 4u << 3 | 4u << 6;
+      if (i < end) {
+        const float4 a = b.hhi[i];
+        const float x = a.x - cx, y = a.y - cy, z = a.z - cz;
+        float sx = b.invf[0] * x + b.invf[3] * y + b.invf[6] * z;
+        float sy = b.invf[1] * x + b.invf[4] * y + b.invf[7] * z;
+        float sz = b.invf[2] * x + b.invf[5] * y + b.invf[8] * z;
+        const float nx = rintf(sx), ny = rintf(sy), nz = rintf(sz);
+        sx -= nx; sy -= ny; sz -= nz;
+        auto norm2 = [&](float u, float w, float t) {
+          const float dx = b.cellf[0] * u + b.cellf[3] * w + b.cellf[6] * t;
+          const float dy = b.cellf[1] * u + b.cellf[4] * w + b.cellf[7] * t;
+          const float dz = b.cellf[2] * u + b.cellf[5] * w + b.cellf[8] * t;
+          return dx * dx + dy * dy + dz * dz;
+        };
+        float r2 = norm2(sx, sy, sz);
+        bool one = true;
+        if (p.mode == 1) {
+          code = (unsigned)((int)nx + 4) | (unsigned)((int)ny + 4) << 3 | (unsigned)((int)nz + 4) << 6;
+        } else {  // the images that rounded fractions may pick for a bead of the voxel
+          const bool tx = fabsf(sx) > p.tie[0], ty = fabsf(sy) > p.tie[1], tz = fabsf(sz) > p.tie[2];
+          one = !(tx || ty || tz);
+          const float ux = sx - copysignf(1.0f, sx), uy = sy - copysignf(1.0f, sy), uz = sz - copysignf(1.0f, sz);
+          for (int k = 1; k < 8 && !one; ++k) {
+            if ((k & 1 && !tx) || (k & 2 && !ty) || (k & 4 && !tz)) continue;
+            r2 = fminf(r2, norm2(k & 1 ? ux : sx, k & 2 ? uy : sy, k & 4 ? uz : sz));
+          }
+        }
+        if (r2 <= p.r_list * p.r_list) {
+          const bool sure = one && p.r_sure > 0.0f && r2 <= p.r_sure * p.r_sure;
+          group = !sure ? 2 : (p.r_near > 0.0f && r2 <= p.r_near * p.r_near ? 0 : 1);
+        }
+      }
+#pragma unroll
+      for (int g = 0; g < 3; ++g) {
+        const unsigned k = __ballot_sync(0xffffffffu, group == g);
+        if (list && group == g) list[at[g] + __popc(k & lt)] = (unsigned)i | code << 20;
+        at[g] += __popc(k);
+        n[g] += __popc(k);
+      }
+    }
+  }
+  if (!list && lane == 0) meta[v] = make_int4(0, n[0] + n[1], n[0] + n[1] + n[2], n[0]);
+}
+
 grx_status build_voxels(grx_box* b) {
   dev_free(b, b->vmeta);
   dev_free(b, b->vlist);
@@ -141,10 +193,15 @@ grx_status build_voxels(grx_box* b) {
   double h = 0.0, half_wmin = 0.0, est = 0.0;
   // host atoms must lie within four cells of the home cell for the 3-bit shifts of mode 1
   bool near_home = true;
-  for (int i = 0; i < nh_atoms && near_home; ++i)
+  for (int i = 0; i < nh_atoms; ++i)
     for (int k = 0; k < 3; ++k) {
       const double f = G.inv[k] * b->h_pos[3 * i] + G.inv[3 + k] * b->h_pos[3 * i + 1] + G.inv[6 + k] * b->h_pos[3 * i + 2];
       if (!(f >= -2.5 && f <= 2.5)) near_home = false;
+      // coordinates that the hi parts do not hold exactly: the tile path serves the box
+      if (!(std::fabs(b->h_pos[3 * i + k]) < (double)kNearCoord)) {
+        refresh_dev(b);
+        return GRX_OK;
+      }
     }
   int mode = 0;
   if (near_home && choose_voxels(C, d.volume, nh_atoms, r_screen, b->vox_max_bytes, true, G, half_wmin, nv, h, est)) mode = 1;
@@ -153,101 +210,38 @@ grx_status build_voxels(grx_box* b) {
     refresh_dev(b);
     return GRX_OK;
   }
-  const double r_list = r_screen + h;
-  const double r_sure = r_screen - 2e-3 - h;  // inside the largest cutoff for every bead of the voxel
-  const int nvox = nv[0] * nv[1] * nv[2];
-  std::vector<std::vector<uint32_t>> lists(nvox);
-  std::vector<int> nsure(nvox, 0);
-  const int ntile = b->ntiles;
-  auto work = [&](int v0, int v1) {
-    std::vector<Cand> sure, maybe;
-    for (int v = v0; v < v1; ++v) {
-      const int ix = v % nv[0], iy = (v / nv[0]) % nv[1], iz = v / (nv[0] * nv[1]);
-      const double f[3] = {(ix + 0.5) / nv[0], (iy + 0.5) / nv[1], (iz + 0.5) / nv[2]};
-      double c[3];
-      for (int j = 0; j < 3; ++j) c[j] = av[j] * f[0] + bv[j] * f[1] + cv[j] * f[2];
-      sure.clear();
-      maybe.clear();
-      for (int t = 0; t < ntile; ++t) {
-        const float4 tc = b->h_tile_c[2 * t];
-        const int4 tr = b->h_tile_r[t];
-        double dv[3] = {tc.x - c[0], tc.y - c[1], tc.z - c[2]};
-        int n[3];
-        if (image(G, dv, n, half_wmin) - tc.w > r_list) continue;
-        for (int i = tr.x; i < tr.y; ++i) {
-          double da[3] = {b->h_pos[3 * i] - c[0], b->h_pos[3 * i + 1] - c[1], b->h_pos[3 * i + 2] - c[2]};
-          int m[3];
-          if (mode == 2) {
-            // the images that rounded fractions may pick for a bead of the voxel: the remainder of
-            // the centre, and across a tie on each axis that the voxel's extent reaches
-            double f[3], v[3];
-            int tie[3], nt = 0;
-            for (int k = 0; k < 3; ++k) {
-              f[k] = G.inv[k] * da[0] + G.inv[3 + k] * da[1] + G.inv[6 + k] * da[2];
-              f[k] -= rnd_away(f[k]);
-              if (std::fabs(f[k]) > 0.5 - (0.5 / nv[k] + kTieMargin)) tie[nt++] = k;
-            }
-            double r2 = 1e300;
-            for (int c = 0; c < (1 << nt); ++c) {
-              double g[3] = {f[0], f[1], f[2]};
-              for (int q = 0; q < nt; ++q)
-                if (c >> q & 1) g[tie[q]] -= g[tie[q]] >= 0.0 ? 1.0 : -1.0;
-              for (int j = 0; j < 3; ++j) v[j] = G.cell[j] * g[0] + G.cell[3 + j] * g[1] + G.cell[6 + j] * g[2];
-              r2 = std::min(r2, v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
-            }
-            const double r = std::sqrt(r2);
-            if (r > r_list) continue;
-            if (nt == 0 && r <= r_sure) sure.push_back({i, (uint32_t)i, (float)r});
-            else maybe.push_back({i, (uint32_t)i, (float)r});
-            continue;
-          }
-          image(G, da, m, half_wmin);
-          // the rounded image is the nearest one for any image within r_list < w_min / 2
-          const double r = std::sqrt(da[0] * da[0] + da[1] * da[1] + da[2] * da[2]);
-          if (r > r_list) continue;
-          bool ok = true;
-          for (int k = 0; k < 3; ++k) ok = ok && m[k] >= -4 && m[k] <= 3;
-          if (!ok) continue;  // never taken: host atoms were checked to lie near the home cell
-          const uint32_t e = (uint32_t)i | ((uint32_t)(m[0] + 4) << 20) | ((uint32_t)(m[1] + 4) << 23) |
-                             ((uint32_t)(m[2] + 4) << 26);
-          if (r <= r_sure) sure.push_back({i, e, (float)r});
-          else maybe.push_back({i, e, (float)r});
-        }
-      }
-      const size_t nf = std::min<size_t>(32, sure.size());
-      std::partial_sort(sure.begin(), sure.begin() + nf, sure.end(),
-                        [](const Cand& x, const Cand& y) { return x.r < y.r || (x.r == y.r && x.e < y.e); });
-      auto by_index = [](const Cand& x, const Cand& y) { return x.i < y.i || (x.i == y.i && x.e < y.e); };
-      std::sort(sure.begin() + nf, sure.end(), by_index);
-      std::sort(maybe.begin(), maybe.end(), by_index);
-      std::vector<uint32_t>& out = lists[v];
-      out.reserve(sure.size() + maybe.size());
-      for (const Cand& p : sure) out.push_back(p.e);
-      for (const Cand& p : maybe) out.push_back(p.e);
-      nsure[v] = (int)sure.size();
-    }
-  };
-  const int nthr = std::max(1, std::min<int>(16, (int)std::thread::hardware_concurrency()));
-  {
-    std::vector<std::thread> th;
-    const int per = (nvox + nthr - 1) / nthr;
-    for (int k = 0; k < nthr; ++k) {
-      const int v0 = k * per, v1 = std::min(nvox, v0 + per);
-      if (v0 < v1) th.emplace_back(work, v0, v1);
-    }
-    for (auto& t : th) t.join();
+  VoxelScan v{};
+  v.mode = mode;
+  for (int k = 0; k < 3; ++k) {
+    v.nv[k] = nv[k];
+    v.tie[k] = (float)(0.5 - (0.5 / nv[k] + kTieMargin));
   }
+  v.r_list = (float)(r_screen + h);
+  v.r_sure = (float)(r_screen - 2e-3 - h);  // inside the largest cutoff for every bead of the voxel
+  v.r_near = (float)std::min((double)v.r_sure, 1.1 * b->sigma_max + h);
+  const int nvox = nv[0] * nv[1] * nv[2];
+  const int grid = (nvox + kVoxelWarps - 1) / kVoxelWarps;
   std::vector<int4> meta(nvox);
+  grx_status st = ensure_scratch(b, nvox * sizeof(int4));
+  if (st) {  // no room to count: the tile path serves the box
+    refresh_dev(b);
+    return GRX_OK;
+  }
+  int4* counts = (int4*)b->scratch;
+  voxel_scan_kernel<<<grid, 32 * kVoxelWarps, 0, b->stream>>>(b->dev, v, counts, nullptr);
+  count_launch();
+  GRX_CHECK_CUDA(cudaGetLastError(), "voxel count launch");
+  GRX_CHECK_CUDA(cudaMemcpyAsync(meta.data(), counts, nvox * sizeof(int4), cudaMemcpyDeviceToHost, b->stream),
+                 "read voxel counts");
+  GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "voxel counts");
   size_t total = 0;
   int maxn = 0;
-  for (int v = 0; v < nvox; ++v) {
-    meta[v] = make_int4((int)total, nsure[v], (int)lists[v].size(), 0);
-    total += lists[v].size();
-    maxn = std::max(maxn, (int)lists[v].size());
+  for (int k = 0; k < nvox; ++k) {  // {first entry, sure, all, near}
+    meta[k].x = (int)total;
+    total += (size_t)meta[k].z;
+    maxn = std::max(maxn, meta[k].z);
   }
-  std::vector<uint32_t> flat;
-  flat.reserve(total);
-  for (const auto& l : lists) flat.insert(flat.end(), l.begin(), l.end());
+  const size_t list_bytes = std::max<size_t>(total, 1) * sizeof(uint32_t);
   // the lattice vectors of the 512 shift codes follow the voxel records
   meta.resize(nvox + 512);
   static_assert(sizeof(int4) == sizeof(float4), "shift vectors share the voxel records' allocation");
@@ -261,13 +255,13 @@ grx_status build_voxels(grx_box* b) {
   if (b->arena) {  // in an arena the lists are optional: take them only with room to spare
     size_t used = 0, largest = 0;
     grx_arena_usage(b->arena, &used, &largest, nullptr);
-    if (largest < meta.size() * sizeof(int4) + flat.size() * sizeof(uint32_t) + kArenaHeadroom) {
+    if (largest < meta.size() * sizeof(int4) + list_bytes + kArenaHeadroom) {
       refresh_dev(b);
       return GRX_OK;
     }
   }
   if (dev_alloc(b, (void**)&b->vmeta, meta.size() * sizeof(int4)) != cudaSuccess ||
-      dev_alloc(b, (void**)&b->vlist, flat.size() * sizeof(uint32_t)) != cudaSuccess) {
+      dev_alloc(b, (void**)&b->vlist, list_bytes) != cudaSuccess) {
     cudaGetLastError();  // no room: the tile path serves the box
     dev_free(b, b->vmeta);
     dev_free(b, b->vlist);
@@ -277,8 +271,10 @@ grx_status build_voxels(grx_box* b) {
     return GRX_OK;
   }
   GRX_CHECK_CUDA(cudaMemcpy(b->vmeta, meta.data(), meta.size() * sizeof(int4), cudaMemcpyHostToDevice), "upload voxels");
-  GRX_CHECK_CUDA(cudaMemcpy(b->vlist, flat.data(), flat.size() * sizeof(uint32_t), cudaMemcpyHostToDevice),
-                 "upload voxel lists");
+  voxel_scan_kernel<<<grid, 32 * kVoxelWarps, 0, b->stream>>>(b->dev, v, b->vmeta, b->vlist);
+  count_launch();
+  GRX_CHECK_CUDA(cudaGetLastError(), "voxel list launch");
+  GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "voxel lists");
   for (int k = 0; k < 3; ++k) b->vn[k] = nv[k];
   b->vchunks = (maxn + 31) / 32;
   b->vox_on = mode;
