@@ -58,6 +58,7 @@ struct CbmcWork {
   long long cfg;    // trial configurations evaluated since the caller last cleared it
   long long cbeads; // their beads
   int ok;       // step constructed
+  int big;      // and its weight (times that of the steps before it) above 1e-150
   int sel;      // chosen (or retraced) trial index
   int nok;      // trials without overlap
   double w;     // averaged weight of the step
@@ -212,27 +213,33 @@ __device__ __noinline__ void trial_pass_excl(const BoxDev& b, WK& W, int nb, int
   trial_pass_body<PREC, CL>(b, W, nb, chain, comp, newmol, excl_comp, excl_mol, -1);
 }
 
-// CBMC weight of one growth step (warp 0 computes, results in W.ok/sel/w/nok/wraw).
-// Insertion: log-sum-exp selection with the uniform u (SelectTrialPosition) and the
+// CBMC weight of one growth step (warp 0 computes, results in W.ok/big/sel/w/nok/wraw).
+// Insertion: log-sum-exp selection with the uniform of word uw (SelectTrialPosition) and the
 // 1e-150 failure test. Retrace (deletion): the first trial without overlap is the
 // existing configuration and no selection is drawn. `stored` is added to the sum
-// before averaging (the reinsertion retrace's StoredR, mc_widom.h:363-366).
+// before averaging over 1 / inv trials (the reinsertion retrace's StoredR, mc_widom.h:363-366).
+// chain: the weight of the steps before, multiplied by this one's. FP64 stays on warp 0: an FP64
+// instruction takes 16 cycles of the SM per warp that issues it, whatever its lanes do.
 template <class WK>
-__device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, double u, double navg,
-                                            bool retrace, double stored = 0.0) {
+__device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, uint32_t uw, double inv,
+                                            bool retrace, double stored = 0.0, double* chain = nullptr) {
   if (threadIdx.x < 32) {
-    const StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u, retrace, W.sel_wa);
+    const StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u01(uw), retrace, W.sel_wa);
     if (threadIdx.x == 0) {
       W.nok = c.nok;
       W.ok = 0;
+      W.big = 0;
       if (c.nok > 0) {
         W.wraw = c.w;
         if (retrace || !(c.w < 1e-150)) {
-          double avg = (c.w + stored) / navg;
+          double avg = (c.w + stored) * inv;
           if (!bias) avg *= exp_move(-beta * (W.te[4 * c.sel + 1] + W.te[4 * c.sel + 3]));
           W.ok = 1;
           W.sel = c.sel;
           W.w = avg;
+          const double all = chain ? *chain * avg : avg;
+          if (chain) *chain = all;
+          W.big = all > 1e-150;
         }
       }
     }
@@ -293,8 +300,11 @@ __device__ __noinline__ void ewald_move(const BoxDev& b, WK& W, int na, double2*
     cr = warp_sum_df(cr);
     if ((tid & 31) == 0) { W.wsum[0][tid >> 5] = df_to(sm); W.wsum[1][tid >> 5] = df_to(cr); }
     __syncthreads();
-    if (tid == 0)
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { same += W.wsum[0][w]; cross += W.wsum[1][w]; }
+    if (tid < 32) {  // one tree instead of a serial FP64 chain over the warps
+      const bool in = tid < (int)(blockDim.x >> 5);
+      same = warp_sum(in ? W.wsum[0][tid] : 0.0);
+      cross = warp_sum(in ? W.wsum[1][tid] : 0.0);
+    }
   }
   if constexpr (CL > 1) {
     const unsigned rank = cluster_rank();
@@ -305,10 +315,9 @@ __device__ __noinline__ void ewald_move(const BoxDev& b, WK& W, int na, double2*
         dst[2 * rank + 1] = cross;
       }
     cluster_sync_all();
-    if (tid == 0) {
-      same = 0.0;
-      cross = 0.0;
-      for (int p = 0; p < CL; ++p) { same += W.ewx[p][0]; cross += W.ewx[p][1]; }
+    if (tid < 32) {
+      same = warp_sum(tid < CL ? W.ewx[tid][0] : 0.0);
+      cross = warp_sum(tid < CL ? W.ewx[tid][1] : 0.0);
     }
   }
   __syncthreads();

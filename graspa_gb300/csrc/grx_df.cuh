@@ -18,13 +18,6 @@ struct df {
   float hi, lo;
 };
 
-__device__ __forceinline__ df df_from(double x) {
-  const float h = __double2float_rn(x);
-  return {h, __double2float_rn(x - (double)h)};
-}
-
-__device__ __forceinline__ double df_to(df a) { return (double)a.hi + (double)a.lo; }
-
 // A float as a double by its bits (the conversion instruction issues at the FP64 rate).
 __device__ __forceinline__ double wide(float x) {
   const unsigned b = __float_as_uint(x);
@@ -32,10 +25,29 @@ __device__ __forceinline__ double wide(float x) {
   return __hiloint2double((int)((b & 0x80000000u) | (((b & 0x7fffffffu) >> 3) + 0x38000000u)), (int)(b << 29));
 }
 
+__device__ __forceinline__ double df_to(df a) { return wide(a.hi) + wide(a.lo); }
+
 __device__ __forceinline__ df fast_two_sum(float a, float b) {  // |a| >= |b|
   const float s = __fadd_rn(a, b);
   const float e = __fsub_rn(b, __fsub_rn(s, a));
   return {s, e};
+}
+
+// A double as a float pair by its bits: the upper 24 significant bits rounded to nearest, the signed
+// remainder of 29 bits as a float. The same pair as rounding and subtracting (ties aside), whose
+// conversions and subtraction issue at the FP64 rate, 64 cycles a warp each.
+__device__ __forceinline__ df df_from(double x) {
+  const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+  const unsigned e = (hi >> 20) & 0x7ffu;
+  if (e - 960u >= 190u) {  // outside the range of two normal floats: zero, tiny, huge, inf, NaN
+    const float h = __double2float_rn(x);
+    return {h, __double2float_rn(x - (double)h)};
+  }
+  const unsigned sign = hi & 0x80000000u;
+  const unsigned top = __funnelshift_l(lo, (hi & 0x7fffffffu) - (896u << 20), 3);
+  const float h = __uint_as_float(sign | (top + ((lo >> 28) & 1u)));
+  const float l = __fmul_rn((float)((int)(lo << 3) >> 3), __uint_as_float(sign | (e - 948u) << 23));
+  return {h, l};
 }
 
 __device__ __forceinline__ df two_sum(float a, float b) {

@@ -148,6 +148,18 @@ static grx_status prepare_gcmc(grx_box* const* boxes, int32_t nboxes, const grx_
       a.big_p = d.mol_fraction * d.pressure * d.fugacity_coeff * b->dev.volume;
       a.step_off = 0;
       a.nsteps_cap = -1;
+      auto threshold = [](double p) {  // words w with w 2^-32 < p
+        return p > 0.0 ? (uint64_t)std::ceil(std::min(p, 2.0) * 4294967296.0) : 0;
+      };
+      a.p_translation = threshold(d.p_translation);
+      a.p_rotation = threshold(d.p_rotation);
+      a.p_reinsertion = threshold(d.p_reinsertion);
+      a.p_identity_swap = threshold(d.p_identity_swap);
+      a.p_swap = threshold(d.p_swap);
+      a.inv_ntrials = 1.0 / d.ntrials;
+      a.inv_norient = ms > 1 ? 1.0 / d.norient : 1.0;
+      a.inv_ideal = 1.0 / d.ideal_rosenbluth;
+      a.beta_p = d.beta * a.big_p;
       ha.push_back(a);
       // eik tables of the moved atoms: FP64 (double2) in the FP64 form, double-float (float4)
       // in the others

@@ -38,7 +38,15 @@ struct GcmcArgs {
   // launch counter + s + step_off; steps taken = min(launch steps, nsteps_cap) (cap < 0: all)
   int64_t step_off;
   int64_t nsteps_cap;
+  // what a step would otherwise form in FP64 on every warp: cumulative move probabilities p as
+  // ceil(p 2^32) against the move word (the same comparison as word 2^-32 < p), reciprocals
+  uint64_t p_translation, p_rotation, p_reinsertion, p_identity_swap, p_swap;
+  double inv_ntrials, inv_norient, inv_ideal;
+  double beta_p;  // beta * big_p
 };
+
+// floor(word 2^-32 n): what the product of the uniform and n in FP64 truncates to (exact below 2^53).
+__device__ __forceinline__ int pick(uint32_t word, int n) { return (int)__umulhi(word, (unsigned)n); }
 
 // sin and cos of an angle in double-float (theta / 2 pi through df_sincos_2pi), out of line so
 // the kernel body keeps its register allocation.
@@ -48,32 +56,30 @@ static __device__ __noinline__ double2 df_sincos_angle(double theta) {
   return make_double2(df_to(sd), df_to(cd));
 }
 
-// RotationAroundAxis (mc_utilities.h:459-481) for a coordinate axis; the mixed and FP32 forms
-// take sin and cos in double-float, the FP64 form in FP64.
+// sin and cos of a rotation angle; the mixed and FP32 forms in double-float, the FP64 form in FP64.
 template <int PREC>
-__device__ __noinline__ double4 rotate_axis_out(double x, double y, double z, double theta, int axis) {
-  double s, c;
-  if constexpr (PREC == GRX_FP64) sincos(theta, &s, &c);
-  else {
-    const double2 sc = df_sincos_angle(theta);
-    s = sc.x;
-    c = sc.y;
+__device__ __forceinline__ double2 rotation_sincos(double theta) {
+  if constexpr (PREC == GRX_FP64) {
+    double s, c;
+    sincos(theta, &s, &c);
+    return make_double2(s, c);
+  } else {
+    return df_sincos_angle(theta);
   }
-  const double w = 1.0 - c;
-  const double ax = axis == 0, ay = axis == 1, az = axis == 2;
-  const double r0 = ax * ax * w + c, r1 = ax * ay * w + az * s, r2 = ax * az * w - ay * s;
-  const double r3 = ax * ay * w - az * s, r4 = ay * ay * w + c, r5 = ay * az * w + ax * s;
-  const double r6 = ax * az * w + ay * s, r7 = ay * az * w - ax * s, r8 = az * az * w + c;
-  const double nx = x * r0 + y * r1 + z * r2;
-  const double ny = x * r3 + y * r4 + z * r5;
-  const double nz = x * r6 + y * r7 + z * r8;
-  return make_double4(nx, ny, nz, 0.0);
 }
 
-template <int PREC>
-__device__ __forceinline__ void rotate_axis(double& x, double& y, double& z, double theta, int axis) {
-  const double4 r = rotate_axis_out<PREC>(x, y, z, theta, axis);
-  x = r.x; y = r.y; z = r.z;
+// RotationAroundAxis (mc_utilities.h:459-481) about the coordinate axes x, y, z in turn: the general
+// matrix leaves one coordinate and mixes the other two with s and c.
+__device__ __forceinline__ void rotate_axes(double& x, double& y, double& z, double2 a, double2 b, double2 c) {
+  double t = y * a.y + z * a.x;
+  z = z * a.y - y * a.x;
+  y = t;
+  t = x * b.y - z * b.x;
+  z = z * b.y + x * b.x;
+  x = t;
+  t = x * c.y + y * c.x;
+  y = y * c.y - x * c.x;
+  x = t;
 }
 
 __device__ __forceinline__ void store_position(const BoxDev& b, int idx, double x, double y, double z) {
@@ -120,7 +126,7 @@ __device__ __forceinline__ void ewald_delta_move(const BoxDev& b, WK& W, int na,
 template <int PREC, int CL, class WK>
 __device__ __noinline__ void identity_swap_step(const BoxDev& b, const GcmcArgs* A, int nm, grx_gcmc_stats* ST, WK& W,
                                                 double2* eik, int* comp_size, uint64_t move, double beta,
-                                                double u_orient, int& s_accept, double* s_e1, double& s_w1,
+                                                uint32_t u_orient, int& s_accept, double* s_e1, double& s_w1,
                                                 double* s_dE, double* s_r1, double& s_wr) {
   const int tid = threadIdx.x;
   uint32_t wx[4];
@@ -129,13 +135,13 @@ __device__ __noinline__ void identity_swap_step(const BoxDev& b, const GcmcArgs*
   for (int e = 0; e < nm; ++e)
     if (comp_size[A[e].comp] >= A[e].ms) have[nh++] = e;
   if (nh > 0) {
-    const int eo = have[min(nh - 1, (int)(u01(wx[0]) * (double)nh))];
-    const int en = min(nm - 1, (int)(u01(wx[1]) * (double)nm));
+    const int eo = have[pick(wx[0], nh)];
+    const int en = pick(wx[1], nm);
     const GcmcArgs& ao = A[eo];
     const GcmcArgs& an = A[en];
     const int mso = ao.ms, msn = an.ms;
     const int No = comp_size[ao.comp] / mso, Nn = comp_size[an.comp] / msn;
-    const int omol = (int)(u01(wx[2]) * (double)No);
+    const int omol = pick(wx[2], No);
     const int o0 = ao.off + omol * mso;
     const bool charged = ao.charged || an.charged;
     if (tid == 0) {
@@ -152,26 +158,24 @@ __device__ __noinline__ void identity_swap_step(const BoxDev& b, const GcmcArgs*
     gen_first_trials(b, W, A[0].d.seed, A[0].d.stream, move, 1, b.charge[an.off], 1.0, b.meta[an.off].x, true, W.mx[0],
                      W.my[0], W.mz[0]);
     trial_pass_excl<PREC, CL>(b, W, 1, 1, an.comp, Nn, ao.comp, omol);
-    step_weight(W, 1, beta, an.bias, 0.0, 1.0, false);
-    bool ok = W.ok && W.w > 1e-150;
+    step_weight(W, 1, beta, an.bias, 0u, 1.0, false);
+    bool ok = W.ok && W.big;
     if (ok && tid == 0) {
       for (int k = 0; k < 4; ++k) s_e1[k] = W.te[k];
       s_w1 = W.w;
       W.mx[mso] = W.mx[0]; W.my[mso] = W.my[0]; W.mz[mso] = W.mz[0]; W.mq[mso] = b.charge[an.off];
     }
     __syncthreads();
-    double rosen = ok ? s_w1 : 0.0;
     double e2[4] = {0, 0, 0, 0};
     if (ok && msn > 1) {
       gen_orientations<PREC>(b, W, A[0].d.seed, A[0].d.stream, move, an.d.norient, msn - 1, an.off, 1.0, 1.0, W.mx[0],
                        W.my[0], W.mz[0], false, nullptr, nullptr, nullptr);
       trial_pass_excl<PREC, CL>(b, W, an.d.norient * (msn - 1), msn - 1, an.comp, Nn, ao.comp, omol);
-      step_weight(W, an.d.norient, beta, an.bias, u_orient, (double)an.d.norient, false);
+      step_weight(W, an.d.norient, beta, an.bias, u_orient, an.inv_norient, false, 0.0, &s_w1);
       ok = W.ok;
       if (ok) {
-        rosen *= W.w;
         for (int k = 0; k < 4; ++k) e2[k] = W.te[4 * W.sel + k];
-        if (rosen <= 1e-150) ok = false;
+        if (!W.big) ok = false;
         if (tid < msn - 1) {
           const Bead& bd = W.beads[W.sel * (msn - 1) + tid];
           W.mx[mso + 1 + tid] = bd.x; W.my[mso + 1 + tid] = bd.y; W.mz[mso + 1 + tid] = bd.z;
@@ -186,23 +190,21 @@ __device__ __noinline__ void identity_swap_step(const BoxDev& b, const GcmcArgs*
       gen_first_trials(b, W, A[0].d.seed, A[0].d.stream, move, 1, b.charge[ao.off], 1.0, b.meta[ao.off].x, true,
                        W.mx[0], W.my[0], W.mz[0]);
       trial_pass<PREC, CL>(b, W, 1, 1, ao.comp, omol);
-      step_weight(W, 1, beta, ao.bias, 0.0, 1.0, true);
+      step_weight(W, 1, beta, ao.bias, 0u, 1.0, true);
       bool ok2 = W.ok;
       if (ok2 && tid == 0) {
         for (int k = 0; k < 4; ++k) s_r1[k] = W.te[k];
         s_wr = W.w;
       }
       __syncthreads();
-      double rosen_old = ok2 ? s_wr : 0.0;
       double r2[4] = {0, 0, 0, 0};
       if (ok2 && mso > 1) {
         gen_orientations<PREC>(b, W, A[0].d.seed, A[0].d.stream, move, ao.d.norient, mso - 1, ao.off, 1.0, 1.0, W.mx[0],
                          W.my[0], W.mz[0], true, W.mx + 1, W.my + 1, W.mz + 1, SLOT_RETRACE);
         trial_pass<PREC, CL>(b, W, ao.d.norient * (mso - 1), mso - 1, ao.comp, omol);
-        step_weight(W, ao.d.norient, beta, ao.bias, 0.0, (double)ao.d.norient, true);
+        step_weight(W, ao.d.norient, beta, ao.bias, 0u, ao.inv_norient, true, 0.0, &s_wr);
         ok2 = W.ok;
         if (ok2) {
-          rosen_old *= W.w;
           for (int k = 0; k < 4; ++k) r2[k] = W.te[4 * W.sel + k];
         }
         __syncthreads();
@@ -217,7 +219,7 @@ __device__ __noinline__ void identity_swap_step(const BoxDev& b, const GcmcArgs*
             if (ao.rigid && ao.charged) same += ao.excl;
             ew = same + 2.0 * cross;
           }
-          rosen *= exp_move(-beta * ew);
+          const double rosen = s_w1 * exp_move(-beta * ew), rosen_old = s_wr;
           const double pre = beta * an.big_p / (1.0 + (double)Nn) * ((double)No / (beta * ao.big_p));
           const double pacc = pre * (rosen / an.d.ideal_rosenbluth) / (rosen_old / ao.d.ideal_rosenbluth);
           s_accept = u01(wx[3]) < pacc;
@@ -309,27 +311,33 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
     draw4_dev(A[0].d.seed, A[0].d.stream, move, SLOT_MOVE, w);
     draw4_dev(A[0].d.seed, A[0].d.stream, move, SLOT_DISP, w2);
     draw4_dev(A[0].d.seed, A[0].d.stream, move, SLOT_SELECT, ws);
-    const int sel = nm > 1 ? min(nm - 1, (int)(u01(w2[3]) * (double)nm)) : 0;
+    const int sel = nm > 1 ? pick(w2[3], nm) : 0;
     const GcmcArgs& a = A[sel];
     const grx_gcmc_desc& d = a.d;
     grx_gcmc_stats& st = ST[sel];
     const int comp = a.comp, ms = a.ms, chain = ms - 1, off = a.off;
     const int N = comp_size[comp] / ms;
-    const int mol = (int)(u01(w[0]) * (double)N);
-    const double r = u01(w[1]);
+    const int mol = pick(w[0], N);
     int kind = -1;
-    if (r < d.p_translation) kind = 0;
-    else if (r < d.p_rotation) kind = 1;
-    else if (r < d.p_reinsertion) kind = 4;
-    else if (IDS && r < d.p_identity_swap) kind = 5;
-    else if (r < d.p_swap) kind = (u01(w[2]) < 0.5) ? 2 : 3;
-    const double uacc = u01(w[3]);
+    if (w[1] < a.p_translation) kind = 0;
+    else if (w[1] < a.p_rotation) kind = 1;
+    else if (w[1] < a.p_reinsertion) kind = 4;
+    else if (IDS && w[1] < a.p_identity_swap) kind = 5;
+    else if (w[1] < a.p_swap) kind = w[2] < 0x80000000u ? 2 : 3;
     if (tid == 0) s_accept = 0;
 
     if ((kind == 0 || kind == 1) && N > 0) {
       // ---------------------------------------------- translation / rotation
       const int m0 = off + mol * ms;
       if (tid == 0) st.attempts[kind]++;
+      double2 ra, rb, rc;
+      if (kind == 1 && tid < 32) {  // the warp that moves the atoms (at most 32): one angle per lane, then shared
+        const int ax = min(tid, 2);
+        const double2 sc = rotation_sincos<PREC>(d.max_rotation[ax] * 2.0 * (u01(ax == 0 ? w2[0] : (ax == 1 ? w2[1] : w2[2])) - 0.5));
+        ra = make_double2(__shfl_sync(kFull, sc.x, 0), __shfl_sync(kFull, sc.y, 0));
+        rb = make_double2(__shfl_sync(kFull, sc.x, 1), __shfl_sync(kFull, sc.y, 1));
+        rc = make_double2(__shfl_sync(kFull, sc.x, 2), __shfl_sync(kFull, sc.y, 2));
+      }
       if (tid < ms) {
         const double4 p = b.pos64[m0 + tid];
         const double4 p0 = b.pos64[m0];
@@ -340,9 +348,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
           nz = p.z + d.max_translation[2] * 2.0 * (u01(w2[2]) - 0.5);
         } else {
           double vx = p.x - p0.x, vy = p.y - p0.y, vz = p.z - p0.z;
-          rotate_axis<PREC>(vx, vy, vz, d.max_rotation[0] * 2.0 * (u01(w2[0]) - 0.5), 0);
-          rotate_axis<PREC>(vx, vy, vz, d.max_rotation[1] * 2.0 * (u01(w2[1]) - 0.5), 1);
-          rotate_axis<PREC>(vx, vy, vz, d.max_rotation[2] * 2.0 * (u01(w2[2]) - 0.5), 2);
+          rotate_axes(vx, vy, vz, ra, rb, rc);
           nx = vx + p0.x; ny = vy + p0.y; nz = vz + p0.z;
         }
         W.mx[tid] = p.x; W.my[tid] = p.y; W.mz[tid] = p.z; W.mq[tid] = -p.w;
@@ -364,7 +370,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
           const double dr = (W.te[1] + W.te[3]) - (W.te[5] + W.te[7]);
           const double ew = same + 2.0 * cross;
           const double pacc = exp_move(-d.beta * (dv + dr + ew));
-          s_accept = uacc < pacc;
+          s_accept = u01(w[3]) < pacc;
           s_dE[0] = dv; s_dE[1] = dr; s_dE[2] = ew;
         }
       }
@@ -393,8 +399,8 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
       gen_first_trials(b, W, d.seed, d.stream, move, d.ntrials, b.charge[off], 1.0, b.meta[off].x, false, 0.0, 0.0,
                        0.0);
       trial_pass<PREC, CL>(b, W, d.ntrials, 1, comp, mol);
-      step_weight(W, d.ntrials, d.beta, a.bias, u01(ws[0]), (double)d.ntrials, false);
-      bool ok = W.ok && W.w > 1e-150;
+      step_weight(W, d.ntrials, d.beta, a.bias, ws[0], a.inv_ntrials, false);
+      bool ok = W.ok && W.big;
       double fx = 0, fy = 0, fz = 0;
       if (ok) {
         const Bead& fb = W.beads[W.sel];
@@ -407,18 +413,16 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
         }
       }
       __syncthreads();
-      double rosen = ok ? s_w1 : 0.0;
       double e2[4] = {0, 0, 0, 0};
       if (ok && chain > 0) {
         gen_orientations<PREC>(b, W, d.seed, d.stream, move, d.norient, chain, off, 1.0, 1.0, fx, fy, fz, false, nullptr,
                          nullptr, nullptr);
         trial_pass<PREC, CL>(b, W, d.norient * chain, chain, comp, mol);
-        step_weight(W, d.norient, d.beta, a.bias, u01(ws[1]), (double)d.norient, false);
+        step_weight(W, d.norient, d.beta, a.bias, ws[1], a.inv_norient, false, 0.0, &s_w1);
         ok = W.ok;
         if (ok) {
-          rosen *= W.w;
           for (int k = 0; k < 4; ++k) e2[k] = W.te[4 * W.sel + k];
-          if (rosen <= 1e-150) ok = false;
+          if (!W.big) ok = false;
           if (tid < chain) {
             const Bead& bd = W.beads[W.sel * chain + tid];
             W.mx[ms + 1 + tid] = bd.x; W.my[ms + 1 + tid] = bd.y; W.mz[ms + 1 + tid] = bd.z;
@@ -431,23 +435,21 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
         gen_first_trials(b, W, d.seed, d.stream, move, 1, b.charge[off], 1.0, b.meta[off].x, true, W.mx[0], W.my[0],
                          W.mz[0]);
         trial_pass<PREC, CL>(b, W, 1, 1, comp, mol);
-        step_weight(W, 1, d.beta, a.bias, 0.0, (double)d.ntrials, true, s_stored);
+        step_weight(W, 1, d.beta, a.bias, 0u, a.inv_ntrials, true, s_stored);
         bool ok2 = W.ok;
         if (ok2 && tid == 0) {
           for (int k = 0; k < 4; ++k) s_r1[k] = W.te[k];
           s_wr = W.w;
         }
         __syncthreads();
-        double rosen_old = ok2 ? s_wr : 0.0;
         double r2[4] = {0, 0, 0, 0};
         if (ok2 && chain > 0) {
           gen_orientations<PREC>(b, W, d.seed, d.stream, move, d.norient, chain, off, 1.0, 1.0, W.mx[0], W.my[0], W.mz[0],
                            true, W.mx + 1, W.my + 1, W.mz + 1, SLOT_RETRACE);
           trial_pass<PREC, CL>(b, W, d.norient * chain, chain, comp, mol);
-          step_weight(W, d.norient, d.beta, a.bias, 0.0, (double)d.norient, true);
+          step_weight(W, d.norient, d.beta, a.bias, 0u, a.inv_norient, true, 0.0, &s_wr);
           ok2 = W.ok;
           if (ok2) {
-            rosen_old *= W.w;
             for (int k = 0; k < 4; ++k) r2[k] = W.te[4 * W.sel + k];
           }
           __syncthreads();
@@ -457,9 +459,8 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
           if (a.charged) ewald_delta_move<PREC, CL>(b, W, 2 * ms, eik, same, cross);
           if (tid == 0) {
             const double ew = a.charged ? same + 2.0 * cross : 0.0;
-            rosen *= exp_move(-d.beta * ew);
-            const double pacc = rosen / rosen_old;
-            s_accept = uacc < pacc;
+            const double rosen = a.charged ? s_w1 * exp_move(-d.beta * ew) : s_w1;
+            s_accept = u01(w[3]) * s_wr < rosen;  // u < W_new / W_old
             s_dE[0] = s_e1[0] + s_e1[2] + e2[0] + e2[2] - (s_r1[0] + s_r1[2] + r2[0] + r2[2]);
             s_dE[1] = s_e1[1] + s_e1[3] + e2[1] + e2[3] - (s_r1[1] + s_r1[3] + r2[1] + r2[3]);
             s_dE[2] = ew;
@@ -491,8 +492,8 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
       gen_first_trials(b, W, d.seed, d.stream, move, d.ntrials, b.charge[off], 1.0, b.meta[off].x, del,
                        W.mx[0], W.my[0], W.mz[0]);
       trial_pass<PREC, CL>(b, W, d.ntrials, 1, comp, newmol);
-      step_weight(W, d.ntrials, d.beta, a.bias, u01(ws[0]), (double)d.ntrials, del);
-      bool ok = W.ok && W.w > 1e-150;
+      step_weight(W, d.ntrials, d.beta, a.bias, ws[0], a.inv_ntrials, del);
+      bool ok = W.ok && W.big;
       double fx = 0, fy = 0, fz = 0;
       if (ok) {
         const Bead& fb = W.beads[W.sel];
@@ -504,18 +505,16 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
         if (!del && tid == 0) { W.mx[0] = fx; W.my[0] = fy; W.mz[0] = fz; W.mq[0] = b.charge[off]; }
       }
       __syncthreads();
-      double rosen = ok ? s_w1 : 0.0;
       double e2[4] = {0, 0, 0, 0};
       if (ok && chain > 0) {
         gen_orientations<PREC>(b, W, d.seed, d.stream, move, d.norient, chain, off, 1.0, 1.0, fx, fy, fz, del,
                          W.mx + 1, W.my + 1, W.mz + 1);
         trial_pass<PREC, CL>(b, W, d.norient * chain, chain, comp, newmol);
-        step_weight(W, d.norient, d.beta, a.bias, u01(ws[1]), (double)d.norient, del);
+        step_weight(W, d.norient, d.beta, a.bias, ws[1], a.inv_norient, del, 0.0, &s_w1);
         ok = W.ok;
         if (ok) {
-          rosen *= W.w;
           for (int k = 0; k < 4; ++k) e2[k] = W.te[4 * W.sel + k];
-          if (rosen <= 1e-150) ok = false;
+          if (!W.big) ok = false;
           if (!del && tid < chain) {
             const Bead& bd = W.beads[W.sel * chain + tid];
             W.mx[1 + tid] = bd.x; W.my[1 + tid] = bd.y; W.mz[1 + tid] = bd.z;
@@ -533,22 +532,23 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
             if (a.rigid) same -= a.excl * (del ? (0.0 - 1.0) : (1.0 - 0.0));
             ew = same + 2.0 * cross;
           }
-          double pacc;
+          // the acceptance quotients with the divisors multiplied over to the other side
+          const double u = u01(w[3]);
+          double rosen = s_w1;
           if (!del) {
-            rosen *= exp_move(-d.beta * ew);
-            rosen *= exp_move(-d.beta * d.tail_insert);
-            pacc = d.beta * a.big_p / (1.0 + (double)N) * rosen / d.ideal_rosenbluth;
-            s_accept = rosen > 1e-150 && uacc < pacc;
+            if (a.charged) rosen *= exp_move(-d.beta * ew);
+            if (d.tail_insert != 0.0) rosen *= exp_move(-d.beta * d.tail_insert);
+            s_accept = rosen > 1e-150 && u * (1.0 + (double)N) < a.beta_p * rosen * a.inv_ideal;
             if (s_accept && (N + 1) * ms > a.cap) {
               s_accept = 0;
               st.capacity_hits++;
             }
           } else {
-            rosen /= exp_move(-d.beta * ew);
-            rosen /= exp_move(d.beta * d.tail_insert);  // the deletion's tail difference is -tail_insert
-            pacc = (double)N / (d.beta * a.big_p) * d.ideal_rosenbluth / rosen;
-            s_accept = uacc < pacc;
+            if (a.charged) rosen *= exp_move(d.beta * ew);
+            if (d.tail_insert != 0.0) rosen *= exp_move(-d.beta * d.tail_insert);  // the deletion's tail is -tail_insert
+            s_accept = u * a.beta_p * rosen < (double)N * d.ideal_rosenbluth;
           }
+          s_w1 = rosen;
           const double ev = s_e1[0] + s_e1[2] + e2[0] + e2[2];
           const double er = s_e1[1] + s_e1[3] + e2[1] + e2[3];
           const double sg = del ? -1.0 : 1.0;
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
         }
       }
       if (!del && tid == 0) {  // RecordRosen of the insertion: W, 0 when the growth failed
-        const double wr = ok ? rosen : 0.0;
+        const double wr = ok ? s_w1 : 0.0;
         st.rosen[0] += wr;
         st.rosen[1] += wr * wr;
         st.rosen[2] += 1.0;
@@ -585,7 +585,7 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
       }
     } else if (IDS && kind == 5) {
       if constexpr (IDS)
-        identity_swap_step<PREC, CL>(b, A, nm, ST, W, eik, comp_size, move, d.beta, u01(ws[1]), s_accept, s_e1,
+        identity_swap_step<PREC, CL>(b, A, nm, ST, W, eik, comp_size, move, d.beta, ws[1], s_accept, s_e1,
                                      s_w1, s_dE, s_r1, s_wr);
     }
     __syncthreads();
