@@ -131,25 +131,47 @@ __global__ void __launch_bounds__(kSkCols) sk_kernel(BoxDev b, SkChunks c, const
   if (jm >= 0) put(jm, make_double2(s0 + s1, s3 - s2));
 }
 
-// Sums the chunks of every active k in order, writes S(k) and adds the Fourier energies
-// (Ewald_Total, ewald_preparation.h:150-161): epart per block {gg, hh, hg}.
+// Sums the chunks of every active k, writes S(k) and adds the Fourier energies (Ewald_Total,
+// ewald_preparation.h:150-161): epart per block {gg, hh, hg}. Bound by the latency of the chunk
+// reads (the sums are in L2): a block takes one k per lane and every eighth chunk per warp, in a
+// fixed order, so there are eight reads in flight for one and eight times the blocks (one k per
+// thread and all chunks behind one another: 51 us for the 110 chunks of a 2300-atom framework).
+constexpr int kSkReduceK = 32;
 __global__ void __launch_bounds__(GRX_THREADS) sk_reduce_kernel(BoxDev b, const double2* part, int nh, int ng,
                                                                 double* epart) {
-  __shared__ double sbuf[32];
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr int W = GRX_THREADS / 32;
+  __shared__ double2 F[W][32], G[W][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int j = blockIdx.x * kSkReduceK + lane;
+  if (part) {
+    double2 f = make_double2(0.0, 0.0), a = f;
+    if (j < b.nact) {
+#pragma unroll 4
+      for (int k = w; k < nh; k += W) {
+        const double2 v = part[(size_t)k * b.nact + j];
+        f.x += v.x; f.y += v.y;
+      }
+#pragma unroll 4
+      for (int k = nh + w; k < nh + ng; k += W) {
+        const double2 v = part[(size_t)k * b.nact + j];
+        a.x += v.x; a.y += v.y;
+      }
+    }
+    F[w][lane] = f;
+    G[w][lane] = a;
+    __syncthreads();
+  }
+  if (w != 0) return;
   double gg = 0.0, hh = 0.0, hg = 0.0;
   if (j < b.nact) {
     const int slot = b.kact[j].w;
     double2 f, a;
     if (part) {
-      f = a = make_double2(0.0, 0.0);
-      for (int k = 0; k < nh; ++k) {
-        const double2 v = part[(size_t)k * b.nact + j];
-        f.x += v.x; f.y += v.y;
-      }
-      for (int k = nh; k < nh + ng; ++k) {
-        const double2 v = part[(size_t)k * b.nact + j];
-        a.x += v.x; a.y += v.y;
+      f = F[0][lane];
+      a = G[0][lane];
+      for (int k = 1; k < W; ++k) {
+        f.x += F[k][lane].x; f.y += F[k][lane].y;
+        a.x += G[k][lane].x; a.y += G[k][lane].y;
       }
       if (b.shared_host) f = b.s_fw[slot];  // a replica reads its parent's
       else b.s_fw[slot] = f;
@@ -164,10 +186,10 @@ __global__ void __launch_bounds__(GRX_THREADS) sk_reduce_kernel(BoxDev b, const 
     hh = t * (f.x * f.x + f.y * f.y);
     hg = t * (f.x * a.x + f.y * a.y) * 2.0;
   }
-  gg = block_sum(gg, sbuf);
-  hh = block_sum(hh, sbuf);
-  hg = block_sum(hg, sbuf);
-  if (threadIdx.x == 0) {
+  gg = warp_sum(gg);
+  hh = warp_sum(hh);
+  hg = warp_sum(hg);
+  if (lane == 0) {
     epart[3 * blockIdx.x] = gg;
     epart[3 * blockIdx.x + 1] = hh;
     epart[3 * blockIdx.x + 2] = hg;
@@ -425,7 +447,7 @@ static grx_status totals(grx_box* b, double* out8, double* pairs, uint8_t* overl
   const int nhost = r.base[r.nhost], nguest = r.n - nhost;
   const int nblk_atoms = (r.n + GRX_THREADS - 1) / GRX_THREADS;
   const int nblk_big = 4 * sms;
-  const int nblk_k = (b->nact + GRX_THREADS - 1) / GRX_THREADS;
+  const int nblk_k = (b->nact + kSkReduceK - 1) / kSkReduceK;
   // framework pairs count only between molecules or components
   int host_comps = 0;
   bool host_pairs = false;
