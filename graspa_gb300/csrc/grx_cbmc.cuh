@@ -43,7 +43,7 @@ struct CbmcWork {
   double ipart[kItems * 4];
   int iflag[kItems];
   int tdead[kCbmcBeads];  // per trial of a pass: early overlap rejection flag (-1: evaluated in full)
-  int qbuf[NW * kQueue];
+  alignas(16) int qbuf[NW * kQueue];  // the warps' pair queues; between passes the quaternions of gen_orientations
   double te[kMaxTrials * 4];
   int tflag[kMaxTrials];
   double sel_wa[kMaxTrials];
@@ -85,57 +85,19 @@ __device__ __noinline__ void gen_first_trials(const BoxDev& b, WK& W, uint64_t s
   __syncthreads();
 }
 
-// Rotate_Quaternions (mc_utilities.h:423-457): uniform rotation from (u, v, w).
-__device__ __forceinline__ void rotate_quaternion(double& x, double& y, double& z, double u, double v,
-                                                  double w) {
-  const double pi = 3.14159265358979323846;
-  double s1, c1, s2, c2;
-  sincos(2 * pi * v, &s1, &c1);
-  sincos(2 * pi * w, &s2, &c2);
-  const double q0 = sqrt(1 - u) * s1;
-  const double q1 = sqrt(1 - u) * c1;
-  const double q2 = sqrt(u) * s2;
-  const double q3 = sqrt(u) * c2;
-  const double a01 = q0 * q1, a02 = q0 * q2, a03 = q0 * q3;
-  const double a11 = q1 * q1, a12 = q1 * q2, a13 = q1 * q3;
-  const double a22 = q2 * q2, a23 = q2 * q3, a33 = q3 * q3;
-  const double r0 = 1.0 - 2.0 * (a22 + a33), r1 = 2.0 * (a12 - a03), r2 = 2.0 * (a13 + a02);
-  const double r3 = 2.0 * (a12 + a03), r4 = 1.0 - 2.0 * (a11 + a33), r5 = 2.0 * (a23 - a01);
-  const double r6 = 2.0 * (a13 - a02), r7 = 2.0 * (a23 + a01), r8 = 1.0 - 2.0 * (a11 + a22);
-  const double nx = x * r0 + y * r1 + z * r2;
-  const double ny = x * r3 + y * r4 + z * r5;
-  const double nz = x * r6 + y * r7 + z * r8;
-  x = nx; y = ny; z = nz;
-}
-
 // Trial orientations about the chosen first bead (fx, fy, fz): the vectors from the
 // component's slot-0 atom to its chain atoms, rotated by Philox quaternions. With
 // `retrace`, orientation 0 is the existing chain (ox/oy/oz arrays, chain atoms).
-// The mixed and FP32 forms rotate in double-float on the FP32 pipe (df_rotate_quaternion),
-// the FP64 form in FP64 (the oracle's arithmetic).
 template <int PREC, class WK>
 __device__ __noinline__ void gen_orientations(const BoxDev& b, WK& W, uint64_t seed, uint32_t stream,
                                                  uint64_t move, int no, int chain, int off, double scale_coul,
                                                  double scale, double fx, double fy, double fz, bool retrace,
                                                  const double* ox, const double* oy, const double* oz,
                                                  uint32_t slot_base = SLOT_ORIENT) {
-  for (int tid = threadIdx.x; tid < no * chain; tid += blockDim.x) {
-    const int o = tid / chain, at = tid % chain;
-    const double q = b.charge[off + 1 + at] * scale_coul;
-    const int type = b.meta[off + 1 + at].x;
-    if (retrace && o == 0) {
-      make_bead(W.beads[tid], ox[at], oy[at], oz[at], q, scale, type, b.prefactor);
-    } else {
-      uint32_t r[4];
-      draw4_dev(seed, stream, move, slot_base + o, r);
-      const double4 t0 = b.pos64[off];
-      const double4 pa = b.pos64[off + 1 + at];
-      double vx = pa.x - t0.x, vy = pa.y - t0.y, vz = pa.z - t0.z;
-      if constexpr (PREC == GRX_FP64) rotate_quaternion(vx, vy, vz, u01(r[0]), u01(r[1]), u01(r[2]));
-      else df_rotate_quaternion(vx, vy, vz, r[0], r[1], r[2]);
-      make_bead(W.beads[tid], fx + vx, fy + vy, fz + vz, q, scale, type, b.prefactor);
-    }
-  }
+  static_assert(sizeof(W.qbuf) >= 2 * kMaxTrials * sizeof(float4), "quaternions in the pair queues");
+  auto draw = [&](int o, uint32_t* r) { draw4_dev(seed, stream, move, slot_base + o, r); };
+  orientation_beads<PREC>(b, W.beads, reinterpret_cast<float4*>(W.qbuf), draw, no, chain, off, scale_coul, scale, fx, fy,
+                          fz, retrace, ox, oy, oz);
   __syncthreads();
 }
 

@@ -199,49 +199,40 @@ __device__ __forceinline__ float4 df_eik(double f, int k, df q) {
   return make_float4(r.hi, r.lo, i.hi, i.lo);
 }
 
-// (x, y, z) rotated by the quaternion of Rotate_Quaternions (mc_utilities.h:423-457, uniform
-// rotation from three uniforms) with the uniforms given as Philox words, in double-float on
-// the FP32 pipe: the same rotation as the FP64 form to ~1e-13 relative.
-__device__ __forceinline__ void df_rotate_quaternion_inl(double& x, double& y, double& z, uint32_t wu, uint32_t wv,
-                                                         uint32_t ww) {
+// The quaternion of Rotate_Quaternions (mc_utilities.h:423-457, uniform rotation from three
+// uniforms) with the uniforms given as Philox words, in double-float on the FP32 pipe, to ~1e-13
+// relative. Half 0: (q0, q1) from u and v, half 1: (q2, q3) from u and w.
+__device__ __forceinline__ float4 df_quaternion_half(uint32_t wu, uint32_t wangle, int half) {
   const df u = df_u01(wu);
-  df s1, c1, s2, c2;
-  df_sincos_2pi(df_u01(wv), s1, c1);
-  df_sincos_2pi(df_u01(ww), s2, c2);
-  const df a = df_sqrt(df_add_f(df{-u.hi, -u.lo}, 1.0f)), b = df_sqrt(u);
-  const df q0 = df_mul(a, s1), q1 = df_mul(a, c1), q2 = df_mul(b, s2), q3 = df_mul(b, c2);
-  const df a01 = df_mul(q0, q1), a02 = df_mul(q0, q2), a03 = df_mul(q0, q3);
-  const df a11 = df_mul(q1, q1), a12 = df_mul(q1, q2), a13 = df_mul(q1, q3);
-  const df a22 = df_mul(q2, q2), a23 = df_mul(q2, q3), a33 = df_mul(q3, q3);
-  auto two = [](df p) { return df{2.0f * p.hi, 2.0f * p.lo}; };
-  auto neg = [](df p) { return df{-p.hi, -p.lo}; };
-  auto one_minus_2 = [&](df p, df q) { return df_add_f(neg(two(df_add(p, q))), 1.0f); };
-  const df r0 = one_minus_2(a22, a33), r1 = two(df_add(a12, neg(a03))), r2 = two(df_add(a13, a02));
-  const df r3 = two(df_add(a12, a03)), r4 = one_minus_2(a11, a33), r5 = two(df_add(a23, neg(a01)));
-  const df r6 = two(df_add(a13, neg(a02))), r7 = two(df_add(a23, a01)), r8 = one_minus_2(a11, a22);
-  const df X = df_from(x), Y = df_from(y), Z = df_from(z);
-  const df nx = df_add(df_add(df_mul(X, r0), df_mul(Y, r1)), df_mul(Z, r2));
-  const df ny = df_add(df_add(df_mul(X, r3), df_mul(Y, r4)), df_mul(Z, r5));
-  const df nz = df_add(df_add(df_mul(X, r6), df_mul(Y, r7)), df_mul(Z, r8));
-  x = df_to(nx);
-  y = df_to(ny);
-  z = df_to(nz);
+  df s, c;
+  df_sincos_2pi(df_u01(wangle), s, c);
+  const df m = df_sqrt(half ? u : df_add_f(df{-u.hi, -u.lo}, 1.0f));
+  const df a = df_mul(m, s), b = df_mul(m, c);
+  return make_float4(a.hi, a.lo, b.hi, b.lo);
 }
 
-// Out of line (the orientation stages run it once per trial on few lanes; a smaller kernel
-// fetches fewer instructions), the result returned in registers.
-static __device__ __noinline__ double4 df_rotate_quaternion_out(double x, double y, double z, uint32_t wu,
-                                                                uint32_t wv, uint32_t ww) {
-  df_rotate_quaternion_inl(x, y, z, wu, wv, ww);
-  return make_double4(x, y, z, 0.0);
+// Component d of (x, y, z) rotated by the quaternion halves q[0], q[1]. With (i, j, k) the axes
+// d, d+1, d+2 and e the vector part, row d of the matrix is 1 - 2 (e_j^2 + e_k^2) at i,
+// 2 (e_i e_j - q0 e_k) at j and 2 (e_i e_k + q0 e_j) at k.
+__device__ __forceinline__ df df_rotated(float4 qa, float4 qb, int d, df x, df y, df z) {
+  const df q0 = {qa.x, qa.y}, q1 = {qa.z, qa.w}, q2 = {qb.x, qb.y}, q3 = {qb.z, qb.w};
+  auto pick3 = [d](df a, df b, df c) { return d == 0 ? a : (d == 1 ? b : c); };
+  const df ei = pick3(q1, q2, q3), ej = pick3(q2, q3, q1), ek = pick3(q3, q1, q2);
+  auto two = [](df p) { return df{2.0f * p.hi, 2.0f * p.lo}; };
+  auto neg = [](df p) { return df{-p.hi, -p.lo}; };
+  const df ti = df_mul(pick3(x, y, z), df_add_f(neg(two(df_add(df_mul(ej, ej), df_mul(ek, ek)))), 1.0f));
+  const df tj = df_mul(pick3(y, z, x), two(df_add(df_mul(ei, ej), neg(df_mul(q0, ek)))));
+  const df tk = df_mul(pick3(z, x, y), two(df_add(df_mul(ei, ek), df_mul(q0, ej))));
+  return df_add(df_add(pick3(ti, tk, tj), pick3(tj, ti, tk)), pick3(tk, tj, ti));  // x, y, z terms in turn
 }
 
 __device__ __forceinline__ void df_rotate_quaternion(double& x, double& y, double& z, uint32_t wu, uint32_t wv,
                                                      uint32_t ww) {
-  const double4 r = df_rotate_quaternion_out(x, y, z, wu, wv, ww);
-  x = r.x;
-  y = r.y;
-  z = r.z;
+  const float4 qa = df_quaternion_half(wu, wv, 0), qb = df_quaternion_half(wu, ww, 1);
+  const df X = df_from(x), Y = df_from(y), Z = df_from(z);
+  x = df_to(df_rotated(qa, qb, 0, X, Y, Z));
+  y = df_to(df_rotated(qa, qb, 1, X, Y, Z));
+  z = df_to(df_rotated(qa, qb, 2, X, Y, Z));
 }
 
 }  // namespace grx

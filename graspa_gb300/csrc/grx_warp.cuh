@@ -1,14 +1,14 @@
 // grx_warp.cuh -- the trial-bead pair engine: tile culling, FP32 screening, warp
 // compaction of in-cutoff pairs and dense evaluation.
 //
-// A work item is (one trial bead, one range of host tiles [+ the guest atoms]) and is
-// processed by one warp. For every 32-atom tile the warp first tests the tile's
-// bounding sphere against the cutoff (orthorhombic cells), then screens the 32 pairs
-// (split-coordinate FP32 in the mixed/FP32 forms, full FP64 in the FP64 form). Pairs
-// inside the screening radius are appended to a per-warp ring buffer in shared
-// memory; every 32 queued pairs are evaluated by all 32 lanes together, so the costly
-// part (FP64 displacement, LJ, real-space Coulomb) runs without idle lanes. The
-// order of every sum is fixed by the ballot order, so results are deterministic.
+// A work item is (one trial bead, one range of host units [+ the guest atoms]) and is
+// processed by one warp. A host unit is a 32-entry chunk of the bead's voxel list or a 32-atom
+// tile, whose bounds are tested against the cutoff first; the 32 pairs of a unit are screened
+// in FP32 (in the FP64 form only where FP32 decides, see pair_screen). Pairs inside the
+// screening radius are appended to a per-warp ring buffer in shared memory; every 32 queued
+// pairs are evaluated by all 32 lanes together, so the costly part (displacement, LJ,
+// real-space Coulomb) runs without idle lanes. The order of every sum is fixed by the ballot
+// order, so results are deterministic.
 #pragma once
 
 #include <limits.h>
@@ -1113,6 +1113,83 @@ static_assert(sizeof(Bead) % 8 == 0, "beads are staged in 8-byte words");
 template <int PREC>
 static inline void launch_trials(const BoxDev& b, const TrialArgs& a, int ntrials, cudaStream_t s) {
   trial_kernel<PREC><<<ntrials * kTrialCtas, kTrialWarps * 32, a.chain * sizeof(Bead), s>>>(b, a);
+}
+
+// Rotate_Quaternions (mc_utilities.h:423-457) in FP64: df_quaternion_half and df_rotated with the
+// uniforms u and v (half 0) or u and w (half 1).
+__device__ __forceinline__ double2 quaternion_half(double u, double angle, int half) {
+  double s, c;
+  sincos(2 * 3.14159265358979323846 * angle, &s, &c);
+  const double m = sqrt(half ? u : 1 - u);
+  return make_double2(m * s, m * c);
+}
+
+__device__ __forceinline__ double rotated(double2 qa, double2 qb, int d, double x, double y, double z) {
+  auto pick3 = [d](double a, double b, double c) { return d == 0 ? a : (d == 1 ? b : c); };
+  const double ei = pick3(qa.y, qb.x, qb.y), ej = pick3(qb.x, qb.y, qa.y), ek = pick3(qb.y, qa.y, qb.x);
+  const double ri = 1.0 - 2.0 * (ej * ej + ek * ek), rj = 2.0 * (ei * ej - qa.x * ek), rk = 2.0 * (ei * ek + qa.x * ej);
+  return x * pick3(ri, rk, rj) + y * pick3(rj, ri, rk) + z * pick3(rk, rj, ri);
+}
+
+// Beads of trial orientations, the whole block: no lane pairs form the quaternions (one sine and
+// cosine each, in `quat`, 2 per orientation), then a warp takes ten beads, a lane one coordinate of
+// one. The mixed and FP32 forms rotate in double-float on the FP32 pipe, the FP64 form in FP64 (the
+// oracle's arithmetic). The stage runs once per move on few lanes, so the length of a lane's chain
+// is its time: with a bead's three coordinates and both sines on one lane it took 17 k of the 205 k
+// cycles of a CO2 move (456 mixed chains 5.70 ms a pass, 5.47 ms so). retrace: orientation 0 is the
+// existing chain ox / oy / oz.
+// draw(o, r): the Philox words of orientation o.
+template <int PREC, class Draw>
+__device__ __forceinline__ void orientation_beads(const BoxDev& b, Bead* beads, float4* quat, Draw draw, int no,
+                                                  int chain, int off, double scale_coul, double scale, double fx,
+                                                  double fy, double fz, bool retrace, const double* ox,
+                                                  const double* oy, const double* oz) {
+  for (int t = threadIdx.x; t < 2 * no; t += blockDim.x) {
+    uint32_t r[4];
+    draw(t >> 1, r);
+    const uint32_t angle = t & 1 ? r[2] : r[1];
+    if constexpr (PREC == GRX_FP64) reinterpret_cast<double2*>(quat)[t] = quaternion_half(u01(r[0]), u01(angle), t & 1);
+    else quat[t] = df_quaternion_half(r[0], angle, t & 1);
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, k = lane / 3, d = lane - 3 * k, nb = no * chain;
+  for (int base = 10 * (int)(threadIdx.x >> 5); base < nb; base += 10 * (int)(blockDim.x >> 5)) {
+    const int t = base + k;
+    const bool live = k < 10 && t < nb;
+    float h = 0.0f, l;
+    if (live) {
+      const int o = t / chain, at = t - o * chain;
+      double c;
+      if (retrace && o == 0) {
+        c = d == 0 ? ox[at] : (d == 1 ? oy[at] : oz[at]);
+      } else {
+        const double4 t0 = b.pos64[off], pa = b.pos64[off + 1 + at];
+        const double x = pa.x - t0.x, y = pa.y - t0.y, z = pa.z - t0.z;
+        if constexpr (PREC == GRX_FP64) {
+          const double2* q = reinterpret_cast<const double2*>(quat) + 2 * o;
+          c = rotated(q[0], q[1], d, x, y, z);
+        } else {
+          c = df_to(df_rotated(quat[2 * o], quat[2 * o + 1], d, df_from(x), df_from(y), df_from(z)));
+        }
+        c += d == 0 ? fx : (d == 1 ? fy : fz);
+      }
+      split_coord(c, h, l);
+      Bead& bd = beads[t];
+      (&bd.x)[d] = c;
+      (&bd.h.x)[d] = h;
+      (&bd.l.x)[d] = l;
+      if (d == 0) {
+        const double q = b.charge[off + 1 + at] * scale_coul;
+        const df pq = df_from(b.prefactor * q);
+        bd.q = q;
+        bd.scale = scale;
+        bd.type = b.meta[off + 1 + at].x;
+        bd.pq = make_float2(pq.hi, pq.lo);
+      }
+    }
+    const unsigned near = __ballot_sync(kFull, fabsf(h) < kNearCoord);
+    if (live && d == 0) beads[t].unit = (scale == 1.0 ? 1 : 0) | (((near >> lane) & 7u) == 7u ? 2 : 0);
+  }
 }
 
 }  // namespace grx

@@ -55,35 +55,12 @@ __device__ bool select_trial_warp(const double* te, const int* tflag, int nt, do
   return true;
 }
 
-// Rotate_Quaternions (mc_utilities.h:423-457): uniform rotation from (u, v, w).
-__device__ __forceinline__ void rotate_quaternion(double& x, double& y, double& z, double u, double v,
-                                                  double w) {
-  const double pi = 3.14159265358979323846;
-  double s1, c1, s2, c2;
-  sincos(2 * pi * v, &s1, &c1);
-  sincos(2 * pi * w, &s2, &c2);
-  const double q0 = sqrt(1 - u) * s1;
-  const double q1 = sqrt(1 - u) * c1;
-  const double q2 = sqrt(u) * s2;
-  const double q3 = sqrt(u) * c2;
-  const double a01 = q0 * q1, a02 = q0 * q2, a03 = q0 * q3;
-  const double a11 = q1 * q1, a12 = q1 * q2, a13 = q1 * q3;
-  const double a22 = q2 * q2, a23 = q2 * q3, a33 = q3 * q3;
-  const double r0 = 1.0 - 2.0 * (a22 + a33), r1 = 2.0 * (a12 - a03), r2 = 2.0 * (a13 + a02);
-  const double r3 = 2.0 * (a12 + a03), r4 = 1.0 - 2.0 * (a11 + a33), r5 = 2.0 * (a23 - a01);
-  const double r6 = 2.0 * (a13 - a02), r7 = 2.0 * (a23 + a01), r8 = 1.0 - 2.0 * (a11 + a22);
-  const double nx = x * r0 + y * r1 + z * r2;
-  const double ny = x * r3 + y * r4 + z * r5;
-  const double nz = x * r6 + y * r7 + z * r8;
-  x = nx; y = ny; z = nz;
-}
-
 template <int PREC>
 __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomArgs a, grx_widom_result* out) {
   __shared__ Bead beads[GRX_MAX_TRIAL_BEADS];
   __shared__ double ipart[kMaxItems * 4];
   __shared__ int iflag[kMaxItems];
-  __shared__ int qbuf[(GRX_THREADS / 32) * kQueue];
+  __shared__ alignas(16) int qbuf[(GRX_THREADS / 32) * kQueue];
   __shared__ int counter;
   __shared__ double te[kMaxTrials * 4];
   __shared__ int tflag[kMaxTrials];
@@ -98,7 +75,6 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
   const int tid = threadIdx.x;
   const int off = b.comp_off[a.comp];
   const int ms = a.molsize, chain = ms - 1;
-  const double4 t0 = b.pos64[off];
   for (int64_t m = blockIdx.x; m < a.n; m += gridDim.x) {
     const uint64_t move = a.first_move + (uint64_t)m;
     uint32_t selw[4];
@@ -151,17 +127,10 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
       // 4. orientations about the chosen first bead (mc_widom.h:255-276)
       const int no = a.norient, nb = no * chain;
       const double fx = newx[0], fy = newy[0], fz = newz[0];
-      if (tid < nb) {
-        const int o = tid / chain, at = tid % chain;
-        uint32_t r[4];
-        draw4(a.seed, a.stream, move, SLOT_ORIENT + o, r);
-        const double4 pa = b.pos64[off + 1 + at];
-        double vx = pa.x - t0.x, vy = pa.y - t0.y, vz = pa.z - t0.z;
-        if constexpr (PREC == GRX_FP64) rotate_quaternion(vx, vy, vz, u01(r[0]), u01(r[1]), u01(r[2]));
-        else df_rotate_quaternion(vx, vy, vz, r[0], r[1], r[2]);
-        make_bead(beads[tid], fx + vx, fy + vy, fz + vz, b.charge[off + 1 + at] * a.scale_coul, a.scale,
-                  b.meta[off + 1 + at].x, b.prefactor);
-      }
+      static_assert(sizeof(qbuf) >= 2 * kMaxTrials * sizeof(float4), "quaternions in the pair queues");
+      auto draw = [&](int o, uint32_t* r) { draw4(a.seed, a.stream, move, SLOT_ORIENT + o, r); };
+      orientation_beads<PREC>(b, beads, reinterpret_cast<float4*>(qbuf), draw, no, chain, off, a.scale_coul, a.scale, fx,
+                              fy, fz, false, nullptr, nullptr, nullptr);
       if (tid == 0) counter = 0;
       if (tid < no) tdead[tid] = 0;
       __syncthreads();

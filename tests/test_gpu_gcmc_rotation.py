@@ -40,6 +40,20 @@ def test_rotation_of_long_molecules(grx_lib, ms, prec):
     assert np.max(np.abs(box.positions(1) - after["pos"][nfw:])) <= 1e-9
 
 
+@pytest.mark.parametrize("prec", ["GRX_FP64", "GRX_MIXED"])
+@pytest.mark.parametrize("ms,norient", [(2, 1), (2, 64), (11, 1), (12, 1), (12, 11), (32, 4)])
+def test_orientations_across_warps(grx_lib, ms, norient, prec):
+    """Orientation beads at the edges of a warp's ten and of the block's eighty: 1, 64, 10, 11, 121
+    and 124 beads, grown and retraced by reinsertions."""
+    s = helix_system(ms)
+    d = params(grx_lib, p_translation=0.2, p_rotation=0.4, p_reinsertion=1.0, max_rotation=0.1, max_translation=0.3,
+               norient=norient)
+    box, st, ost, after = run_pair(grx_lib, s, d, 60, getattr(grx_lib, prec))
+    assert list(st.attempts) == list(ost.attempts) and list(st.accepted) == list(ost.accepted)
+    assert st.attempts[4] > 20
+    assert np.max(np.abs(box.positions(1) - after["pos"][s["comp_start"][1]:])) <= 1e-9
+
+
 @pytest.mark.parametrize("edges", [(0.0, 0.0, 0.0, 1.0), (0.0, 1.0, 1.0, 1.0), (0.1, 0.1, 0.1, 0.1), (1.0, 1.0, 1.0, 1.0),
                                    (-1.0, 0.3, 0.3, 7.0)])
 def test_move_choice_edges(grx_lib, edges):
