@@ -72,16 +72,8 @@ template <class WK>
 __device__ __noinline__ void gen_first_trials(const BoxDev& b, WK& W, uint64_t seed, uint32_t stream,
                                                  uint64_t move, int nt, double q, double scale, int type,
                                                  bool retrace, double ox, double oy, double oz) {
-  for (int t = threadIdx.x; t < nt; t += blockDim.x) {
-    if (retrace && t == 0) {
-      make_bead(W.beads[0], ox, oy, oz, q, scale, type, b.prefactor);
-    } else {
-      uint32_t r[4];
-      draw4_dev(seed, stream, move, SLOT_FIRST + t, r);
-      make_bead(W.beads[t], b.cell[0] * u01(r[0]), b.cell[4] * u01(r[1]), b.cell[8] * u01(r[2]), q, scale, type,
-                b.prefactor);
-    }
-  }
+  auto draw = [&](int t, uint32_t* r) { draw4_dev(seed, stream, move, SLOT_FIRST + t, r); };
+  first_beads(b, W.beads, draw, nt, q, scale, type, retrace, ox, oy, oz);
   __syncthreads();
 }
 

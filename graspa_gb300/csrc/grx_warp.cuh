@@ -1131,6 +1131,51 @@ __device__ __forceinline__ double rotated(double2 qa, double2 qb, int d, double 
   return x * pick3(ri, rk, rj) + y * pick3(rj, ri, rk) + z * pick3(rk, rj, ri);
 }
 
+// make_bead by three lanes, 3 k + d of a warp the coordinate c of bead k along d (the whole warp
+// calls; live: the lane has a coordinate). FP64 issues once for the three coordinates.
+__device__ __forceinline__ void put_bead(const BoxDev& b, Bead& bd, int lane, int d, bool live, double c, double q,
+                                         double scale, int type) {
+  float h = 0.0f, l;
+  if (live) {
+    split_coord(c, h, l);
+    (&bd.x)[d] = c;
+    (&bd.h.x)[d] = h;
+    (&bd.l.x)[d] = l;
+    if (d == 0) {
+      const df pq = df_from(b.prefactor * q);
+      bd.q = q;
+      bd.scale = scale;
+      bd.type = type;
+      bd.pq = make_float2(pq.hi, pq.lo);
+    }
+  }
+  const unsigned near = __ballot_sync(kFull, fabsf(h) < kNearCoord);
+  if (live && d == 0) bd.unit = (scale == 1.0 ? 1 : 0) | (((near >> lane) & 7u) == 7u ? 2 : 0);
+}
+
+// First-bead trials of a growth, the whole block: cell diagonal x Philox uniforms
+// (mc_widom.h:133-139), a lane per coordinate. retrace: trial 0 is the bead (ox, oy, oz).
+template <class Draw>
+__device__ __forceinline__ void first_beads(const BoxDev& b, Bead* beads, Draw draw, int nt, double q, double scale,
+                                            int type, bool retrace, double ox, double oy, double oz) {
+  const int lane = threadIdx.x & 31, k = lane / 3, d = lane - 3 * k;
+  for (int base = 10 * (int)(threadIdx.x >> 5); base < nt; base += 10 * (int)(blockDim.x >> 5)) {
+    const int t = base + k;
+    const bool live = k < 10 && t < nt;
+    double c = 0.0;
+    if (live) {
+      if (retrace && t == 0) {
+        c = d == 0 ? ox : (d == 1 ? oy : oz);
+      } else {
+        uint32_t r[4];
+        draw(t, r);
+        c = b.cell[4 * d] * u01(d == 0 ? r[0] : (d == 1 ? r[1] : r[2]));
+      }
+    }
+    put_bead(b, beads[live ? t : 0], lane, d, live, c, q, scale, type);
+  }
+}
+
 // Beads of trial orientations, the whole block: no lane pairs form the quaternions (one sine and
 // cosine each, in `quat`, 2 per orientation), then a warp takes ten beads, a lane one coordinate of
 // one. The mixed and FP32 forms rotate in double-float on the FP32 pipe, the FP64 form in FP64 (the
@@ -1156,39 +1201,27 @@ __device__ __forceinline__ void orientation_beads(const BoxDev& b, Bead* beads, 
   for (int base = 10 * (int)(threadIdx.x >> 5); base < nb; base += 10 * (int)(blockDim.x >> 5)) {
     const int t = base + k;
     const bool live = k < 10 && t < nb;
-    float h = 0.0f, l;
+    double c = 0.0, q = 0.0;
+    int type = 0;
     if (live) {
       const int o = t / chain, at = t - o * chain;
-      double c;
       if (retrace && o == 0) {
         c = d == 0 ? ox[at] : (d == 1 ? oy[at] : oz[at]);
       } else {
         const double4 t0 = b.pos64[off], pa = b.pos64[off + 1 + at];
         const double x = pa.x - t0.x, y = pa.y - t0.y, z = pa.z - t0.z;
         if constexpr (PREC == GRX_FP64) {
-          const double2* q = reinterpret_cast<const double2*>(quat) + 2 * o;
-          c = rotated(q[0], q[1], d, x, y, z);
+          const double2* p = reinterpret_cast<const double2*>(quat) + 2 * o;
+          c = rotated(p[0], p[1], d, x, y, z);
         } else {
           c = df_to(df_rotated(quat[2 * o], quat[2 * o + 1], d, df_from(x), df_from(y), df_from(z)));
         }
         c += d == 0 ? fx : (d == 1 ? fy : fz);
       }
-      split_coord(c, h, l);
-      Bead& bd = beads[t];
-      (&bd.x)[d] = c;
-      (&bd.h.x)[d] = h;
-      (&bd.l.x)[d] = l;
-      if (d == 0) {
-        const double q = b.charge[off + 1 + at] * scale_coul;
-        const df pq = df_from(b.prefactor * q);
-        bd.q = q;
-        bd.scale = scale;
-        bd.type = b.meta[off + 1 + at].x;
-        bd.pq = make_float2(pq.hi, pq.lo);
-      }
+      q = b.charge[off + 1 + at] * scale_coul;
+      type = b.meta[off + 1 + at].x;
     }
-    const unsigned near = __ballot_sync(kFull, fabsf(h) < kNearCoord);
-    if (live && d == 0) beads[t].unit = (scale == 1.0 ? 1 : 0) | (((near >> lane) & 7u) == 7u ? 2 : 0);
+    put_bead(b, beads[live ? t : 0], lane, d, live, c, q, scale, type);
   }
 }
 

@@ -89,12 +89,8 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
     // 1. first-bead trials (mc_widom.h:133-139)
     const int nt = a.ntrials;
     if (tid < nt) tdead[tid] = 0;
-    if (tid < nt) {
-      uint32_t r[4];
-      draw4(a.seed, a.stream, move, SLOT_FIRST + tid, r);
-      make_bead(beads[tid], b.cell[0] * u01(r[0]), b.cell[4] * u01(r[1]), b.cell[8] * u01(r[2]),
-                b.charge[off] * a.scale_coul, a.scale, b.meta[off].x, b.prefactor);
-    }
+    auto draw_first = [&](int t, uint32_t* r) { draw4(a.seed, a.stream, move, SLOT_FIRST + t, r); };
+    first_beads(b, beads, draw_first, nt, b.charge[off] * a.scale_coul, a.scale, b.meta[off].x, false, 0.0, 0.0, 0.0);
     __syncthreads();
     // 2. pair energies of the first-bead trials
     {
