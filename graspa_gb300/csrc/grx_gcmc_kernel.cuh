@@ -39,7 +39,9 @@ struct GcmcArgs {
   int64_t step_off;
   int64_t nsteps_cap;
   // what a step would otherwise form in FP64 on every warp: cumulative move probabilities p as
-  // ceil(p 2^32) against the move word (the same comparison as word 2^-32 < p), reciprocals
+  // ceil(p 2^32) against the move word (the same comparison as word 2^-32 < p), reciprocals. With
+  // the acceptance on one warp and the axis rotations below: 456 CO2 chains 5.92 -> 5.69 ms a pass,
+  // 64 CH4/Xe boxes 3.36 -> 2.85 ms
   uint64_t p_translation, p_rotation, p_reinsertion, p_identity_swap, p_swap;
   double inv_ntrials, inv_norient, inv_ideal;
   double beta_p;  // beta * big_p
