@@ -250,11 +250,6 @@ __device__ __forceinline__ float vdw32(float4 f, float rr) {
 }
 
 // CoulombReal(), maths.cuh:496-500, with q already multiplied by scaleCoul.
-__device__ __forceinline__ double coul64(const BoxDev& b, double qq, double rr) {
-  const double r = sqrt(rr);
-  return b.prefactor * qq * erfc(b.alpha * r) / r;
-}
-
 __device__ __forceinline__ float coul32(const BoxDev& b, float qq, float rr) {
   const float r = sqrtf(rr);
   return (float)b.prefactor * qq * erfcf((float)b.alpha * r) / r;
