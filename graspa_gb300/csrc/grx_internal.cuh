@@ -85,7 +85,7 @@ struct BoxDev {
   const unsigned short* htype;   // host atoms: type | 0x8000 when scale != 1
   const int4* vmeta;     // per voxel {first entry, sure atoms, all atoms, 0}
   const unsigned* vlist; // entries: storage index | lattice shift << 20
-  const float4* vshift;  // lattice vector of every shift code, hi parts
+  const float4* vshift;  // lattice vector of every shift code
   int vox;               // 0 tile path, 1 entries carry their image, 2 images by rounded fractions
   int vn[3];             // voxels along a, b, c
   int vchunks;           // 32-entry chunks of the longest list

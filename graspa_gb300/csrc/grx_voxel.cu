@@ -249,7 +249,7 @@ grx_status build_voxels(grx_box* b) {
   for (int c = 0; c < 512; ++c) {
     const double n[3] = {(c & 7) - 4.0, ((c >> 3) & 7) - 4.0, (c >> 6) - 4.0};
     float v[3];
-    for (int k = 0; k < 3; ++k) v[k] = (float)(n[0] * d.cell_hi[k] + n[1] * d.cell_hi[3 + k] + n[2] * d.cell_hi[6 + k]);
+    for (int k = 0; k < 3; ++k) v[k] = (float)(n[0] * d.cell[k] + n[1] * d.cell[3 + k] + n[2] * d.cell[6 + k]);
     shift[c] = make_float4(v[0], v[1], v[2], 0.0f);
   }
   if (b->arena) {  // in an arena the lists are optional: take them only with room to spare
