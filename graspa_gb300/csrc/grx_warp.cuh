@@ -529,8 +529,8 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
             pass = qx * qx + qy * qy + qz * qz <= b.cull_r * b.cull_r;
             one_image = trl.w != 0 && fabsf(dx) + th.x + 1e-2f < 0.5f * b.cellf[0] &&
                         fabsf(dy) + th.y + 1e-2f < 0.5f * b.cellf[4] && fabsf(dz) + th.z + 1e-2f < 0.5f * b.cellf[8];
-            sx = nx * b.cell_hi[0]; sy = ny * b.cell_hi[4]; sz = nz * b.cell_hi[8];
-            // far images: n times the dropped low part of the cell would pass the screen's guard band
+            // the whole edges: n times their low parts alone would pass the screen's guard band
+            sx = nx * b.cellf[0]; sy = ny * b.cellf[4]; sz = nz * b.cellf[8];
             if (PREC == GRX_FP64) one_image = one_image && fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz)) <= 4.0f;
           } else {
             const float fx = b.invf[0] * dx + b.invf[3] * dy + b.invf[6] * dz;

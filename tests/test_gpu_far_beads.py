@@ -1,9 +1,9 @@
-"""Beads many cells from the home cell (unwrapped positions) on voxel lists: pairs next to the cutoff
-must survive the FP32 screen at any distance. Beads sit 1e-4 to 2e-3 A inside the cutoff of a
+"""Beads many cells from the home cell (unwrapped positions) on voxel lists and on tiles: pairs next to
+the cutoff must survive the FP32 screen at any distance. Beads sit 1e-4 to 2e-3 A inside the cutoff of a
 framework atom's image, up to 60 cells out (2,400 A), on a thinned framework (12 atoms, LJ unshifted),
 so that one lost pair is a large part of a trial's energy.
 
-Bars, with M the sum of the magnitudes of a trial's pair terms (no atom nearer than 10 A, where a term
+Bars, with M the sum of the magnitudes of a trial's pair terms (no atom nearer than 9 A, where a term
 changes by at most 2.5 of itself per A): a displacement at 2,400 A carries 1e-12 A on either side, so
 1e-11 M for FP64; 1e-6 kT (and 1e-6 M) for the mixed form; the FP32 form keeps a displacement to 1e-6 A
 and its functions to 1e-5: 1e-4 M. The smallest term of every trial is at least twice its bar (checked).
@@ -19,12 +19,16 @@ pytestmark = pytest.mark.gpu
 LATTICES = [(0, 0, 0), (0, 0, 5), (12, 0, 0), (0, 0, 25), (0, 0, 40), (20, -20, 10), (-30, 25, 30), (0, 0, 60)]
 
 
-def _system(which):
-    """Twelve framework atoms of the system's framework, charges of both signs, no LJ shift."""
+def _system(which, path):
+    """Twelve framework atoms of the system's framework (spread, or in a cluster: a tile with one image),
+    no LJ shift."""
     s = {"silica": synth.silica_co2, "triclinic": lambda: synth.adsorbate_system("CO2", 3, n_atoms=1500),
          "skewed": lambda: synth.adsorbate_system("CO2", 11, n_atoms=1500)}[which]()
     n, rng = s["comp_start"][1], np.random.default_rng(2)
     keep = np.sort(rng.choice(n, 12, replace=False))
+    if path == "tiles":
+        middle = 0.5 * np.array(s["cell"]).reshape(3, 3).sum(0)
+        keep = np.sort(np.argsort(np.linalg.norm(s["pos"][:n] - middle, axis=1))[:12])
     s["molsize"] = [12] + list(s["molsize"][1:])
     synth._set_atoms(s, s["pos"][keep], s["type"][keep], s["charge"][keep], [np.zeros((0, 3))])
     s["shift"] = np.zeros_like(s["shift"])
@@ -46,10 +50,13 @@ def _terms(s, p, q, ty):
 
 @pytest.mark.parametrize("prec", ["fp64", "mixed", "fp32"])
 @pytest.mark.parametrize("which", ["silica", "triclinic", "skewed"])
-def test_pairs_at_the_cutoff_far_from_home(grx_lib, which, prec):
-    s = _system(which)
+@pytest.mark.parametrize("path", ["lists", "tiles"])
+def test_pairs_at_the_cutoff_far_from_home(grx_lib, path, which, prec):
+    s = _system(which, path)
     box = grx_lib.Box(s, capacity=[12, 64])
     assert box.voxel_lists()[0]
+    if path == "tiles":
+        box.set_voxel_lists(0)
     cell = np.array(s["cell"]).reshape(3, 3)
     rng = np.random.default_rng(9)
     n = 600
@@ -62,7 +69,7 @@ def test_pairs_at_the_cutoff_far_from_home(grx_lib, which, prec):
     q, ty = np.full(n, tm["charge"][-1]), np.full(n, tm["type"][-1])
     lj, co, r = _terms(s, p, q, ty)
     least = np.where(co != 0, np.abs(co), np.inf).min(1)
-    keep = (r.min(1) > 10.0) & (least > 0.01)
+    keep = (r.min(1) > 9.0) & (least > 0.01)
     p, q, ty, lj, co, least = p[keep], q[keep], ty[keep], lj[keep], co[keep], least[keep]
     n = len(p)
     assert n >= 60
