@@ -25,8 +25,12 @@ void set_error(const char* fmt, ...) {
   va_end(ap);
 }
 
+// The status of a failed runtime call. Its error is reported here, so it is taken off the runtime too
+// (a context-wide one stays): callers that go on without the memory they asked for (totals in one
+// chunk, boxes without voxel lists) would meet it again at their next launch check.
 grx_status cuda_status(cudaError_t e, const char* what) {
   set_error("%s: %s", what, cudaGetErrorString(e));
+  cudaGetLastError();
   if (e == cudaErrorMemoryAllocation) return GRX_ERR_OUT_OF_MEMORY;
   if (e == cudaErrorNoDevice || e == cudaErrorInsufficientDriver) return GRX_ERR_NO_DEVICE;
   return GRX_ERR_CUDA;
