@@ -86,6 +86,8 @@ grx_status ensure_pinned(grx_box* b, size_t bytes) {
   return GRX_OK;
 }
 
+cudaError_t uploads_done() { return cudaStreamSynchronize(nullptr); }
+
 static bool plain_host(const void* p) {
   cudaPointerAttributes a;
   if (!p) return false;  // the runtime reports it
@@ -749,7 +751,7 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
     cudaMemcpy(b->kcol, b->h_kcol.data(), b->h_kcol.size() * sizeof(int4), cudaMemcpyHostToDevice);
     cudaMemcpy(b->kgroup, b->h_kgroup.data(), b->h_kgroup.size() * sizeof(int2), cudaMemcpyHostToDevice);
   }
-  if ((e = cudaStreamSynchronize(nullptr)) != cudaSuccess) return fail(e, "box upload");
+  if ((e = uploads_done()) != cudaSuccess) return fail(e, "box upload");
   if (!ff.no_charges) {
     grx_status st = build_coulomb_table(b, g.alpha, ff.cutoff_coul_sq);
     if (st) {
@@ -761,6 +763,7 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
       diag += 0.5 * std::sqrt(g.cell[3 * k] * g.cell[3 * k] + g.cell[3 * k + 1] * g.cell[3 * k + 1] +
                               g.cell[3 * k + 2] * g.cell[3 * k + 2]);
     attach_tables64(b, g.alpha, ff.cutoff_coul_sq, diag * diag);
+    if ((e = uploads_done()) != cudaSuccess) return fail(e, "table upload");
   }
   refresh_dev(b);
   *out = b;
@@ -1025,7 +1028,10 @@ grx_status grx_box_set_component(grx_box* b, int32_t comp, const grx_atoms* a, i
   if (comp < b->nhost) {
     grx_status st = build_tiles(b);
     if (st) return st;
-    st = build_voxels(b);
+  }
+  GRX_CHECK_CUDA(uploads_done(), "grx_box_set_component");
+  if (comp < b->nhost) {
+    grx_status st = build_voxels(b);
     if (st) return st;
   }
   b->sk_valid = false;
@@ -1080,6 +1086,7 @@ grx_status grx_ewald_set_structure_factors(grx_box* b, const double* s_fw, const
   GRX_CHECK_CUDA(cudaMemcpy(b->s_fw, s_fw, b->nvec * sizeof(double2), cudaMemcpyDefault), "set S_fw");
   GRX_CHECK_CUDA(cudaMemcpy(b->s_ads, s_ads, b->nvec * sizeof(double2), cudaMemcpyDefault), "set S_ads");
   GRX_CHECK_CUDA(cudaMemcpy(b->s_tmp, s_ads, b->nvec * sizeof(double2), cudaMemcpyDefault), "set S_tmp");
+  GRX_CHECK_CUDA(uploads_done(), "grx_ewald_set_structure_factors");
   b->sk_valid = true;
   b->ewdf_valid = false;
   return GRX_OK;

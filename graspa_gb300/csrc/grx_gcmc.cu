@@ -452,6 +452,7 @@ extern "C" grx_status grx_gcmc_batch_set_box_steps(grx_gcmc_batch* B, const uint
   }
   GRX_CHECK_CUDA(cudaMemcpy(B->d_args, B->h_args.data(), B->nentries * sizeof(GcmcArgs), cudaMemcpyHostToDevice),
                  "upload box steps");
+  GRX_CHECK_CUDA(uploads_done(), "upload box steps");
   drop_graph(B);
   return GRX_OK;
 }
@@ -527,6 +528,7 @@ static grx_status upload_mult(grx_gcmc_batch* B, int mult) {
     hb[i] = B->boxes[i]->dev;
   }
   GRX_CHECK_CUDA(cudaMemcpy(B->d_boxes, hb.data(), nb * sizeof(BoxDev), cudaMemcpyHostToDevice), "shape upload");
+  GRX_CHECK_CUDA(uploads_done(), "shape upload");
   return GRX_OK;
 }
 

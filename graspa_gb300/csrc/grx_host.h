@@ -126,6 +126,10 @@ grx_status ensure_results(grx_box* b, size_t n);
 // CUDA runtime knows (device, managed, pinned) through it.
 grx_status fetch(void* dst, const void* src, size_t bytes, const char* what);
 grx_status deliver(void* dst, const void* src, size_t bytes, const char* what);
+// A cudaMemcpy from pageable memory may return with its last part still on the way to the device, and
+// a non-blocking stream is not ordered behind the default stream that carries it: what uploads this
+// way ends with this wait, since the calls that follow start their kernels with no copy before them.
+cudaError_t uploads_done();
 void refresh_dev(grx_box* b);
 int sm_count(grx_box* b);
 void* arena_alloc(grx_arena* a, size_t bytes);

@@ -270,7 +270,9 @@ grx_status build_voxels(grx_box* b) {
     refresh_dev(b);
     return GRX_OK;
   }
-  GRX_CHECK_CUDA(cudaMemcpy(b->vmeta, meta.data(), meta.size() * sizeof(int4), cudaMemcpyHostToDevice), "upload voxels");
+  // on the box's stream: the kernel takes its write offsets from these records
+  GRX_CHECK_CUDA(cudaMemcpyAsync(b->vmeta, meta.data(), meta.size() * sizeof(int4), cudaMemcpyHostToDevice, b->stream),
+                 "upload voxels");
   voxel_scan_kernel<<<grid, 32 * kVoxelWarps, 0, b->stream>>>(b->dev, v, b->vmeta, b->vlist);
   count_launch();
   GRX_CHECK_CUDA(cudaGetLastError(), "voxel list launch");
