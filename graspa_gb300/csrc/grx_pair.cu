@@ -134,21 +134,23 @@ grx_status grx_single_body_energy(grx_box* b, const grx_trials* old_mol, const g
   if (!st) st = ensure_pinned(b, bead_bytes + 8 * sizeof(double) + 8);
   if (st) return st;
   Bead* beads = (Bead*)b->pinned;
-  make_beads(hn, 0, ms, b->dev.prefactor, beads);
-  make_beads(ho, 0, ms, b->dev.prefactor, beads + ms);
-  // two trials: the new molecule and the old one, each without the atoms of its own molecule id
+  // up to two trials, the new molecule and the old one, each without the atoms of its own molecule id.
+  // Only what is asked for runs: the other side may hold anything (its types index the pair tables).
+  const int nconf = (do_new ? 1 : 0) + (do_old ? 1 : 0);
+  if (do_new) make_beads(hn, 0, ms, b->dev.prefactor, beads);
+  if (do_old) make_beads(ho, 0, ms, b->dev.prefactor, beads + (nconf - 1) * ms);
   TrialArgs a{};
   a.beads = beads;
   a.chain = (int)ms;
   a.component = component;
-  a.mol[0] = (int)new_mol->molid;
+  a.mol[0] = (int)(do_new ? new_mol->molid : old_mol->molid);
   a.mol[1] = (int)old_mol->molid;
   a.split = 1;
   a.excl_comp = -1;
   a.excl_mol = -1;
   a.out = (double*)((char*)b->pinned + bead_bytes);
   a.over = (unsigned char*)(a.out + 8);
-  run_trials(b, a, 2, prec == GRX_MIXED ? kMixed64 : (int)prec);
+  run_trials(b, a, nconf, prec == GRX_MIXED ? kMixed64 : (int)prec);
   GRX_CHECK_CUDA(cudaGetLastError(), "single body launch");
   GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "single body");
   const double* r = a.out;
@@ -158,7 +160,7 @@ grx_status grx_single_body_energy(grx_box* b, const grx_trials* old_mol, const g
   for (int q = 0; q < 4; ++q) {
     double d = 0.0;
     if (do_new) d += r[q];
-    if (do_old) d -= r[4 + q];
+    if (do_old) d -= r[4 * (nconf - 1) + q];
     e[host_slot + q] = d;
   }
   const int flag = do_new && a.over[0];
