@@ -150,7 +150,7 @@ grx_status grx_single_body_energy(grx_box* b, const grx_trials* old_mol, const g
   a.excl_mol = -1;
   a.out = (double*)((char*)b->pinned + bead_bytes);
   a.over = (unsigned char*)(a.out + 8);
-  run_trials(b, a, nconf, prec == GRX_MIXED ? kMixed64 : (int)prec);
+  run_trials(b, a, nconf, prec == GRX_FP64 ? (int)GRX_FP64 : (prec == GRX_MIXED ? kMixed64 : (int)GRX_FP32));
   GRX_CHECK_CUDA(cudaGetLastError(), "single body launch");
   GRX_CHECK_CUDA(cudaStreamSynchronize(b->stream), "single body");
   const double* r = a.out;

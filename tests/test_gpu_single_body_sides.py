@@ -31,3 +31,15 @@ def test_sides_of_a_delta(grx_lib, component, beads, lists, prec):
     assert np.array_equal(only_new + only_old, both)
     assert np.any(only_new != 0) and np.any(only_old != 0)
     assert f_new == flag and f_old == 0
+
+
+def test_any_other_precision_is_fp32(grx_lib):
+    """The entry point takes every value past the two wider forms as FP32."""
+    s = synth.silica_co2(n_co2=4)
+    nfw = s["comp_start"][1]
+    box = grx_lib.Box(s, capacity=[nfw, 64])
+    old = dict(pos=s["pos"][nfw:nfw + 3], charge=s["charge"][nfw:nfw + 3], type=s["type"][nfw:nfw + 3], molid=0)
+    new = dict(old, pos=old["pos"] + 0.2)
+    want, _ = box.single_body(old, new, 1, prec=grx_lib.GRX_FP32)
+    for prec in (3, 4, -1):
+        assert np.array_equal(box.single_body(old, new, 1, prec=prec)[0], want), prec
