@@ -8,7 +8,7 @@
 #include "grx_internal.cuh"
 
 namespace grx {
-// Device copies of the FP64 tables of one (device, alpha, cutoff^2, largest image distance^2):
+// Device copies of the FP64 tables of one (device, alpha, range of g, range of h):
 // freed when the last holder (a box, or an arena for its boxes) lets go.
 struct Tables64 {
   int device = 0;

@@ -103,11 +103,12 @@ void attach_tables64(grx_box* b, double alpha, double cut2, double smax) {
   if (!(alpha > 0.0) || !(cut2 > kTableMin) || !std::isfinite(smax) || smax > 1e12) return;
   // whole octaves of h, so that cells of similar size share a table
   double top = kTableMin;
-  while (top <= std::max(smax, cut2) * (1.0 + 1e-6)) top *= 2.0;
-  // past alpha^2 s = 20 (erfc below 3e-10) the Gaussian tail would need finer pieces: library functions
-  const double gtop = std::min(cut2 * (1.0 + 1e-9), 20.0 / (alpha * alpha));
+  while (top <= smax * (1.0 + 1e-6)) top *= 2.0;
+  // g to the cutoff, or to the longest image distance (the cutoff may be infinite). Past alpha^2 s = 20
+  // (erfc below 3e-10) the Gaussian tail would need finer pieces: library functions
+  const double gtop = std::min({cut2 * (1.0 + 1e-9), top, 20.0 / (alpha * alpha)});
   if (!(gtop > kTableMin)) return;
-  const std::tuple<int, double, double, double> key(b->device, alpha, cut2, top);
+  const std::tuple<int, double, double, double> key(b->device, alpha, gtop, top);
   std::lock_guard<std::mutex> lock(g_mutex);
   for (auto it = g_live.begin(); it != g_live.end();) it = it->second.expired() ? g_live.erase(it) : std::next(it);
   auto it = g_live.find(key);
