@@ -62,35 +62,37 @@ __global__ void eik_tables_kernel(BoxDev b, CompRanges r, int first, double2* ex
 // four real sums with Re Z and Im Z give both +kz and -kz, two FP64 FMAs per (k, atom) where
 // the direct product of three factors takes ten. FP64 issue (two lanes per SM and clock)
 // bounds it. Chunks hold framework or adsorbate atoms only; their partial S(k) go to `part`
-// [chunk][active k], or straight into the structure factors when there is one chunk of each.
+// [chunk][active k].
 constexpr int kSkCols = 128;
 constexpr int kSkRows = 32;
 constexpr int kSkTile = 32;
 
 struct SkChunks {
-  int n, nhost, n_host_chunks;  // atoms, framework atoms, chunks of them (0 when the framework's S is a parent's)
-  int host_len, guest_len;      // atoms per chunk
+  int n, nhost, n_host_chunks, n_chunks;  // atoms, framework atoms, chunks of them (0 when the framework's S is a parent's), all chunks
+  int host_len, guest_len;                // atoms per chunk
+  __device__ __forceinline__ void range(int k, int& a0, int& a1) const {
+    const bool host = k < n_host_chunks;
+    a0 = host ? k * host_len : nhost + (k - n_host_chunks) * guest_len;
+    a1 = host ? min(a0 + host_len, nhost) : min(a0 + guest_len, n);
+  }
 };
+constexpr int kSkSums = GRX_THREADS / 32;  // sums per k that the chunks are spread over (the warps of sk_reduce_kernel)
 
-__global__ void __launch_bounds__(kSkCols) sk_kernel(BoxDev b, SkChunks c, const KRow* rows, const int2* groups,
-                                                     const double2* ex, const double2* ey, const double2* ez,
-                                                     double2* part) {
-  __shared__ double2 P[kSkRows][kSkTile + 1];
-  __shared__ KRow R[kSkRows];
-  const int tid = threadIdx.x;
-  const int2 g = groups[blockIdx.x];
-  const int nr = g.y - g.x;
+// The rows of the block's group in R, the row of this thread's column; returns |kz| of the column.
+__device__ __forceinline__ int sk_column(const KRow* rows, int2 g, KRow* R, int& row) {
+  const int tid = threadIdx.x, nr = g.y - g.x;
   for (int k = tid; k < nr; k += blockDim.x) R[k] = rows[g.x + k];
   __syncthreads();
-  int row = 0;
+  row = 0;
   while (row + 1 < nr && tid >= R[row + 1].col) ++row;
-  const int az = tid - R[row].col;
-  const bool live = az < R[row].ncol;
-  const int chunk = blockIdx.y;
-  const bool host = chunk < c.n_host_chunks;
-  const int a0 = host ? chunk * c.host_len : c.nhost + (chunk - c.n_host_chunks) * c.guest_len;
-  const int a1 = host ? min(a0 + c.host_len, c.nhost) : min(a0 + c.guest_len, c.n);
-  const int kz1 = b.kmax[2] + 1;
+  return tid - R[row].col;
+}
+
+// S(+kz) and S(-kz) of this thread's column over the atoms [a0, a1), by the whole block.
+__device__ __forceinline__ void sk_sums(const BoxDev& b, int n, double2 (*P)[kSkTile + 1], const KRow* R, int nr, int row,
+                                        int az, bool live, int a0, int a1, const double2* ex, const double2* ey,
+                                        const double2* ez, double2& plus, double2& minus) {
+  const int tid = threadIdx.x, kz1 = b.kmax[2] + 1;
   const double2* z = ez + (live ? az : 0);
   double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
   for (int t0 = a0; t0 < a1; t0 += kSkTile) {
@@ -98,9 +100,9 @@ __global__ void __launch_bounds__(kSkCols) sk_kernel(BoxDev b, SkChunks c, const
       const int k = e / kSkTile, at = e % kSkTile, j = t0 + at;
       double2 v = make_double2(0.0, 0.0);
       if (j < a1) {
-        double2 y = ey[(size_t)abs(R[k].ky) * c.n + j];
+        double2 y = ey[(size_t)abs(R[k].ky) * n + j];
         if (R[k].ky < 0) y.y = -y.y;
-        v = cmul(ex[(size_t)R[k].kx * c.n + j], y);
+        v = cmul(ex[(size_t)R[k].kx * n + j], y);
       }
       P[k][at] = v;
     }
@@ -119,16 +121,69 @@ __global__ void __launch_bounds__(kSkCols) sk_kernel(BoxDev b, SkChunks c, const
     }
     __syncthreads();
   }
+  plus = make_double2(s0 - s1, s2 + s3);
+  minus = make_double2(s0 + s1, s3 - s2);
+}
+
+__global__ void __launch_bounds__(kSkCols) sk_kernel(BoxDev b, SkChunks c, const KRow* rows, const int2* groups,
+                                                     const double2* ex, const double2* ey, const double2* ez,
+                                                     double2* part) {
+  __shared__ double2 P[kSkRows][kSkTile + 1];
+  __shared__ KRow R[kSkRows];
+  const int2 g = groups[blockIdx.x];
+  int row;
+  const int az = sk_column(rows, g, R, row);
+  const bool live = az < R[row].ncol;
+  const int chunk = blockIdx.y;
+  int a0, a1;
+  c.range(chunk, a0, a1);
+  double2 plus, minus;
+  sk_sums(b, c.n, P, R, g.y - g.x, row, az, live, a0, a1, ex, ey, ez, plus, minus);
   if (!live) return;
-  double2* out = part ? part + (size_t)chunk * b.nact : nullptr;
-  double2* in_place = host ? b.s_fw : b.s_ads;
-  auto put = [&](int j, double2 v) {
-    if (out) out[j] = v;
-    else in_place[b.kact[j].w] = v;
-  };
+  double2* out = part + (size_t)chunk * b.nact;
   const int jp = R[row].index(az), jm = az ? R[row].index(-az) : -1;
-  if (jp >= 0) put(jp, make_double2(s0 - s1, s2 + s3));
-  if (jm >= 0) put(jm, make_double2(s0 + s1, s3 - s2));
+  if (jp >= 0) out[jp] = plus;
+  if (jm >= 0) out[jm] = minus;
+}
+
+// Without room for the chunks' partial sums: a block walks the chunks of one kind (blockIdx.y 0 the
+// framework's, 1 the adsorbates') behind one another and adds them up as sk_reduce_kernel does,
+// every eighth chunk to one of eight sums, so that S(k) is the same to the last bit whatever the
+// memory has room for.
+__global__ void __launch_bounds__(kSkCols) sk_in_place_kernel(BoxDev b, SkChunks c, const KRow* rows,
+                                                              const int2* groups, const double2* ex, const double2* ey,
+                                                              const double2* ez) {
+  __shared__ double2 P[kSkRows][kSkTile + 1];
+  __shared__ KRow R[kSkRows];
+  const int2 g = groups[blockIdx.x];
+  int row;
+  const int az = sk_column(rows, g, R, row);
+  const bool live = az < R[row].ncol;
+  const bool host = blockIdx.y == 0;
+  const int first = host ? 0 : c.n_host_chunks, end = host ? c.n_host_chunks : c.n_chunks;
+  if (first == end) return;
+  double2 sp[kSkSums], sm[kSkSums];
+  for (int w = 0; w < kSkSums; ++w) sp[w] = sm[w] = make_double2(0.0, 0.0);
+  for (int k0 = first; k0 < end; k0 += kSkSums)
+#pragma unroll
+    for (int w = 0; w < kSkSums; ++w) {
+      if (k0 + w >= end) break;
+      int a0, a1;
+      c.range(k0 + w, a0, a1);
+      double2 plus, minus;
+      sk_sums(b, c.n, P, R, g.y - g.x, row, az, live, a0, a1, ex, ey, ez, plus, minus);
+      sp[w].x += plus.x; sp[w].y += plus.y;
+      sm[w].x += minus.x; sm[w].y += minus.y;
+    }
+  if (!live) return;
+  for (int w = 1; w < kSkSums; ++w) {
+    sp[0].x += sp[w].x; sp[0].y += sp[w].y;
+    sm[0].x += sm[w].x; sm[0].y += sm[w].y;
+  }
+  double2* out = host ? b.s_fw : b.s_ads;
+  const int jp = R[row].index(az), jm = az ? R[row].index(-az) : -1;
+  if (jp >= 0) out[b.kact[jp].w] = sp[0];
+  if (jm >= 0) out[b.kact[jm].w] = sm[0];
 }
 
 // Sums the chunks of every active k, writes S(k) and adds the Fourier energies (Ewald_Total,
@@ -140,7 +195,7 @@ __global__ void __launch_bounds__(kSkCols) sk_kernel(BoxDev b, SkChunks c, const
 constexpr int kSkReduceK = 32;
 __global__ void __launch_bounds__(GRX_THREADS) sk_reduce_kernel(BoxDev b, const double2* part, int nh, int ng,
                                                                 double* epart) {
-  constexpr int W = GRX_THREADS / 32;
+  constexpr int W = kSkSums;
   __shared__ double2 F[W][32], G[W][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int j = blockIdx.x * kSkReduceK + lane;
@@ -490,11 +545,7 @@ static grx_status totals(grx_box* b, double* out8, double* pairs, uint8_t* overl
   }
   const size_t fixed = ntab * sizeof(double2) + n_out * sizeof(double);
   st = ensure_scratch(b, fixed + part_bytes);
-  if (st == GRX_ERR_OUT_OF_MEMORY && part_bytes) {  // one chunk of each kind writes S(k) in place
-    ck.host_len = std::max(kSkTile, fw_atoms);
-    ck.guest_len = std::max(kSkTile, nguest);
-    ck.n_host_chunks = fw_atoms ? 1 : 0;
-    nchunks = ck.n_host_chunks + (nguest ? 1 : 0);
+  if (st == GRX_ERR_OUT_OF_MEMORY && part_bytes) {  // the same sums, written in place chunk after chunk
     part_bytes = 0;
     st = ensure_scratch(b, fixed);
   }
@@ -514,8 +565,11 @@ static grx_status totals(grx_box* b, double* out8, double* pairs, uint8_t* overl
     const int first = b->parent ? nhost : 0;
     if (r.n > first)
       eik_tables_kernel<<<dim3((r.n - first + 127) / 128, 3), 128, 0, s>>>(b->dev, r, first, ex, ey, ez);
-    if (nchunks)
+    ck.n_chunks = nchunks;
+    if (part)
       sk_kernel<<<dim3(b->n_kgroups, nchunks), kSkCols, 0, s>>>(b->dev, ck, b->krow, b->kgroup, ex, ey, ez, part);
+    else if (nchunks)
+      sk_in_place_kernel<<<dim3(b->n_kgroups, 2), kSkCols, 0, s>>>(b->dev, ck, b->krow, b->kgroup, ex, ey, ez);
     count_launch((r.n > first) + (nchunks > 0));
   }
   if (b->nact > 0) {
