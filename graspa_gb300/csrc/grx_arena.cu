@@ -7,7 +7,6 @@
 #include <map>
 #include <mutex>
 #include <unordered_map>
-#include <vector>
 
 #include "grx_host.h"
 
@@ -20,26 +19,11 @@ struct grx_arena {
   std::unordered_map<size_t, size_t> used_;   // offset -> length
   size_t in_use = 0;
   size_t peak = 0;
-  std::vector<std::shared_ptr<const grx::Tables64>> kept_;  // FP64 tables of its boxes, at most kArenaTables
 };
 
 namespace grx {
 
 static constexpr size_t kArenaAlign = 256;
-static constexpr size_t kArenaTables = 16;
-
-// The oldest kept tables make room for new ones beyond the bound.
-void arena_keep(grx_arena* a, const std::shared_ptr<const Tables64>& t) {
-  std::shared_ptr<const Tables64> old;  // released after the lock
-  std::lock_guard<std::mutex> g(a->m);
-  for (const auto& k : a->kept_)
-    if (k == t) return;
-  if (a->kept_.size() >= kArenaTables) {
-    old = a->kept_.front();
-    a->kept_.erase(a->kept_.begin());
-  }
-  a->kept_.push_back(t);
-}
 
 void* arena_alloc(grx_arena* a, size_t bytes) {
   const size_t need = (std::max<size_t>(bytes, 1) + kArenaAlign - 1) / kArenaAlign * kArenaAlign;

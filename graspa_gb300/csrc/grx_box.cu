@@ -758,11 +758,11 @@ static grx_status box_create(const grx_box_desc* desc, grx_arena* arena, grx_box
       grx_box_destroy(b);
       return st;
     }
-    double diag = 0.0;  // no image picked by rounded fractions is longer than half the summed edges
-    for (int k = 0; k < 3; ++k)
-      diag += 0.5 * std::sqrt(g.cell[3 * k] * g.cell[3 * k] + g.cell[3 * k + 1] * g.cell[3 * k + 1] +
-                              g.cell[3 * k + 2] * g.cell[3 * k + 2]);
-    attach_tables64(b, g.alpha, ff.cutoff_coul_sq, diag * diag);
+    st = attach_tables64(b, g.alpha, ff.cutoff_coul_sq, g.cell);
+    if (st) {
+      grx_box_destroy(b);
+      return st;
+    }
     if ((e = uploads_done()) != cudaSuccess) return fail(e, "table upload");
   }
   refresh_dev(b);
@@ -804,6 +804,7 @@ grx_status grx_box_footprint(const grx_box_desc* desc, size_t* bytes) {
     std::memcpy(&lb, &s_lo, 4);
     std::memcpy(&hb, &s_hi, 4);
     t += al(2 * (size_t)((int)(hb >> 17) - (int)(lb >> 17) + 2) * sizeof(float4));
+    t += al(tables64_bytes(desc->geometry.alpha, desc->forcefield.cutoff_coul_sq, desc->geometry.cell));
   }
   t += al((size_t)1 << 20) + al(1024 * sizeof(grx_widom_result));  // first scratch and result buffers
   *bytes = t;

@@ -8,11 +8,12 @@
 #include "grx_internal.cuh"
 
 namespace grx {
-// Device copies of the FP64 tables of one (device, alpha, range of g, range of h):
-// freed when the last holder (a box, or an arena for its boxes) lets go.
+// Device copy of the FP64 tables of one (device, arena, alpha, range of g, range of h), shared by the
+// boxes that use them and given back (to the arena, which costs the device no wait) with the last one.
 struct Tables64 {
   int device = 0;
-  double2* g = nullptr;
+  grx_arena* arena = nullptr;
+  double2* g = nullptr;  // g's pieces, h's behind them
   double2* h = nullptr;
   int g_base = 0, g_n = 0, h_base = 0, h_n = 0;
   ~Tables64();
@@ -140,11 +141,11 @@ cudaError_t dev_alloc(grx_box* b, void** p, size_t bytes);
 // for replicas) and marks them valid.
 grx_status ewald_df_refresh(grx_box* b);
 void dev_free(grx_box* b, void* p);
-// The FP64 Coulomb tables of the box (grx_table.cu); without device memory for them the box
-// runs on the library functions.
-void attach_tables64(grx_box* b, double alpha, double cut2, double smax);
-// Keeps the tables of an arena's boxes until the arena goes (retiring a box must not free device memory).
-void arena_keep(grx_arena* a, const std::shared_ptr<const Tables64>& t);
+// The FP64 Coulomb tables of the box (grx_table.cu). In an arena they are part of the box
+// (tables64_bytes of its footprint); elsewhere, without device memory for them, the box runs on the
+// library functions.
+grx_status attach_tables64(grx_box* b, double alpha, double cut2, const double* cell);
+size_t tables64_bytes(double alpha, double cut2, const double* cell);
 // Voxel candidate lists of the machine's host atoms (grx_voxel.cu), rebuilt after the tiles.
 grx_status build_voxels(grx_box* b);
 }  // namespace grx

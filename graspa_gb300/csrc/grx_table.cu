@@ -18,8 +18,10 @@
 #include <cmath>
 #include <cstring>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "grx_host.h"
@@ -58,9 +60,11 @@ double centre_value(double alpha, double s, bool complement, double ex) {
   return q + (std::fma(-q, r, f) + df - q * dr) / r;
 }
 
+int pieces(double smax, int shift) { return (high_word(smax) >> shift) - (high_word(kTableMin) >> shift) + 1; }
+
 void fit(double alpha, double smax, bool complement, int shift, int& base, int& n, std::vector<double>& tab) {
   base = high_word(kTableMin) >> shift;
-  n = (high_word(smax) >> shift) - base + 1;
+  n = pieces(smax, shift);
   tab.assign(6 * (size_t)n, 0.0);
   const double a2 = alpha * alpha, K = alpha / std::sqrt(3.14159265358979323846) * (complement ? 1.0 : -1.0);
   for (int k = 0; k < n; ++k) {
@@ -84,53 +88,105 @@ void fit(double alpha, double smax, bool complement, int shift, int& base, int& 
   }
 }
 
-std::mutex g_mutex;
-std::map<std::tuple<int, double, double, double>, std::weak_ptr<const Tables64>> g_live;
+// Ranges of g and h for a box, 0 where it has no tables (it runs on the library functions then).
+struct Range64 {
+  double g = 0.0, h = 0.0;
+  bool any() const { return g > 0.0; }
+};
 
-}  // namespace
-
-Tables64::~Tables64() {
-  int prev = -1;
-  cudaGetDevice(&prev);
-  if (prev != device) cudaSetDevice(device);
-  cudaFree(g);
-  cudaFree(h);
-  if (prev >= 0 && prev != device) cudaSetDevice(prev);
-}
-
-void attach_tables64(grx_box* b, double alpha, double cut2, double smax) {
-  b->t64.reset();
-  if (!(alpha > 0.0) || !(cut2 > kTableMin) || !std::isfinite(smax) || smax > 1e12) return;
+Range64 range64(double alpha, double cut2, const double* cell) {
+  double diag = 0.0;  // no image picked by rounded fractions is longer than half the summed edges
+  for (int k = 0; k < 3; ++k)
+    diag += 0.5 * std::sqrt(cell[3 * k] * cell[3 * k] + cell[3 * k + 1] * cell[3 * k + 1] + cell[3 * k + 2] * cell[3 * k + 2]);
+  const double smax = diag * diag;
+  if (!(alpha > 0.0) || !(cut2 > kTableMin) || !std::isfinite(smax) || smax > 1e12) return {};
   // whole octaves of h, so that cells of similar size share a table
   double top = kTableMin;
   while (top <= smax * (1.0 + 1e-6)) top *= 2.0;
   // g to the cutoff, or to the longest image distance (the cutoff may be infinite). Past alpha^2 s = 20
   // (erfc below 3e-10) the Gaussian tail would need finer pieces: library functions
   const double gtop = std::min({cut2 * (1.0 + 1e-9), top, 20.0 / (alpha * alpha)});
-  if (!(gtop > kTableMin)) return;
-  const std::tuple<int, double, double, double> key(b->device, alpha, gtop, top);
+  if (!(gtop > kTableMin)) return {};
+  return {gtop, top};
+}
+
+constexpr size_t kPieceBytes = 6 * sizeof(double);
+
+// The fitted pieces, g then h, of the last few ranges: a serving process creates boxes of few kinds
+// over and over, and a fit evaluates some 8,000 pieces on the host.
+using Fitted = std::shared_ptr<const std::vector<double>>;
+using FitKey = std::tuple<double, double, double>;
+constexpr size_t kFits = 16;
+
+std::mutex g_mutex;
+std::map<std::tuple<int, const grx_arena*, double, double, double>, std::weak_ptr<const Tables64>> g_live;
+std::vector<std::pair<FitKey, Fitted>> g_fits;  // at most kFits, the oldest first
+
+Fitted fitted(double alpha, const Range64& r) {
+  const FitKey key(alpha, r.g, r.h);
+  for (const auto& f : g_fits)
+    if (f.first == key) return f.second;
+  int base, n;
+  std::vector<double> g, h;
+  fit(alpha, r.g, true, kShiftG64, base, n, g);
+  fit(alpha, r.h, false, kShiftH64, base, n, h);
+  g.insert(g.end(), h.begin(), h.end());
+  if (g_fits.size() >= kFits) g_fits.erase(g_fits.begin());
+  g_fits.emplace_back(key, std::make_shared<const std::vector<double>>(std::move(g)));
+  return g_fits.back().second;
+}
+
+}  // namespace
+
+Tables64::~Tables64() {
+  if (arena) {
+    arena_free(arena, g);
+    return;
+  }
+  int prev = -1;
+  cudaGetDevice(&prev);
+  if (prev != device) cudaSetDevice(device);
+  cudaFree(g);
+  if (prev >= 0 && prev != device) cudaSetDevice(prev);
+}
+
+size_t tables64_bytes(double alpha, double cut2, const double* cell) {
+  const Range64 r = range64(alpha, cut2, cell);
+  return r.any() ? (size_t)(pieces(r.g, kShiftG64) + pieces(r.h, kShiftH64)) * kPieceBytes : 0;
+}
+
+grx_status attach_tables64(grx_box* b, double alpha, double cut2, const double* cell) {
+  b->t64.reset();
+  const Range64 r = range64(alpha, cut2, cell);
+  if (!r.any()) return GRX_OK;
   std::lock_guard<std::mutex> lock(g_mutex);
   for (auto it = g_live.begin(); it != g_live.end();) it = it->second.expired() ? g_live.erase(it) : std::next(it);
-  auto it = g_live.find(key);
-  std::shared_ptr<const Tables64> t = it != g_live.end() ? it->second.lock() : nullptr;
-  if (!t) {
-    auto n = std::make_shared<Tables64>();
-    n->device = b->device;
-    std::vector<double> g, h;
-    fit(alpha, gtop, true, kShiftG64, n->g_base, n->g_n, g);
-    fit(alpha, top, false, kShiftH64, n->h_base, n->h_n, h);
-    if (cudaMalloc((void**)&n->g, g.size() * sizeof(double)) != cudaSuccess ||
-        cudaMalloc((void**)&n->h, h.size() * sizeof(double)) != cudaSuccess ||
-        cudaMemcpy(n->g, g.data(), g.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(n->h, h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
-      cudaGetLastError();
-      return;  // the library functions serve the box
+  std::weak_ptr<const Tables64>& live = g_live[std::make_tuple(b->device, (const grx_arena*)b->arena, alpha, r.g, r.h)];
+  b->t64 = live.lock();
+  if (b->t64) return GRX_OK;
+  const Fitted tab = fitted(alpha, r);
+  auto n = std::make_shared<Tables64>();
+  n->device = b->device;
+  n->arena = b->arena;
+  n->g_base = high_word(kTableMin) >> kShiftG64;
+  n->g_n = pieces(r.g, kShiftG64);
+  n->h_base = high_word(kTableMin) >> kShiftH64;
+  n->h_n = pieces(r.h, kShiftH64);
+  const size_t bytes = tab->size() * sizeof(double);
+  if (dev_alloc(b, (void**)&n->g, bytes) != cudaSuccess) {
+    n->g = nullptr;
+    if (b->arena) {  // counted in grx_box_footprint; a box's arithmetic must not depend on its neighbours
+      set_error("FP64 tables: %zu bytes do not fit the arena", bytes);
+      return GRX_ERR_OUT_OF_MEMORY;
     }
-    t = n;
-    g_live[key] = t;
+    cudaGetLastError();
+    return GRX_OK;  // the library functions serve the box
   }
-  b->t64 = t;
-  if (b->arena) arena_keep(b->arena, t);
+  n->h = n->g + 3 * (size_t)n->g_n;
+  GRX_CHECK_CUDA(cudaMemcpy(n->g, tab->data(), bytes, cudaMemcpyHostToDevice), "upload FP64 tables");
+  b->t64 = n;
+  live = b->t64;
+  return GRX_OK;
 }
 
 }  // namespace grx

@@ -233,8 +233,10 @@ grx_status grx_arena_destroy(grx_arena* arena);      /* every box in it destroye
 grx_status grx_arena_usage(grx_arena* arena, size_t* in_use, size_t* largest_free, size_t* peak);
 grx_status grx_box_create_in(const grx_box_desc* desc, grx_arena* arena, grx_box** out);
 /* Upper estimate of the device bytes a box of this description needs, including its
- * first scratch and Widom result buffers. The framework's voxel candidate lists (up to
- * 32 MB, grx_box_set_voxel_lists) come on top when the arena or device has room for
+ * first scratch and Widom result buffers and its FP64 Coulomb tables (0.2 to 0.5 MB; boxes
+ * of one alpha, cutoff and similar cells hold them once per arena; outside an arena a box
+ * does without them when the device has no room). The framework's voxel candidate lists
+ * (up to 32 MB, grx_box_set_voxel_lists) come on top when the arena or device has room for
  * them; without room the box keeps the tile path, so this is the admission minimum. */
 grx_status grx_box_footprint(const grx_box_desc* desc, size_t* bytes);
 /* All later work of the box goes to this stream (cudaStream_t, NULL = default). */
