@@ -779,13 +779,18 @@ static __device__ __noinline__ StepChoice choose_trial(const double* te, const i
   if (m0) c.sel = __ffs(m0) - 1;
   else if (m1) c.sel = 31 + __ffs(m1);
   else c.sel = ok1 ? 63 - __clz(ok1) : 31 - __clz(ok0);  // rounding left the sum below u * sum: the last one
-  const bool finite = scale < INFINITY;  // weights beyond the range of exp: one by one
+  const bool finite = scale < INFINITY;
 #pragma unroll 1
   for (int r = 0; r < 2; ++r) {
     const int t = lane + 32 * r;
     if (t < nt) wa[t] = finite ? scale * e[r] : (ok[r] ? exp_move(lw[r]) : 0.0);
   }
-  c.w = mx > -INFINITY || mx != mx ? scale * sum : 0.0;  // every energy +inf: no weight
+  if (finite) {
+    c.w = mx > -INFINITY ? scale * sum : 0.0;  // every energy +inf: no weight
+  } else {  // a maximum that exp does not hold, or no number: the sum of the weights as they are
+    c.w = (lane < nt ? wa[lane] : 0.0) + (lane + 32 < nt ? wa[lane + 32] : 0.0);
+    for (int o = 16; o > 0; o >>= 1) c.w += __shfl_xor_sync(kFull, c.w, o);
+  }
   __syncwarp();
   return c;
 }
