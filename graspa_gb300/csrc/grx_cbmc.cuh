@@ -193,7 +193,7 @@ __device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, u
           W.w = avg;
           const double all = chain ? *chain * avg : avg;
           if (chain) *chain = all;
-          W.big = all > 1e-150;
+          W.big = chain ? !(all <= 1e-150) : all > 1e-150;  // apart for NaN: recorded when it is the chain's
         }
       }
     }

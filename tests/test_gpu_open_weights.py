@@ -45,7 +45,7 @@ def test_weights_that_are_not_finite(grx_lib, guest_type, value, ntrials):
     assert odd.any() == (value != -np.inf)
 
 
-@pytest.mark.parametrize("value", [np.inf])
+@pytest.mark.parametrize("value", [np.inf, np.nan])
 def test_recorded_weights_that_are_not_finite(grx_lib, value):
     """GCMC: a chain's undefined or infinite weight is recorded in the insertions' weights."""
     s = _system(3, value)
