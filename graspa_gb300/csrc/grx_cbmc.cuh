@@ -178,7 +178,8 @@ template <class WK>
 __device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, uint32_t uw, double inv,
                                             bool retrace, double stored = 0.0, double* chain = nullptr) {
   if (threadIdx.x < 32) {
-    const StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u01(uw), retrace, W.sel_wa);
+    StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u01(uw), retrace, W.sel_wa);
+    c.w = step_sum(c, W.sel_wa, nt);
     if (threadIdx.x == 0) {
       W.nok = c.nok;
       W.ok = 0;

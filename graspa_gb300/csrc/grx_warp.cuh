@@ -779,20 +779,29 @@ static __device__ __noinline__ StepChoice choose_trial(const double* te, const i
   if (m0) c.sel = __ffs(m0) - 1;
   else if (m1) c.sel = 31 + __ffs(m1);
   else c.sel = ok1 ? 63 - __clz(ok1) : 31 - __clz(ok0);  // rounding left the sum below u * sum: the last one
-  const bool finite = scale < INFINITY;
+  const bool finite = scale < INFINITY;  // weights beyond the range of exp: one by one
 #pragma unroll 1
   for (int r = 0; r < 2; ++r) {
     const int t = lane + 32 * r;
     if (t < nt) wa[t] = finite ? scale * e[r] : (ok[r] ? exp_move(lw[r]) : 0.0);
   }
-  if (finite) {
-    c.w = mx > -INFINITY ? scale * sum : 0.0;  // every energy +inf: no weight
-  } else {  // a maximum that exp does not hold, or no number: the sum of the weights as they are
-    c.w = (lane < nt ? wa[lane] : 0.0) + (lane + 32 < nt ? wa[lane + 32] : 0.0);
-    for (int o = 16; o > 0; o >>= 1) c.w += __shfl_xor_sync(kFull, c.w, o);
-  }
+  c.w = mx > -INFINITY || mx != mx ? scale * sum : 0.0;  // every energy +inf: no weight
   __syncwarp();
   return c;
+}
+
+// The weight sum of a step by the warp that chose: beyond the range of exp (and for energies that are no
+// numbers) the sum of the weights as they are, since exp of the maximum times the shifted sum is no
+// number where a weight is infinite. Apart from choose_trial, which this branch inside made slower (456
+// CO2 chains by 0.8 %). Every lane reads what it wrote.
+static __device__ __noinline__ double weight_sum(const double* wa, int nt) {
+  const int lane = threadIdx.x & 31;
+  double w = (lane < nt ? wa[lane] : 0.0) + (lane + 32 < nt ? wa[lane + 32] : 0.0);
+  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(kFull, w, o);
+  return w;
+}
+__device__ __forceinline__ double step_sum(const StepChoice& c, const double* wa, int nt) {
+  return c.w < INFINITY ? c.w : weight_sum(wa, nt);
 }
 
 // Live adsorbate atoms of the box, and the 32-atom work units a bead pass covers

@@ -45,7 +45,8 @@ struct WidomArgs {
 // Weight of one CBMC step by one warp (insertion branch); true when a trial was chosen.
 __device__ bool select_trial_warp(const double* te, const int* tflag, int nt, double beta, int bias,
                                   double u, double navg, int& sel, double& wavg, int& nok, double* wa) {
-  const StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false, wa);
+  StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false, wa);
+  c.w = step_sum(c, wa, nt);
   nok = c.nok;
   if ((threadIdx.x & 31) != 0 || c.nok == 0 || c.w < 1e-150) return false;
   sel = c.sel;
