@@ -205,7 +205,11 @@ grx_status build_voxels(grx_box* b) {
     }
   int mode = 0;
   if (near_home && choose_voxels(C, d.volume, nh_atoms, r_screen, b->vox_max_bytes, true, G, half_wmin, nv, h, est)) mode = 1;
-  else if (choose_voxels(C, d.volume, nh_atoms, r_screen, b->vox_max_bytes, false, G, half_wmin, nv, h, est)) mode = 2;
+  // not in an arena: its users size it by the footprints of their boxes, and such cells have never
+  // taken lists on top of theirs
+  else if (!b->arena &&
+           choose_voxels(C, d.volume, nh_atoms, r_screen, b->vox_max_bytes, false, G, half_wmin, nv, h, est))
+    mode = 2;
   if (!mode) {
     refresh_dev(b);
     return GRX_OK;

@@ -212,10 +212,11 @@ grx_status grx_box_create_replica(grx_box* parent, grx_box** out);
  * voxel first. The pair engine then walks a bead's voxel list instead of culling the
  * framework's 32-atom tiles (the cutoff tests stay exact, so results change only in the
  * summation order). In a cell narrower than twice the list radius an entry's image is the
- * one of rounded fractions, as on the tile path. Built by default when the lists fit 32 MB;
- * mode 0 frees them (tile path), mode 1 rebuilds them. Refused on a box with replicas (they
- * share the lists). No counterpart in the reference (it tests every framework atom per
- * trial). get: on (0/1), voxels per axis, list entries. */
+ * one of rounded fractions, as on the tile path; boxes in an arena keep the tile path
+ * there. Built by default when the lists fit 32 MB; mode 0 frees them (tile path), mode 1
+ * rebuilds them. Refused on a box with replicas (they share the lists). No counterpart in
+ * the reference (it tests every framework atom per trial). get: on (0/1), voxels per axis,
+ * list entries. */
 grx_status grx_box_set_voxel_lists(grx_box* box, int32_t mode);
 grx_status grx_box_get_voxel_lists(grx_box* box, int32_t* on, int32_t* dims, int64_t* entries);
 
@@ -236,8 +237,9 @@ grx_status grx_box_create_in(const grx_box_desc* desc, grx_arena* arena, grx_box
  * first scratch and Widom result buffers and its FP64 Coulomb tables (0.2 to 0.5 MB; boxes
  * of one alpha, cutoff and similar cells hold them once per arena; outside an arena a box
  * does without them when the device has no room). The framework's voxel candidate lists
- * (up to 32 MB, grx_box_set_voxel_lists) come on top when the arena or device has room for
- * them; without room the box keeps the tile path, so this is the admission minimum. */
+ * (up to 32 MB, grx_box_set_voxel_lists; in an arena only for cells wider than twice the
+ * list radius) come on top when the arena or device has room for them; without room the
+ * box keeps the tile path, so this is the admission minimum. */
 grx_status grx_box_footprint(const grx_box_desc* desc, size_t* bytes);
 /* All later work of the box goes to this stream (cudaStream_t, NULL = default). */
 grx_status grx_box_set_stream(grx_box* box, void* cuda_stream);

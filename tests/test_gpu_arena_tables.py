@@ -72,8 +72,20 @@ def test_footprint_holds_the_tables(grx_lib):
     assert np.array_equal(_energies(grx_lib, b), _energies(grx_lib, plain))
     b.close()
     arena.close()
-    small = grx_lib.Arena(used - (1 << 20) - 200_000)  # without its scratch, room for all but the tables
+    small = grx_lib.Arena(used - 200_000)  # room for all but the tables
     with pytest.raises(grx_lib.GrxError, match="memory"):
         _box(grx_lib, small)
     assert small.usage()[0] == 0
     small.close()
+
+
+def test_narrow_boxes_fit_by_their_footprint(grx_lib):
+    """An arena of 24 footprints takes 24 boxes of a cell narrower than twice the list radius: no lists
+    (4 to 9 MB a box) on top of the footprint."""
+    fp = grx_lib.box_footprint(_system(), CAP)
+    arena = grx_lib.Arena(24 * fp)
+    boxes = [grx_lib.Box(_system(), capacity=CAP, arena=arena) for _ in range(24)]
+    assert not any(b.voxel_lists()[0] for b in boxes)
+    for b in boxes:
+        b.close()
+    arena.close()
