@@ -512,6 +512,9 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
         if (pass && b.cull) {
           const float4 tc = b.tile_c[2 * tl];
           float dx = tc.x - bx, dy = tc.y - by, dz = tc.z - bz;
+          // FP64: the hi parts of bead and tile hold their coordinates to 2^-13 A (below 2 kNearCoord)
+          const bool exact = (bd.unit & 2) && fmaxf(fmaxf(fabsf(dx), fabsf(dy)), fabsf(dz)) + tc.w < kNearCoord;
+          bool near4;
           const float lim = b.cull_r + tc.w;
           const float m = tc.w + 1e-2f;
           if (b.cubic) {
@@ -531,7 +534,7 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
                         fabsf(dy) + th.y + 1e-2f < 0.5f * b.cellf[4] && fabsf(dz) + th.z + 1e-2f < 0.5f * b.cellf[8];
             // the whole edges: n times their low parts alone would pass the screen's guard band
             sx = nx * b.cellf[0]; sy = ny * b.cellf[4]; sz = nz * b.cellf[8];
-            if (PREC == GRX_FP64) one_image = one_image && fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz)) <= 4.0f;
+            near4 = fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz)) <= 4.0f;
           } else {
             const float fx = b.invf[0] * dx + b.invf[3] * dy + b.invf[6] * dz;
             const float fy = b.invf[1] * dx + b.invf[4] * dy + b.invf[7] * dz;
@@ -551,8 +554,9 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
             }
             one_image = trl.w != 0 && rx + m / b.wperp[0] < 0.5f - 1e-4f &&
                         ry + m / b.wperp[1] < 0.5f - 1e-4f && rz + m / b.wperp[2] < 0.5f - 1e-4f;
-            if (PREC == GRX_FP64) one_image = one_image && fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz)) <= 4.0f;
+            near4 = fmaxf(fmaxf(fabsf(nx), fabsf(ny)), fabsf(nz)) <= 4.0f;
           }
+          if (PREC == GRX_FP64) one_image = one_image && near4 && exact;
         }
         mask = __ballot_sync(kFull, pass);
       }

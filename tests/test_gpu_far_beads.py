@@ -81,3 +81,27 @@ def test_pairs_at_the_cutoff_far_from_home(grx_lib, path, which, prec):
     for lattice in LATTICES:
         e, _ = box.trial_energies(p + np.array(lattice) @ cell, q, ty, 10 ** 6, n, 1, 1, prec=grx_lib.PRECISIONS[prec])
         assert np.all(np.abs(e[:, :2] - want) <= bar), (lattice, int((np.abs(e[:, :2] - want) > bar).any(1).sum()))
+
+
+def test_pairs_at_the_cutoff_in_a_wide_cell(grx_lib):
+    """FP64 on tiles in a cell of 80,000 A, whose coordinates the hi parts hold to 4e-3 A only. Bar:
+    displacements carry 1.5e-11 A, a term changes by at most 2.5 of itself per A: 1e-10 M."""
+    s = _system("silica", "tiles")
+    s["pos"] = s["pos"] - s["pos"][0] + np.array([70011.3, 68123.7, 71987.1])
+    s["cell"] = synth.orthorhombic_cell(80000.0, 80000.0, 80000.0)
+    box = grx_lib.Box(s, capacity=[12, 64])
+    assert not box.voxel_lists()[0]
+    rng = np.random.default_rng(9)
+    n = 400
+    v = rng.normal(size=(n, 3))
+    v /= np.linalg.norm(v, axis=1, keepdims=True)
+    p = s["pos"][rng.integers(0, 12, n)] + (s["cutoff_coul"] - rng.uniform(1e-4, 2e-3, n))[:, None] * v
+    tm = s["templates"][1]
+    q, ty = np.full(n, tm["charge"][-1]), np.full(n, tm["type"][-1])
+    lj, co, r = _terms(s, p, q, ty)
+    k = r.min(1) > 9.0
+    assert k.sum() >= 60
+    e, _ = box.trial_energies(p[k], q[k], ty[k], 10 ** 6, int(k.sum()), 1, 1, prec=grx_lib.GRX_FP64)
+    want = np.stack([lj[k].sum(1), co[k].sum(1)], 1)
+    mag = np.stack([np.abs(lj[k]).sum(1), np.abs(co[k]).sum(1)], 1)
+    assert np.all(np.abs(e[:, :2] - want) <= 1e-10 * mag)
