@@ -169,10 +169,8 @@ void refresh_dev(grx_box* b) {
   const grx_box* h = b->parent ? b->parent : b;
   d.hpos64 = h->pos64;
   d.hhi = h->hi;
-  d.hlo = h->lo;
   d.hmeta = h->meta;
   d.hscale = h->scale;
-  d.hqdf = h->qdf;
   d.hrec = h->hrec;
   d.htype = h->htype;
   d.shared_host = b->parent ? 1 : 0;

@@ -71,10 +71,8 @@ struct BoxDev {
   // when the box is a replica sharing its framework (guests are always the box's own)
   const double4* hpos64;
   const float4* hhi;
-  const float4* hlo;
   const int2* hmeta;
   const double* hscale;
-  const float2* hqdf;
   int shared_host;       // 1: host atoms, tiles, tables and framework S(k) belong to a parent
   // spatial tiles of host atoms (32 atoms each, k-d order)
   const float4* tile_c;  // per tile: {x, y, z, bounding radius}, {box half extents, 0}
@@ -83,7 +81,7 @@ struct BoxDev {
   // voxel candidate lists of host atoms (grx_voxel.cu); used instead of the tiles when vox
   const float4* hrec;            // host atoms: {hi xyz, q hi}, {lo xyz, q lo} per atom
   const unsigned short* htype;   // host atoms: type | 0x8000 when scale != 1
-  const int4* vmeta;     // per voxel {first entry, sure atoms, all atoms, 0}
+  const int4* vmeta;     // per voxel {first entry, sure atoms, all atoms, near ones of the sure}
   const unsigned* vlist; // entries: storage index | lattice shift << 20
   const float4* vshift;  // lattice vector of every shift code
   int vox;               // 0 tile path, 1 entries carry their image, 2 images by rounded fractions

@@ -1,10 +1,10 @@
 // grx_noalloc.cu -- trial energies without any device allocation at call time.
 //
-// grx_trial_energies grows a per-box scratch buffer with cudaMalloc when a call needs
+// grx_trial_energies grows a per-box pinned buffer with cudaMallocHost when a call needs
 // more than the last one. Some callers cannot allow that: a Monte Carlo loop that
-// must never stall the device (cudaMalloc and cudaFree can synchronize the whole
-// GPU and hold up other jobs' streams), or a host application whose device memory
-// all belongs to its own pool allocator. For them, grx_trial_energies_noalloc does
+// must never stall the device (CUDA allocations can synchronize the whole GPU and hold
+// up other jobs' streams), or a host application whose memory all belongs to its own
+// pool allocators. For them, grx_trial_energies_noalloc does
 // the same work with its scratch in one file-scope device array of fixed size,
 // GRX_NOALLOC_SCRATCH_BYTES, which every GPU that loads this library holds until the
 // process exits.

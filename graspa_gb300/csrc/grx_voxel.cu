@@ -36,7 +36,7 @@ namespace grx {
 namespace {
 
 struct Geo {
-  double cell[9], inv[9], w[3];
+  double inv[9], w[3];
 };
 
 constexpr double kMargin = 0.02;                  // A, on the voxel bounding radius
@@ -182,12 +182,8 @@ grx_status build_voxels(grx_box* b) {
   }
   const BoxDev& d = b->dev;
   Geo G;
-  for (int k = 0; k < 9; ++k) {
-    G.cell[k] = d.cell[k];
-    G.inv[k] = d.inv[k];
-  }
+  for (int k = 0; k < 9; ++k) G.inv[k] = d.inv[k];
   const double* C = d.cell;
-  const double av[3] = {C[0], C[1], C[2]}, bv[3] = {C[3], C[4], C[5]}, cv[3] = {C[6], C[7], C[8]};
   const double r_screen = std::sqrt((double)d.screen2);
   int nv[3] = {0, 0, 0};
   double h = 0.0, half_wmin = 0.0, est = 0.0;

@@ -175,8 +175,8 @@ __device__ __forceinline__ df lj_df(const BoxDev& b, int row, df rr) {
 // order >= 2 are ~1e-4 of g, so they are summed in FP32; the first two orders keep their low
 // parts, not renormalised in between (|c0| > |c1 t| and |c1| > |t tail| hold on every piece).
 // 26 instructions and two 16-byte loads; the normalised form took 44 and four. On the CO2-silica
-// batch of 456 chains x 50 steps, with the accumulation below: 7.13 -> 6.77 ms, 20,000 Widom
-// insertions 6.61 -> 5.85 ms.
+// batch of 456 chains x 50 steps, with the accumulation below: 7.16 -> 6.79 ms, 20,000 Widom
+// insertions 6.60 -> 5.79 ms.
 __device__ __forceinline__ df coul_table_df(const BoxDev& b, int k, df s) {
   float4 c0, c1;
   load32(b.ctabf + 2 * k, c0, c1);
@@ -212,11 +212,6 @@ static __device__ __noinline__ double coul_g_cold(const BoxDev& b, double rr) {
 // Accumulators of one lane: FP64 for the FP64 and FP32 forms, double-float for mixed.
 template <int PREC> struct LaneAcc { double v = 0.0, r = 0.0; };
 template <> struct LaneAcc<GRX_MIXED> { df v = {0.f, 0.f}, r = {0.f, 0.f}; };
-
-template <int PREC> __device__ __forceinline__ double acc_value(const LaneAcc<PREC>& a, bool vdw) {
-  if constexpr (PREC == GRX_MIXED) return vdw ? df_to(a.v) : df_to(a.r);
-  else return vdw ? a.v : a.r;
-}
 
 // Dense evaluation of one screened pair in the split forms, from its displacement (dh, dl): exact
 // cutoff tests, LJ, real Coulomb, overlap flag (VDW_Coulomb.cu:1287-1322). row: type pair; sc1: the
