@@ -179,12 +179,12 @@ __device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, u
                                             bool retrace, double stored = 0.0, double* chain = nullptr) {
   if (threadIdx.x < 32) {
     StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u01(uw), retrace, W.sel_wa);
-    c.w = step_sum(c, W.sel_wa, nt);
     if (threadIdx.x == 0) {
       W.nok = c.nok;
       W.ok = 0;
       W.big = 0;
       if (c.nok > 0) {
+        c.w = step_sum(c, W.sel_wa, nt);
         W.wraw = c.w;
         if (retrace || !(c.w < 1e-150)) {
           double avg = (c.w + stored) * inv;

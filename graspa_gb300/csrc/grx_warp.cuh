@@ -789,18 +789,17 @@ static __device__ __noinline__ StepChoice choose_trial(const double* te, const i
   return c;
 }
 
-// The weight sum of a step by the warp that chose: beyond the range of exp (and for energies that are no
-// numbers) the sum of the weights as they are, since exp of the maximum times the shifted sum is no
-// number where a weight is infinite. Apart from choose_trial, which this branch inside made slower (456
-// CO2 chains by 0.8 %). Every lane reads what it wrote.
-static __device__ __noinline__ double weight_sum(const double* wa, int nt) {
-  const int lane = threadIdx.x & 31;
-  double w = (lane < nt ? wa[lane] : 0.0) + (lane + 32 < nt ? wa[lane + 32] : 0.0);
-  for (int o = 16; o > 0; o >>= 1) w += __shfl_xor_sync(kFull, w, o);
-  return w;
-}
+// The weight sum of a step, by the lane that uses it. Beyond the range of exp, where a weight is infinite,
+// exp of the maximum times the shifted sum is no number: the sum of the weights as they are. (Inside
+// choose_trial this branch cost 456 CO2 chains 0.8 %.)
 __device__ __forceinline__ double step_sum(const StepChoice& c, const double* wa, int nt) {
-  return c.w < INFINITY ? c.w : weight_sum(wa, nt);
+  double w = c.w;
+  if (w != w) {
+    w = 0.0;
+#pragma unroll 1
+    for (int t = 0; t < nt; ++t) w += wa[t];
+  }
+  return w;
 }
 
 // Live adsorbate atoms of the box, and the 32-atom work units a bead pass covers

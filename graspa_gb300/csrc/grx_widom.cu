@@ -46,9 +46,10 @@ struct WidomArgs {
 __device__ bool select_trial_warp(const double* te, const int* tflag, int nt, double beta, int bias,
                                   double u, double navg, int& sel, double& wavg, int& nok, double* wa) {
   StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false, wa);
-  c.w = step_sum(c, wa, nt);
   nok = c.nok;
-  if ((threadIdx.x & 31) != 0 || c.nok == 0 || c.w < 1e-150) return false;
+  if ((threadIdx.x & 31) != 0 || c.nok == 0) return false;
+  c.w = step_sum(c, wa, nt);
+  if (c.w < 1e-150) return false;
   sel = c.sel;
   double avg = c.w / navg;
   if (!bias) avg *= exp(-beta * (te[4 * c.sel + 1] + te[4 * c.sel + 3]));
