@@ -428,7 +428,7 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
       // the bead in the home cell, for the screen: the hi parts of the m cells taken off (grid
       // multiples, exact below 4096 A), then their low parts, which grow with m (1.2e-4 A a cell and
       // vector at most, against a guard band of 2e-3 A). Left out, silica beads 40 cells away were
-      // up to 3.4e-3 A off and lost pairs at the cutoff; so 4e-4 A at any distance.
+      // up to 3.4e-3 A off and lost pairs at the cutoff; so 4e-4 A, to 4096 A out.
       auto home = [&](float h, int k) {
         h = __fmaf_rn(-mz, b.cell_hi[6 + k], __fmaf_rn(-my, b.cell_hi[3 + k], __fmaf_rn(-mx, b.cell_hi[k], h)));
         return h - (mx * b.cell_lo[k] + my * b.cell_lo[3 + k] + mz * b.cell_lo[6 + k]);
