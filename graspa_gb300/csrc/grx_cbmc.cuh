@@ -46,7 +46,6 @@ struct CbmcWork {
   alignas(16) int qbuf[NW * kQueue];  // the warps' pair queues; between passes the quaternions of gen_orientations
   double te[kMaxTrials * 4];
   int tflag[kMaxTrials];
-  double sel_wa[kMaxTrials];
   // moved atoms of the Ewald delta: [0, n_old) leave (charge stored negated),
   // [n_old, n_old + n_new) arrive
   double mx[2 * kMolWork], my[2 * kMolWork], mz[2 * kMolWork], mq[2 * kMolWork];
@@ -62,7 +61,6 @@ struct CbmcWork {
   int sel;      // chosen (or retraced) trial index
   int nok;      // trials without overlap
   double w;     // averaged weight of the step
-  double wraw;  // unaveraged weight sum of the step (reinsertion StoredR)
 };
 
 // ---------------------------------------------------------------- trials
@@ -167,7 +165,7 @@ __device__ __noinline__ void trial_pass_excl(const BoxDev& b, WK& W, int nb, int
   trial_pass_body<PREC, CL>(b, W, nb, chain, comp, newmol, excl_comp, excl_mol, -1);
 }
 
-// CBMC weight of one growth step (warp 0 computes, results in W.ok/big/sel/w/nok/wraw).
+// CBMC weight of one growth step (warp 0 computes, results in W.ok/big/sel/w/nok).
 // Insertion: log-sum-exp selection with the uniform of word uw (SelectTrialPosition) and the
 // 1e-150 failure test. Retrace (deletion): the first trial without overlap is the
 // existing configuration and no selection is drawn. `stored` is added to the sum
@@ -178,14 +176,13 @@ template <class WK>
 __device__ __noinline__ void step_weight(WK& W, int nt, double beta, int bias, uint32_t uw, double inv,
                                             bool retrace, double stored = 0.0, double* chain = nullptr) {
   if (threadIdx.x < 32) {
-    StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u01(uw), retrace, W.sel_wa);
+    StepChoice c = choose_trial(W.te, W.tflag, nt, beta, bias, u01(uw), retrace);
+    if (c.w != c.w) c.w = plain_weights(W.te, W.tflag, nt, beta, bias, -1).x;
     if (threadIdx.x == 0) {
       W.nok = c.nok;
       W.ok = 0;
       W.big = 0;
       if (c.nok > 0) {
-        c.w = step_sum(c, W.sel_wa, nt);
-        W.wraw = c.w;
         if (retrace || !(c.w < 1e-150)) {
           double avg = (c.w + stored) * inv;
           if (!bias) avg *= exp_move(-beta * (W.te[4 * c.sel + 1] + W.te[4 * c.sel + 3]));

@@ -410,8 +410,11 @@ __global__ void __launch_bounds__(NW * 32, 24 / NW) gcmc_kernel(const BoxDev* bo
         if (tid == 0) {
           for (int k = 0; k < 4; ++k) s_e1[k] = W.te[4 * W.sel + k];
           s_w1 = W.w;
-          s_stored = W.wraw - W.sel_wa[W.sel];  // StoredR (mc_widom.h:363)
           W.mx[ms] = fx; W.my[ms] = fy; W.mz[ms] = fz;
+        }
+        if (tid < 32) {
+          const double2 w = plain_weights(W.te, W.tflag, d.ntrials, d.beta, a.bias, W.sel);
+          if (tid == 0) s_stored = w.y;  // StoredR (mc_widom.h:363)
         }
       }
       __syncthreads();

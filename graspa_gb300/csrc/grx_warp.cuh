@@ -703,17 +703,24 @@ __device__ __forceinline__ void warp_store(const LaneAcc<PREC>& h, const LaneAcc
 // Selection and weight of one CBMC step over nt <= 64 trials by one warp (SelectTrialPosition,
 // mc_widom.h:14-39, and the sums of CBMC_FirstBead_Finish, :330-376): the trial without overlap
 // that the uniform u picks from the shifted weights (with `retrace` the first one), the number of
-// trials without overlap and the unshifted weight sum; wa[t] is trial t's weight. Every trial is
-// two lanes' worth at most, the cumulative sum a warp scan and the unshifted weights the shifted
-// ones times exp(max), so a step is one exp and five additions deep; a serial walk over the trials
+// trials without overlap and the unshifted weight sum. Every trial is
+// two lanes' worth at most, the cumulative sum a warp scan and the unshifted sum the shifted
+// one times exp(max), so a step is one exp and five additions deep; a serial walk over the trials
 // took two exps and three additions per trial, each a full FP64 latency on one lane.
 struct StepChoice {
   int sel, nok;
   double w;
 };
 
+// The exponent of trial t.
+__device__ __forceinline__ double trial_exponent(const double* te, int t, double beta, int bias) {
+  double tot = te[4 * t] + te[4 * t + 2];
+  if (bias) tot += te[4 * t + 1] + te[4 * t + 3];
+  return __dmul_rn(-beta, tot);
+}
+
 static __device__ __noinline__ StepChoice choose_trial(const double* te, const int* tflag, int nt, double beta, int bias,
-                                                       double u, bool retrace, double* wa) {
+                                                       double u, bool retrace) {
   const int lane = threadIdx.x & 31;
   double lw[2], e[2] = {0.0, 0.0};
   bool ok[2];
@@ -725,9 +732,7 @@ static __device__ __noinline__ StepChoice choose_trial(const double* te, const i
     ok[r] = t < nt && !tflag[t];
     lw[r] = 0.0;
     if (ok[r]) {
-      double tot = te[4 * t] + te[4 * t + 2];
-      if (bias) tot += te[4 * t + 1] + te[4 * t + 3];
-      lw[r] = __dmul_rn(-beta, tot);
+      lw[r] = trial_exponent(te, t, beta, bias);
       const long long w = __double_as_longlong(lw[r]);
       top = max(top, w ^ ((w >> 63) & 0x7fffffffffffffffll));
     }
@@ -737,11 +742,7 @@ static __device__ __noinline__ StepChoice choose_trial(const double* te, const i
   c.nok = __popc(ok0) + __popc(ok1);
   c.sel = -1;
   c.w = 0.0;
-  if (c.nok == 0) {
-    for (int t = lane; t < nt; t += 32) wa[t] = 0.0;
-    __syncwarp();
-    return c;
-  }
+  if (c.nok == 0) return c;
   for (int o = 16; o > 0; o >>= 1) top = max(top, __shfl_xor_sync(kFull, top, o));
   const double mx = __longlong_as_double(top ^ ((top >> 63) & 0x7fffffffffffffffll));
   double scale;
@@ -778,28 +779,34 @@ static __device__ __noinline__ StepChoice choose_trial(const double* te, const i
   if (m0) c.sel = __ffs(m0) - 1;
   else if (m1) c.sel = 31 + __ffs(m1);
   else c.sel = ok1 ? 63 - __clz(ok1) : 31 - __clz(ok0);  // rounding left the sum below u * sum: the last one
-  const bool finite = scale < INFINITY;  // weights beyond the range of exp: one by one
-#pragma unroll 1
-  for (int r = 0; r < 2; ++r) {
-    const int t = lane + 32 * r;
-    if (t < nt) wa[t] = finite ? scale * e[r] : (ok[r] ? exp_move(lw[r]) : 0.0);
-  }
   c.w = mx > -INFINITY || mx != mx ? scale * sum : 0.0;  // every energy +inf: no weight
-  __syncwarp();
   return c;
 }
 
-// The weight sum of a step, by the lane that uses it. Beyond the range of exp, where a weight is infinite,
-// exp of the maximum times the shifted sum is no number: the sum of the weights as they are. (Inside
-// choose_trial this branch cost 456 CO2 chains 0.8 %.)
-__device__ __forceinline__ double step_sum(const StepChoice& c, const double* wa, int nt) {
-  double w = c.w;
-  if (w != w) {
-    w = 0.0;
+// The weights of a step as they are, by one warp: {their sum in the order of the trials, what it leaves
+// over the weight of trial sel}. Where a trial outweighs the rest by 1e15 that remainder is roundings of the
+// sum, and a reinsertion's retrace weight (StoredR) is made of it: it has to come from this order, as
+// the oracle's and the host layer's do, and not from the shifted sum, which rounds elsewhere (5 of 60
+// chains of 40 reinsertions beside charged atoms took other decisions). A chain of nt FP64 additions:
+// 2.6 % of a pass of 64 CH4/Xe boxes. Also the sum beyond the range of exp, where exp of the maximum
+// times the shifted sum is no number.
+static __device__ __noinline__ double2 plain_weights(const double* te, const int* tflag, int nt, double beta, int bias,
+                                                     int sel) {
+  const int lane = threadIdx.x & 31;
+  double x[2] = {0.0, 0.0};
 #pragma unroll 1
-    for (int t = 0; t < nt; ++t) w += wa[t];
+  for (int r = 0; r < 2; ++r) {
+    const int t = lane + 32 * r;
+    if (t < nt && !tflag[t]) x[r] = exp_move(trial_exponent(te, t, beta, bias));
   }
-  return w;
+  double w = 0.0, ws = 0.0;
+#pragma unroll 1
+  for (int t = 0; t < nt; ++t) {
+    const double v = __shfl_sync(kFull, t < 32 ? x[0] : x[1], t & 31);
+    w += v;
+    if (t == sel) ws = v;
+  }
+  return make_double2(w, w - ws);
 }
 
 // Live adsorbate atoms of the box, and the 32-atom work units a bead pass covers

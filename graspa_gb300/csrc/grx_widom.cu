@@ -44,12 +44,11 @@ struct WidomArgs {
 
 // Weight of one CBMC step by one warp (insertion branch); true when a trial was chosen.
 __device__ bool select_trial_warp(const double* te, const int* tflag, int nt, double beta, int bias,
-                                  double u, double navg, int& sel, double& wavg, int& nok, double* wa) {
-  StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false, wa);
+                                  double u, double navg, int& sel, double& wavg, int& nok) {
+  StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false);
+  if (c.w != c.w) c.w = plain_weights(te, tflag, nt, beta, bias, -1).x;
   nok = c.nok;
-  if ((threadIdx.x & 31) != 0 || c.nok == 0) return false;
-  c.w = step_sum(c, wa, nt);
-  if (c.w < 1e-150) return false;
+  if ((threadIdx.x & 31) != 0 || c.nok == 0 || c.w < 1e-150) return false;
   sel = c.sel;
   double avg = c.w / navg;
   if (!bias) avg *= exp(-beta * (te[4 * c.sel + 1] + te[4 * c.sel + 3]));
@@ -71,7 +70,6 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
   __shared__ double newx[GRX_MAX_MOLSIZE], newy[GRX_MAX_MOLSIZE], newz[GRX_MAX_MOLSIZE], newq[GRX_MAX_MOLSIZE];
   __shared__ grx_widom_result res;
   __shared__ int s_ok;
-  __shared__ double sel_wa[kMaxTrials];
   extern __shared__ double2 eik_s[];
 
   const int tid = threadIdx.x;
@@ -108,7 +106,7 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
       int sel = -1, nok = 0;
       double w = 0.0;
       const bool ok = select_trial_warp(te, tflag, nt, a.beta, b.vdw_real_bias, u01(selw[0]), (double)nt, sel, w,
-                                        nok, sel_wa);
+                                        nok);
       if (tid == 0) res.n_ok_first = nok;
       if (ok && w > 1e-150) {
         s_ok = 1;
@@ -143,7 +141,7 @@ __global__ void __launch_bounds__(GRX_THREADS, 3) widom_kernel(BoxDev b, WidomAr
         int sel = -1, nok = 0;
         double w = 0.0;
         const bool ok = select_trial_warp(te, tflag, no, a.beta, b.vdw_real_bias, u01(selw[1]), (double)no, sel, w,
-                                          nok, sel_wa);
+                                          nok);
         if (tid == 0) res.n_ok_orient = nok;
         if (tid == 0 && ok) {
           res.sel_orient = sel;
