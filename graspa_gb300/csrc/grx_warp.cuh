@@ -425,15 +425,14 @@ __device__ __forceinline__ void warp_item(const BoxDev& b, const Bead& bd, int t
       const int iy = min(b.vn[1] - 1, max(0, (int)((fy - my) * (float)b.vn[1])));
       const int iz = min(b.vn[2] - 1, max(0, (int)((fz - mz) * (float)b.vn[2])));
       const int4 vm = b.vmeta[(iz * b.vn[1] + iy) * b.vn[0] + ix];
-      // the bead in the home cell, for the screen: the hi parts of the m cells taken off (grid
-      // multiples, exact below 4096 A), then their low parts, which grow with m (1.2e-4 A a cell and
-      // vector at most, against a guard band of 2e-3 A). Left out, silica beads 40 cells away were
-      // up to 3.4e-3 A off and lost pairs at the cutoff; so 4e-4 A, to 4096 A out.
-      auto home = [&](float h, int k) {
-        h = __fmaf_rn(-mz, b.cell_hi[6 + k], __fmaf_rn(-my, b.cell_hi[3 + k], __fmaf_rn(-mx, b.cell_hi[k], h)));
-        return h - (mx * b.cell_lo[k] + my * b.cell_lo[3 + k] + mz * b.cell_lo[6 + k]);
-      };
-      const float3 wh = make_float3(home(bd.h.x, 0), home(bd.h.y, 1), home(bd.h.z, 2));
+      // the bead in the home cell, for the screen, by whole cell vectors. (Their hi parts alone, exact in
+      // FP32, leave out up to 1.2e-4 A a cell and vector against a guard band of 2e-3 A: silica beads 40
+      // cells away were 3.4e-3 A off and lost pairs at the cutoff. So they are 4e-4 A off there and
+      // 1e-3 A at 200 cells; hi and low parts apart would give 5e-4 A there, for 9 FMAs and 9 loads an
+      // item more.)
+      const float3 wh = make_float3(bd.h.x - (mx * b.cellf[0] + my * b.cellf[3] + mz * b.cellf[6]),
+                                    bd.h.y - (mx * b.cellf[1] + my * b.cellf[4] + mz * b.cellf[7]),
+                                    bd.h.z - (mx * b.cellf[2] + my * b.cellf[5] + mz * b.cellf[8]));
       const bool hcheck = component < b.nhost || (excl_comp >= 0 && excl_comp < b.nhost);
       int ch = t0;
       const int cend = min(t1, (vm.z + 31) >> 5);

@@ -42,11 +42,19 @@ struct WidomArgs {
   uint32_t stream;
 };
 
+// choose_trial with the weights beyond the range of exp, out of line: the rare branch inlined into the
+// kernel's two steps spilled registers of its body.
+static __device__ __noinline__ StepChoice choose_step(const double* te, const int* tflag, int nt, double beta, int bias,
+                                                      double u) {
+  StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false);
+  if (c.w != c.w) c.w = plain_weights(te, tflag, nt, beta, bias, -1).x;
+  return c;
+}
+
 // Weight of one CBMC step by one warp (insertion branch); true when a trial was chosen.
 __device__ bool select_trial_warp(const double* te, const int* tflag, int nt, double beta, int bias,
                                   double u, double navg, int& sel, double& wavg, int& nok) {
-  StepChoice c = choose_trial(te, tflag, nt, beta, bias, u, false);
-  if (c.w != c.w) c.w = plain_weights(te, tflag, nt, beta, bias, -1).x;
+  const StepChoice c = choose_step(te, tflag, nt, beta, bias, u);
   nok = c.nok;
   if ((threadIdx.x & 31) != 0 || c.nok == 0 || c.w < 1e-150) return false;
   sel = c.sel;
