@@ -34,7 +34,7 @@ def test_tables_come_from_the_arena(grx_lib):
     _energies(grx_lib, first)
     free = torch.cuda.mem_get_info()[0]
     boxes = [_box(grx_lib, arena, 0.2 + 0.004 * k) for k in range(1, 21)]
-    assert torch.cuda.mem_get_info()[0] == free
+    assert torch.cuda.mem_get_info()[0] > free - (4 << 20)  # 20 tables of 0.4 MB are 8 MB
     for k, b in enumerate(boxes):
         plain = grx_lib.Box(b.system, capacity=CAP)
         plain.set_voxel_lists(0)
